@@ -68,8 +68,7 @@ struct Ctrl {
   int abort_flag;
   alignas(16) float sc[kFp8 ? 4 : 1][2][kFp8 ? BT : 4];  // per epilogue warp, double buffered
   alignas(16) uint16_t xpose[4][32 * 32];  // per epilogue warp: output transpose tile
-  int tile_start[kMaxExperts + 1];
-  int row_start[kMaxExperts + 1];
+  alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
 };
 
 // kGated (16-bit inputs, token tiles up to 128): a tile pairs the 128 gate features j0.. with the
@@ -126,8 +125,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    build_tile_prefix<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->row_start,
-                          ctrl->tile_start);
+    build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
@@ -152,9 +150,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const int total_tiles = ctrl->tile_start[p.num_experts];
-  const int* tile_start = ctrl->tile_start;
-  const int* row_start = ctrl->row_start;
+  const TileWalk walk = tile_walk_at(ctrl->walk, p.num_experts);
+  const int total_tiles = walk.total;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -164,7 +161,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<BT>(tile_start, row_start, t, cursor, ti, p.w_experts);
+        locate_tile<BT>(walk, t, cursor, ti, p.w_experts);
         const int n0 = ti.n_tile * kFeat;
         for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
           if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
@@ -203,7 +200,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
       constexpr uint32_t kWStep = !kWKn ? 32u : (kFp8 ? 4096u : 2048u);   // bytes per 32-byte K step
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<BT>(tile_start, row_start, t, cursor, ti, p.w_experts);
+        locate_tile<BT>(walk, t, cursor, ti, p.w_experts);
         uint32_t a = acc_it % kAccStages;
         // A partly filled token tile multiplies only its valid columns (UMMA N in steps of 16).
         const uint32_t n_eff = (uint32_t)((ti.valid + 15) & ~15);
@@ -286,7 +283,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       TileInfo ti;
-      locate_tile<BT>(tile_start, row_start, t, cursor, ti, p.w_experts);
+      locate_tile<BT>(walk, t, cursor, ti, p.w_experts);
       const int feat = ti.n_tile * kFeat + et;
       const int n_out = kGated ? (p.n >> 1) : p.n;
       const bool feat_ok = feat < n_out;
@@ -372,7 +369,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
           } else if (t + (int)gridDim.x < total_tiles) {
             int cursor2 = cursor;
             TileInfo tn;
-            locate_tile<BT>(tile_start, row_start, t + gridDim.x, cursor2, tn, p.w_experts);
+            locate_tile<BT>(walk, t + gridDim.x, cursor2, tn, p.w_experts);
             fetch_group(tn, 0, pre);
             pre_valid = true;
           }
@@ -451,6 +448,7 @@ template <int BT, bool kFp8, bool kWKn, bool kGated = false>
 int launch_tc(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams& p, int grid,
               cudaStream_t st) {
   auto kern = grouped_gemm_tc_kernel<BT, kFp8, kWKn, kGated>;
+  static_assert(smem_bytes<BT, kFp8, kGated>() <= kMaxSmem, "shared memory");
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, smem_bytes<BT, kFp8, kGated>())) return rc;
   kern<<<grid, kTcThreads, smem_bytes<BT, kFp8, kGated>(), st>>>(ta, tw, p);
@@ -488,6 +486,7 @@ struct PairXchg {
 };
 constexpr size_t kPairGatedSmem = 1024 + (size_t)kPairGatedStages * kPairStageBytes + kEpiWarps * 2 * kPairXBuf +
                                   sizeof(PairXchg) + sizeof(Ctrl<kPairTok, false>);
+static_assert(kPairSmem <= kMaxSmem && kPairGatedSmem <= kMaxSmem, "shared memory");
 
 template <bool kWKn, bool kGated>
 __global__ void __launch_bounds__(kTcThreads, 1)
@@ -509,7 +508,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int pair_tiles = kGated ? p.n_tiles : (p.n_tiles + 1) / 2;
 
   if (warp == 0) {
-    build_tile_prefix<kPairTok>(p.rows_per_expert, p.num_experts, pair_tiles, ctrl->row_start, ctrl->tile_start);
+    build_tile_walk<kPairTok>(p.rows_per_expert, p.num_experts, pair_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
@@ -542,9 +541,8 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const int total_tiles = ctrl->tile_start[p.num_experts];
-  const int* tile_start = ctrl->tile_start;
-  const int* row_start = ctrl->row_start;
+  const TileWalk walk = tile_walk_at(ctrl->walk, p.num_experts);
+  const int total_tiles = walk.total;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -554,7 +552,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool ok = true;
       for (int t = walker; t < total_tiles && ok; t += walkers) {
         TileInfo ti;
-        locate_tile<kPairTok>(tile_start, row_start, t, cursor, ti, p.w_experts);
+        locate_tile<kPairTok>(walk, t, cursor, ti, p.w_experts);
         // past N: the load is zero-filled
         const int n0 = kGated ? (cta == 0 ? 0 : (p.n >> 1)) + ti.n_tile * kFeat : (ti.n_tile * 2 + (int)cta) * kFeat;
         const int row = ti.row0 + (int)cta * 128;
@@ -622,7 +620,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     bool ok = true;
     for (int t = walker; t < total_tiles && ok; t += walkers) {
       TileInfo ti;
-      locate_tile<kPairTok>(tile_start, row_start, t, cursor, ti, p.w_experts);
+      locate_tile<kPairTok>(walk, t, cursor, ti, p.w_experts);
       const int n_tile = kGated ? ti.n_tile : ti.n_tile * 2 + (int)cta;
       // the feature (row of W and of the bias) this thread's accumulator lane belongs to
       const int feat = (kGated && cta == 1 ? (p.n >> 1) : 0) + n_tile * kFeat + q * 32 + lane;

@@ -12,27 +12,64 @@ namespace {
 
 constexpr int kFeat = 128;          // features per tile (UMMA M)
 constexpr int kMaxExperts = 1024;
+constexpr size_t kMaxSmem = 227 * 1024;   // dynamic shared memory of a CTA
 
 struct TileInfo {
   int e, n_tile, m_tile, row0, valid;   // e: index of the weights the tile multiplies with
 };
+
+// The tile walk of a CTA, in shared memory: row and tile prefix sums over the experts that have
+// rows (decode batches leave most experts of a layer empty; walking over those, an element at a
+// time in every role, cost more than a tile's multiplications), and those experts' ids.
+struct TileWalk {
+  const int* tile_start;     // [n + 1] first tile of an expert, then the number of tiles
+  const int* row_start;      // [n + 1]
+  const uint16_t* expert;    // [n]
+  int n;                     // experts with rows
+  int total;                 // tiles
+};
+__host__ __device__ constexpr int tile_walk_bytes(int num_experts) {
+  return ((2 * (num_experts + 1) + 1) * 4 + 2 * num_experts + 15) & ~15;
+}
+__device__ __forceinline__ TileWalk tile_walk_at(const void* mem, int num_experts) {
+  TileWalk w;
+  const int* p = reinterpret_cast<const int*>(mem);
+  w.n = p[0];
+  w.tile_start = p + 1;
+  w.row_start = w.tile_start + num_experts + 1;
+  w.expert = reinterpret_cast<const uint16_t*>(w.row_start + num_experts + 1);
+  w.total = w.tile_start[w.n];
+  return w;
+}
 
 // Tiles of one expert are numbered feature-tile-major with the token tiles
 // adjacent, so CTAs that run at the same time share a weight tile in L2.
 // With w_experts > 0 the row segments outnumber the weight sets: segment s multiplies with
 // weights s % w_experts (the segments are the (source rank, local expert) pairs of an
 // expert-parallel exchange, source-major).
+// `cursor` is the position in the walk of the caller's previous tile; t does not decrease.
 template <int BT>
-__device__ __forceinline__ void locate_tile(const int* tile_start, const int* row_start, int t,
-                                            int& cursor, TileInfo& ti, int w_experts = 0) {
-  while (t >= tile_start[cursor + 1]) ++cursor;
-  const int local = t - tile_start[cursor];
-  const int rows = row_start[cursor + 1] - row_start[cursor];
+__device__ __forceinline__ void locate_tile(const TileWalk& w, int t, int& cursor, TileInfo& ti, int w_experts = 0) {
+  if (t >= w.tile_start[cursor + 1]) {
+    ++cursor;
+    if (t >= w.tile_start[cursor + 1]) {   // further than the next one: bisect
+      int lo = cursor + 1, hi = w.n - 1;
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (w.tile_start[mid] <= t) lo = mid;
+        else hi = mid - 1;
+      }
+      cursor = lo;
+    }
+  }
+  const int local = t - w.tile_start[cursor];
+  const int rows = w.row_start[cursor + 1] - w.row_start[cursor];
   const int m_tiles = (rows + BT - 1) / BT;
-  ti.e = w_experts > 0 ? cursor % w_experts : cursor;
-  ti.n_tile = local / m_tiles;
+  const int e = w.expert[cursor];
+  ti.e = w_experts > 0 ? e % w_experts : e;
+  ti.n_tile = m_tiles == 1 ? local : local / m_tiles;
   ti.m_tile = local - ti.n_tile * m_tiles;
-  ti.row0 = row_start[cursor] + ti.m_tile * BT;
+  ti.row0 = w.row_start[cursor] + ti.m_tile * BT;
   const int left = rows - ti.m_tile * BT;
   ti.valid = left < BT ? left : BT;
 }
@@ -94,32 +131,60 @@ __device__ __forceinline__ void store_block_transposed(uint16_t* xp, const float
   __syncwarp();
 }
 
-// Warp-cooperative prefix sums over the experts: row_start[e], tile_start[e]
-// (tiles of expert e = ceil(rows_e / BT) * n_tiles).  Called by one full warp.
+// Fills the tile walk at `mem` (tiles of expert e = ceil(rows_e / BT) * n_tiles).  Called by one
+// full warp; a lane takes eight consecutive experts of every 256, so that their loads are in
+// flight together and one scan serves them all.
 template <int BT>
-__device__ __forceinline__ void build_tile_prefix(const int32_t* rows_per_expert, int num_experts,
-                                                  int n_tiles, int* row_start, int* tile_start) {
+__device__ __forceinline__ void build_tile_walk(const int32_t* rows_per_expert, int num_experts, int n_tiles, void* mem) {
   const int lane = threadIdx.x & 31;
-  int carry_r = 0, carry_t = 0;
-  if (lane == 0) { row_start[0] = 0; tile_start[0] = 0; }
-  for (int base = 0; base < num_experts; base += 32) {
-    const int e = base + lane;
-    int r = (e < num_experts) ? rows_per_expert[e] : 0;
-    if (r < 0) r = 0;
-    int tl = ((r + BT - 1) / BT) * n_tiles;
-    int ir = r, it = tl;
+  int* head = reinterpret_cast<int*>(mem);
+  int* tile_start = head + 1;
+  int* row_start = tile_start + num_experts + 1;
+  uint16_t* expert = reinterpret_cast<uint16_t*>(row_start + num_experts + 1);
+  int carry_r = 0, carry_t = 0, carry_n = 0;
+  for (int base = 0; base < num_experts; base += 256) {
+    int r[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = base + lane * 8 + i;
+      r[i] = e < num_experts ? rows_per_expert[e] : 0;
+    }
+    int sum_r = 0, sum_t = 0, sum_n = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (r[i] < 0) r[i] = 0;
+      sum_r += r[i];
+      sum_t += ((r[i] + BT - 1) / BT) * n_tiles;
+      sum_n += r[i] > 0 ? 1 : 0;
+    }
+    int ir = sum_r, it = sum_t, in = sum_n;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const int o_r = __shfl_up_sync(0xffffffffu, ir, d);
       const int o_t = __shfl_up_sync(0xffffffffu, it, d);
-      if (lane >= d) { ir += o_r; it += o_t; }
+      const int o_n = __shfl_up_sync(0xffffffffu, in, d);
+      if (lane >= d) { ir += o_r; it += o_t; in += o_n; }
     }
-    if (e < num_experts) {
-      row_start[e + 1] = carry_r + ir;
-      tile_start[e + 1] = carry_t + it;
+    int row = carry_r + ir - sum_r, tile = carry_t + it - sum_t, pos = carry_n + in - sum_n;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      if (r[i] > 0) {
+        row_start[pos] = row;
+        tile_start[pos] = tile;
+        expert[pos] = (uint16_t)(base + lane * 8 + i);
+        ++pos;
+        row += r[i];
+        tile += ((r[i] + BT - 1) / BT) * n_tiles;
+      }
     }
     carry_r += __shfl_sync(0xffffffffu, ir, 31);
     carry_t += __shfl_sync(0xffffffffu, it, 31);
+    carry_n += __shfl_sync(0xffffffffu, in, 31);
+  }
+  if (lane == 0) {
+    head[0] = carry_n;
+    row_start[carry_n] = carry_r;
+    tile_start[carry_n] = carry_t;
   }
 }
 

@@ -67,8 +67,7 @@ struct DqCtrl {
   uint64_t sfw_empty[2];
   uint32_t tmem_base;
   int abort_flag;
-  int tile_start[kMaxExperts + 1];
-  int row_start[kMaxExperts + 1];
+  alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
   alignas(16) uint16_t xpose[4][32 * 32];  // per epilogue warp: output transpose tile
 };
 
@@ -192,8 +191,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    build_tile_prefix<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->row_start,
-                          ctrl->tile_start);
+    build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
@@ -221,9 +219,8 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const int total_tiles = ctrl->tile_start[p.num_experts];
-  const int* tile_start = ctrl->tile_start;
-  const int* row_start = ctrl->row_start;
+  const TileWalk walk = tile_walk_at(ctrl->walk, p.num_experts);
+  const int total_tiles = walk.total;
   const int num_st = (p.num_kb + kSub - 1) / kSub;   // stages per tile
 
   if (warp == 0) {
@@ -234,7 +231,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+        locate_tile<BT>(walk, t, cursor, ti);
         const int n0 = ti.n_tile * kFeat;
         for (int si = 0; si < num_st; ++si) {
           if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
@@ -263,7 +260,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t smem_base = ptx::smem_u32(smem);
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+        locate_tile<BT>(walk, t, cursor, ti);
         const uint32_t a = acc_it & 1;
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_empty[a], ((acc_it >> 1) & 1) ^ 1, abort_flag))) break;
         ptx::tc_fence_after();
@@ -318,14 +315,14 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
     };
     TileInfo ti, ti_next;
     if (staged && (int)blockIdx.x < total_tiles) {
-      locate_tile<BT>(tile_start, row_start, blockIdx.x, cursor_next, ti_next);
+      locate_tile<BT>(walk, blockIdx.x, cursor_next, ti_next);
       if (!stage_scales(ti_next, 0u)) { *abort_flag = 1; ok = false; }
     }
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_seq) {
-      locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+      locate_tile<BT>(walk, t, cursor, ti);
       const int t_next = t + gridDim.x;
       if (staged && t_next < total_tiles) {
-        locate_tile<BT>(tile_start, row_start, t_next, cursor_next, ti_next);
+        locate_tile<BT>(walk, t_next, cursor_next, ti_next);
         if (!stage_scales(ti_next, tile_seq + 1)) { *abort_flag = 1; ok = false; break; }
       }
       const uint32_t b = tile_seq & 1;
@@ -384,7 +381,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
     bool ok = true;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       TileInfo ti;
-      locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+      locate_tile<BT>(walk, t, cursor, ti);
       const int feat = ti.n_tile * kFeat + et;
       const bool feat_ok = feat < p.n;
       float bias_v = 0.f;

@@ -73,8 +73,7 @@ struct TCtrl {
   uint64_t acc_empty[kTAcc];
   uint32_t tmem_base;
   int abort_flag;
-  int tile_start[kMaxExperts + 1];
-  int row_start[kMaxExperts + 1];
+  alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
 };
 
 constexpr size_t kTSmem = 1024 + (size_t)kTStages * kTStageBytes + sizeof(TCtrl);
@@ -90,7 +89,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    build_tile_prefix<kTTok>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->row_start, ctrl->tile_start);
+    build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
@@ -115,9 +114,8 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const int* tile_start = ctrl->tile_start;
-  const int* row_start = ctrl->row_start;
-  const int total_tiles = tile_start[p.num_experts];
+  const TileWalk walk = tile_walk_at(ctrl->walk, p.num_experts);
+  const int total_tiles = walk.total;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -127,7 +125,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<kTTok>(tile_start, row_start, t, cursor, ti, p.w_experts);
+        locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
         const int n0 = ti.n_tile * kFeat;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
@@ -204,7 +202,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       TileInfo ti;
-      locate_tile<kTTok>(tile_start, row_start, t, cursor, ti, p.w_experts);
+      locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
       float acc[kTCols];
 #pragma unroll
       for (int i = 0; i < kTCols; ++i) acc[i] = 0.f;
@@ -220,7 +218,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
         } else if (t + (int)gridDim.x < total_tiles) {
           int cursor2 = cursor;
           TileInfo tn;
-          locate_tile<kTTok>(tile_start, row_start, t + gridDim.x, cursor2, tn, p.w_experts);
+          locate_tile<kTTok>(walk, t + gridDim.x, cursor2, tn, p.w_experts);
           fetch_group(tn, 0, pre);
           pre_valid = true;
         }
@@ -315,8 +313,7 @@ struct T2Ctrl {
   int abort_flag;
   float xchg[2][2][128];   // gated epilogue: group maxima exchanged between the two warps of a token row
   uint64_t xbar[4];        // ... and the barrier of each such pair of warps (one per lane quarter)
-  int tile_start[kMaxExperts + 1];
-  int row_start[kMaxExperts + 1];
+  alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
 };
 // store tiles (3-stage form): per epilogue warp its 32 token rows x 128 features in 16 bits
 constexpr size_t kT2XposeBytes = 8 * 32 * kT2RowPitch;
@@ -325,6 +322,7 @@ constexpr size_t kT2Smem = 1024 + kT2Ring + ((sizeof(T2Ctrl) + 15) & ~(size_t)15
 static_assert(kT2XposeBytes <= kT2StageBytes + 24 * 1024, "store tiles must fit the fourth stage's room");
 constexpr size_t kT2SmemStaged = 1024 + (size_t)kT2StagesStaged * kT2StageBytes + kT2XposeBytes +
                                  ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
+static_assert(kT2Smem <= kMaxSmem && kT2SmemStaged <= kMaxSmem, "shared memory");
 
 //
 // kGated (the first grouped GEMM of a SiLU layer with block-scaled fp8 experts): a tile pairs the
@@ -352,7 +350,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int up_block0 = p.n_tiles / 2;        // gated: first 128-feature block of the up half
 
   if (warp == 0) {
-    build_tile_prefix<kTTok>(p.rows_per_expert, p.num_experts, n_tiles2, ctrl->row_start, ctrl->tile_start);
+    build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, n_tiles2, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
@@ -378,9 +376,8 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const int* tile_start = ctrl->tile_start;
-  const int* row_start = ctrl->row_start;
-  const int total_tiles = tile_start[p.num_experts];
+  const TileWalk walk = tile_walk_at(ctrl->walk, p.num_experts);
+  const int total_tiles = walk.total;
 
   if (warp < 4) {
     ptx::setmaxnreg_dec<kT2LowRegs>();
@@ -391,7 +388,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       bool ok = true;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<kTTok>(tile_start, row_start, t, cursor, ti, p.w_experts);
+        locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
         const int n0 = kGated ? ti.n_tile * 128 : ti.n_tile * 256;
         const int n1 = kGated ? (up_block0 + ti.n_tile) * 128 : n0 + 128;
         for (int kb = 0; kb < p.num_kb; ++kb) {
@@ -497,7 +494,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       TileInfo ti;
-      locate_tile<kTTok>(tile_start, row_start, t, cursor, ti, p.w_experts);
+      locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
       float acc[128];
 #pragma unroll
       for (int i = 0; i < 128; ++i) acc[i] = 0.f;
@@ -511,7 +508,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
         } else if (t + (int)gridDim.x < total_tiles) {
           int cursor2 = cursor;
           TileInfo tn;
-          locate_tile<kTTok>(tile_start, row_start, t + gridDim.x, cursor2, tn, p.w_experts);
+          locate_tile<kTTok>(walk, t + gridDim.x, cursor2, tn, p.w_experts);
           fetch_group(tn, 0, pre);
           pre_valid = true;
         }

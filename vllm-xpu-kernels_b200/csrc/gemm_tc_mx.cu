@@ -15,17 +15,17 @@
 //               the 16U4_ALIGN16B tensor-map type, which spreads every 8 packed
 //               bytes into a 16-byte slot (the operand format the MMA reads),
 //               128-byte swizzle; activation tile BT rows x 128 bytes.
-//   warp 1    : MMA issuer, owns tensor memory
-//   warps 2-5 : scale feeders: bring the e8m0 bytes of the tile's 128 weight rows
+//   warp 1    : MMA issuer, owns tensor memory; also copies the scale factors of each
+//               K block from shared to tensor memory (tcgen05.cp, which replicates them
+//               over the four lane quarters as the MMA wants them)
+//   warps 2-5 : scale preparers: bring the e8m0 bytes of the tile's 128 weight rows
 //               (one contiguous piece of the scale tensor) into shared memory
 //               with cp.async one tile ahead, read the tokens' scale words (one
-//               coalesced 32-bit word per token and K block) a few K blocks
-//               ahead, and write both to tensor memory (tcgen05.st), one copy
-//               per lane quarter as the MMA wants.
-//               When K is not a multiple of 128 (that tensor-map type needs it)
-//               they also spread the last, partial block, which then arrives
-//               through a plain byte tensor map.
-//   warps 6-9 : epilogue
+//               coalesced 32-bit word per token and K block) a group of K blocks
+//               ahead, and write both to a ring of groups in the layout tcgen05.cp
+//               reads
+//   warps 6-9 : epilogue.  When K is not a multiple of 128 (the weights' tensor-map type
+//               needs it) they also bring and spread the last, partial block of a tile.
 //
 // The same kernel (kW8) multiplies per-tensor-scaled fp8 weights ([E,K,N], e4m3 or
 // e5m2, one fp32 scale per expert: the reference's w8a16 recipe,
@@ -50,14 +50,15 @@ namespace b200moe {
 namespace {
 
 constexpr int kMxWBytes = 16384;    // 128 rows x 128 codes in 16-byte slots of 16
-constexpr int kMxRawBytes = 8192;   // 128 rows x 64 packed bytes
 constexpr int kMxWTx = 8192;        // the spreading load reports the packed bytes it read to its barrier
 constexpr int kMxThreads = 320;
 constexpr int kMxMaxStages = 8;
-constexpr int kMxGroup = 2;         // K blocks per token-scale prefetch group (read two groups ahead)
-constexpr int kMxSfwCap = 24576 + 16;    // largest weight-scale piece (128 rows x K/32 bytes) staged in shared memory
+constexpr int kMxGroup = 4;         // K blocks per scale group (one hand-over from the scale preparers)
+constexpr int kMxSlots = 4;         // scale groups in the ring, at most
+constexpr int kMxSfwCap = 24576 + 32;    // largest weight-scale piece (128 rows x K/32 bytes) staged in shared memory
 
 struct MxParams {
+  const uint8_t* w;         // [E, N, K/2]: the partial K block's source
   const uint8_t* w_scale;   // [E, N, K/32] e8m0; kW8 with w8_block: [E, K/32, N]; else unused
   const float* w_tensor_scale;  // kW8 without w8_block: [E] fp32, multiplies the result
   int w8_block;             // kW8: 1 = MXFP8 weights (scales per 32 K rows), 0 = one scale per expert
@@ -70,10 +71,9 @@ struct MxParams {
   int n, k, num_experts;
   int n_tiles, num_kb;
   int terms;       // activation planes (1 or 2)
-  int tail;        // 1: the last K block is partial and comes through the byte map
-  int stages, stage_bytes;
+  int tail;        // 1: the last K block is partial, its weights are brought by the epilogue warps
+  int stages;
   int sfw_bytes;   // bytes of one staged weight-scale buffer
-  int raw_shared;  // 1: one buffer for the partial K block after the staging buffers, 0: one per stage
   uint32_t tmem_cols;
   uint32_t idesc;
   int out_f16;
@@ -83,20 +83,26 @@ struct MxParams {
 
 struct MxCtrl {
   uint64_t full[kMxMaxStages];
-  uint64_t sf_full[kMxMaxStages];
   uint64_t empty[kMxMaxStages];
+  uint64_t sf_full[kMxSlots];
+  uint64_t sf_empty[kMxSlots];
   uint64_t acc_full[2];
   uint64_t acc_empty[2];
   uint64_t sfw_full[2];
   uint64_t sfw_empty[2];
+  uint64_t tail_full;    // the tile's partial block has been spread
   uint32_t tmem_base;
   int abort_flag;
   alignas(16) uint16_t xpose[4][32 * 32];
 };
-// Shared memory after the pipeline stages: one buffer for the partial K block
-// (when the stages do not carry their own), MxCtrl, the tile walk's prefix arrays
-// (2 x (experts + 1) ints) and two weight-scale staging buffers.
-__host__ __device__ inline int mx_prefix_bytes(int num_experts) { return ((num_experts + 1) * 4 + 15) & ~15; }
+// Shared memory after the pipeline stages: one buffer for the partial K block, the ring
+// of scale groups, MxCtrl, the tile walk and two weight-scale staging buffers.
+// One group of the scale ring: per K block 512 bytes for the weight rows and 512 per 128 token rows.
+template <int kNT>
+__host__ __device__ constexpr int mx_slot_bytes() { return kMxGroup * 512 * (kNT > 128 ? 3 : 2); }
+// Wide token tiles give the room of two groups to another pipeline stage.
+template <int kNT>
+__host__ __device__ constexpr int mx_slots() { return kNT > 128 ? 2 : kMxSlots; }
 
 // Weight scales of a tile's rows: one contiguous piece of the scale tensor,
 // copied to staging buffer (seq & 1) asynchronously by the 128 feeder threads
@@ -148,41 +154,35 @@ __device__ __forceinline__ bool stage_w_scales_kn(const MxParams& p, MxCtrl* ctr
 template <int BT, int kTerms, int kSub, bool kW8>
 __global__ void __launch_bounds__(kMxThreads, 1)
 grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                       const __grid_constant__ CUtensorMap tmap_w,
-                       const __grid_constant__ CUtensorMap tmap_raw, const MxParams p) {
-  static_assert(kSub == 1 || kSub == kMxGroup, "a stage holds one K block or one prefetch group");
+                       const __grid_constant__ CUtensorMap tmap_w, const MxParams p) {
+  static_assert(kMxGroup % kSub == 0, "a scale group is a whole number of stages");
   constexpr int kChunk = BT >= 32 ? 32 : 16;
   constexpr int kNT = kTerms * BT;                  // UMMA N: the planes side by side
-  constexpr int kW = kNT >= 32 ? kNT / 32 : 1;       // token-scale columns (words per lane and K block)
+  constexpr int kTokChunks = kNT > 128 ? 2 : 1;      // 512-byte scale chunks of the tokens per K block
   constexpr uint32_t kSfBase = 2 * kNT;
-  // scale columns per K block: the weight rows' four, then the tokens' kW; the region of a K
-  // block starts on a multiple of 8 columns
-  constexpr int kSfPer = kW <= 4 ? 8 : 16;
-  constexpr int kSfCols = kSfPer * kSub;            // scale columns of one stage
+  constexpr int kSfPer = kTokChunks == 1 ? 8 : 16;   // scale columns of a K block: the weight rows' four, then the tokens'
+  constexpr int kSlotBytes = mx_slot_bytes<kNT>(), kSlots = mx_slots<kNT>();
   constexpr int kABytes = kNT * 128;                // activation bytes of one K block (all planes)
-  constexpr int kAOff = kSub * kMxWBytes;           // stage: [W blocks][A blocks][raw tail]
-  constexpr int kRawOff = kSub * (kMxWBytes + kABytes);
+  constexpr int kAOff = kSub * kMxWBytes;           // stage: [W blocks][A blocks]
+  constexpr int kStageBytes = kSub * (kMxWBytes + kABytes);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int stages = p.stages;
-  const int stage_bytes = p.stage_bytes;
-  uint8_t* raw_one = smem + stages * stage_bytes;   // used when p.raw_shared (1024-byte aligned)
-  uint8_t* ctrl_at = raw_one + (p.raw_shared ? kMxRawBytes : 0);
+  uint8_t* tail_w = smem + stages * kStageBytes;   // the weights of the partial K block, if there is one
+  uint8_t* sf_ring = tail_w + (p.tail ? kMxWBytes : 0);
+  uint8_t* ctrl_at = sf_ring + kSlots * kSlotBytes;
   MxCtrl* ctrl = reinterpret_cast<MxCtrl*>(ctrl_at);
   uint8_t* after = ctrl_at + ((sizeof(MxCtrl) + 15) & ~(size_t)15);
-  int* tile_start_w = reinterpret_cast<int*>(after);
-  int* row_start_w = reinterpret_cast<int*>(after + mx_prefix_bytes(p.num_experts));
-  uint8_t* sfw = after + 2 * mx_prefix_bytes(p.num_experts);
+  uint8_t* sfw = after + tile_walk_bytes(p.num_experts);
   volatile int* abort_flag = &ctrl->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    build_tile_prefix<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, row_start_w, tile_start_w);
+    build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, after);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
-      ptx::prefetch_tensormap(&tmap_raw);
     }
   } else if (warp == 1) {
     ptx::tmem_alloc(&ctrl->tmem_base, p.tmem_cols);
@@ -190,8 +190,11 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
   } else if (warp == 2 && lane == 0) {
     for (int s = 0; s < kMxMaxStages; ++s) {
       ptx::mbar_init(&ctrl->full[s], 1);
-      ptx::mbar_init(&ctrl->sf_full[s], 4);
       ptx::mbar_init(&ctrl->empty[s], 1);
+    }
+    for (int g = 0; g < kMxSlots; ++g) {
+      ptx::mbar_init(&ctrl->sf_full[g], 4);
+      ptx::mbar_init(&ctrl->sf_empty[g], 1);
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(&ctrl->acc_full[a], 1);
@@ -199,6 +202,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
       ptx::mbar_init(&ctrl->sfw_full[a], 128);
       ptx::mbar_init(&ctrl->sfw_empty[a], 4);
     }
+    ptx::mbar_init(&ctrl->tail_full, 4);
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
@@ -207,150 +211,171 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const int* tile_start = tile_start_w;
-  const int* row_start = row_start_w;
-  const int total_tiles = tile_start[p.num_experts];
+  const TileWalk walk = tile_walk_at(after, p.num_experts);
+  const int total_tiles = walk.total;
   const int tail_kb = (!kW8 && p.tail) ? p.num_kb - 1 : -1;
   constexpr int kWTx = kW8 ? kMxWBytes : kMxWTx;   // bytes a weight-tile load reports
-  const int num_st = (p.num_kb + kSub - 1) / kSub;   // stages per tile
+  const int n_groups = (p.num_kb + kMxGroup - 1) / kMxGroup;
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      uint32_t s = 0, ph = 0;
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 1;
       int cursor = 0;
       bool ok = true;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t st0 = ptx::smem_u32(smem);
+      uint32_t st = st0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+        locate_tile<BT>(walk, t, cursor, ti);
         const int n0 = ti.n_tile * kFeat;
-        for (int si = 0; si < num_st; ++si) {
-          if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* st = smem + s * stage_bytes;
-          const int kb0 = si * kSub;
-          const int nsub = (p.num_kb - kb0) < kSub ? (p.num_kb - kb0) : kSub;
-          ptx::mbar_expect_tx(&ctrl->full[s], nsub * (kWTx + kABytes));
+        for (int kb0 = 0; kb0 < p.num_kb; kb0 += kSub) {
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          const uint32_t full = full0 + 8 * s;
+          const bool whole = kb0 + kSub < p.num_kb || (tail_kb < 0 && kb0 + kSub == p.num_kb);
+          if (whole) {
+            ptx::mbar_expect_tx_s(full, kSub * (kWTx + kABytes));
 #pragma unroll
-          for (int sub = 0; sub < kSub; ++sub) {
-            const int kb = kb0 + sub;
-            if (sub < nsub) {
-              if (kW8)   // 128 K rows x 128 features, one byte each; rows past K are zero-filled
-                ptx::tma_load_3d(st + sub * kMxWBytes, &tmap_w, &ctrl->full[s], n0, kb * 128, ti.e);
-              else if (kb == tail_kb)
-                ptx::tma_load_3d(p.raw_shared ? raw_one : st + kRawOff, &tmap_raw, &ctrl->full[s], kb * 64, n0, ti.e);
-              else
-                ptx::tma_load_3d(st + sub * kMxWBytes, &tmap_w, &ctrl->full[s], kb * 128, n0, ti.e);
-#pragma unroll
-              for (int term = 0; term < kTerms; ++term)
-                ptx::tma_load_3d(st + kAOff + sub * kABytes + term * (BT * 128), &tmap_a, &ctrl->full[s],
-                                 kb * 128, ti.row0, term);
+            for (int sub = 0; sub < kSub; ++sub) {
+              // kW8: 128 K rows x 128 features, one byte each; rows past K are zero-filled
+              if (kW8) ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, n0, (kb0 + sub) * 128, ti.e);
+              else ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, (kb0 + sub) * 128, n0, ti.e);
+              ptx::tma_load_3d_s(st + kAOff + sub * kABytes, &tmap_a, full, (kb0 + sub) * 128, ti.row0, 0);   // all planes
+            }
+          } else {
+            // a tile's last stage: fewer K blocks, or the partial one (only its tokens come this way)
+            const int nsub = p.num_kb - kb0;
+            ptx::mbar_expect_tx_s(full, nsub * (kWTx + kABytes) - (tail_kb >= 0 ? kWTx : 0));
+            for (int sub = 0; sub < nsub; ++sub) {
+              const int kb = kb0 + sub;
+              if (kW8) ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, n0, kb * 128, ti.e);
+              else if (kb != tail_kb) ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, kb * 128, n0, ti.e);
+              ptx::tma_load_3d_s(st + kAOff + sub * kABytes, &tmap_a, full, kb * 128, ti.row0, 0);
             }
           }
-          if (++s == (uint32_t)stages) { s = 0; ph ^= 1; }
+          st += kStageBytes;
+          if (++s == (uint32_t)stages) { s = 0; ph ^= 1; st = st0; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    // (the whole warp runs the loop with the same values; one elected lane issues)
-    {
-      uint32_t s = 0, ph = 0, acc_it = 0;
+    // One thread.  A K block is one asm statement on descriptors that differ by an addition from
+    // the ring's first: the issuer is a serial chain, and with token tiles of 16 and 64 the chain,
+    // not the tensor pipe (38 to 64 cycles per instruction), sets the rate.
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 0, acc_it = 0, slot = 0, slot_ph = 0;
       int cursor = 0;
       bool ok = true;
-      const uint32_t smem_base = ptx::smem_u32(smem);
-      uint32_t idesc_j[4];
-#pragma unroll
-      for (uint32_t j = 0; j < 4; ++j) idesc_j[j] = (p.idesc & ~(0x3fu << 17)) | (j << 29) | (j << 4);
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t sf_full0 = ptx::smem_u32(&ctrl->sf_full[0]), sf_empty0 = ptx::smem_u32(&ctrl->sf_empty[0]);
+      const uint32_t tail_full = ptx::smem_u32(&ctrl->tail_full);
+      const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
+      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kAOff, 16, 1024);
+      const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kW8 ? 16384 : 16, 1024);
+      const uint64_t tdesc = ptx::make_smem_desc(ptx::smem_u32(tail_w), 16, 1024);
+      const uint64_t sfdesc0 = ptx::make_smem_desc_plain(ptx::smem_u32(sf_ring), 128);
+      uint64_t wdesc = wdesc0, adesc = adesc0, sfdesc = sfdesc0;
+      const int whole_kb = tail_kb >= 0 ? tail_kb : p.num_kb;   // K blocks before the partial one
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
-        locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+        locate_tile<BT>(walk, t, cursor, ti);
         const uint32_t a = acc_it & 1;
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_empty[a], ((acc_it >> 1) & 1) ^ 1, abort_flag))) break;
-        ptx::tc_fence_after();
-        const uint32_t d_tmem = tmem_base + a * kNT;
         // A partly filled token tile multiplies only up to its last valid column (UMMA N in
         // steps of 16; with two planes the second one's columns follow the first one's BT).
         const uint32_t n_eff = (uint32_t)((kTerms - 1) * BT + ((ti.valid + 15) & ~15));
-        const uint32_t n_bits = (n_eff >> 3) << 17;
-        for (int si = 0; si < num_st; ++si) {
-          bool go = ptx::mbar_wait(&ctrl->full[s], ph, abort_flag);
-          if (go) go = ptx::mbar_wait(&ctrl->sf_full[s], ph, abort_flag);
-          if (!__all_sync(0xffffffffu, go)) { ok = false; break; }
+        const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((n_eff >> 3) << 17);
+        const uint32_t d_tmem = tmem_base + a * kNT;
+        if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, ((acc_it >> 1) & 1) ^ 1, abort_flag)) break;
+        ptx::tc_fence_after();
+        auto wait_stage = [&]() {
+          const bool go = ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag);
           ptx::tc_fence_after();
-          // Every operand descriptor of the stage is the first weight block's plus a
-          // compile-time offset (the address field counts 16-byte units).
-          const uint64_t desc0 = ptx::make_smem_desc(smem_base + s * stage_bytes, 16, 1024);
-          const uint64_t desc0w = kW8 ? ptx::make_smem_desc(smem_base + s * stage_bytes, 16384, 1024) : desc0;
-          const uint32_t sf0 = tmem_base + kSfBase + s * kSfCols;
-          const int kb0 = si * kSub;
+          return go;
+        };
+        // scales first: tcgen05.cp and tcgen05.mma of one thread execute in issue order
+        auto issue = [&](int u, uint64_t w, uint32_t accumulate) {
+          ptx::umma_mx_block<kTokChunks, kW8 ? 4096 / 16 : 32 / 16>(
+              d_tmem, w, adesc + (u % kSub) * (kABytes >> 4), idesc, accumulate,
+              tmem_base + kSfBase + u * kSfPer, sfdesc + u * 32, sfdesc + kMxGroup * 32 + u * (kTokChunks * 32));
+        };
+        auto release_stage = [&]() {
+          ptx::umma_commit(empty0 + 8 * s);
+          wdesc += kStageBytes >> 4;
+          adesc += kStageBytes >> 4;
+          if (++s == (uint32_t)stages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
+        };
+        for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += kMxGroup) {
+          if (!ptx::mbar_wait_s(sf_full0 + 8 * slot, slot_ph, abort_flag)) { ok = false; break; }
+          if (kb0 + kMxGroup <= whole_kb) {
 #pragma unroll
-          for (int sub = 0; sub < kSub; ++sub) {
-            if (kb0 + sub < p.num_kb) {
-              // The planes' activation tiles are adjacent in the stage: one K-major
-              // operand of kNT rows; their results land in adjacent column blocks.
-              const uint32_t sfa = sf0 + kSfPer * sub;
+            for (int u = 0; u < kMxGroup; ++u) {
+              if (u % kSub == 0 && !wait_stage()) { ok = false; break; }
+              issue(u, wdesc + (u % kSub) * (kMxWBytes >> 4), (kb0 > 0 || u > 0) ? 1u : 0u);
+              if (u % kSub == kSub - 1) release_stage();
+            }
+          } else {   // the tile's last, partial group (and the partial K block)
 #pragma unroll
-              for (uint32_t j = 0; j < 4; ++j) {
-                // K-major e2m1 tile: 32 codes further is 32 bytes; MN-major byte tile: 32 K rows
-                const uint64_t wdesc = desc0w + (uint64_t)((sub * kMxWBytes + j * (kW8 ? 4096 : 32)) >> 4);
-                const uint64_t adesc = desc0 + (uint64_t)((kAOff + sub * kABytes + j * 32) >> 4);
-                ptx::umma_mx_elect(d_tmem, wdesc, adesc, idesc_j[j] | n_bits, (kb0 + sub > 0 || j > 0) ? 1u : 0u, sfa, sfa + 4);
+            for (int u = 0; u < kMxGroup; ++u) {
+              const int kb = kb0 + u;
+              if (kb < p.num_kb) {
+                if (u % kSub == 0 && !wait_stage()) { ok = false; break; }
+                if (kb == tail_kb) {
+                  if (!ptx::mbar_wait_s(tail_full, acc_it & 1, abort_flag)) { ok = false; break; }
+                  ptx::tc_fence_after();
+                }
+                issue(u, kb == tail_kb ? tdesc : wdesc + (u % kSub) * (kMxWBytes >> 4), kb > 0 ? 1u : 0u);
+                if (u % kSub == kSub - 1 || kb == p.num_kb - 1) release_stage();
               }
             }
           }
-          ptx::umma_commit_elect(&ctrl->empty[s]);
-          if (++s == (uint32_t)stages) { s = 0; ph ^= 1; }
+          if (!ok) break;
+          ptx::umma_commit(sf_empty0 + 8 * slot);
+          sfdesc += kSlotBytes >> 4;
+          if (++slot == kSlots) { slot = 0; slot_ph ^= 1; sfdesc = sfdesc0; }
         }
-        if (ok) { ptx::umma_commit_elect(&ctrl->acc_full[a]); ++acc_it; }
+        if (ok) { ptx::umma_commit(acc_full0 + 8 * a); ++acc_it; }
       }
     }
+    __syncwarp();
   } else if (warp < 6) {
-    // ------------------------------ scale feeders ------------------------------
-    const int q = warp & 3;                       // lane quarter this warp may write
-    const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
-    const int ft = (warp - 2) * 32 + lane;         // 0..127: tile row spread by this thread (tail
-                                                   // block), index in the cooperative copies
+    // ------------------------------ scale preparers ------------------------------
+    const int ft = (warp - 2) * 32 + lane;         // 0..127: index in the cooperative copies
+    // The weight row whose scales this thread lays out: the word of row r goes to byte
+    // (r % 32) * 16 + (r / 32) * 4 of a K block's chunk, so these rows make a warp's stores contiguous.
+    const int wrow = (warp - 2) * 8 + (lane >> 2) + 32 * (lane & 3);
     const int kgroups = p.k / 32;
-    const int n_groups = (p.num_kb + kMxGroup - 1) / kMxGroup;
     const int64_t plane_words = (int64_t)p.num_kb * p.m;
-    uint32_t s = 0, ph = 0;
+    constexpr int kPer = (kMxGroup * kNT + 127) / 128;   // token words per thread and group
+    uint32_t slot = 0, slot_ph = 0;
     int cursor = 0, cursor_next = 0, cursor_la = 0;
     bool ok = true;
 
-    // Token scales of kMxGroup K blocks: word [plane][kb][row], coalesced over the
-    // lanes.  They are read two groups ahead of their use (cur <- nxt <- nx2), by a
-    // look-ahead position (la_*) that runs over the same (tile, group) sequence.
-    uint32_t cur_b[kMxGroup][kW], nxt_b[kMxGroup][kW], nx2_b[kMxGroup][kW];
-    auto fetch_b = [&](const TileInfo& ti, int g, uint32_t (&db)[kMxGroup][kW]) {
+    // Token scales of one group: word [plane][kb][row], coalesced over the lanes, read one group
+    // ahead of their use by a look-ahead position (la_*) that runs over the same sequence.
+    // (Two register sets that change roles: a move from one to the other would wait for the loads.)
+    uint32_t tok_a[kPer], tok_b[kPer];
+    bool odd = false;
+    auto fetch_b = [&](const TileInfo& ti, int g, uint32_t (&db)[kPer]) {
 #pragma unroll
-      for (int u = 0; u < kMxGroup; ++u) {
-        const int kb = g * kMxGroup + u;
-#pragma unroll
-        for (int j = 0; j < kW; ++j) {
-          const int n = lane + 32 * j;              // row of the side-by-side token operand
-          const int term = n / BT, tok = n % BT;
-          uint32_t v = 0x7f7f7f7fu;
-          if (kb < p.num_kb && term < kTerms && tok < ti.valid)
-            v = p.a_scale[term * plane_words + (int64_t)kb * p.m + ti.row0 + tok];
-          db[u][j] = v;
-        }
+      for (int i = 0; i < kPer; ++i) {
+        const int x = ft + 128 * i;
+        const int n = x % kNT;                      // row of the side-by-side token operand
+        const int kb = g * kMxGroup + x / kNT;
+        const int term = n / BT, tok = n % BT;
+        db[i] = (x < kMxGroup * kNT && kb < p.num_kb && tok < ti.valid)
+                    ? __ldg(p.a_scale + term * plane_words + (int64_t)kb * p.m + ti.row0 + tok) : 0x7f7f7f7fu;
       }
     };
     int la_t = blockIdx.x, la_g = 0;
     TileInfo la_ti;
     bool la_valid = la_t < total_tiles;
-    if (la_valid) locate_tile<BT>(tile_start, row_start, la_t, cursor_la, la_ti);
-#define B200_MX_LA_ADVANCE()                                                              \
-  do {                                                                                    \
-    if (++la_g == n_groups) {                                                             \
-      la_g = 0;                                                                           \
-      la_t += gridDim.x;                                                                  \
-      la_valid = la_t < total_tiles;                                                      \
-      if (la_valid) locate_tile<BT>(tile_start, row_start, la_t, cursor_la, la_ti);       \
-    }                                                                                     \
-  } while (0)
-    if (la_valid) { fetch_b(la_ti, la_g, cur_b); B200_MX_LA_ADVANCE(); }
-    if (la_valid) { fetch_b(la_ti, la_g, nxt_b); B200_MX_LA_ADVANCE(); }
+    if (la_valid) {
+      locate_tile<BT>(walk, la_t, cursor_la, la_ti);
+      fetch_b(la_ti, 0, tok_a);
+    }
 
     uint32_t tile_seq = 0;
     TileInfo ti, ti_next;
@@ -360,14 +385,14 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
                  : stage_w_scales(p, ctrl, sfw, tn, seq, ft, kgroups, abort_flag);
     };
     if (staged && (int)blockIdx.x < total_tiles) {
-      locate_tile<BT>(tile_start, row_start, blockIdx.x, cursor_next, ti_next);
+      locate_tile<BT>(walk, blockIdx.x, cursor_next, ti_next);
       if (!stage(ti_next, 0u)) { *abort_flag = 1; ok = false; }
     }
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_seq) {
-      locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+      locate_tile<BT>(walk, t, cursor, ti);
       const int t_next = t + gridDim.x;
       if (staged && t_next < total_tiles) {
-        locate_tile<BT>(tile_start, row_start, t_next, cursor_next, ti_next);
+        locate_tile<BT>(walk, t_next, cursor_next, ti_next);
         if (!stage(ti_next, tile_seq + 1)) {
           *abort_flag = 1; ok = false; break;
         }
@@ -377,98 +402,73 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
         *abort_flag = 1; ok = false; break;
       }
       const uint32_t sfw_s = ptx::smem_u32(sfw + b * p.sfw_bytes);
-      const int n0 = ti.n_tile * kFeat;
-      for (int g = 0; g < n_groups && ok; ++g) {
-        if (la_valid) { fetch_b(la_ti, la_g, nx2_b); B200_MX_LA_ADVANCE(); }
+      const bool row_ok = ti.n_tile * kFeat + wrow < p.n;
+      auto group = [&](int g, const uint32_t (&use)[kPer], uint32_t (&fill)[kPer]) {
+        if (++la_g == n_groups) {
+          la_g = 0;
+          la_t += gridDim.x;
+          la_valid = la_t < total_tiles;
+          if (la_valid) locate_tile<BT>(walk, la_t, cursor_la, la_ti);
+        }
+        if (la_valid) fetch_b(la_ti, la_g, fill);
+        // this row's scale bytes of the group's four K blocks, one word each; bytes of groups past
+        // the row's end become 0x7f
+        uint32_t wa[kMxGroup];
+        const int left = kgroups - 16 * g;
+        if (!kW8) {
+          const uint32_t addr = sfw_s + wrow * kgroups + 16 * g;   // any alignment: aligned words and a funnel shift
+          uint32_t v[kMxGroup + 1];
 #pragma unroll
-        for (int u = 0; u < kMxGroup; ++u) {
-          const int kb = g * kMxGroup + u;
-          const int sub = u % kSub;                  // position of this K block in its stage
-          if (kb < p.num_kb && ok) {
-            // Four scale bytes per row from the staged piece: two aligned words and a
-            // funnel shift (rows are K/32 bytes apart, any alignment); bytes of groups
-            // past the row end become 0x7f.
-            uint32_t wa[4];
-            const int left = kgroups - 4 * kb;
-            const uint32_t keep = left >= 4 ? 0xffffffffu : ((1u << (8 * left)) - 1u);
+          for (int u = 0; u <= kMxGroup; ++u) v[u] = ptx::lds32((addr & ~3u) + 4 * u);
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const int row = lane + 32 * j;
-              if (!kW8) {
-                const uint32_t addr = sfw_s + row * kgroups + 4 * kb;
-                const uint32_t lo = ptx::lds32(addr & ~3u), hi = ptx::lds32((addr & ~3u) + 4);
-                const uint32_t v = __funnelshift_r(lo, hi, (addr & 3u) * 8);
-                wa[j] = (n0 + row < p.n) ? ((v & keep) | (0x7f7f7f7fu & ~keep)) : 0x7f7f7f7fu;
-              } else if (p.w8_block) {
-                // staged as [group][128 features]: one byte per group of this K block
-                uint32_t v = 0;
+          for (int u = 0; u < kMxGroup; ++u) wa[u] = __funnelshift_r(v[u], v[u + 1], (addr & 3u) * 8);
+        } else if (p.w8_block) {
+          // staged as [group][128 features]: one byte per group
 #pragma unroll
-                for (int gq = 0; gq < 4; ++gq)
-                  if (gq < left) v |= ptx::lds8(sfw_s + (4 * kb + gq) * 128 + row) << (8 * gq);
-                wa[j] = (n0 + row < p.n) ? (v | (0x7f7f7f7fu & ~keep)) : 0x7f7f7f7fu;
-              } else {
-                wa[j] = 0x7f7f7f7fu;   // per-tensor scale: applied in the epilogue
-              }
-            }
-            if (sub == 0) {   // the stage's scale columns and weight buffer are free again
-              if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag))) {
-                *abort_flag = 1; ok = false;
-              }
-              ptx::tc_fence_after();
-            }
-            if (ok) {
-              const uint32_t col = tmem_base + kSfBase + s * kSfCols + kSfPer * sub + lane_sel;
-              {
-                // eight columns at once: the weight rows' four, then the tokens' (unused ones 2^0)
-                uint32_t r8[8];
+          for (int u = 0; u < kMxGroup; ++u) {
+            wa[u] = 0;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) { r8[j] = wa[j]; r8[4 + j] = j < kW ? cur_b[u][j < kW ? j : 0] : 0x7f7f7f7fu; }
-                ptx::tmem_st_32x8(col, r8);
-                if (kW > 4)   // token tiles wider than 128 columns: their remaining scale columns
-                  ptx::tmem_st_32x4(col + 8, cur_b[u][4 < kW ? 4 : 0], 5 < kW ? cur_b[u][5 < kW ? 5 : 0] : 0x7f7f7f7fu,
-                                    0x7f7f7f7fu, 0x7f7f7f7fu);
-              }
-              if (kb == tail_kb) {
-                // Spread the partial block: row ft, 64 packed bytes -> eight 16-byte
-                // slots (8 data bytes each), slot index xor-ed with (ft & 7).
-                if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->full[s], ph, abort_flag))) {
-                  *abort_flag = 1; ok = false;
-                } else {
-                  const uint32_t st = ptx::smem_u32(smem + s * stage_bytes);
-                  const uint32_t src = (p.raw_shared ? ptx::smem_u32(raw_one) : st + kRawOff) + ft * 64;
-                  const uint32_t dst = st + sub * kMxWBytes + (ft >> 3) * 1024 + (ft & 7) * 128;
-#pragma unroll
-                  for (int c = 0; c < 4; ++c) {
-                    const uint4 v = ptx::lds128(src + c * 16);
-                    ptx::sts64(dst + (((2 * c) ^ (ft & 7)) << 4), v.x, v.y);
-                    ptx::sts64(dst + (((2 * c + 1) ^ (ft & 7)) << 4), v.z, v.w);
-                  }
-                  ptx::fence_proxy_async();
-                }
-              }
-              if (sub == kSub - 1 || kb == p.num_kb - 1) {   // last K block of the stage
-                ptx::tmem_wait_st();
-                ptx::tc_fence_before();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&ctrl->sf_full[s]);
-                if (++s == (uint32_t)stages) { s = 0; ph ^= 1; }
-              }
-            }
+            for (int q = 0; q < 4; ++q)
+              if (4 * u + q < left) wa[u] |= ptx::lds8(sfw_s + (16 * g + 4 * u + q) * 128 + wrow) << (8 * q);
           }
         }
 #pragma unroll
-        for (int u = 0; u < kMxGroup; ++u)
+        for (int u = 0; u < kMxGroup; ++u) {
+          const int lu = left - 4 * u;
+          const uint32_t keep = lu >= 4 ? 0xffffffffu : (lu <= 0 ? 0u : ((1u << (8 * lu)) - 1u));
+          if (!staged || !row_ok) wa[u] = 0x7f7f7f7fu;   // per-tensor scale: applied in the epilogue
+          else wa[u] = (wa[u] & keep) | (0x7f7f7f7fu & ~keep);
+        }
+        // the ring slot's previous group has been copied to tensor memory
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->sf_empty[slot], slot_ph ^ 1, abort_flag))) {
+          *abort_flag = 1;
+          return false;
+        }
+        const uint32_t ring = ptx::smem_u32(sf_ring) + slot * kSlotBytes;
 #pragma unroll
-          for (int j = 0; j < kW; ++j) { cur_b[u][j] = nxt_b[u][j]; nxt_b[u][j] = nx2_b[u][j]; }
-      }
+        for (int u = 0; u < kMxGroup; ++u) ptx::sts32(ring + u * 512 + (wrow & 31) * 16 + (wrow >> 5) * 4, wa[u]);
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) {
+          const int x = ft + 128 * i;
+          const int n = x % kNT, u = x / kNT;
+          if (x < kMxGroup * kNT)
+            ptx::sts32(ring + kMxGroup * 512 + u * (kTokChunks * 512) + (n >> 7) * 512 + (n & 31) * 16 +
+                       ((n >> 5) & 3) * 4, use[i]);
+        }
+        ptx::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&ctrl->sf_full[slot]);
+        if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
+        return true;
+      };
+      for (int g = 0; g < n_groups && ok; ++g, odd = !odd) ok = odd ? group(g, tok_b, tok_a) : group(g, tok_a, tok_b);
+      if (!ok) break;
       if (staged) {
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&ctrl->sfw_empty[b]);
       }
     }
-#undef B200_MX_LA_ADVANCE
-    if (warp == 2 && lane == 0)
-    ptx::cp_async_wait_all();
+    ptx::cp_async_wait_all();   // staged pieces of an aborted walk
   } else {
     // ------------------------------ epilogue ----------------------------------
     const int q = warp & 3;
@@ -476,17 +476,55 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
     const int n_out = p.swiglu ? p.n / 2 : p.n;
     uint32_t acc_it = 0;
-    int cursor = 0;
+    int cursor = 0, cursor_next = 0;
     bool ok = true;
+    // The partial K block (K = 64 past a multiple of 128): row et's 32 packed bytes, fetched a tile
+    // ahead; the other half of the block's codes stay zero, like the tokens' there.
+    uint4 tail_q[2] = {};
+    auto fetch_tail = [&](const TileInfo& tn) {
+      const int f = tn.n_tile * kFeat + et;
+      const uint4* src = reinterpret_cast<const uint4*>(p.w + ((int64_t)tn.e * p.n + f) * (p.k / 2) + tail_kb * 64);
+      tail_q[0] = f < p.n ? __ldg(src) : make_uint4(0, 0, 0, 0);
+      tail_q[1] = f < p.n ? __ldg(src + 1) : make_uint4(0, 0, 0, 0);
+    };
+    if (tail_kb >= 0) {
+      const uint32_t dst = ptx::smem_u32(tail_w) + (et >> 3) * 1024 + (et & 7) * 128;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) ptx::sts128(dst + c * 16, make_uint4(0, 0, 0, 0));
+      if ((int)blockIdx.x < total_tiles) {
+        TileInfo tn;
+        locate_tile<BT>(walk, blockIdx.x, cursor_next, tn);
+        fetch_tail(tn);
+      }
+    }
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
       TileInfo ti;
-      locate_tile<BT>(tile_start, row_start, t, cursor, ti);
+      locate_tile<BT>(walk, t, cursor, ti);
       const int feat = ti.n_tile * kFeat + et;
       const bool feat_ok = feat < p.n;
       float bias_v = 0.f;
       if (p.bias != nullptr && feat_ok) bias_v = load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + feat);
       const float w_mul = (kW8 && !p.w8_block) ? p.w_tensor_scale[ti.e] : 1.0f;
       const uint32_t a = acc_it & 1;
+      if (tail_kb >= 0) {
+        // The previous tile's MMAs are complete (its accumulator has been waited for): write this
+        // tile's partial block, row et: 32 packed bytes -> four of the row's eight 16-byte slots
+        // (8 data bytes each), slot index xor-ed with (et & 7).
+        const uint32_t dst = ptx::smem_u32(tail_w) + (et >> 3) * 1024 + (et & 7) * 128;
+        ptx::sts64(dst + ((0 ^ (et & 7)) << 4), tail_q[0].x, tail_q[0].y);
+        ptx::sts64(dst + ((1 ^ (et & 7)) << 4), tail_q[0].z, tail_q[0].w);
+        ptx::sts64(dst + ((2 ^ (et & 7)) << 4), tail_q[1].x, tail_q[1].y);
+        ptx::sts64(dst + ((3 ^ (et & 7)) << 4), tail_q[1].z, tail_q[1].w);
+        ptx::fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&ctrl->tail_full);
+        const int t_next = t + gridDim.x;
+        if (t_next < total_tiles) {
+          TileInfo tn;
+          locate_tile<BT>(walk, t_next, cursor_next, tn);
+          fetch_tail(tn);
+        }
+      }
       // a whole tile's MMAs away: poll from one lane, sleeping in between, so that the
       // wait does not take issue slots from the feeder warp on the same scheduler
       if (!ptx::mbar_wait_warp(&ctrl->acc_full[a], (acc_it >> 1) & 1, abort_flag, 128)) { ok = false; break; }
@@ -556,33 +594,20 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 template <int BT, int kTerms, int kSub, bool kW8>
-int launch_mx(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& traw, MxParams& p,
-              int grid, cudaStream_t st) {
+int launch_mx(const CUtensorMap& ta, const CUtensorMap& tw, MxParams& p, int grid, cudaStream_t st) {
   auto kern = grouped_gemm_mx_kernel<BT, kTerms, kSub, kW8>;
-  const uint32_t need = 2 * kTerms * BT + kMxMaxStages * (kTerms * BT > 128 ? 16 : 8) * kSub;
+  const uint32_t need = 2 * kTerms * BT + kMxGroup * (kTerms * BT > 128 ? 16 : 8);
   p.tmem_cols = need <= 128 ? 128u : (need <= 256 ? 256u : 512u);
-  // The partial K block's packed bytes get one buffer for the whole CTA when a tile
-  // has at least as many stages as the pipeline (its next use then comes after
-  // the previous one was consumed), else one per stage.
   const int body = kSub * (kMxWBytes + kTerms * BT * 128);
-  const int fixed = 1024 + (int)((sizeof(MxCtrl) + 15) & ~(size_t)15) + 2 * mx_prefix_bytes(p.num_experts) +
-                    2 * p.sfw_bytes;
-  const int budget = 227 * 1024 - fixed;
-  const int num_st = (p.num_kb + kSub - 1) / kSub;
-  p.raw_shared = 0;
-  p.stage_bytes = body + (p.tail ? kMxRawBytes : 0);
-  p.stages = budget / p.stage_bytes;
-  if (p.tail) {
-    int st_shared = (budget - kMxRawBytes) / body;
-    if (st_shared > kMxMaxStages) st_shared = kMxMaxStages;
-    if (st_shared > p.stages && num_st >= st_shared) { p.raw_shared = 1; p.stage_bytes = body; p.stages = st_shared; }
-  }
+  const int fixed = 1024 + (p.tail ? kMxWBytes : 0) + mx_slots<kTerms * BT>() * mx_slot_bytes<kTerms * BT>() +
+                    (int)((sizeof(MxCtrl) + 15) & ~(size_t)15) + tile_walk_bytes(p.num_experts) + 2 * p.sfw_bytes;
+  p.stages = (227 * 1024 - fixed) / body;
   if (p.stages > kMxMaxStages) p.stages = kMxMaxStages;
   if (p.stages < 2) return fail(B200MOE_E_UNSUPPORTED, "block-scaled GEMM: tile does not fit shared memory");
-  const size_t smem = (size_t)fixed + (size_t)p.stages * p.stage_bytes + (p.raw_shared ? kMxRawBytes : 0);
+  const size_t smem = (size_t)fixed + (size_t)p.stages * body;
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, smem)) return rc;
-  kern<<<grid, kMxThreads, smem, st>>>(ta, tw, traw, p);
+  kern<<<grid, kMxThreads, smem, st>>>(ta, tw, p);
   B200_LAUNCH_OK("grouped_gemm_mx_kernel");
   return B200MOE_OK;
 }
@@ -616,6 +641,7 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   if (a->m == 0 || a->n == 0) return B200MOE_OK;
 
   MxParams p;
+  p.w = reinterpret_cast<const uint8_t*>(a->w);
   p.w_scale = reinterpret_cast<const uint8_t*>(a->w_scale);
   p.w_tensor_scale = reinterpret_cast<const float*>(a->w_scale);
   p.a_scale = reinterpret_cast<const uint32_t*>(a->a_scale);
@@ -639,7 +665,7 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
     // tensor) are staged in shared memory: every tile's piece must start on a
     // 16-byte boundary and two pieces must fit.
     const int kgroups = a->k / 32;
-    const int piece = ((128 * kgroups + 15) & ~15) + 16;
+    const int piece = ((128 * kgroups + 15) & ~15) + 32;   // the last row's words are read past its end
     if (((uintptr_t)a->w_scale & 15) != 0 || ((int64_t)a->n * kgroups) % 16 != 0 || piece > kMxSfwCap)
       return fail(B200MOE_E_UNSUPPORTED,
                   "block-scaled GEMM: N * K / 32 must be a multiple of 16, K at most 6144, scales 16-byte aligned");
@@ -661,11 +687,11 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   const uint32_t a_fmt = w4 ? 5u : (a->w_format == B200MOE_W_FP8E5M2_TENSOR_KN ? 1u : 0u);
   p.idesc = ptx::make_idesc_mx(a_fmt, 0u, kFeat, (uint32_t)(bt * p.terms)) | (w8 ? (1u << 15) : 0u);
 
-  CUtensorMap ta, tw, traw;
+  CUtensorMap ta, tw;
   {
     cuuint64_t dims[3] = {(cuuint64_t)a->k, (cuuint64_t)a->m, (cuuint64_t)p.terms};
     cuuint64_t strides[2] = {(cuuint64_t)a->k, (cuuint64_t)a->k * (cuuint64_t)a->m};
-    cuuint32_t box[3] = {128, (cuuint32_t)bt, 1};
+    cuuint32_t box[3] = {128, (cuuint32_t)bt, (cuuint32_t)p.terms};
     int rc = encode_map(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->a, dims, strides, box);
     if (rc) return rc;
   }
@@ -675,7 +701,6 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
     cuuint32_t box[3] = {128, 128, 1};
     int rc = encode_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->w, dims, strides, box);
     if (rc) return rc;
-    traw = tw;
   } else {
     {
       // Whole 128-code blocks only: this tensor-map type wants the inner extent to be
@@ -684,14 +709,6 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
       cuuint64_t strides[2] = {(cuuint64_t)(a->k / 2), (cuuint64_t)(a->k / 2) * a->n};
       cuuint32_t box[3] = {128, (cuuint32_t)kFeat, 1};
       int rc = encode_map(&tw, CU_TENSOR_MAP_DATA_TYPE_16U4_ALIGN16B, 3, a->w, dims, strides, box);
-      if (rc) return rc;
-    }
-    {
-      cuuint64_t dims[3] = {(cuuint64_t)(a->k / 2), (cuuint64_t)a->n, (cuuint64_t)a->num_experts};
-      cuuint64_t strides[2] = {(cuuint64_t)(a->k / 2), (cuuint64_t)(a->k / 2) * a->n};
-      cuuint32_t box[3] = {64, (cuuint32_t)kFeat, 1};
-      int rc = encode_map(&traw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->w, dims, strides, box,
-                          CU_TENSOR_MAP_SWIZZLE_NONE);
       if (rc) return rc;
     }
   }
@@ -703,14 +720,14 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   // Small token tiles move two K blocks per pipeline stage.
 #define B200_MX_CASES(W8)                                                              \
   if (x2) {                                                                            \
-    if (bt == 16) return launch_mx<16, 2, 2, W8>(ta, tw, traw, p, grid, st);           \
-    if (bt == 96) return launch_mx<96, 2, 1, W8>(ta, tw, traw, p, grid, st);           \
-    return launch_mx<64, 2, 1, W8>(ta, tw, traw, p, grid, st);                         \
+    if (bt == 16) return launch_mx<16, 2, 2, W8>(ta, tw, p, grid, st);                 \
+    if (bt == 96) return launch_mx<96, 2, 1, W8>(ta, tw, p, grid, st);                 \
+    return launch_mx<64, 2, 1, W8>(ta, tw, p, grid, st);                               \
   }                                                                                    \
-  if (bt == 192) return launch_mx<192, 1, 1, W8>(ta, tw, traw, p, grid, st);           \
-  if (bt == 16) return launch_mx<16, 1, 2, W8>(ta, tw, traw, p, grid, st);             \
-  if (bt == 64) return launch_mx<64, 1, 2, W8>(ta, tw, traw, p, grid, st);             \
-  return launch_mx<128, 1, 1, W8>(ta, tw, traw, p, grid, st);
+  if (bt == 192) return launch_mx<192, 1, 1, W8>(ta, tw, p, grid, st);                 \
+  if (bt == 16) return launch_mx<16, 1, 2, W8>(ta, tw, p, grid, st);                   \
+  if (bt == 64) return launch_mx<64, 1, 2, W8>(ta, tw, p, grid, st);                   \
+  return launch_mx<128, 1, 1, W8>(ta, tw, p, grid, st);
   if (w8) { B200_MX_CASES(true) }
   B200_MX_CASES(false)
 #undef B200_MX_CASES

@@ -94,6 +94,49 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
   return true;
 }
 
+// The wait of the producer and issuer loops, which are single threads whose instruction chain
+// bounds a CTA's streaming rate: barriers are 32-bit shared addresses and only the first poll is
+// inline (measured on a loop of one wait, one expect_tx and one load: 198 instead of 378 cycles).
+// Same budget and abort rules as mbar_wait.
+__device__ __forceinline__ bool mbar_try_wait_s(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+static __device__ __noinline__ bool mbar_wait_rest(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  const long long t0 = clock64();
+  uint32_t spins = 0;
+  while (!mbar_try_wait_s(bar, parity)) {
+    if ((++spins & 0xff) == 0) {
+      if (*abort_flag != 0) return false;
+      if (clock64() - t0 > kWaitBudgetCycles) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
+__device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  return mbar_try_wait_s(bar, parity) || mbar_wait_rest(bar, parity, abort_flag);
+}
+__device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+// True in one lane of a converged warp.  Code under it issues TMA and MMA instructions about twice
+// as fast as under `lane == 0`: the compiler knows that a single lane runs it.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t one;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+  return one != 0;
+}
+
 // Warp-level wait: lane 0 polls (sleeping `sleep_ns` between polls when non-zero),
 // the other lanes wait at the warp barrier, which also orders their later reads
 // after the barrier's completion.  Keeps the polling traffic of long waits off
@@ -139,6 +182,30 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
       ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0),
       "r"(c1), "r"(c2)
       : "memory");
+}
+
+// The same with 32-bit shared addresses.
+__device__ __forceinline__ void tma_load_2d_s(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_s(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1,
+                                              int c2) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];"
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
+      : "memory");
+}
+
+// Brings a tile into L2 only.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2)
+               : "memory");
 }
 
 // ---- CTA pairs (a cluster of two CTAs working on one tcgen05.mma tile) ----------------
@@ -356,6 +423,12 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr, uint32_t 
   return d;
 }
 
+// The same without a swizzle: rows of 16 bytes, eight rows (one 128-byte core matrix) after
+// another, core matrices `sbo_bytes` apart.
+__device__ __forceinline__ uint64_t make_smem_desc_plain(uint32_t smem_addr, uint32_t sbo_bytes) {
+  return (uint64_t)((smem_addr >> 4) & 0x3fff) | ((uint64_t)((sbo_bytes >> 4) & 0x3fff) << 32) | ((uint64_t)1 << 46);
+}
+
 // Instruction descriptor of tcgen05.mma kind::f16 / kind::f8f6f4, fp32 accumulate.
 // fmt: kind::f16 -> 0 = f16, 1 = bf16; kind::f8f6f4 -> 0 = e4m3, 1 = e5m2.
 // major: 0 = K-major, 1 = MN-major.
@@ -373,24 +446,55 @@ __host__ __device__ constexpr uint32_t make_idesc_mx(uint32_t a_fmt, uint32_t b_
                                                      uint32_t N) {
   return (a_fmt << 7) | (b_fmt << 10) | ((N >> 3) << 17) | (1u << 23) | ((M >> 4) << 24);
 }
-// tcgen05.mma and tcgen05.commit for a warp that runs the issue loop convergently (all lanes
-// hold the same operands): one elected lane issues.  A warp-uniform loop lets the compiler keep
-// descriptors and barrier addresses in uniform registers (measured on the fp8 kernel: 4 MMAs
-// and 2 commits issue in 370 instead of 640 cycles).  A commit makes `bar` receive one arrival
-// when all MMAs issued so far by that lane have completed.
-//
 // Block-scaled form: D[tmem_d] (+)= (A * 2^(sfa-127)) * (B * 2^(sfb-127)) over K = 32; sfa / sfb
 // are tensor-memory addresses of the scale columns (one byte per row, replicated in the four
-// lane quarters).
-__device__ __forceinline__ void umma_mx_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                              uint32_t idesc, uint32_t accumulate, uint32_t sfa,
-                                              uint32_t sfb) {
-  asm volatile(
-      "{\n\t.reg .pred pe, pa;\n\telect.sync _|pe, 0xffffffff;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
-      "@pe tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], pa;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
-      : "memory");
+// lane quarters).  Issued by one thread (elect_one), like umma_commit.
+//
+// One 128-wide K block in one statement: the block's scale chunks are copied from shared to tensor
+// memory (tcgen05.cp 32x128b.warpx4: 32 rows of 16 bytes -> four columns, replicated in the four
+// lane quarters; the weight rows' to column sf, the tokens' kTokChunks chunks to the columns after
+// them), then the four K = 32 instructions run on scale bytes 0..3 of those columns.  kWStep:
+// 16-byte units between the K steps of the weight operand (the tokens' are 32 bytes apart).
+template <int kTokChunks, int kWStep>
+__device__ __forceinline__ void umma_mx_block(uint32_t tmem_d, uint64_t wdesc, uint64_t adesc, uint32_t idesc,
+                                                    uint32_t accumulate, uint32_t sf, uint64_t sfw_desc,
+                                                    uint64_t sfa_desc) {
+#define B200_MX_MMA4                                                                                             \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [t], pa;\n\t"             \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w1, a1, i1, [%5], [t], 1;\n\t"              \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w2, a2, i2, [%5], [t], 1;\n\t"              \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w3, a3, i3, [%5], [t], 1;\n\t}"
+#define B200_MX_HEAD                                                                                             \
+      "{\n\t.reg .pred pa;\n\t.reg .b32 t, i1, i2, i3;\n\t.reg .b64 w1, w2, w3, a1, a2, a3;\n\t"              \
+      "setp.ne.b32 pa, %4, 0;\n\tadd.u32 t, %5, 4;\n\t"                                                          \
+      "add.u64 w1, %1, %8;\n\tadd.u64 w2, %1, %9;\n\tadd.u64 w3, %1, %10;\n\t"                                   \
+      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"                                       \
+      "or.b32 i1, %3, 0x20000010;\n\tor.b32 i2, %3, 0x40000020;\n\tor.b32 i3, %3, 0x60000030;\n\t"               \
+      "tcgen05.cp.cta_group::1.32x128b.warpx4 [%5], %6;\n\t"                                                 \
+      "tcgen05.cp.cta_group::1.32x128b.warpx4 [t], %7;\n\t"
+  if (kTokChunks == 1) {
+    asm volatile(B200_MX_HEAD B200_MX_MMA4
+                 ::"r"(tmem_d), "l"(wdesc), "l"(adesc), "r"(idesc), "r"(accumulate), "r"(sf), "l"(sfw_desc),
+                 "l"(sfa_desc), "n"(kWStep), "n"(2 * kWStep), "n"(3 * kWStep)
+                 : "memory");
+  } else {
+    asm volatile(B200_MX_HEAD
+                 "{\n\t.reg .b32 t2;\n\t.reg .b64 c2;\n\tadd.u32 t2, %5, 8;\n\tadd.u64 c2, %7, 32;\n\t"
+                 "tcgen05.cp.cta_group::1.32x128b.warpx4 [t2], c2;\n\t}\n\t" B200_MX_MMA4
+                 ::"r"(tmem_d), "l"(wdesc), "l"(adesc), "r"(idesc), "r"(accumulate), "r"(sf), "l"(sfw_desc),
+                 "l"(sfa_desc), "n"(kWStep), "n"(2 * kWStep), "n"(3 * kWStep)
+                 : "memory");
+  }
+#undef B200_MX_MMA4
+#undef B200_MX_HEAD
 }
+// A commit makes the barrier receive one arrival when all tcgen05 operations issued so far by this
+// thread have completed.
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// tcgen05.mma and tcgen05.commit for a warp that runs the issue loop convergently (all lanes
+// hold the same operands): one elected lane issues.
 template <bool kFp8>
 __device__ __forceinline__ void umma_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
                                            uint32_t idesc, uint32_t accumulate) {
@@ -455,6 +559,9 @@ __device__ __forceinline__ void sts64(uint32_t addr, uint32_t a, uint32_t b) {
 }
 __device__ __forceinline__ void sts16(uint32_t addr, uint16_t v) {
   asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
+}
+__device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
+  asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void sts32f(uint32_t addr, float v) {
   asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
