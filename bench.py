@@ -381,19 +381,21 @@ def time_gemms(cfg, layer, ids, T, dev, iters, ep_world=1, ep_rank=0):
 
 def launches_per_step(cfg, T, layer, ep_world, transport) -> int:
     """Kernels of this repository launched by one step, counted from the code path taken:
-    routing 1; sort 1 (<= 2048 slots) or 3; row copy (+quant) 1; gemm1 1; activation (+quant) 1
-    unless fused into gemm1; MX activation quantisers 2; gemm2 1; gather 1.  Expert parallelism
+    routing 1; sort 3 and row copy (+quant) 1, or one kernel for both (<= 2048 slots, top-k <= 8);
+    gemm1 1; activation (+quant) 1 unless fused into gemm1; MX quantiser of gemm2's input 1; gemm2 1;
+    gather 1.  Expert parallelism
     over peer memory: routing 1, dispatch sort 1|3 + dispatch 1, mask 1, the local layer without
     its gather, combine 1, final gather 1."""
     local = layer.local if ep_world > 1 else layer
     act = 0 if local.fuses_activation(T * cfg.K) else 1
-    mx = 2 if getattr(local, "mx_acts", False) else 0
+    mx = 1 if getattr(local, "mx_acts", False) else 0
     sort = lambda slots: 1 if slots <= 2048 else 3
+    place = lambda slots: 1 if slots <= 2048 and cfg.K <= 8 else sort(slots) + 1
     if ep_world == 1:
-        return 1 + sort(T * cfg.K) + 1 + 1 + act + mx + 1 + 1
+        return 1 + place(T * cfg.K) + 1 + act + mx + 1 + 1
     if transport == "peer":
-        return 1 + sort(T * ep_world) + 1 + 1 + sort(ep_world * T * cfg.K) + 1 + 1 + act + mx + 1 + 1 + 1
-    return 1 + sort(T * ep_world) + 1 + sort(T * ep_world * cfg.K) + 1 + 1 + act + mx + 1 + 1 + 1
+        return 1 + sort(T * ep_world) + 1 + 1 + place(ep_world * T * cfg.K) + 1 + act + mx + 1 + 1 + 1
+    return 1 + place(T * ep_world) + place(T * ep_world * cfg.K) + 1 + act + mx + 1 + 1 + 1
 
 
 def stage_times(cfg, layer, step, x, logits, bias, reps=5):

@@ -294,6 +294,17 @@ int b200moe_remap_quant_fp8(const void* hidden, b200moe_dtype dtype,
                             int total_experts, int local_experts,
                             void* workspace, size_t workspace_bytes,
                             b200moe_stream stream);
+/* The same with MXFP8 planes (b200moe_quant_mxfp8) instead of fp8: codes
+ * [planes][T*K,H], scale words [planes][ceil(H/128)][T*K]. */
+int b200moe_remap_quant_mxfp8(const void* hidden, b200moe_dtype dtype,
+                              void* remapped_q, void* remapped_scales, int planes,
+                              const int32_t* expert_map,
+                              int32_t* rows_per_expert, int32_t* row_map,
+                              const void* topk_ids, b200moe_dtype ids_dtype,
+                              int64_t num_rows, int hidden_size, int topk,
+                              int total_experts, int local_experts,
+                              void* workspace, size_t workspace_bytes,
+                              b200moe_stream stream);
 
 /* ------------------------------------------------------------------------- */
 /* Grouped GEMM                                                               */

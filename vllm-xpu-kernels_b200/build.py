@@ -29,7 +29,7 @@ INCLUDE = HERE.parent / "include"
 
 CU_SOURCES = ["abi.cu", "routing.cu", "permute.cu", "ep.cu", "elementwise.cu", "fused_quant.cu", "gemm.cu",
               "gemm_check.cu", "gemm_tc.cu", "gemm_tc_dq.cu", "gemm_tc_mx.cu", "gemm_tc_fp8t.cu"]
-SHIMS = {"_C": "c_ops.cpp", "_moe_C": "moe_ops.cpp", "_xpu_C": "xpu_ops.cpp"}
+SHIMS = {"_C": ["c_ops.cpp"], "_moe_C": ["moe_ops.cpp"], "_xpu_C": ["xpu_ops.cpp", "layer.cpp"]}
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3",
               "-std=c++17", "-Xcompiler", "-fPIC", "--threads", "2"]
@@ -88,16 +88,16 @@ def build_shims(force: bool = False) -> None:
     abi = int(torch._C._GLIBCXX_USE_CXX11_ABI)
     common = ["g++", "-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-DTORCH_API_INCLUDE_EXTENSION_H",
               f"-D_GLIBCXX_USE_CXX11_ABI={abi}", "-Wno-deprecated-declarations"] + inc
-    headers = [CSRC / "torch" / "shim.h", INCLUDE / "b200moe.h"]
+    headers = list((CSRC / "torch").glob("*.h")) + [INCLUDE / "b200moe.h"]
     jobs = []
-    for name, src in SHIMS.items():
+    for name, sources in SHIMS.items():
         out = PKG / f"{name}.so"
-        srcp = CSRC / "torch" / src
-        if force or not _newer(out, [srcp] + headers):
-            jobs.append(common + ["-shared", str(srcp), "-o", str(out),
+        srcs = [CSRC / "torch" / src for src in sources]
+        if force or not _newer(out, srcs + headers):
+            jobs.append(common + ["-shared", *map(str, srcs), "-o", str(out),
                                   "-fvisibility=default",
                                   "-L", str(PKG), "-lb200moe", "-L", torch_lib, "-ltorch", "-ltorch_cpu",
-                                  "-lc10", "-lc10_cuda", "-ltorch_cuda",
+                                  "-lc10", "-lc10_cuda", "-ltorch_cuda", "-ltorch_python",
                                   "-Wl,-rpath,$ORIGIN", f"-Wl,-rpath,{torch_lib}"])
     with ThreadPoolExecutor(max_workers=3) as pool:
         list(pool.map(_run, jobs))

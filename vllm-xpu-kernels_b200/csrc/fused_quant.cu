@@ -70,6 +70,8 @@ constexpr int kRows = 4;
 template <typename T, bool kGated, int kFmt>
 __global__ void __launch_bounds__(1024)
 group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Vec16<T>::N;
   const int64_t r0 = (int64_t)blockIdx.x * kRows;
   if (a.rows_per_segment != nullptr) {
@@ -183,6 +185,8 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 silu_mul_static_quant_kernel(uint8_t* __restrict__ out, const T* __restrict__ in,
                              const float* __restrict__ scale, int d, bool vec_ok) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int N = Vec16<T>::N;
   const int64_t r = blockIdx.x;
   const T* g = in + r * 2 * (int64_t)d;
@@ -214,13 +218,18 @@ template <bool kGated, int kFmt>
 int launch_group_quant(b200moe_dtype dtype, const GroupQuantArgs& a, int64_t rows, cudaStream_t st,
                        const char* name) {
   if (dtype == B200MOE_BF16) {
-    group_quant_kernel<__nv_bfloat16, kGated, kFmt><<<(unsigned)((rows + kRows - 1) / kRows), threads_for(a.hidden / 8), 0, st>>>(a, rows);
+    B200_LAUNCHED("group_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<__nv_bfloat16, kGated, kFmt>,
+        dim3((unsigned)((rows + kRows - 1) / kRows)), dim3(threads_for(a.hidden / 8)), 0, st,
+        a, rows));
   } else if (dtype == B200MOE_F16) {
-    group_quant_kernel<__half, kGated, kFmt><<<(unsigned)((rows + kRows - 1) / kRows), threads_for(a.hidden / 8), 0, st>>>(a, rows);
+    B200_LAUNCHED("group_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<__half, kGated, kFmt>,
+        dim3((unsigned)((rows + kRows - 1) / kRows)), dim3(threads_for(a.hidden / 8)), 0, st,
+        a, rows));
   } else {
-    group_quant_kernel<float, kGated, kFmt><<<(unsigned)((rows + kRows - 1) / kRows), threads_for(a.hidden / 4), 0, st>>>(a, rows);
+    B200_LAUNCHED("group_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<float, kGated, kFmt>,
+        dim3((unsigned)((rows + kRows - 1) / kRows)), dim3(threads_for(a.hidden / 4)), 0, st,
+        a, rows));
   }
-  B200_LAUNCH_OK(name);
   return B200MOE_OK;
 }
 
@@ -299,11 +308,12 @@ extern "C" int b200moe_silu_and_mul_quant(void* out, const void* in, b200moe_dty
   B200_CHECK_ARG(out && in && scale, "silu_and_mul_quant: null pointer");
   const bool vec_ok = d % 8 == 0 && aligned16(in) && (((uintptr_t)out & 7) == 0);
   if (dtype == B200MOE_BF16)
-    silu_mul_static_quant_kernel<__nv_bfloat16><<<(unsigned)rows, 256, 0, as_stream(stream)>>>(
-        (uint8_t*)out, (const __nv_bfloat16*)in, scale, d, vec_ok);
+    B200_LAUNCHED("silu_mul_static_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, silu_mul_static_quant_kernel<__nv_bfloat16>,
+        dim3((unsigned)rows), dim3(256), 0, as_stream(stream),
+        (uint8_t*)out, (const __nv_bfloat16*)in, scale, d, vec_ok));
   else
-    silu_mul_static_quant_kernel<__half><<<(unsigned)rows, 256, 0, as_stream(stream)>>>(
-        (uint8_t*)out, (const __half*)in, scale, d, vec_ok);
-  B200_LAUNCH_OK("silu_and_mul_quant");
+    B200_LAUNCHED("silu_mul_static_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, silu_mul_static_quant_kernel<__half>,
+        dim3((unsigned)rows), dim3(256), 0, as_stream(stream),
+        (uint8_t*)out, (const __half*)in, scale, d, vec_ok));
   return B200MOE_OK;
 }

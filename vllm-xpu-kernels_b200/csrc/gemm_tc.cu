@@ -125,6 +125,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
+    pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
@@ -145,6 +146,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
+  pdl_wait();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -434,6 +436,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 
   // Teardown: everyone meets here, also after an aborted wait.
+  pdl_trigger();
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -451,8 +454,7 @@ int launch_tc(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams& p, i
   static_assert(smem_bytes<BT, kFp8, kGated>() <= kMaxSmem, "shared memory");
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, smem_bytes<BT, kFp8, kGated>())) return rc;
-  kern<<<grid, kTcThreads, smem_bytes<BT, kFp8, kGated>(), st>>>(ta, tw, p);
-  B200_LAUNCH_OK("grouped_gemm_tc_kernel");
+  B200_LAUNCHED("grouped_gemm_tc_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kTcThreads), smem_bytes<BT, kFp8, kGated>(), st, ta, tw, p));
   return B200MOE_OK;
 }
 
@@ -508,6 +510,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int pair_tiles = kGated ? p.n_tiles : (p.n_tiles + 1) / 2;
 
   if (warp == 0) {
+    pdl_wait();
     build_tile_walk<kPairTok>(p.rows_per_expert, p.num_experts, pair_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
@@ -535,6 +538,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
+  pdl_wait();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::cluster_sync();   // both CTAs' barriers and tensor memory exist before either signals the other
@@ -714,6 +718,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
   // Teardown: neither CTA frees tensor memory or leaves while the other may still use its
   // shared memory, its barriers or MMAs in flight (every thread of both CTAs gets here after
   // bounded waits).
+  pdl_trigger();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::cluster_sync();
@@ -733,9 +738,11 @@ int launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams&
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, kSmem)) return rc;
   cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.blockDim = dim3(kTcThreads); cfg.dynamicSmemBytes = kSmem; cfg.stream = st;
   cfg.attrs = attr; cfg.numAttrs = 1;
   static std::atomic<int> resident[kMaxDevices];
@@ -752,6 +759,7 @@ int launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams&
   if (pairs < 0) return B200MOE_E_UNSUPPORTED;   // the caller takes the single-CTA kernel
   if (pairs > max_pairs) pairs = max_pairs;
   cfg.gridDim = dim3(2 * pairs);
+  cfg.numAttrs = p.m <= kEarlyLaunchRows ? 2 : 1;
   B200_CUDA_OK(cudaLaunchKernelEx(&cfg, kern, ta, tw, p));
   return B200MOE_OK;
 }

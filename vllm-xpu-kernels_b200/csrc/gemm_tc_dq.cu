@@ -191,6 +191,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
+    pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
@@ -214,6 +215,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
+  pdl_wait();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -436,6 +438,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   }
 
+  pdl_trigger();
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -457,8 +460,7 @@ int launch_dq(const CUtensorMap& ta, const CUtensorMap& tw, DqParams& p, int gri
   const size_t smem = (size_t)fixed + (size_t)p.stages * p.stage_bytes;
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, smem)) return rc;
-  kern<<<grid, kDqThreads, smem, st>>>(ta, tw, p);
-  B200_LAUNCH_OK("grouped_gemm_dq_kernel");
+  B200_LAUNCHED("grouped_gemm_dq_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kDqThreads), smem, st, ta, tw, p));
   return B200MOE_OK;
 }
 

@@ -89,6 +89,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
+    pdl_wait();
     build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
@@ -109,6 +110,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
+  pdl_wait();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -274,6 +276,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
   }
 
   // Teardown: everyone meets here, also after an aborted wait.
+  pdl_trigger();
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -350,6 +353,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int up_block0 = p.n_tiles / 2;        // gated: first 128-feature block of the up half
 
   if (warp == 0) {
+    pdl_wait();
     build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, n_tiles2, ctrl->walk);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
@@ -371,6 +375,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
+  pdl_wait();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -672,6 +677,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
     }
   }
 
+  pdl_trigger();
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -688,8 +694,7 @@ int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, const TParams& 
   static SmemConfig configured;
   const size_t smem = p.stages == kT2Stages ? kT2Smem : kT2SmemStaged;
   if (int rc = configured.ensure(kern, kT2SmemStaged > kT2Smem ? kT2SmemStaged : kT2Smem)) return rc;
-  kern<<<grid, kT2Threads, smem, st>>>(ta, tw, p);
-  B200_LAUNCH_OK("grouped_gemm_fp8t256_kernel");
+  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), smem, st, ta, tw, p));
   return B200MOE_OK;
 }
 
@@ -698,8 +703,7 @@ int launch_fp8t(const CUtensorMap& ta, const CUtensorMap& tw, const TParams& p, 
   auto kern = grouped_gemm_fp8t_kernel<kWKn>;
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, kTSmem)) return rc;
-  kern<<<grid, kTThreads, kTSmem, st>>>(ta, tw, p);
-  B200_LAUNCH_OK("grouped_gemm_fp8t_kernel");
+  B200_LAUNCHED("grouped_gemm_fp8t_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kTThreads), kTSmem, st, ta, tw, p));
   return B200MOE_OK;
 }
 

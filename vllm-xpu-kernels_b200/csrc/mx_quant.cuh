@@ -1,0 +1,44 @@
+// MXFP8 activation quantisation shared by the quantiser and the permutation: per 32 consecutive
+// values one power-of-two scale 2^(b-127) (stored as the e8m0 byte b, the smallest power of two
+// with amax / scale <= 448, at least 2^-33) and e4m3 codes of x / scale.
+#pragma once
+
+#include "common.cuh"
+
+namespace b200moe {
+namespace {
+
+// A lane holds 8 values, four lanes one group of 32, sixteen lanes (aligned in the warp) one
+// 128-wide block; all lanes of the warp call it.  Writes the codes, leaves the residual
+// v - code * scale in v (what a second plane quantises) and returns the block's scale word: byte g
+// of it is group g's scale, 0x7f (2^0) for groups whose lanes are not `active`.
+//
+// amax / 448 <= 2^e is amax <= 1.75 * 2^(e + 8), a comparison of exponent and mantissa; scale and
+// inverse are then exact powers of two (the divisions this replaces gave the same bits).
+__device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes) {
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  const uint32_t bits = __float_as_uint(amax);
+  int e = (int)(bits >> 23) - 8 + ((bits & 0x007fffffu) > 0x00600000u ? 1 : 0);   // biased exponent of the scale
+  e = e < 94 ? 94 : e;
+  if (bits >= 0x7f800000u) e = 255;   // an infinity in the group: the scale byte is NaN
+  const float sc = __uint_as_float((uint32_t)e << 23), inv = e == 255 ? 0.f : __uint_as_float((uint32_t)(254 - e) << 23);
+  uint32_t c[2] = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const uint32_t o = f32_to_e4m3(fminf(fmaxf(__fmul_rn(v[i], inv), -448.f), 448.f));
+    c[i >> 2] |= o << (8 * (i & 3));
+    v[i] = __fsub_rn(v[i], __fmul_rn(e4m3_to_f32((uint8_t)o), sc));
+  }
+  codes = make_uint2(c[0], c[1]);
+  const uint32_t byte = (active ? (uint32_t)e : 0x7fu) << (8 * ((threadIdx.x >> 2) & 3));
+  uint32_t word = byte | __shfl_xor_sync(0xffffffffu, byte, 4);
+  word |= __shfl_xor_sync(0xffffffffu, word, 8);
+  return word;
+}
+
+}  // namespace
+}  // namespace b200moe

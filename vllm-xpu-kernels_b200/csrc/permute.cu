@@ -20,65 +20,70 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "mx_quant.cuh"
 #include "sort.cuh"
 
 namespace b200moe {
 namespace {
 
-// ------------------------- row copy ------------------------------------------
-// One block per token: the row is read once and written to its K destinations.
-__global__ void __launch_bounds__(256)
-remap_copy_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                  const uint8_t* __restrict__ src_s, uint8_t* __restrict__ dst_s,
-                  const int32_t* __restrict__ row_map, int row_bytes,
-                  int scale_row_bytes, int K) {
-  const int64_t tok = blockIdx.x;
-  __shared__ int dest[32];
-  if (threadIdx.x < K) dest[threadIdx.x] = row_map[tok * K + threadIdx.x];
-  __syncthreads();
-  const uint8_t* s = src + tok * (int64_t)row_bytes;
-  const int nvec = row_bytes >> 4;
+// ------------------------- row copies ------------------------------------------
+// One block per token: its row is read once and written to its K destinations (`dest` in shared
+// memory, negative = none), as it is, quantised to e4m3 per 1x128 group, or as MXFP8 planes.
+struct RowJob {
+  const void* src;
+  void* dst;
+  const void* src_s;     // copy: the caller's scale rows, or null
+  void* dst_s;           // copy: their destination; fp8: fp32 [rows, H/128]; mx: words [planes][ceil(H/128)][rows]
+  int row_bytes;         // copy
+  int scale_row_bytes;   // copy
+  int H;                 // quantised forms: values per row
+  int K;
+  int64_t rows;          // mx: rows of a plane (T * K)
+  int planes;            // mx: 1 or 2
+};
+
+__device__ __forceinline__ void copy_row(const RowJob& a, int64_t tok, const int* dest) {
+  const uint8_t* s = reinterpret_cast<const uint8_t*>(a.src) + tok * (int64_t)a.row_bytes;
+  uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst);
+  const int nvec = a.row_bytes >> 4;
   for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
     const vec16 v = ld16(s + (int64_t)j * 16);
-    for (int k = 0; k < K; ++k) {
+    for (int k = 0; k < a.K; ++k) {
       const int r = dest[k];
-      if (r >= 0) st16(dst + (int64_t)r * row_bytes + (int64_t)j * 16, v);
+      if (r >= 0) st16(dst + (int64_t)r * a.row_bytes + (int64_t)j * 16, v);
     }
   }
-  if (src_s != nullptr) {
-    const uint8_t* ss = src_s + tok * (int64_t)scale_row_bytes;
-    if ((scale_row_bytes & 3) == 0) {
-      for (int j = threadIdx.x; j < (scale_row_bytes >> 2); j += blockDim.x) {
+  if (a.src_s != nullptr) {
+    const uint8_t* ss = reinterpret_cast<const uint8_t*>(a.src_s) + tok * (int64_t)a.scale_row_bytes;
+    uint8_t* dst_s = reinterpret_cast<uint8_t*>(a.dst_s);
+    if ((a.scale_row_bytes & 3) == 0) {
+      for (int j = threadIdx.x; j < (a.scale_row_bytes >> 2); j += blockDim.x) {
         const uint32_t v = reinterpret_cast<const uint32_t*>(ss)[j];
-        for (int k = 0; k < K; ++k) {
+        for (int k = 0; k < a.K; ++k) {
           const int r = dest[k];
-          if (r >= 0) reinterpret_cast<uint32_t*>(dst_s + (int64_t)r * scale_row_bytes)[j] = v;
+          if (r >= 0) reinterpret_cast<uint32_t*>(dst_s + (int64_t)r * a.scale_row_bytes)[j] = v;
         }
       }
     } else {
-      for (int j = threadIdx.x; j < scale_row_bytes; j += blockDim.x) {
+      for (int j = threadIdx.x; j < a.scale_row_bytes; j += blockDim.x) {
         const uint8_t v = ss[j];
-        for (int k = 0; k < K; ++k) {
+        for (int k = 0; k < a.K; ++k) {
           const int r = dest[k];
-          if (r >= 0) dst_s[(int64_t)r * scale_row_bytes + j] = v;
+          if (r >= 0) dst_s[(int64_t)r * a.scale_row_bytes + j] = v;
         }
       }
     }
   }
 }
 
-// Row copy fused with the per-1x128 dynamic e4m3 quantisation.  A lane holds 8
-// consecutive elements, 16 lanes cover one 128-wide group.
+// Per-1x128 dynamic e4m3 quantisation.  A lane holds 8 consecutive elements, 16 lanes
+// cover one 128-wide group.
 template <typename T>
-__global__ void __launch_bounds__(256)
-remap_quant_kernel(const T* __restrict__ src, uint8_t* __restrict__ dst_q,
-                   float* __restrict__ dst_s, const int32_t* __restrict__ row_map,
-                   int H, int K) {
-  const int64_t tok = blockIdx.x;
-  __shared__ int dest[32];
-  if (threadIdx.x < K) dest[threadIdx.x] = row_map[tok * K + threadIdx.x];
-  __syncthreads();
-  const T* s = src + tok * (int64_t)H;
+__device__ __forceinline__ void quant_row_fp8(const RowJob& a, int64_t tok, const int* dest) {
+  const int H = a.H;
+  const T* s = reinterpret_cast<const T*>(a.src) + tok * (int64_t)H;
+  uint8_t* dst_q = reinterpret_cast<uint8_t*>(a.dst);
+  float* dst_s = reinterpret_cast<float*>(a.dst_s);
   const int groups = H / 128;
   const int nvec = H / 8;
   // Full warps iterate together so the 16-lane shuffles stay converged.
@@ -114,7 +119,7 @@ remap_quant_kernel(const T* __restrict__ src, uint8_t* __restrict__ dst_q,
         hi |= (uint32_t)f32_to_e4m3(q) << (8 * i);
       }
       const int g = j / 16;
-      for (int k = 0; k < K; ++k) {
+      for (int k = 0; k < a.K; ++k) {
         const int r = dest[k];
         if (r >= 0) {
           *reinterpret_cast<uint2*>(dst_q + (int64_t)r * H + (int64_t)j * 8) = make_uint2(lo, hi);
@@ -125,7 +130,125 @@ remap_quant_kernel(const T* __restrict__ src, uint8_t* __restrict__ dst_q,
   }
 }
 
+// MXFP8 planes (mx_quant.cuh); sixteen lanes cover a 128-wide K block, whose first lane writes its
+// scale word.
+template <typename T>
+__device__ __forceinline__ void quant_row_mx(const RowJob& a, int64_t tok, const int* dest) {
+  const int H = a.H;
+  const T* s = reinterpret_cast<const T*>(a.src) + tok * (int64_t)H;
+  uint8_t* dst_q = reinterpret_cast<uint8_t*>(a.dst);
+  uint32_t* dst_s = reinterpret_cast<uint32_t*>(a.dst_s);
+  const int nvec = H / 8, num_kb = (H + 127) / 128;
+  for (int j0 = (threadIdx.x & ~31); j0 < num_kb * 16; j0 += blockDim.x) {
+    const int j = j0 + (threadIdx.x & 31);
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0.f;
+    if (j < nvec) {
+      const vec16 in = ld16(s + (int64_t)j * 8);
+      const T* e = reinterpret_cast<const T*>(&in);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = to_f32<T>(e[i]);
+    }
+    for (int p = 0; p < a.planes; ++p) {
+      uint2 codes;
+      const uint32_t word = mx_quant_lane(v, j < nvec, codes);
+      for (int k = 0; k < a.K; ++k) {
+        const int r = dest[k];
+        if (r >= 0) {
+          if (j < nvec) *reinterpret_cast<uint2*>(dst_q + (p * a.rows + r) * H + (int64_t)j * 8) = codes;
+          if ((j & 15) == 0 && j < num_kb * 16) dst_s[((int64_t)p * num_kb + (j >> 4)) * a.rows + r] = word;
+        }
+      }
+    }
+  }
+}
+
+enum RowForm { kRowCopy = 0, kRowFp8 = 1, kRowMx = 2 };
+template <typename T, int kForm>
+__device__ __forceinline__ void place_row(const RowJob& a, int64_t tok, const int* dest) {
+  if (kForm == kRowCopy) copy_row(a, tok, dest);
+  else if (kForm == kRowFp8) quant_row_fp8<T>(a, tok, dest);
+  else quant_row_mx<T>(a, tok, dest);
+}
+
+template <typename T, int kForm>
+__global__ void __launch_bounds__(256)
+remap_rows_kernel(const RowJob a, const int32_t* __restrict__ row_map) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ int dest[32];
+  const int64_t tok = blockIdx.x;
+  if (threadIdx.x < a.K) dest[threadIdx.x] = row_map[tok * a.K + threadIdx.x];
+  __syncthreads();
+  place_row<T, kForm>(a, tok, dest);
+}
+
+// Up to kBlockSlots routed slots: the bookkeeping and the rows in one launch.  A block finds its
+// token's positions by itself: the position of slot i is the number of slots with a smaller bucket
+// plus the number of earlier slots with the same one, counted over all slots by the block's threads
+// (2048 slots x 8 are 64 comparisons a thread).  One more block counts the rows per expert.  The
+// separate sort, a single block that everything waited for, took 6 to 10 us of a decode step and
+// its launch; this form takes 3 us.  K up to kSmallK, else the sort.
+constexpr int kSmallK = 8;
+template <typename T, int kForm>
+__global__ void __launch_bounds__(256)
+remap_small_kernel(const SortParams p, const RowJob a, int32_t* __restrict__ rows_per_expert,
+                   int32_t* __restrict__ row_map) {
+  __shared__ int dest[32];
+  __shared__ uint32_t part[8][kSmallK / 2];
+  __shared__ int hist[kMaxBuckets];
+  pdl_trigger();
+  pdl_wait();
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int numel = (int)p.numel, K = a.K;
+  if (blockIdx.x == gridDim.x - 1) {
+    for (int e = t; e < p.n_buckets; e += 256) hist[e] = 0;
+    __syncthreads();
+    for (int i = t; i < numel; i += 256) {
+      const int b = bucket_of(p, i);
+      if (b >= 0) atomicAdd(&hist[b], 1);
+    }
+    __syncthreads();
+    for (int e = t; e < p.n_buckets; e += 256) rows_per_expert[e] = hist[e];
+    return;
+  }
+  const int64_t tok = blockIdx.x;
+  const int slot0 = (int)tok * K;
+  int own[kSmallK];
+#pragma unroll
+  for (int k = 0; k < kSmallK; ++k) own[k] = k < K ? bucket_of(p, slot0 + k) : -1;
+  uint32_t cnt[kSmallK / 2];   // two 16-bit counters a word
+#pragma unroll
+  for (int k = 0; k < kSmallK / 2; ++k) cnt[k] = 0;
+  for (int i = t; i < numel; i += 256) {
+    const int b = bucket_of(p, i);
+    if (b < 0) continue;
+#pragma unroll
+    for (int k = 0; k < kSmallK; ++k)
+      if (b < own[k] || (b == own[k] && i < slot0 + k)) cnt[k >> 1] += 1u << (16 * (k & 1));
+  }
+#pragma unroll
+  for (int k = 0; k < kSmallK / 2; ++k) {
+    cnt[k] = __reduce_add_sync(0xffffffffu, cnt[k]);
+    if (lane == 0) part[warp][k] = cnt[k];
+  }
+  __syncthreads();
+  if (t < K) {
+    uint32_t sum = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) sum += part[w][t >> 1];
+    const int pos = bucket_of(p, slot0 + t) < 0 ? -1 : (int)((sum >> (16 * (t & 1))) & 0xffffu);
+    dest[t] = pos;
+    row_map[slot0 + t] = pos;
+  }
+  __syncthreads();
+  place_row<T, kForm>(a, tok, dest);
+}
+
 __global__ void init_expert_map_kernel(int32_t* map, int n_local, int ep_rank, int total) {
+  pdl_trigger();
+  pdl_wait();
   const int g = blockIdx.x * blockDim.x + threadIdx.x;
   if (g < total) {
     const int lo = ep_rank * n_local;
@@ -138,24 +261,40 @@ int check_ids_dtype(b200moe_dtype t, const char* name) {
   return fail(B200MOE_E_BADARG, "%s: topk_ids must be int64 or int32", name);
 }
 
-int remap_bookkeeping(const int32_t* expert_map, int32_t* rows_per_expert,
-                      int32_t* row_map, const void* topk_ids, b200moe_dtype ids_dtype,
-                      int64_t num_rows, int topk, int total_experts, int local_experts,
-                      void* workspace, size_t workspace_bytes, cudaStream_t st) {
+int remap_params(SortParams& p, const int32_t* expert_map, const int32_t* rows_per_expert, const int32_t* row_map,
+                 const void* topk_ids, b200moe_dtype ids_dtype, int64_t num_rows, int topk, int total_experts,
+                 int local_experts) {
   if (check_ids_dtype(ids_dtype, "remap_hidden_states")) return B200MOE_E_BADARG;
   B200_CHECK_ARG(topk >= 1 && topk <= 32, "Unsupported TopK value");
   B200_CHECK_ARG(local_experts >= 1 && local_experts <= kMaxBuckets,
                  "local_experts_num exceeds the maximum supported number");
   B200_CHECK_ARG(rows_per_expert && row_map && topk_ids, "remap_hidden_states: null pointer");
-  SortParams p;
   p.ids = topk_ids; p.ids_dtype = ids_dtype; p.map = expert_map;
   p.numel = num_rows * topk;
   p.id_limit = expert_map ? total_experts : local_experts;
   p.n_buckets = local_experts;
   p.block_size = 1;
+  return B200MOE_OK;
+}
+
+// Bookkeeping and rows: one launch where the slots fit one block's count, else the sort and a
+// kernel that places the rows.
+template <typename T, int kForm>
+int remap_rows(const SortParams& p, const RowJob& job, int32_t* rows_per_expert, int32_t* row_map, int64_t num_rows,
+               void* workspace, size_t workspace_bytes, cudaStream_t st) {
+  const bool early = p.numel <= kEarlyLaunchRows;
+  if (p.numel > 0 && p.numel <= kBlockSlots && job.K <= kSmallK) {
+    B200_LAUNCHED("remap_small_kernel", launch_pdl(early, remap_small_kernel<T, kForm>, dim3((unsigned)num_rows + 1),
+                                                   dim3(256), 0, st, p, job, rows_per_expert, row_map));
+    return B200MOE_OK;
+  }
   AlignOut ao = {};
   RemapOut ro = {rows_per_expert, row_map};
-  return run_sort<1>(p, ao, ro, workspace, workspace_bytes, st);
+  if (int rc = run_sort<1>(p, ao, ro, workspace, workspace_bytes, st)) return rc;
+  if (num_rows == 0) return B200MOE_OK;
+  B200_LAUNCHED("remap_rows_kernel", launch_pdl(early, remap_rows_kernel<T, kForm>, dim3((unsigned)num_rows),
+                                                dim3(256), 0, st, job, row_map));
+  return B200MOE_OK;
 }
 
 }  // namespace
@@ -235,6 +374,8 @@ __device__ __forceinline__ void copy_bytes(unsigned char* dst, const unsigned ch
 // index maps.  Block 0 first turns the per-expert counts into the int64 offsets.
 __global__ void __launch_bounds__(kBlockThreads)
 prologue_expand_kernel(PrologueArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int scan[kMaxBuckets + 1];
   __shared__ int warp_tot[kWarps];
   if (blockIdx.x == 0) {
@@ -366,8 +507,8 @@ extern "C" int b200moe_fused_moe_prologue(
   a.num_tokens = num_rows; a.topk = topk; a.experts = num_experts_on_rank;
   const int64_t want = (int64_t)n < 1 ? 1 : (int64_t)n;
   const int grid = (int)(want < 148 * 8 ? want : 148 * 8);
-  prologue_expand_kernel<<<grid, kBlockThreads, 0, st>>>(a);
-  B200_LAUNCH_OK("prologue_expand_kernel");
+  B200_LAUNCHED("prologue_expand_kernel", launch_pdl(n <= kEarlyLaunchRows, prologue_expand_kernel, dim3(grid), dim3(kBlockThreads), 0, st,
+      a));
   return B200MOE_OK;
 }
 
@@ -397,8 +538,9 @@ extern "C" int b200moe_moe_lora_align_block_size(
                      sorted_token_ids, expert_ids, num_tokens_post_pad};
   const size_t smem = (size_t)(kWarps * num_experts + num_experts + 1 + kWarps) * sizeof(int);
   // lora_ids has max_loras + 1 entries: every adapter slot plus a possible -1
-  lora_align_kernel<<<max_loras + 1, kBlockThreads, smem, as_stream(stream)>>>(p, a);
-  B200_LAUNCH_OK("lora_align_kernel");
+  B200_LAUNCHED("lora_align_kernel", launch_pdl(true, lora_align_kernel,
+      dim3(max_loras + 1), dim3(kBlockThreads), smem, as_stream(stream),
+      p, a));
   return B200MOE_OK;
 }
 
@@ -411,6 +553,8 @@ __global__ void __launch_bounds__(1024)
 batched_align_kernel(const int32_t* __restrict__ counts, int B, int max_tokens, int block,
                      int32_t* __restrict__ sorted_ids, int32_t* __restrict__ block_ids,
                      int32_t* __restrict__ num_post_pad) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int warp_sums[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int blocks_per_batch = (max_tokens + block - 1) / block;
@@ -455,9 +599,8 @@ extern "C" int b200moe_batched_moe_align_block_size(int max_tokens_per_batch, in
   B200_CHECK_ARG(block_size >= 1 && max_tokens_per_batch >= 0, "batched_moe_align_block_size: bad sizes");
   B200_CHECK_ARG(batch_num_tokens && sorted_ids && batch_ids && num_tokens_post_pad,
                  "batched_moe_align_block_size: null pointer");
-  batched_align_kernel<<<1, 1024, 0, as_stream(stream)>>>(batch_num_tokens, num_batches, max_tokens_per_batch,
-                                                          block_size, sorted_ids, batch_ids, num_tokens_post_pad);
-  B200_LAUNCH_OK("batched_align_kernel");
+  B200_LAUNCHED("batched_align_kernel", launch_pdl(true, batched_align_kernel, dim3(1), dim3(1024), 0, as_stream(stream),
+      batch_num_tokens, num_batches, max_tokens_per_batch, block_size, sorted_ids, batch_ids, num_tokens_post_pad));
   return B200MOE_OK;
 }
 
@@ -467,9 +610,9 @@ extern "C" int b200moe_init_expert_map(int32_t* expert_map, int num_local_expert
   B200_CHECK_ARG(num_local_experts >= 1 && ep_size >= 1 && ep_rank >= 0 && ep_rank < ep_size,
                  "init_expert_map: bad ep_rank/ep_size");
   const int total = num_local_experts * ep_size;
-  init_expert_map_kernel<<<(total + 255) / 256, 256, 0, as_stream(stream)>>>(
-      expert_map, num_local_experts, ep_rank, total);
-  B200_LAUNCH_OK("init_expert_map_kernel");
+  B200_LAUNCHED("init_expert_map_kernel", launch_pdl(true, init_expert_map_kernel,
+      dim3((total + 255) / 256), dim3(256), 0, as_stream(stream),
+      expert_map, num_local_experts, ep_rank, total));
   return B200MOE_OK;
 }
 
@@ -487,20 +630,17 @@ extern "C" int b200moe_remap_hidden_states(
   B200_CHECK_ARG(((int64_t)hidden_size * elem_bytes) % 16 == 0,
                  "hidden_size must be divisible by ElemsPerItem");
   B200_CHECK_ARG(num_rows >= 0, "remap_hidden_states: negative num_rows");
-  cudaStream_t st = as_stream(stream);
-  int rc = remap_bookkeeping(expert_map, rows_per_expert, row_map, topk_ids, ids_dtype,
-                             num_rows, topk, total_experts, local_experts, workspace,
-                             workspace_bytes, st);
-  if (rc != B200MOE_OK || num_rows == 0) return rc;
-  B200_CHECK_ARG(hidden && remapped, "remap_hidden_states: null pointer");
+  SortParams p;
+  if (int rc = remap_params(p, expert_map, rows_per_expert, row_map, topk_ids, ids_dtype, num_rows, topk,
+                            total_experts, local_experts)) return rc;
+  B200_CHECK_ARG(num_rows == 0 || (hidden && remapped), "remap_hidden_states: null pointer");
   B200_CHECK_ARG(((uintptr_t)hidden & 15) == 0 && ((uintptr_t)remapped & 15) == 0,
                  "remap_hidden_states: buffers must be 16-byte aligned");
-  remap_copy_kernel<<<(unsigned)num_rows, 256, 0, st>>>(
-      (const uint8_t*)hidden, (uint8_t*)remapped, (const uint8_t*)scales,
-      (uint8_t*)remapped_scales, row_map, hidden_size * elem_bytes,
-      scale_cols * scale_elem_bytes, topk);
-  B200_LAUNCH_OK("remap_copy_kernel");
-  return B200MOE_OK;
+  RowJob job = {};
+  job.src = hidden; job.dst = remapped; job.src_s = scales; job.dst_s = remapped_scales;
+  job.row_bytes = hidden_size * elem_bytes; job.scale_row_bytes = scale_cols * scale_elem_bytes; job.K = topk;
+  return remap_rows<uint8_t, kRowCopy>(p, job, rows_per_expert, row_map, num_rows, workspace, workspace_bytes,
+                                       as_stream(stream));
 }
 
 extern "C" int b200moe_remap_quant_fp8(
@@ -512,24 +652,39 @@ extern "C" int b200moe_remap_quant_fp8(
   B200_CHECK_ARG(dtype == B200MOE_BF16 || dtype == B200MOE_F16,
                  "remap_quant_fp8: activations must be bfloat16 or float16");
   B200_CHECK_ARG(hidden_size % 128 == 0, "remap_quant_fp8: hidden_size must be a multiple of 128");
-  cudaStream_t st = as_stream(stream);
-  int rc = remap_bookkeeping(expert_map, rows_per_expert, row_map, topk_ids, ids_dtype,
-                             num_rows, topk, total_experts, local_experts, workspace,
-                             workspace_bytes, st);
-  if (rc != B200MOE_OK || num_rows == 0) return rc;
-  B200_CHECK_ARG(hidden && remapped_q && remapped_scales, "remap_quant_fp8: null pointer");
+  SortParams p;
+  if (int rc = remap_params(p, expert_map, rows_per_expert, row_map, topk_ids, ids_dtype, num_rows, topk,
+                            total_experts, local_experts)) return rc;
+  B200_CHECK_ARG(num_rows == 0 || (hidden && remapped_q && remapped_scales), "remap_quant_fp8: null pointer");
   B200_CHECK_ARG(((uintptr_t)hidden & 15) == 0 && ((uintptr_t)remapped_q & 7) == 0,
                  "remap_quant_fp8: buffers must be 16-byte aligned");
-  if (dtype == B200MOE_BF16)
-    remap_quant_kernel<__nv_bfloat16><<<(unsigned)num_rows, 256, 0, st>>>(
-        (const __nv_bfloat16*)hidden, (uint8_t*)remapped_q, remapped_scales, row_map,
-        hidden_size, topk);
-  else
-    remap_quant_kernel<__half><<<(unsigned)num_rows, 256, 0, st>>>(
-        (const __half*)hidden, (uint8_t*)remapped_q, remapped_scales, row_map, hidden_size,
-        topk);
-  B200_LAUNCH_OK("remap_quant_kernel");
-  return B200MOE_OK;
+  RowJob job = {};
+  job.src = hidden; job.dst = remapped_q; job.dst_s = remapped_scales; job.H = hidden_size; job.K = topk;
+  auto run = dtype == B200MOE_BF16 ? remap_rows<__nv_bfloat16, kRowFp8> : remap_rows<__half, kRowFp8>;
+  return run(p, job, rows_per_expert, row_map, num_rows, workspace, workspace_bytes, as_stream(stream));
+}
+
+extern "C" int b200moe_remap_quant_mxfp8(
+    const void* hidden, b200moe_dtype dtype, void* remapped_q, void* remapped_scales, int planes,
+    const int32_t* expert_map, int32_t* rows_per_expert, int32_t* row_map,
+    const void* topk_ids, b200moe_dtype ids_dtype, int64_t num_rows, int hidden_size,
+    int topk, int total_experts, int local_experts, void* workspace,
+    size_t workspace_bytes, b200moe_stream stream) {
+  B200_CHECK_ARG(dtype == B200MOE_BF16 || dtype == B200MOE_F16,
+                 "remap_quant_mxfp8: activations must be bfloat16 or float16");
+  B200_CHECK_ARG(hidden_size % 32 == 0, "remap_quant_mxfp8: hidden_size must be a multiple of 32");
+  B200_CHECK_ARG(planes == 1 || planes == 2, "remap_quant_mxfp8: one or two planes");
+  SortParams p;
+  if (int rc = remap_params(p, expert_map, rows_per_expert, row_map, topk_ids, ids_dtype, num_rows, topk,
+                            total_experts, local_experts)) return rc;
+  B200_CHECK_ARG(num_rows == 0 || (hidden && remapped_q && remapped_scales), "remap_quant_mxfp8: null pointer");
+  B200_CHECK_ARG(((uintptr_t)hidden & 15) == 0 && ((uintptr_t)remapped_q & 7) == 0,
+                 "remap_quant_mxfp8: buffers must be 16-byte aligned");
+  RowJob job = {};
+  job.src = hidden; job.dst = remapped_q; job.dst_s = remapped_scales; job.H = hidden_size; job.K = topk;
+  job.rows = num_rows * topk; job.planes = planes;
+  auto run = dtype == B200MOE_BF16 ? remap_rows<__nv_bfloat16, kRowMx> : remap_rows<__half, kRowMx>;
+  return run(p, job, rows_per_expert, row_map, num_rows, workspace, workspace_bytes, as_stream(stream));
 }
 
 // ---------------------------------------------------------------------------

@@ -37,6 +37,8 @@ topk_gating_kernel(const T* __restrict__ gating, float* __restrict__ out_w,
                    void* __restrict__ out_idx, b200moe_dtype idx_dtype,
                    int32_t* __restrict__ out_src, const float* __restrict__ bias,
                    int64_t num_rows, int E, int K, bool renorm, float rsf) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int kRowsPerWarp = 32 / R;
   const int lane = threadIdx.x & 31;
   const int warp = threadIdx.x >> 5;
@@ -150,9 +152,9 @@ int launch_gating(const T* gating, float* w, void* idx, b200moe_dtype idx_dtype,
   {                                                                             \
     constexpr int rows_per_block = kWarpsPerBlock * (32 / R_);                  \
     const unsigned grid = (unsigned)((T_ + rows_per_block - 1) / rows_per_block); \
-    topk_gating_kernel<T, R_, VPT_, kMode>                                      \
-        <<<grid, kWarpsPerBlock * 32, 0, st>>>(gating, w, idx, idx_dtype, src,  \
-                                               bias, T_, E, K, renorm, rsf);    \
+    B200_LAUNCHED("topk_gating_kernel", launch_pdl(T_ * K <= kEarlyLaunchRows, topk_gating_kernel<T, R_, VPT_, kMode>, \
+        dim3(grid), dim3(kWarpsPerBlock * 32), 0, st, \
+        gating, w, idx, idx_dtype, src, bias, T_, E, K, renorm, rsf));    \
   }
   if (E <= 1) B200_GATING_CASE(1, 1)
   else if (E <= 2) B200_GATING_CASE(2, 1)
@@ -166,7 +168,6 @@ int launch_gating(const T* gating, float* w, void* idx, b200moe_dtype idx_dtype,
   else if (E <= 512) B200_GATING_CASE(32, 16)
   else B200_GATING_CASE(32, 32)
 #undef B200_GATING_CASE
-  B200_LAUNCH_OK("topk_gating_kernel");
   return B200MOE_OK;
 }
 
@@ -216,6 +217,8 @@ grouped_topk_kernel(const T* __restrict__ scores, const T* __restrict__ swb,
                     T* __restrict__ out_val, int32_t* __restrict__ out_idx,
                     int64_t num_tokens, int E, int n_group, int topk_group, int K,
                     bool renorm, double rsf) {
+  pdl_trigger();
+  pdl_wait();
   const int lane = threadIdx.x & 31;
   const int64_t tok = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   if (tok >= num_tokens) return;  // whole warp leaves together
@@ -406,10 +409,9 @@ extern "C" int b200moe_grouped_topk(void* topk_values, int32_t* topk_indices,
   cudaStream_t st = as_stream(stream);
   const unsigned grid = (unsigned)((num_tokens + kWarpsPerBlock - 1) / kWarpsPerBlock);
 #define B200_GT_CASE(VPT_)                                                     \
-  grouped_topk_kernel<scalar_t, VPT_><<<grid, kWarpsPerBlock * 32, 0, st>>>(   \
-      (const scalar_t*)scores, (const scalar_t*)scores_with_bias,              \
-      (scalar_t*)topk_values, topk_indices, num_tokens, num_experts, n_group,  \
-      topk_group, topk, renormalize != 0, routed_scaling_factor)
+  B200_LAUNCHED("grouped_topk_kernel", launch_pdl(num_tokens * topk <= kEarlyLaunchRows, grouped_topk_kernel<scalar_t, VPT_>, \
+      dim3(grid), dim3(kWarpsPerBlock * 32), 0, st, \
+      (const scalar_t*)scores, (const scalar_t*)scores_with_bias, (scalar_t*)topk_values, topk_indices, num_tokens, num_experts, n_group, topk_group, topk, renormalize != 0, routed_scaling_factor))
   switch (dtype) {
     case B200MOE_F32: case B200MOE_F16: case B200MOE_BF16: break;
     default:
@@ -425,7 +427,6 @@ extern "C" int b200moe_grouped_topk(void* topk_values, int32_t* topk_indices,
     else B200_GT_CASE(32);
   });
 #undef B200_GT_CASE
-  B200_LAUNCH_OK("grouped_topk_kernel");
   return B200MOE_OK;
 }
 
@@ -448,6 +449,8 @@ softplus_sqrt_hash_kernel(const T* __restrict__ gating, float* __restrict__ out_
                           int32_t* __restrict__ out_src, const void* __restrict__ input_ids,
                           const void* __restrict__ tid2eid, int64_t num_rows, int E, int K,
                           bool renorm, float rsf) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (row >= num_rows) return;
   const int64_t tok = load_index(input_ids, idx_dtype, row);
@@ -491,10 +494,10 @@ extern "C" int b200moe_topk_softplus_sqrt(float* topk_weights, void* topk_indice
   B200_CHECK_ARG(topk_weights && topk_indices && token_expert_indices && gating, "topk_softplus_sqrt: null pointer");
   const unsigned grid = (unsigned)((num_tokens + 127) / 128);
   B200_DISPATCH_FLOAT(gating_dtype, "topk_softplus_sqrt", {
-    b200moe::softplus_sqrt_hash_kernel<scalar_t><<<grid, 128, 0, b200moe::as_stream(stream)>>>(
+    B200_LAUNCHED("softplus_sqrt_hash_kernel", b200moe::launch_pdl(num_tokens * topk <= b200moe::kEarlyLaunchRows, b200moe::softplus_sqrt_hash_kernel<scalar_t>,
+        dim3(grid), dim3(128), 0, b200moe::as_stream(stream),
         (const scalar_t*)gating, topk_weights, topk_indices, index_dtype, token_expert_indices, input_ids,
-        tid2eid, num_tokens, num_experts, topk, renormalize != 0, (float)routed_scaling_factor);
+        tid2eid, num_tokens, num_experts, topk, renormalize != 0, (float)routed_scaling_factor));
   });
-  B200_LAUNCH_OK("softplus_sqrt_hash_kernel");
   return B200MOE_OK;
 }

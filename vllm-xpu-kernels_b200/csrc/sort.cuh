@@ -162,6 +162,8 @@ struct RemapOut {
 template <int kMode>
 __global__ void __launch_bounds__(kBlockThreads)
 sort_single_block_kernel(SortParams p, AlignOut ao, RemapOut ro) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ int smem[];
   int* hist = smem;                              // [kWarps][n_buckets]
   int* base = hist + kWarps * p.n_buckets;       // [n_buckets + 1]
@@ -251,6 +253,8 @@ struct LoraAlignArgs {
 
 __global__ void __launch_bounds__(kBlockThreads)
 lora_align_kernel(SortParams p, LoraAlignArgs a) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ int smem[];
   const int nb = p.n_buckets;
   int* hist = smem;                        // [kWarps][nb]
@@ -333,6 +337,8 @@ lora_align_kernel(SortParams p, LoraAlignArgs a) {
 __global__ void __launch_bounds__(kBlockThreads)
 sort_count_kernel(SortParams p, int n_chunks, int* counts, int32_t* fill,
                   int64_t fill_len) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ int smem[];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int nb = p.n_buckets;
@@ -363,6 +369,8 @@ template <int kMode>
 __global__ void __launch_bounds__(1024)
 sort_scan_kernel(SortParams p, int n_chunks, int* counts, int* base_out,
                  AlignOut ao, RemapOut ro) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ int base[kMaxBuckets + 1];
   __shared__ int sizes[kMaxBuckets];
   __shared__ int warp_tot[32];
@@ -426,6 +434,8 @@ template <int kMode>
 __global__ void __launch_bounds__(kBlockThreads)
 sort_rank_kernel(SortParams p, int n_chunks, const int* counts, const int* base,
                  AlignOut ao, RemapOut ro) {
+  pdl_trigger();
+  pdl_wait();
   extern __shared__ int smem[];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const int nb = p.n_buckets;
@@ -452,8 +462,9 @@ int run_sort(const SortParams& p, const AlignOut& ao, const RemapOut& ro,
   const int nb = p.n_buckets;
   if (p.numel <= kBlockSlots) {
     const size_t smem = (size_t)(kWarps * nb + nb + 1 + kWarps) * sizeof(int);
-    sort_single_block_kernel<kMode><<<1, kBlockThreads, smem, st>>>(p, ao, ro);
-    B200_LAUNCH_OK("sort_single_block_kernel");
+    B200_LAUNCHED("sort_single_block_kernel", launch_pdl(p.numel <= kEarlyLaunchRows, sort_single_block_kernel<kMode>,
+        dim3(1), dim3(kBlockThreads), smem, st,
+        p, ao, ro));
     return B200MOE_OK;
   }
   const size_t need = b200moe_sort_workspace_bytes(p.numel, nb);
@@ -465,13 +476,12 @@ int run_sort(const SortParams& p, const AlignOut& ao, const RemapOut& ro,
   int* counts = reinterpret_cast<int*>(workspace);
   int* base = counts + (size_t)nb * n_chunks;
   const size_t smem = (size_t)kWarps * nb * sizeof(int);
-  sort_count_kernel<<<n_blocks, kBlockThreads, smem, st>>>(
-      p, n_chunks, counts, kMode == 0 ? ao.sorted : nullptr, kMode == 0 ? ao.sorted_len : 0);
-  B200_LAUNCH_OK("sort_count_kernel");
-  sort_scan_kernel<kMode><<<1, 1024, 0, st>>>(p, n_chunks, counts, base, ao, ro);
-  B200_LAUNCH_OK("sort_scan_kernel");
-  sort_rank_kernel<kMode><<<n_blocks, kBlockThreads, smem, st>>>(p, n_chunks, counts, base, ao, ro);
-  B200_LAUNCH_OK("sort_rank_kernel");
+  B200_LAUNCHED("sort_count_kernel", launch_pdl(p.numel <= kEarlyLaunchRows, sort_count_kernel, dim3(n_blocks), dim3(kBlockThreads), smem, st,
+      p, n_chunks, counts, kMode == 0 ? ao.sorted : nullptr, kMode == 0 ? ao.sorted_len : 0));
+  B200_LAUNCHED("sort_scan_kernel", launch_pdl(p.numel <= kEarlyLaunchRows, sort_scan_kernel<kMode>, dim3(1), dim3(1024), 0, st,
+      p, n_chunks, counts, base, ao, ro));
+  B200_LAUNCHED("sort_rank_kernel", launch_pdl(p.numel <= kEarlyLaunchRows, sort_rank_kernel<kMode>, dim3(n_blocks), dim3(kBlockThreads), smem, st,
+      p, n_chunks, counts, base, ao, ro));
   return B200MOE_OK;
 }
 

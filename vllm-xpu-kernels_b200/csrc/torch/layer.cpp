@@ -1,0 +1,486 @@
+// The host side of one fused-MoE layer call in native code: permutation (+ quantisation), gemm1,
+// activation, gemm2 and the top-k reduction are launched from one function of the extension
+// module, with the intermediates carved out of one workspace.  The stages are the reference's
+// (vllm_xpu_kernels/fused_moe_interface.py:328-419 of vllm-xpu-kernels).
+//
+// A decode step is bound by the host as much as by the GPU: as seven torch ops with their Python
+// wrappers, argument checks and buffer look-ups, a call took 50 to 80 us of host time; here the
+// launches are what is left (about 2 us each).
+#include "layer.h"
+
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <map>
+#include <memory>
+#include <mutex>
+#include <utility>
+#include <vector>
+
+namespace b200shim {
+namespace {
+
+enum ActKind { kSilu = 0, kGelu, kGeluTanh, kSwigluOai, kRelu2NoMul, kSwigluStep };
+enum Form { kUnfused = 0, kEpilogue = 1, kFp8 = 2 };   // what gemm1 does besides multiplying
+
+struct Plan {
+  at::Tensor w13, w2;
+  std::optional<at::Tensor> s13, b13, s2, b2;
+  int64_t inter = 0, experts = 0, total_experts = 0;
+  int topk = 0, act = 0, inter_scale = 1, planes = 1;
+  bool block_fp8 = false, mx = false;
+  double clamp = 0.0;
+  // the weights as described for the last (hidden size, activation type): the checks run once
+  int64_t hidden = -1;
+  at::ScalarType act_dtype = at::kFloat;
+  WeightDesc d13{}, d2{};
+};
+const char* const kPlanName = "b200moe.layer_plan";
+
+// ------------------------------- workspace ------------------------------------
+// One grow-only buffer per (device, stream), shared by all layers: the calls of a stream run one
+// after the other, so the next one may overwrite what the previous one left.  At most kMaxSlabs
+// streams keep one (the least recently used is given back).  All are given back with the last layer
+// object, but for buffers that a CUDA graph has captured, which stay until workspace_clear().
+constexpr size_t kMaxSlabs = 8;
+struct Slab {
+  at::Tensor mem;
+  uint64_t used = 0;
+  bool captured = false;
+};
+std::mutex g_mutex;
+auto& g_slabs = *new std::map<std::pair<int, int64_t>, Slab>();   // (never destroyed: CUDA may be gone at exit)
+auto& g_captured = *new std::vector<at::Tensor>();
+uint64_t g_tick = 0;
+int64_t g_plans = 0;
+
+void clear_slabs(bool captured_too) {
+  std::lock_guard<std::mutex> lock(g_mutex);
+  for (auto it = g_slabs.begin(); it != g_slabs.end();)
+    it = (captured_too || !it->second.captured) ? g_slabs.erase(it) : std::next(it);
+  if (captured_too) g_captured.clear();
+}
+
+at::Tensor workspace(const c10::cuda::CUDAStream& stream, size_t bytes, bool persistent) {
+  const auto options = at::TensorOptions().dtype(at::kByte).device(stream.device());
+  if (!persistent) return at::empty({(int64_t)bytes}, options);
+  std::lock_guard<std::mutex> lock(g_mutex);
+  const std::pair<int, int64_t> key(stream.device_index(), (int64_t)stream.id());
+  Slab& slab = g_slabs[key];
+  if (!slab.mem.defined() || (size_t)slab.mem.numel() < bytes) {
+    if (slab.captured) g_captured.push_back(slab.mem);
+    slab.captured = false;
+    slab.mem = at::Tensor();
+    slab.mem = at::empty({(int64_t)((bytes + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1))}, options);
+    while (g_slabs.size() > kMaxSlabs) {
+      auto oldest = g_slabs.end();
+      for (auto it = g_slabs.begin(); it != g_slabs.end(); ++it)
+        if (it->first != key && (oldest == g_slabs.end() || it->second.used < oldest->second.used)) oldest = it;
+      if (oldest->second.captured) g_captured.push_back(oldest->second.mem);
+      g_slabs.erase(oldest);
+    }
+  }
+  if (!slab.captured && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+    slab.captured = true;
+  slab.used = ++g_tick;
+  return slab.mem;
+}
+
+// Offsets into a workspace whose size is known once everything has been laid out.
+struct Layout {
+  size_t end = 0;
+  size_t take(size_t bytes) {
+    const size_t at = end;
+    end += (bytes + 255) & ~(size_t)255;
+    return at;
+  }
+};
+
+b200moe_dtype dtype16(at::ScalarType t, const char* what) {
+  if (t == at::kBFloat16) return B200MOE_BF16;
+  if (t == at::kHalf) return B200MOE_F16;
+  TORCH_CHECK(false, what, " must be bfloat16 or float16");
+  return B200MOE_BF16;
+}
+
+void describe(Plan& p, int64_t hidden, at::ScalarType out_dtype) {
+  if (p.hidden == hidden && p.act_dtype == out_dtype) return;
+  const at::ScalarType a = (p.block_fp8 || p.mx) ? at::kFloat8_e4m3fn : out_dtype;
+  p.d13 = describe_weights(p.w13, p.s13, 2 * p.inter, hidden, p.experts, 0, a);
+  p.d2 = describe_weights(p.w2, p.s2, hidden, p.inter * p.inter_scale, p.experts, 0, a);
+  for (const auto* b : {&p.b13, &p.b2}) {
+    if (!b->has_value()) continue;
+    TORCH_CHECK((*b)->dim() == 2, "ptr_bias must be 2D [num_experts, N]");
+    TORCH_CHECK((*b)->is_contiguous(), "ptr_bias must be contiguous");
+    TORCH_CHECK((*b)->size(0) == p.experts, "ptr_bias.size(0) must match num_experts");
+    TORCH_CHECK((*b)->size(1) == (b == &p.b13 ? 2 * p.inter : hidden), "ptr_bias.size(1) must match N");
+    TORCH_CHECK((*b)->scalar_type() == out_dtype, "ptr_bias must have ptr_D's dtype");
+  }
+  p.hidden = hidden;
+  p.act_dtype = out_dtype;
+}
+
+// What a call brings along besides its tensors.
+struct CallOptions {
+  int form = kUnfused;
+  int64_t rows_hint = 0;
+  int max_ctas = 0;
+  PyObject* hook = nullptr;   // called with a stage's name after it has been launched
+};
+void mark(const CallOptions& o, const char* stage) {
+  if (o.hook == nullptr) return;
+  PyObject* r = PyObject_CallFunction(o.hook, "s", stage);
+  if (r == nullptr) throw python_error();
+  Py_DECREF(r);
+}
+
+// gemm1 (+ activation) and gemm2 on expert-major rows.
+struct Experts {
+  const Plan& p;
+  const CallOptions& o;
+  b200moe_dtype out;          // 16-bit type between the stages
+  at::ScalarType out_scalar;
+  int64_t M, hidden;
+  int segments;               // row segments (a multiple of the experts)
+  int device;
+  b200moe_stream stream;
+  bool a_fp8;                 // gemm1's rows are e4m3 with 1x128 scales
+  int64_t inter2() const { return p.inter * p.inter_scale; }
+  // offsets
+  size_t g1 = 0, act = 0, act_q = 0, act_s = 0;
+
+  void lay_out(Layout& l) {
+    if (o.form == kUnfused) g1 = l.take(M * 2 * p.inter * 2);
+  }
+  void lay_out_second(Layout& l) {
+    const int64_t I = p.inter, I2 = o.form == kUnfused ? inter2() : I;
+    const bool direct_fp8 = p.block_fp8 && (o.form == kFp8 || (p.act == kSilu && I % 128 == 0));
+    if (!direct_fp8) act = l.take(M * I2 * 2);
+    if (p.block_fp8) {
+      act_q = l.take(M * I2);
+      act_s = l.take(M * (I2 / 128) * 4);
+    } else if (p.mx) {
+      act_q = l.take((size_t)p.planes * M * I2);
+      act_s = l.take((size_t)p.planes * ((I2 + 127) / 128) * M * 4);
+    }
+  }
+
+  void gemm(bool first, const void* a, b200moe_dtype a_dtype, const void* a_scale, void* d, b200moe_dtype d_dtype,
+            void* d_scale, const int32_t* rows, b200moe_epilogue epi) const {
+    b200moe_gemm_args g = {};
+    const WeightDesc& w = first ? p.d13 : p.d2;
+    const at::Tensor& wt = first ? p.w13 : p.w2;
+    const auto& sc = first ? p.s13 : p.s2;
+    const auto& bias = first ? p.b13 : p.b2;
+    g.a = a; g.a_dtype = a_dtype; g.a_scale = a_scale;
+    g.w = wt.data_ptr(); g.w_format = w.format; g.group_size = w.group;
+    g.w_scale = sc.has_value() ? sc->data_ptr() : nullptr;
+    g.bias = bias.has_value() ? bias->data_ptr() : nullptr;
+    g.d = d; g.d_dtype = d_dtype; g.d_scale = (float*)d_scale; g.mid_dtype = out;
+    g.rows_per_expert = rows;
+    g.m = M; g.n = (int)(first ? 2 * p.inter : hidden); g.k = (int)(first ? hidden : inter2());
+    g.num_experts = segments;
+    g.w_experts = segments != p.experts ? (int)p.experts : 0;
+    g.epilogue = epi;
+    g.act_alpha = 1.702f; g.act_limit = 7.0f;
+    g.clamp_limit = epi != B200MOE_EPI_NONE && p.clamp > 0 ? (float)p.clamp : 0.f;
+    g.status = device_status_word(device);
+    g.max_ctas = o.max_ctas; g.rows_hint = o.rows_hint;
+    check_status(b200moe_grouped_gemm(&g, stream));
+  }
+
+  void run(uint8_t* ws, const void* a, const void* a_scale, const int32_t* rows, void* d) const {
+    const int64_t I = p.inter, I2 = inter2();
+    const b200moe_dtype mx_dtype = p.planes == 2 ? B200MOE_FP8_E4M3_X2 : B200MOE_FP8_E4M3;
+    const b200moe_dtype a_dtype = a_fp8 ? B200MOE_FP8_E4M3 : p.mx ? mx_dtype : out;
+    bool fp8_ready = false;
+    if (o.form == kFp8) {
+      gemm(true, a, a_dtype, a_scale, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, rows, B200MOE_EPI_SILU_MUL);
+      mark(o, "gemm1");
+      fp8_ready = true;
+    } else if (o.form == kEpilogue) {
+      gemm(true, a, a_dtype, a_scale, ws + act, out, nullptr, rows,
+           p.act == kSilu ? B200MOE_EPI_SILU_MUL : B200MOE_EPI_SWIGLUOAI);
+      mark(o, "gemm1");
+    } else {
+      gemm(true, a, a_dtype, a_scale, ws + g1, out, nullptr, rows, B200MOE_EPI_NONE);
+      mark(o, "gemm1");
+      if (p.clamp > 0) {
+        at::Tensor t = at::from_blob(ws + g1, {M, 2 * I},
+                                     at::TensorOptions().dtype(out_scalar).device(at::kCUDA, device));
+        t.narrow(1, 0, I).clamp_max_(p.clamp);
+        t.narrow(1, I, I).clamp_(-p.clamp, p.clamp);
+      }
+      if (p.block_fp8 && p.act == kSilu && I % 128 == 0) {
+        // SiLU, multiply and the 1x128 e4m3 quantisation of gemm2's input in one pass over the rows
+        // that the experts' segments use (the buffers may be sized for a worst case)
+        check_status(b200moe_silu_and_mul_per_block_quant_ragged(ws + act_q, (float*)(ws + act_s), ws + g1, out, M,
+                                                                 (int)I, rows, segments, stream));
+        fp8_ready = true;
+      } else {
+        void *to = ws + act, *from = ws + g1;
+        switch (p.act) {
+          case kSilu: check_status(b200moe_silu_and_mul(to, from, out, M, (int)I, stream)); break;
+          case kGelu: check_status(b200moe_gelu_and_mul(to, from, out, M, (int)I, stream)); break;
+          case kGeluTanh: check_status(b200moe_gelu_tanh_and_mul(to, from, out, M, (int)I, stream)); break;
+          case kSwigluOai:
+            check_status(b200moe_swigluoai_and_mul(to, from, out, M, (int)I, 1.702f, 7.0f, stream)); break;
+          case kRelu2NoMul: check_status(b200moe_relu2_no_mul(to, from, out, M, (int)I2, stream)); break;
+          default: check_status(b200moe_swiglustep_and_mul(to, from, out, M, (int)I, 7.0f, stream)); break;
+        }
+      }
+    }
+    mark(o, "activation");
+    if (p.block_fp8) {
+      if (!fp8_ready)
+        check_status(b200moe_per_token_group_fp8_quant(ws + act, out, ws + act_q, (float*)(ws + act_s), M, (int)I2, 128,
+                                                       1e-10f, 0, I2 / 128, 1, stream));
+      gemm(false, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, d, out, nullptr, rows, B200MOE_EPI_NONE);
+    } else if (p.mx) {
+      check_status(b200moe_quant_mxfp8(ws + act, out, ws + act_q, ws + act_s, M, (int)I2, p.planes, stream));
+      gemm(false, ws + act_q, mx_dtype, ws + act_s, d, out, nullptr, rows, B200MOE_EPI_NONE);
+    } else {
+      gemm(false, ws + act, out, nullptr, d, out, nullptr, rows, B200MOE_EPI_NONE);
+    }
+    mark(o, "gemm2");
+  }
+};
+
+const at::Tensor& tensor_arg(PyObject* o, const char* name) {
+  TORCH_CHECK_TYPE(THPVariable_Check(o), name, " must be a tensor");
+  return THPVariable_Unpack(o);
+}
+std::optional<at::Tensor> optional_arg(PyObject* o, const char* name) {
+  if (o == Py_None) return std::nullopt;
+  return tensor_arg(o, name);
+}
+int64_t int_arg(PyObject* o) {
+  const int64_t v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw python_error();
+  return v;
+}
+Plan* plan_arg(PyObject* o) {
+  Plan* p = (Plan*)PyCapsule_GetPointer(o, kPlanName);
+  if (p == nullptr) throw python_error();
+  return p;
+}
+void need_cuda(const at::Tensor& t, const char* name) {
+  TORCH_CHECK_NOT_IMPLEMENTED(t.is_cuda(), name, " must be a CUDA tensor: the layer has no CPU path");
+}
+
+void free_plan(PyObject* capsule) {
+  delete (Plan*)PyCapsule_GetPointer(capsule, kPlanName);
+  bool last;
+  { std::lock_guard<std::mutex> lock(g_mutex); last = --g_plans == 0; }
+  if (last) clear_slabs(false);
+}
+
+// layer_plan(w13, s13, b13, w2, s2, b2, inter, topk, experts, total_experts, act, inter_scale,
+//            block_fp8, mx, planes, clamp)
+PyObject* layer_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 16, "layer_plan takes 16 arguments");
+  auto p = std::make_unique<Plan>();
+  p->w13 = tensor_arg(a[0], "w13"); p->s13 = optional_arg(a[1], "w13_scales"); p->b13 = optional_arg(a[2], "w13_bias");
+  p->w2 = tensor_arg(a[3], "w2"); p->s2 = optional_arg(a[4], "w2_scales"); p->b2 = optional_arg(a[5], "w2_bias");
+  p->inter = int_arg(a[6]); p->topk = (int)int_arg(a[7]); p->experts = int_arg(a[8]); p->total_experts = int_arg(a[9]);
+  p->act = (int)int_arg(a[10]); p->inter_scale = (int)int_arg(a[11]);
+  p->block_fp8 = int_arg(a[12]) != 0; p->mx = int_arg(a[13]) != 0; p->planes = (int)int_arg(a[14]);
+  p->clamp = PyFloat_AsDouble(a[15]);
+  if (PyErr_Occurred()) throw python_error();
+  PyObject* capsule = PyCapsule_New(p.get(), kPlanName, free_plan);
+  if (capsule == nullptr) throw python_error();
+  p.release();
+  std::lock_guard<std::mutex> lock(g_mutex);
+  ++g_plans;
+  return capsule;
+  END_HANDLE_TH_ERRORS
+}
+
+// layer_run(plan, form, output | None, hidden, topk_weights, topk_ids, expert_map | None, a1q_scale | None,
+//           rows_hint, max_ctas, persistent, hook | None, out_dtype | None)
+// With output None the reduction is left to the caller: returns (rows [T*K, hidden], row map [T, K]),
+// valid until the next layer call on the stream.
+PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 13, "layer_run takes 13 arguments");
+  Plan& p = *plan_arg(a[0]);
+  CallOptions o;
+  o.form = (int)int_arg(a[1]);
+  o.rows_hint = int_arg(a[8]);
+  o.max_ctas = (int)int_arg(a[9]);
+  o.hook = a[11] == Py_None ? nullptr : a[11];
+  const bool gather = a[2] != Py_None;
+  const at::Tensor& x = tensor_arg(a[3], "hidden_states");
+  const at::Tensor& ids = tensor_arg(a[5], "topk_ids");
+  const std::optional<at::Tensor> map = optional_arg(a[6], "expert_map"), a1q = optional_arg(a[7], "a1q_scale");
+  need_cuda(x, "hidden_states");
+  TORCH_CHECK(x.dim() == 2, "hidden_states must be [num_rows, hidden_size]");
+  const int64_t T = x.size(0), H = x.size(1), K = p.topk, M = T * K;
+  at::ScalarType od = x.scalar_type();
+  if (gather) od = tensor_arg(a[2], "output").scalar_type();
+  else if (a[12] != Py_None) od = ((THPDtype*)a[12])->scalar_type;
+  TORCH_CHECK_NOT_IMPLEMENTED(!(a1q.has_value() && x.scalar_type() != od && !p.block_fp8),
+              // The reference forwards caller-quantised activations and their scales to gemm1 for
+              // every recipe; here only the block-scaled fp8 kernels take them (1x128 fp32 scales).
+              "a1q_scale with pre-quantised hidden_states is built for block-scaled fp8 weights only; "
+              "pass 16-bit hidden_states instead");
+  const b200moe_dtype out = dtype16(od, "ptr_D");
+  if (map.has_value()) {
+    TORCH_CHECK(map->scalar_type() == at::kInt, "expert_map must be int32");
+    TORCH_CHECK(map->size(0) == p.total_experts, "expert_map must be [total_experts_num]");
+  }
+  TORCH_CHECK(ids.scalar_type() == at::kLong || ids.scalar_type() == at::kInt, "topk_ids must be int64 or int32");
+  TORCH_CHECK(ids.dim() == 2 && ids.size(0) == T && ids.size(1) == K, "topk_ids must be [num_rows, TopK]");
+  TORCH_CHECK(x.is_contiguous() && ids.is_contiguous(), "remap_hidden_states expects contiguous tensors");
+  if (p.experts > 1024) throw std::runtime_error("local_experts_num exceeds the maximum supported number");
+  if (a1q.has_value())
+    TORCH_CHECK(a1q->is_contiguous() && a1q->dim() == 2, "remap_hidden_states expects contiguous scales");
+  if (gather) {
+    const at::Tensor& y = tensor_arg(a[2], "output");
+    const at::Tensor& w = tensor_arg(a[4], "topk_weights");
+    TORCH_CHECK(w.scalar_type() == at::kFloat, "topk_weights must be float32");
+    TORCH_CHECK(y.is_cuda() && w.is_cuda() && y.is_contiguous() && w.is_contiguous(),
+                "moe_gather expects contiguous tensors");
+    TORCH_CHECK(y.dim() == 2 && y.size(0) == T && y.size(1) == H && w.numel() == M,
+                "output must be [num_rows, hidden_size], topk_weights [num_rows, TopK]");
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  const b200moe_stream st = (b200moe_stream)stream.stream();
+  describe(p, H, od);
+  raise_if_timed_out(device_status_word(x.get_device()));   // an earlier call on this device gave up a wait
+  if (o.rows_hint == 0 && map.has_value() && p.total_experts > p.experts)
+    o.rows_hint = std::max<int64_t>(1, M * p.experts / p.total_experts);   // the other ranks' share is masked
+  mark(o, "routing");
+
+  const bool quant_fp8 = p.block_fp8 && !a1q.has_value();
+  if (!p.mx && !p.block_fp8)
+    TORCH_CHECK(x.scalar_type() == od, "ptr_A and ptr_D must have the same dtype");
+  // (16-bit rows with caller-made scales: the scales are permuted and left unused)
+  const bool a_fp8 = quant_fp8 || (p.block_fp8 && x.scalar_type() == at::kFloat8_e4m3fn);
+  Experts e{p, o, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8};
+  Layout l;
+  const size_t rows_at = l.take(p.experts * 4), map_at = l.take(M * 4);
+  const size_t sort_bytes = b200moe_sort_workspace_bytes(M, (int)p.experts);
+  const size_t sort_at = l.take(sort_bytes);
+  const size_t a_at = l.end;
+  size_t as_at = a_at;
+  if (quant_fp8) {
+    l.take(M * H);
+    as_at = l.take(M * (H / 128) * 4);
+  } else if (p.mx) {
+    l.take((size_t)p.planes * M * H);
+    as_at = l.take((size_t)p.planes * ((H + 127) / 128) * M * 4);
+  } else {
+    l.take(M * H * x.element_size());
+    if (a1q.has_value()) as_at = l.take(M * a1q->size(1) * a1q->element_size());
+  }
+  e.lay_out(l);
+  // gemm2's rows take the place of gemm1's operands (and, unfused, of its output) where they fit
+  size_t d_at = a_at;
+  if (l.end - a_at < (size_t)M * H * 2) d_at = l.take(M * H * 2);
+  e.lay_out_second(l);
+  at::Tensor mem = workspace(stream, l.end, a[10] == Py_True);
+  uint8_t* ws = mem.data_ptr<uint8_t>();
+  int32_t *rows = (int32_t*)(ws + rows_at), *row_map = (int32_t*)(ws + map_at);
+  const int32_t* emap = map.has_value() ? map->data_ptr<int32_t>() : nullptr;
+  if (quant_fp8)
+    check_status(b200moe_remap_quant_fp8(x.data_ptr(), float_dtype(x, "b200_remap_quant_fp8"), ws + a_at,
+                                         (float*)(ws + as_at), emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T,
+                                         (int)H, (int)K, (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes,
+                                         st));
+  else if (p.mx)
+    check_status(b200moe_remap_quant_mxfp8(x.data_ptr(), float_dtype(x, "hidden_states"), ws + a_at, ws + as_at,
+                                           p.planes, emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T, (int)H,
+                                           (int)K, (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes, st));
+  else
+    check_status(b200moe_remap_hidden_states(
+        x.data_ptr(), a1q.has_value() ? a1q->data_ptr() : nullptr, ws + a_at, a1q.has_value() ? ws + as_at : nullptr,
+        emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T, (int)H, (int)x.element_size(),
+        a1q.has_value() ? (int)a1q->size(1) : 0, a1q.has_value() ? (int)a1q->element_size() : 0, (int)K,
+        (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes, st));
+  mark(o, "permute");
+  e.run(ws, ws + a_at, (a_fp8 || p.mx) ? ws + as_at : nullptr, rows, ws + d_at);
+  if (gather) {
+    const at::Tensor& y = THPVariable_Unpack(a[2]);
+    const at::Tensor& w = THPVariable_Unpack(a[4]);
+    check_status(b200moe_moe_gather(y.data_ptr(), ws + d_at, w.data_ptr<float>(), row_map, out, T, (int)H, (int)K, st));
+    mark(o, "gather");
+    Py_RETURN_NONE;
+  }
+  auto view = [&](size_t at, int64_t r, int64_t c, at::ScalarType t) {
+    return mem.narrow(0, (int64_t)at, r * c * (int64_t)c10::elementSize(t)).view(t).view({r, c});
+  };
+  PyObject* y = THPVariable_Wrap(view(d_at, M, H, od));
+  PyObject* m = THPVariable_Wrap(view(map_at, T, K, at::kInt));
+  return Py_BuildValue("(NN)", y, m);
+  END_HANDLE_TH_ERRORS
+}
+
+// layer_experts(plan, form, output_rows, rows, rows_per_segment, a_scale | None, rows_hint, max_ctas,
+//               persistent, hook | None): gemm1, activation and gemm2 on rows that are grouped already.
+PyObject* layer_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
+  HANDLE_TH_ERRORS
+  TORCH_CHECK(n == 10, "layer_experts takes 10 arguments");
+  Plan& p = *plan_arg(a[0]);
+  CallOptions o;
+  o.form = (int)int_arg(a[1]);
+  o.rows_hint = int_arg(a[6]);
+  o.max_ctas = (int)int_arg(a[7]);
+  o.hook = a[9] == Py_None ? nullptr : a[9];
+  const at::Tensor &y = tensor_arg(a[2], "output_rows"), &x = tensor_arg(a[3], "rows"),
+                   &rows = tensor_arg(a[4], "rows_per_segment");
+  const std::optional<at::Tensor> scale = optional_arg(a[5], "a1q_scale");
+  need_cuda(x, "rows");
+  const int64_t M = x.size(0), H = x.size(1), segments = rows.numel();
+  TORCH_CHECK(x.dim() == 2 && y.dim() == 2 && y.size(0) == M && y.size(1) == H, "ptr_A.size(0) must match ptr_D.size(0)");
+  TORCH_CHECK(x.is_contiguous() && y.is_contiguous(), "ptr_A must be contiguous");
+  TORCH_CHECK(rows.scalar_type() == at::kInt && rows.is_contiguous() && segments > 0 && segments % p.experts == 0,
+              "rows_per_expert must be int32 [num_experts]");
+  const b200moe_dtype out = dtype16(y.scalar_type(), "ptr_D");
+  if (p.block_fp8) {
+    TORCH_CHECK(scale.has_value() && x.scalar_type() == at::kFloat8_e4m3fn && scale->scalar_type() == at::kFloat &&
+                    scale->is_contiguous() && scale->dim() == 2 && scale->size(0) == M && scale->size(1) == H / 128,
+                "ptr_A_scale must be float32 [Total_M, K / 128]");
+  } else {
+    TORCH_CHECK(x.scalar_type() == y.scalar_type(), "ptr_A and ptr_D must have the same dtype");
+  }
+  const c10::cuda::CUDAGuard guard(x.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  describe(p, H, y.scalar_type());
+  raise_if_timed_out(device_status_word(x.get_device()));
+  Experts e{p, o, out, y.scalar_type(), M, H, (int)segments, (int)x.get_device(), (b200moe_stream)stream.stream(),
+            p.block_fp8};
+  Layout l;
+  e.lay_out(l);
+  e.lay_out_second(l);
+  at::Tensor mem = workspace(stream, l.end, a[8] == Py_True);
+  e.run(mem.data_ptr<uint8_t>(), x.data_ptr(), scale.has_value() ? scale->data_ptr() : nullptr,
+        rows.data_ptr<int32_t>(), y.data_ptr());
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* workspace_clear(PyObject*, PyObject*) {
+  HANDLE_TH_ERRORS
+  clear_slabs(true);
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+}  // namespace
+
+PyMethodDef* layer_methods() {
+  static PyMethodDef methods[] = {
+      {"layer_plan", (PyCFunction)(void (*)(void))layer_plan, METH_FASTCALL, nullptr},
+      {"layer_run", (PyCFunction)(void (*)(void))layer_run, METH_FASTCALL, nullptr},
+      {"layer_experts", (PyCFunction)(void (*)(void))layer_experts, METH_FASTCALL, nullptr},
+      {"workspace_clear", workspace_clear, METH_NOARGS, nullptr},
+      {nullptr, nullptr, 0, nullptr}};
+  return methods;
+}
+
+}  // namespace b200shim

@@ -22,6 +22,15 @@
     return PyModule_Create(&module);                                         \
   }
 
+// The same with a table of module functions.
+#define B200_REGISTER_EXTENSION_METHODS(NAME, METHODS)                       \
+  PyMODINIT_FUNC PyInit_##NAME() {                                           \
+    static struct PyModuleDef module = {PyModuleDef_HEAD_INIT, #NAME,       \
+                                        nullptr, 0, METHODS, nullptr,       \
+                                        nullptr, nullptr, nullptr};         \
+    return PyModule_Create(&module);                                         \
+  }
+
 namespace b200shim {
 
 inline b200moe_stream current_stream() {

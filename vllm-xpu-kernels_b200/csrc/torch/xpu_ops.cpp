@@ -8,6 +8,8 @@
 
 #include <mutex>
 
+#include "layer.h"
+
 using namespace b200shim;
 
 namespace {
@@ -19,6 +21,10 @@ namespace {
 constexpr int kMaxStatusDevices = 64;
 std::mutex g_status_mutex;
 at::Tensor g_status[kMaxStatusDevices];
+
+}  // namespace
+
+namespace b200shim {
 
 int32_t* device_status_word(int device) {
   TORCH_CHECK(device >= 0 && device < kMaxStatusDevices, "device index out of range");
@@ -37,17 +43,12 @@ void raise_if_timed_out(int32_t* word) {
   }
 }
 
-// layout: 0 = as the reference infers it from shapes, 1 = [E,N,K], 2 = [E,K,N]
-at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>& ptr_A_scale,
-                             at::Tensor& ptr_B, const std::optional<at::Tensor>& ptr_B_scale,
-                             const std::optional<at::Tensor>& ptr_bias, at::Tensor& ptr_D,
-                             at::Tensor& rows_per_expert, int64_t N, int64_t K, int64_t num_experts,
-                             int64_t layout, int64_t epilogue, double alpha, double limit,
-                             double clamp_limit, int64_t impl, int64_t max_ctas, bool allow_segments,
-                             int64_t rows_hint = 0, const std::optional<at::Tensor>& ptr_D_scale = std::nullopt,
-                             bool mid_f16 = false) {
-  check_cuda(ptr_A, "ptr_A");
-  const auto A_dtype = ptr_A.scalar_type();
+}  // namespace b200shim
+
+namespace b200shim {
+
+WeightDesc describe_weights(const at::Tensor& ptr_B, const std::optional<at::Tensor>& ptr_B_scale, int64_t N, int64_t K,
+                            int64_t num_experts, int64_t layout, at::ScalarType A_dtype) {
   const auto B_dtype = ptr_B.scalar_type();
   const bool is_weight_fp8 = (B_dtype == at::kFloat8_e4m3fn) || (B_dtype == at::kFloat8_e5m2);
   const bool is_B_mxfp4 = (B_dtype == at::kFloat4_e2m1fn_x2) && ptr_B_scale.has_value();
@@ -58,16 +59,8 @@ at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>&
   const bool is_B_fp8_block = is_weight_fp8 && !is_B_mxfp8 && ptr_B_scale.has_value() && ptr_B_scale->dim() == 3;
 
   TORCH_CHECK(N % 8 == 0, "N must be divisible by 8");
-  TORCH_CHECK(ptr_A.dim() == 2, "ptr_A must be 2D [Total_M, K]");
   TORCH_CHECK(ptr_B.dim() == 3, "ptr_B must be 3D");
-  TORCH_CHECK(ptr_D.dim() == 2, "ptr_D must be 2D [Total_M, N]");
-  if (ptr_bias.has_value()) TORCH_CHECK(ptr_bias->dim() == 2, "ptr_bias must be 2D [num_experts, N]");
-  TORCH_CHECK(ptr_A.is_contiguous(), "ptr_A must be contiguous");
   TORCH_CHECK(ptr_B.is_contiguous(), "ptr_B must be contiguous");
-  TORCH_CHECK(ptr_D.is_contiguous(), "ptr_D must be contiguous");
-  if (ptr_bias.has_value()) TORCH_CHECK(ptr_bias->is_contiguous(), "ptr_bias must be contiguous");
-
-  const int64_t A_total_M = ptr_A.size(0), A_K = ptr_A.size(1);
   const int64_t B_E = ptr_B.size(0);
   int64_t B_K = ptr_B.size(1), B_N = ptr_B.size(2);
   b200moe_weight_format fmt;
@@ -94,27 +87,9 @@ at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>&
     fmt = B200MOE_W_BF16_KN;
     if (layout == 1) { fmt = B200MOE_W_BF16_NK; B_K = ptr_B.size(2); B_N = ptr_B.size(1); }
   }
-  const int64_t D_total_M = ptr_D.size(0), D_N = ptr_D.size(1);
-  const int64_t n_out = epilogue ? N / 2 : N;
   TORCH_CHECK(B_E == num_experts, "ptr_B.size(0) must match num_experts");
-  // Extended op only: rows_per_expert may hold a multiple of num_experts segments; segment s
-  // then multiplies with weight set s % num_experts (b200moe_gemm_args.w_experts).
-  const int64_t segments = rows_per_expert.numel();
-  TORCH_CHECK(rows_per_expert.scalar_type() == at::kInt && rows_per_expert.is_contiguous() &&
-              (segments == num_experts || (allow_segments && segments > 0 && segments % num_experts == 0)),
-              "rows_per_expert must be int32 [num_experts]");
-  TORCH_CHECK(A_total_M == D_total_M || ((is_B_mxfp4 || (is_weight_fp8 && !is_B_fp8_block)) && A_dtype == at::kFloat8_e4m3fn && A_total_M == 2 * D_total_M),
-              "ptr_A.size(0) must match ptr_D.size(0)");
-  TORCH_CHECK(A_K == B_K && B_K == K, "ptr_A K dimension must match ptr_B logical K dimension and K");
-  TORCH_CHECK(B_N == N && D_N == n_out, "ptr_B logical N dimension must match ptr_D N dimension and N");
-  if (ptr_bias.has_value()) {
-    TORCH_CHECK(ptr_bias->size(0) == num_experts, "ptr_bias.size(0) must match num_experts");
-    TORCH_CHECK(ptr_bias->size(1) == N, "ptr_bias.size(1) must match N");
-    TORCH_CHECK(ptr_bias->scalar_type() == ptr_D.scalar_type() ||
-                    (ptr_D.scalar_type() == at::kFloat8_e4m3fn &&
-                     ptr_bias->scalar_type() == (mid_f16 ? at::kHalf : at::kBFloat16)),
-                "ptr_bias must have ptr_D's dtype");
-  }
+  TORCH_CHECK(B_K == K, "ptr_A K dimension must match ptr_B logical K dimension and K");
+  TORCH_CHECK(B_N == N, "ptr_B logical N dimension must match ptr_D N dimension and N");
   int64_t group_size = 0;
   if (is_B_int4) {
     TORCH_CHECK(ptr_B_scale->is_contiguous(), "ptr_scales must be contiguous");
@@ -158,13 +133,60 @@ at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>&
     TORCH_CHECK(B_dtype == A_dtype, "w16a16 grouped gemm needs weights of the activation dtype");
   }
 
+  return {fmt, (int)group_size, is_weight_fp8, is_B_mxfp4, is_B_fp8_block};
+}
+
+}  // namespace b200shim
+
+namespace {
+
+// layout: 0 = as the reference infers it from shapes, 1 = [E,N,K], 2 = [E,K,N]
+at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>& ptr_A_scale,
+                             at::Tensor& ptr_B, const std::optional<at::Tensor>& ptr_B_scale,
+                             const std::optional<at::Tensor>& ptr_bias, at::Tensor& ptr_D,
+                             at::Tensor& rows_per_expert, int64_t N, int64_t K, int64_t num_experts,
+                             int64_t layout, int64_t epilogue, double alpha, double limit,
+                             double clamp_limit, int64_t impl, int64_t max_ctas, bool allow_segments,
+                             int64_t rows_hint = 0, const std::optional<at::Tensor>& ptr_D_scale = std::nullopt,
+                             bool mid_f16 = false) {
+  check_cuda(ptr_A, "ptr_A");
+  const auto A_dtype = ptr_A.scalar_type();
+  TORCH_CHECK(ptr_A.dim() == 2, "ptr_A must be 2D [Total_M, K]");
+  TORCH_CHECK(ptr_D.dim() == 2, "ptr_D must be 2D [Total_M, N]");
+  if (ptr_bias.has_value()) TORCH_CHECK(ptr_bias->dim() == 2, "ptr_bias must be 2D [num_experts, N]");
+  TORCH_CHECK(ptr_A.is_contiguous(), "ptr_A must be contiguous");
+  TORCH_CHECK(ptr_D.is_contiguous(), "ptr_D must be contiguous");
+  if (ptr_bias.has_value()) TORCH_CHECK(ptr_bias->is_contiguous(), "ptr_bias must be contiguous");
+
+  const int64_t A_total_M = ptr_A.size(0), A_K = ptr_A.size(1);
+  const WeightDesc w = describe_weights(ptr_B, ptr_B_scale, N, K, num_experts, layout, A_dtype);
+  const int64_t D_total_M = ptr_D.size(0), D_N = ptr_D.size(1);
+  const int64_t n_out = epilogue ? N / 2 : N;
+  // Extended op only: rows_per_expert may hold a multiple of num_experts segments; segment s
+  // then multiplies with weight set s % num_experts (b200moe_gemm_args.w_experts).
+  const int64_t segments = rows_per_expert.numel();
+  TORCH_CHECK(rows_per_expert.scalar_type() == at::kInt && rows_per_expert.is_contiguous() &&
+              (segments == num_experts || (allow_segments && segments > 0 && segments % num_experts == 0)),
+              "rows_per_expert must be int32 [num_experts]");
+  TORCH_CHECK(A_total_M == D_total_M || ((w.mxfp4 || (w.fp8 && !w.fp8_block)) && A_dtype == at::kFloat8_e4m3fn && A_total_M == 2 * D_total_M),
+              "ptr_A.size(0) must match ptr_D.size(0)");
+  TORCH_CHECK(A_K == K, "ptr_A K dimension must match ptr_B logical K dimension and K");
+  TORCH_CHECK(D_N == n_out, "ptr_B logical N dimension must match ptr_D N dimension and N");
+  if (ptr_bias.has_value()) {
+    TORCH_CHECK(ptr_bias->size(0) == num_experts, "ptr_bias.size(0) must match num_experts");
+    TORCH_CHECK(ptr_bias->size(1) == N, "ptr_bias.size(1) must match N");
+    TORCH_CHECK(ptr_bias->scalar_type() == ptr_D.scalar_type() ||
+                    (ptr_D.scalar_type() == at::kFloat8_e4m3fn &&
+                     ptr_bias->scalar_type() == (mid_f16 ? at::kHalf : at::kBFloat16)),
+                "ptr_bias must have ptr_D's dtype");
+  }
   b200moe_gemm_args g = {};
   g.a = ptr_A.data_ptr();
   if (A_dtype == at::kFloat8_e4m3fn) {
-    TORCH_CHECK((is_weight_fp8 || is_B_mxfp4) && ptr_A_scale.has_value(),
+    TORCH_CHECK((w.fp8 || w.mxfp4) && ptr_A_scale.has_value(),
                 "fp8 activations need fp8 or mxfp4 weights and ptr_A_scale");
     g.a_dtype = B200MOE_FP8_E4M3;
-    if (is_B_mxfp4 || !is_B_fp8_block) {
+    if (w.mxfp4 || !w.fp8_block) {
       // ptr_A [planes * Total_M, K] (planes = 1 or 2, the second the residual), scales
       // int32 [planes, ceil(K / 128), Total_M]: the outputs of _C::b200_quant_mxfp8.
       const int64_t planes = A_total_M / D_total_M;
@@ -191,14 +213,14 @@ at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>&
               "ptr_D must be bfloat16 or float16");
   if (d_quant) {
     // extended op only: quantised output of the fused SiLU epilogue, scales [Total_M, N / 256]
-    TORCH_CHECK(allow_segments && epilogue == 1 && ptr_D_scale.has_value() && is_B_fp8_block &&
+    TORCH_CHECK(allow_segments && epilogue == 1 && ptr_D_scale.has_value() && w.fp8_block &&
                 A_dtype == at::kFloat8_e4m3fn, "float8_e4m3fn ptr_D needs the SiLU epilogue, ptr_D_scale, fp8 "
                 "activations and block-scaled fp8 weights");
     TORCH_CHECK(N % 256 == 0 && ptr_D_scale->scalar_type() == at::kFloat && ptr_D_scale->is_contiguous() &&
                 ptr_D_scale->numel() == D_total_M * (N / 256), "ptr_D_scale must be float32 [Total_M, N / 256]");
   }
   g.w = ptr_B.data_ptr();
-  g.w_format = fmt;
+  g.w_format = w.format;
   g.w_scale = ptr_B_scale.has_value() ? ptr_B_scale->data_ptr() : nullptr;
   g.bias = ptr_bias.has_value() ? ptr_bias->data_ptr() : nullptr;
   g.d = ptr_D.data_ptr();
@@ -215,7 +237,7 @@ at::Tensor grouped_gemm_impl(at::Tensor& ptr_A, const std::optional<at::Tensor>&
   g.status = status_word;
   g.impl = (int)impl;
   g.max_ctas = (int)max_ctas;
-  g.group_size = (int)group_size;
+  g.group_size = w.group;
   g.rows_hint = rows_hint;
   const c10::cuda::CUDAGuard guard(ptr_A.device());
   check_status(b200moe_grouped_gemm(&g, current_stream()));
@@ -287,4 +309,4 @@ TORCH_LIBRARY_IMPL(_xpu_C, CUDA, m) {
   m.impl("b200_selftest_bounded_wait", &b200_selftest_bounded_wait);
 }
 
-B200_REGISTER_EXTENSION(_xpu_C)
+B200_REGISTER_EXTENSION_METHODS(_xpu_C, b200shim::layer_methods())

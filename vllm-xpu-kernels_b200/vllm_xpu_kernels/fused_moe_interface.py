@@ -31,15 +31,10 @@ except ImportError as e:  # native libraries not built
     FUSEDMOE_UNAVAILABLE_REASON = str(e)
     FUSEDMOE_AVAILABLE = False
 
-from .moe_utils import quant_act_xpu
-
 REF_FUSED_MOE_ENV = "VLLM_XPU_FUSED_MOE_USE_REF"
 USE_MXFP4_FP8_ENV = "VLLM_XPU_FUSED_MOE_USE_MXFP4_FP8"
 FP8_BLOCK_SIZE = 128
 FP8_FUSED_MIN_ROWS = 512   # routed rows per expert from which gemm1 of an fp8 layer fuses SiLU + quantisation
-
-# Epilogue codes of torch.ops._xpu_C.b200_grouped_gemm (b200moe_epilogue).
-_EPI_NONE, _EPI_SILU, _EPI_SWIGLUOAI = 0, 1, 2
 
 
 def _require_native():
@@ -124,23 +119,19 @@ def compute_num_tokens_per_block(num_tokens, num_experts_per_node):
 
 
 # Intermediates of a layer call (permuted rows, the two GEMM outputs, scales, index maps) live
-# in one grow-only pool per device, shared by all layer objects: layers of a model run one after
-# the other on a stream, so the next call may overwrite what the previous one left.  A caller
-# that runs layer calls concurrently on several streams of one device must pass
-# ``persistent_workspace=False`` (fresh torch allocations per call, as the reference does).
-_WORKSPACE = {}
+# in one grow-only workspace per device and stream, shared by all layer objects: layers of a model
+# run one after the other on a stream, so the next call may overwrite what the previous one left
+# (csrc/torch/layer.cpp; given back with the last layer object).  ``persistent_workspace=False``
+# takes a fresh torch allocation per call instead, as the reference does.
+class _Workspace:
+    """The workspaces as a whole; ``clear()`` gives them back."""
+
+    @staticmethod
+    def clear():
+        _xpu_C.workspace_clear()
 
 
-def _pooled(name, shape, dtype, device):
-    n = 1
-    for d in shape:
-        n *= int(d)
-    key = (device, name, dtype)
-    buf = _WORKSPACE.get(key)
-    if buf is None or buf.numel() < n:
-        buf = torch.empty(max(n, 1), dtype=dtype, device=device)
-        _WORKSPACE[key] = buf
-    return buf[:n].view(shape)
+_WORKSPACE = _Workspace()
 
 
 def _signed_nibbles(w):
@@ -161,6 +152,15 @@ def _activation_kind(activation):
     if activation == "swigluoai" or ("SWIGLUOAI" in str(activation)):
         return "swigluoai"
     raise ValueError(f"Unsupported FusedMoe activation: {activation}.")
+
+
+# Attributes of a layer that its native plan holds: setting one of them makes a new plan.
+_PLAN_FIELDS = frozenset((
+    "w13", "gemm1_wei_scales", "w13_bias", "w2", "gemm2_wei_scales", "w2_bias", "inter_size", "n_experts_per_token",
+    "num_experts", "total_experts_num", "inter_size_scale", "is_block_fp8", "mx_acts", "mx_planes", "gemm1_clamp_limit"))
+
+# Codes of the activations in csrc/torch/layer.cpp.
+_ACT_CODES = {"silu": 0, "gelu": 1, "gelu_tanh": 2, "swigluoai": 3, "relu2_no_mul": 4, "swiglustep": 5}
 
 
 def _activation_op(kind):
@@ -195,9 +195,8 @@ class XpuFusedMoe:
     ``True`` forces it wherever a kernel has it, ``False`` never fuses.
 
     ``persistent_workspace`` (not in the reference; keyword only, default
-    True): intermediates come from one grow-only pool per device shared by all
-    layer objects instead of fresh allocations per call; a layer object (and
-    the pool) must then be used from one stream at a time.
+    True): intermediates come from one grow-only workspace per device and
+    stream, shared by all layer objects, instead of fresh allocations per call.
 
     ``mxfp4_activations`` (not in the reference; keyword only) chooses what the
     MXFP4 (and per-tensor fp8, and MXFP8, whose default is one plane as its recipe
@@ -334,7 +333,7 @@ class XpuFusedMoe:
             raise ValueError("the block-scaled MXFP4 GEMM has no fused SiLU epilogue")
         if fuse_activation and self._act_kind not in ("silu", "swigluoai"):
             raise ValueError(f"no fused epilogue for the {self._act_kind} activation")
-        self.act_func = _activation_op(self._act_kind)
+        self._native_plan = None
 
         self.expert_map = expert_map
         if self.expert_map is None and self.ep_size > 1:
@@ -359,14 +358,21 @@ class XpuFusedMoe:
         # benchmark does (benchmark/src/fused_moe_interface_.py:12-40)
         self.stage_hook = None
 
-    def _mark(self, name):
-        if self.stage_hook is not None:
-            self.stage_hook(name)
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        if name in _PLAN_FIELDS:
+            object.__setattr__(self, "_native_plan", None)
 
-    def _buf(self, name, shape, dtype, device):
-        if self.persistent_workspace:
-            return _pooled(name, shape, dtype, device)
-        return torch.empty(shape, dtype=dtype, device=device)
+    def _plan(self):
+        """The layer as csrc/torch/layer.cpp sees it (tensors, sizes, recipe); made on first use."""
+        if self._native_plan is None:
+            clamp = self.gemm1_clamp_limit
+            self._native_plan = _xpu_C.layer_plan(
+                self.w13, self.gemm1_wei_scales, self.w13_bias, self.w2, self.gemm2_wei_scales, self.w2_bias,
+                self.inter_size, self.n_experts_per_token, self.num_experts, self.total_experts_num,
+                _ACT_CODES[self._act_kind], self.inter_size_scale, self.is_block_fp8, self.mx_acts, self.mx_planes,
+                float(clamp) if clamp is not None and clamp > 0 else 0.0)
+        return self._native_plan
 
     def apply(self, output, hidden_states, topk_weights, topk_ids,
               expert_map=None, a1q_scale=None):
@@ -378,73 +384,25 @@ class XpuFusedMoe:
         [planes, ceil(cols / 128), rows]); planes = 2 adds the residual plane."""
         rows, cols = x.shape
         planes = self.mx_planes
-        q = self._buf(f"mxq{cols}", (planes * rows, cols), torch.float8_e4m3fn, x.device)
-        s = self._buf(f"mxs{cols}", (planes, (cols + 127) // 128, rows), torch.int32, x.device)
+        q = torch.empty((planes * rows, cols), dtype=torch.float8_e4m3fn, device=x.device)
+        s = torch.empty((planes, (cols + 127) // 128, rows), dtype=torch.int32, device=x.device)
         torch.ops._C.b200_quant_mxfp8(x, q, s)
         return q, s
 
-    # The stages below are the reference's eight steps (:328-419); what differs
-    # is inside the ops and, for block fp8, that activations really are
-    # quantised to e4m3 per 1x128 group and multiplied on the fp8 tensor cores.
+    # The stages are the reference's eight steps (:328-419), launched from native code; what
+    # differs is inside the kernels and, for block fp8, that activations really are quantised
+    # to e4m3 per 1x128 group and multiplied on the fp8 tensor cores.
     def _apply_kernel(self, output, hidden_states, topk_weights, topk_ids,
                       expert_map=None, a1q_scale=None, gather=True, out_dtype=None):
         """With ``gather=False`` the last stage is left to the caller: returns the expert-major
         rows ``[T*K, hidden]`` after gemm2 and the row map ``[T, K]`` (valid until the next
-        layer call on this device)."""
-        self._mark("routing")
-        num_rows, hidden_size = hidden_states.shape
-        K = self.n_experts_per_token
-        num_moe_inputs = K * num_rows
-        dev = hidden_states.device
-        E = self.num_experts
-        I = self.inter_size
+        layer call on this stream)."""
         if expert_map is None and self.ep_size > 1:
             expert_map = self.expert_map
-        if out_dtype is None:
-            out_dtype = output.dtype if output is not None else hidden_states.dtype
-        if (a1q_scale is not None and hidden_states.dtype != out_dtype and not self.is_block_fp8):
-            # The reference forwards caller-quantised activations and their scales to gemm1 for
-            # every recipe; here only the block-scaled fp8 kernels take them (1x128 fp32 scales).
-            raise NotImplementedError(
-                f"a1q_scale with pre-quantised hidden_states is built for block-scaled fp8 weights only "
-                f"(recipe of this layer: {self.recipe}); pass 16-bit hidden_states instead")
-
-        rows_per_expert = self._buf("rows_per_expert", (E,), torch.int32, dev)
-        row_map = self._buf("row_map", (num_rows, K), torch.int32, dev)
-
-        quant_acts = self.is_block_fp8
-        if quant_acts and a1q_scale is None:
-            # permute + dynamic 1x128 e4m3 quantisation in one pass
-            remapped = self._buf("remapped", (num_moe_inputs, hidden_size), torch.float8_e4m3fn, dev)
-            remapped_scales = self._buf("remapped_scales", (num_moe_inputs, hidden_size // FP8_BLOCK_SIZE),
-                                        torch.float32, dev)
-            torch.ops._moe_C.b200_remap_quant_fp8(
-                hidden_states, remapped, remapped_scales, expert_map, rows_per_expert,
-                row_map, topk_ids, self.total_experts_num, self.local_experts_num)
-        else:
-            if a1q_scale is not None:
-                remapped_scales = self._buf("remapped_scales", (num_moe_inputs, a1q_scale.shape[1]),
-                                            a1q_scale.dtype, dev)
-            else:
-                remapped_scales = None
-            remapped = self._buf("remapped", (num_moe_inputs, hidden_size), hidden_states.dtype, dev)
-            torch.ops._moe_C.remap_hidden_states(
-                hidden_states=hidden_states, hidden_states_scales=a1q_scale,
-                remapped_hidden_states=remapped,
-                remapped_hidden_states_scales=remapped_scales, expert_map=expert_map,
-                rows_per_expert=rows_per_expert,
-                unpermuted_row_to_permuted_row=row_map, topk_ids=topk_ids,
-                total_experts_num=self.total_experts_num,
-                local_experts_num=self.local_experts_num)
-
-        self._mark("permute")
-        a_scale1 = remapped_scales if quant_acts else None
-        gemm2_output = self._buf("gemm2_output", (num_moe_inputs, hidden_size), out_dtype, dev)
-        self._experts(gemm2_output, remapped, a_scale1, rows_per_expert)
-        if not gather:
-            return gemm2_output, row_map
-        torch.ops._moe_C.moe_gather(output, gemm2_output, topk_weights, row_map, E)
-        self._mark("gather")
+        return _xpu_C.layer_run(
+            self._native_plan or self._plan(), self._form(hidden_states.shape[0] * self.n_experts_per_token),
+            output if gather else None, hidden_states, topk_weights, topk_ids, expert_map, a1q_scale, self.rows_hint,
+            self.gemm_max_ctas, self.persistent_workspace, self.stage_hook, out_dtype)
 
     def apply_sorted(self, output_rows, rows, rows_per_segment, a1q_scale=None):
         """The experts alone (gemm1 -> activation -> gemm2) on rows that are already grouped:
@@ -461,7 +419,9 @@ class XpuFusedMoe:
             raise NotImplementedError("apply_sorted: 16-bit or block-scaled fp8 weights only")
         if rows.shape[0] == 0:
             return
-        self._experts(output_rows, rows, a1q_scale if self.is_block_fp8 else None, rows_per_segment)
+        _xpu_C.layer_experts(self._plan(), self._form(rows.shape[0]), output_rows, rows, rows_per_segment,
+                             a1q_scale if self.is_block_fp8 else None, self.rows_hint, self.gemm_max_ctas,
+                             self.persistent_workspace, self.stage_hook)
 
     def fuses_activation(self, num_moe_inputs):
         """Which form gemm1 takes for a call with `num_moe_inputs` routed rows: "fp8" (SiLU and the
@@ -476,77 +436,10 @@ class XpuFusedMoe:
             return "epilogue"
         return None
 
-    def _experts(self, gemm2_output, remapped, a_scale1, rows_per_expert):
-        """gemm1 (+ activation) and gemm2 on permuted rows; writes gemm2_output [rows, hidden]."""
-        num_moe_inputs, hidden_size = remapped.shape
-        dev = remapped.device
-        E = self.num_experts
-        I = self.inter_size
-        quant_acts = self.is_block_fp8
-        output = gemm2_output
-        if self.mx_acts:
-            remapped, a_scale1 = self._quant_mx(remapped)
-        clamp = float(self.gemm1_clamp_limit) if (self.gemm1_clamp_limit is not None
-                                                   and self.gemm1_clamp_limit > 0) else 0.0
-
-        # ---- gemm1 (+ activation) ----
+    def _form(self, num_moe_inputs):
+        """`fuses_activation` as the code csrc/torch/layer.cpp takes."""
         fused = self.fuses_activation(num_moe_inputs)
-        if fused == "fp8":
-            act_output = None
-            act_q = self._buf("act_q", (num_moe_inputs, I), torch.float8_e4m3fn, dev)
-            gemm2_act_scale = self._buf("act_q_scale", (num_moe_inputs, I // FP8_BLOCK_SIZE), torch.float32, dev)
-            torch.ops._xpu_C.b200_grouped_gemm(
-                remapped, a_scale1, self.w13, self.gemm1_wei_scales, self.w13_bias, act_q,
-                rows_per_expert, 2 * I, hidden_size, E, 0, _EPI_SILU, 1.702, 7.0, clamp, 0,
-                self.gemm_max_ctas, self.rows_hint, gemm2_act_scale, output.dtype == torch.float16)
-            self._mark("gemm1")
-        elif fused == "epilogue":
-            act_output = self._buf("act_output", (num_moe_inputs, I), output.dtype, dev)
-            torch.ops._xpu_C.b200_grouped_gemm(
-                remapped, a_scale1, self.w13, self.gemm1_wei_scales, self.w13_bias, act_output,
-                rows_per_expert, 2 * I, hidden_size, E, 0,
-                _EPI_SILU if self._act_kind == "silu" else _EPI_SWIGLUOAI, 1.702, 7.0, clamp, 0,
-                self.gemm_max_ctas, self.rows_hint)
-            self._mark("gemm1")
-        else:
-            gemm1_output = self._buf("gemm1_output", (num_moe_inputs, 2 * I), output.dtype, dev)
-            torch.ops._xpu_C.b200_grouped_gemm(
-                remapped, a_scale1, self.w13, self.gemm1_wei_scales, self.w13_bias, gemm1_output,
-                rows_per_expert, 2 * I, hidden_size, E, 0, _EPI_NONE, 1.702, 7.0, 0.0, 0,
-                self.gemm_max_ctas, self.rows_hint)
-            self._mark("gemm1")
-            if clamp > 0:
-                gate = gemm1_output[:, :I]
-                up = gemm1_output[:, I:]
-                gate.clamp_(max=clamp)
-                up.clamp_(min=-clamp, max=clamp)
-            if quant_acts and self._act_kind == "silu" and I % FP8_BLOCK_SIZE == 0:
-                # SiLU, multiply and the 1x128 e4m3 quantisation of gemm2's input in one pass
-                act_output = None
-                act_q = self._buf("act_q", (num_moe_inputs, I), torch.float8_e4m3fn, dev)
-                gemm2_act_scale = self._buf("act_q_scale", (num_moe_inputs, I // FP8_BLOCK_SIZE), torch.float32, dev)
-                # (only the rows the experts' segments use: the buffers may be sized for a worst case)
-                torch.ops._C.b200_silu_and_mul_block_quant_rows(act_q, gemm1_output, gemm2_act_scale,
-                                                                rows_per_expert)
-            else:
-                act_output = self._buf("act_output", (num_moe_inputs, I * self.inter_size_scale), output.dtype, dev)
-                self.act_func(act_output, gemm1_output)
-
-        self._mark("activation")
-        # ---- gemm2 ----
-        if quant_acts and act_output is None:
-            pass   # already quantised together with the activation
-        elif quant_acts:
-            act_q, gemm2_act_scale = quant_act_xpu(act_output, self.recipe)
-        elif self.mx_acts:
-            act_q, gemm2_act_scale = self._quant_mx(act_output)
-        else:
-            act_q, gemm2_act_scale = act_output, None
-        torch.ops._xpu_C.b200_grouped_gemm(
-            act_q, gemm2_act_scale, self.w2, self.gemm2_wei_scales, self.w2_bias, gemm2_output,
-            rows_per_expert, hidden_size, I * self.inter_size_scale, E, 0, _EPI_NONE, 1.702, 7.0, 0.0, 0,
-            self.gemm_max_ctas, self.rows_hint)
-        self._mark("gemm2")
+        return 0 if fused is None else (2 if fused == "fp8" else 1)
 
 
 def xpu_fused_moe(hidden_states,
