@@ -54,11 +54,11 @@ __global__ void __launch_bounds__(64) bounded_wait_selftest_kernel(int32_t* stat
   volatile int* af = &abort_flag;
   bool ok = true;
   if (threadIdx.x == 0) {
-    ok = ptx::mbar_wait(&bar, 0, af, false, budget_cycles);   // phase 0 never completes
+    ok = ptx::mbar_wait(&bar, 0, af, budget_cycles);   // phase 0 never completes
   } else if (threadIdx.x == 32) {
     // a second role, as the MMA issuer beside the producer: it polls the same barrier and
     // must leave through the abort flag once the first wait has given up
-    ok = ptx::mbar_wait(&bar, 0, af, false, 4 * budget_cycles);
+    ok = ptx::mbar_wait(&bar, 0, af, 4 * budget_cycles);
   }
   __syncthreads();
   if (threadIdx.x == 0 && *af != 0 && status != nullptr) {

@@ -37,7 +37,7 @@ namespace {
 
 constexpr int kWTileBytes = 16384;  // 128 rows x 128 bytes, or the same area K-by-N
 constexpr int kMaxAccStages = 8;
-constexpr int kMaxStages = 8;
+constexpr int kMaxStages = 11;
 
 struct TcParams {
   const float* a_scale;
@@ -157,49 +157,58 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      uint32_t it = 0, s = 0, ph = 0;
+    // (one thread here and in the issuer; their instruction chains bound a CTA's streaming rate
+    // at decode sizes, so addresses and descriptors advance by additions)
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 1;
       int cursor = 0;
       bool ok = true;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t st0 = ptx::smem_u32(smem);
+      uint32_t st = st0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti, p.w_experts);
         const int n0 = ti.n_tile * kFeat;
-        for (int kb = 0; kb < p.num_kb; ++kb, ++it) {
-          if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* wdst = smem + s * kStageBytes;
-          uint8_t* adst = wdst + kAOff;
-          ptx::mbar_expect_tx(&ctrl->full[s], kStageBytes);
+        for (int kb = 0; kb < p.num_kb; ++kb) {
+          const uint32_t full = full0 + 8 * s;
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          ptx::mbar_expect_tx_s(full, kStageBytes);
           const int k0 = kb * kElemsPerKb;
 #pragma unroll
           for (int half = 0; half < (kGated ? 2 : 1); ++half) {   // gate tile, then (gated) the up tile
-            uint8_t* wd = wdst + half * kWTileBytes;
+            const uint32_t wd = st + half * kWTileBytes;
             const int nn = n0 + half * (p.n >> 1);
             if (!kWKn) {
-              ptx::tma_load_3d(wd, &tmap_w, &ctrl->full[s], k0, nn, ti.e);
+              ptx::tma_load_3d_s(wd, &tmap_w, full, k0, nn, ti.e);
             } else if (kFp8) {
-              ptx::tma_load_3d(wd, &tmap_w, &ctrl->full[s], nn, k0, ti.e);
+              ptx::tma_load_3d_s(wd, &tmap_w, full, nn, k0, ti.e);
             } else {
-              ptx::tma_load_3d(wd, &tmap_w, &ctrl->full[s], nn, k0, ti.e);
-              ptx::tma_load_3d(wd + kWTileBytes / 2, &tmap_w, &ctrl->full[s], nn + 64, k0, ti.e);
+              ptx::tma_load_3d_s(wd, &tmap_w, full, nn, k0, ti.e);
+              ptx::tma_load_3d_s(wd + kWTileBytes / 2, &tmap_w, full, nn + 64, k0, ti.e);
             }
           }
-          ptx::tma_load_2d(adst, &tmap_a, &ctrl->full[s], k0, ti.row0);
-          if (++s == (uint32_t)kStages) { s = 0; ph ^= 1; }
+          ptx::tma_load_2d_s(st + kAOff, &tmap_a, full, k0, ti.row0);
+          st += kStageBytes;
+          if (++s == (uint32_t)kStages) { s = 0; ph ^= 1; st = st0; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    // (the whole warp runs the loop with the same values; one elected lane issues)
-    {
+    if (ptx::elect_one()) {
       uint32_t s = 0, ph = 0, acc_it = 0;
       int cursor = 0;
       bool ok = true;
-      const uint32_t smem_base = ptx::smem_u32(smem);
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
       // leading-dimension byte offset of the weight operand: K-major 16, MN-major 8192 (16-bit) / 16384 (fp8)
       constexpr uint32_t kWLbo = !kWKn ? 16u : (kFp8 ? 16384u : 8192u);
-      constexpr uint32_t kWStep = !kWKn ? 32u : (kFp8 ? 4096u : 2048u);   // bytes per 32-byte K step
+      constexpr int kWStep = (!kWKn ? 32 : (kFp8 ? 4096 : 2048)) / 16;   // 16-byte units per 32-byte K step
+      const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kWLbo, 1024);
+      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kAOff, 16, 1024);
+      uint64_t wdesc = wdesc0, adesc = adesc0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti, p.w_experts);
@@ -209,40 +218,31 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((n_eff >> 3) << 17);
         constexpr bool per_block = kFp8;
         if (!per_block) {
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_empty[a], ((acc_it / kAccStages) & 1) ^ 1, abort_flag))) break;
+          if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, ((acc_it / kAccStages) & 1) ^ 1, abort_flag)) break;
           ptx::tc_fence_after();
         }
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          bool go = true;
           if (per_block) {
             a = acc_it % kAccStages;
-            go = ptx::mbar_wait(&ctrl->acc_empty[a], ((acc_it / kAccStages) & 1) ^ 1, abort_flag);
+            if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, ((acc_it / kAccStages) & 1) ^ 1, abort_flag)) { ok = false; break; }
           }
-          if (go) go = ptx::mbar_wait(&ctrl->full[s], ph, abort_flag);
-          if (!__all_sync(0xffffffffu, go)) { ok = false; break; }
+          if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
-          // every operand descriptor of the stage = one base descriptor + a compile-time
-          // offset (the address field counts 16-byte units), so the issue loop is adds only
-          const uint32_t st_addr = smem_base + s * kStageBytes;
-          const uint64_t wdesc0 = ptx::make_smem_desc(st_addr, kWLbo, 1024);
-          const uint64_t adesc0 = ptx::make_smem_desc(st_addr + kAOff, 16, 1024);
           const uint32_t d_tmem = tmem_base + a * kAccCols;
+          const uint32_t accumulate = per_block ? 0u : (kb > 0 ? 1u : 0u);
 #pragma unroll
-          for (int half = 0; half < (kGated ? 2 : 1); ++half) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const uint32_t accumulate = per_block ? (j > 0) : (kb > 0 || j > 0);
-              ptx::umma_elect<kFp8>(d_tmem + half * BT, wdesc0 + (uint64_t)((half * kWTileBytes + j * kWStep) >> 4),
-                                    adesc0 + (uint64_t)((j * 32) >> 4), idesc, accumulate);
-            }
-          }
-          ptx::umma_commit_elect(&ctrl->empty[s]);
-          if (per_block) { ptx::umma_commit_elect(&ctrl->acc_full[a]); ++acc_it; }
-          if (++s == (uint32_t)kStages) { s = 0; ph ^= 1; }
+          for (int half = 0; half < (kGated ? 2 : 1); ++half)
+            ptx::umma_block<kFp8, kWStep, 2>(d_tmem + half * BT, wdesc + half * (kWTileBytes >> 4), adesc, idesc, accumulate);
+          ptx::umma_commit(empty0 + 8 * s);
+          if (per_block) { ptx::umma_commit(acc_full0 + 8 * a); ++acc_it; }
+          wdesc += kStageBytes >> 4;
+          adesc += kStageBytes >> 4;
+          if (++s == (uint32_t)kStages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
         }
-        if (!per_block && ok) { ptx::umma_commit_elect(&ctrl->acc_full[a]); ++acc_it; }
+        if (!per_block && ok) { ptx::umma_commit(acc_full0 + 8 * a); ++acc_it; }
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------ epilogue ----------------------------------
     const int q = warp & 3;                 // TMEM lane quarter this warp may read
@@ -550,10 +550,14 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      uint32_t s = 0, ph = 0;
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 1;
       int cursor = 0;
       bool ok = true;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t bar0 = ptx::map_to_cta(full0, 0);   // the even CTA's barriers count the bytes of both CTAs
+      const uint32_t st0 = ptx::smem_u32(smem);
+      uint32_t st = st0;
       for (int t = walker; t < total_tiles && ok; t += walkers) {
         TileInfo ti;
         locate_tile<kPairTok>(walk, t, cursor, ti, p.w_experts);
@@ -561,52 +565,52 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int n0 = kGated ? (cta == 0 ? 0 : (p.n >> 1)) + ti.n_tile * kFeat : (ti.n_tile * 2 + (int)cta) * kFeat;
         const int row = ti.row0 + (int)cta * 128;
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* wdst = smem + s * kPairStageBytes;
-          // the even CTA's barrier counts the bytes of both CTAs
-          if (cta == 0) ptx::mbar_expect_tx(&ctrl->full[s], 2 * kPairStageBytes);
-          const uint32_t bar = ptx::map_to_cta(ptx::smem_u32(&ctrl->full[s]), 0);
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (cta == 0) ptx::mbar_expect_tx_s(full0 + 8 * s, 2 * kPairStageBytes);
+          const uint32_t bar = bar0 + 8 * s;
           const int k0 = kb * 64;
           if (!kWKn) {
-            ptx::tma_load_3d_pair(wdst, &tmap_w, bar, k0, n0, ti.e);
+            ptx::tma_load_3d_pair(st, &tmap_w, bar, k0, n0, ti.e);
           } else {
-            ptx::tma_load_3d_pair(wdst, &tmap_w, bar, n0, k0, ti.e);
-            ptx::tma_load_3d_pair(wdst + kWTileBytes / 2, &tmap_w, bar, n0 + 64, k0, ti.e);
+            ptx::tma_load_3d_pair(st, &tmap_w, bar, n0, k0, ti.e);
+            ptx::tma_load_3d_pair(st + kWTileBytes / 2, &tmap_w, bar, n0 + 64, k0, ti.e);
           }
-          ptx::tma_load_2d_pair(wdst + kWTileBytes, &tmap_a, bar, k0, row);
-          if (++s == (uint32_t)kStagesP) { s = 0; ph ^= 1; }
+          ptx::tma_load_2d_pair(st + kWTileBytes, &tmap_a, bar, k0, row);
+          st += kPairStageBytes;
+          if (++s == (uint32_t)kStagesP) { s = 0; ph ^= 1; st = st0; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (even CTA) -----------------------
-    if (cta == 0) {
+    if (cta == 0 && ptx::elect_one()) {
       uint32_t s = 0, ph = 0, acc_it = 0;
       bool ok = true;
-      const uint32_t smem_base = ptx::smem_u32(smem);
-      constexpr uint32_t kWLbo = !kWKn ? 16u : 8192u;
-      constexpr uint32_t kWStep = !kWKn ? 32u : 2048u;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
+      constexpr int kWStep = (!kWKn ? 32 : 2048) / 16;
+      const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kWKn ? 8192u : 16u, 1024);
+      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kWTileBytes, 16, 1024);
+      uint64_t wdesc = wdesc0, adesc = adesc0;
       const uint32_t idesc = (p.idesc & ~((0x3fu << 17) | (0x1fu << 24))) | ((256u >> 3) << 17) | ((256u >> 4) << 24);
       for (int t = walker; t < total_tiles && ok; t += walkers) {
         const uint32_t a = acc_it & 1;
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_empty[a], ((acc_it >> 1) & 1) ^ 1, abort_flag))) break;
+        if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, ((acc_it >> 1) & 1) ^ 1, abort_flag)) break;
         ptx::tc_fence_after();
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->full[s], ph, abort_flag))) { ok = false; break; }
+          if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
-          const uint32_t st_addr = smem_base + s * kPairStageBytes;
-          const uint64_t wdesc0 = ptx::make_smem_desc(st_addr, kWLbo, 1024);
-          const uint64_t adesc0 = ptx::make_smem_desc(st_addr + kWTileBytes, 16, 1024);
-#pragma unroll
-          for (int j = 0; j < 4; ++j)
-            ptx::umma_f16_pair_elect(tmem_base + a * kPairTok, wdesc0 + (uint64_t)((j * kWStep) >> 4),
-                                     adesc0 + (uint64_t)((j * 32) >> 4), idesc, (kb > 0 || j > 0) ? 1u : 0u);
-          ptx::umma_commit_pair_elect(&ctrl->empty[s]);
-          if (++s == (uint32_t)kStagesP) { s = 0; ph ^= 1; }
+          ptx::umma_f16_pair_block<kWStep, 2>(tmem_base + a * kPairTok, wdesc, adesc, idesc, kb > 0 ? 1u : 0u);
+          ptx::umma_commit_pair(empty0 + 8 * s);
+          wdesc += kPairStageBytes >> 4;
+          adesc += kPairStageBytes >> 4;
+          if (++s == (uint32_t)kStagesP) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
         }
-        if (ok) { ptx::umma_commit_pair_elect(&ctrl->acc_full[a]); ++acc_it; }
+        if (ok) { ptx::umma_commit_pair(acc_full0 + 8 * a); ++acc_it; }
       }
     }
+    __syncwarp();
   } else {
     // ------------------------------ epilogue ----------------------------------
     const int q = warp & 3;

@@ -227,70 +227,68 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      uint32_t s = 0, ph = 0;
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 1;
       int cursor = 0;
       bool ok = true;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full_raw[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti);
         const int n0 = ti.n_tile * kFeat;
         for (int si = 0; si < num_st; ++si) {
-          if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* st = smem + s * stage_bytes;
+          const uint32_t full = full0 + 8 * s;
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          const uint32_t st = ptx::smem_u32(smem) + s * stage_bytes;
           const int kb0 = si * kSub;
           const int nsub = (p.num_kb - kb0) < kSub ? (p.num_kb - kb0) : kSub;
-          ptx::mbar_expect_tx(&ctrl->full_raw[s], nsub * (kRawBytes + kABytes));
+          ptx::mbar_expect_tx_s(full, nsub * (kRawBytes + kABytes));
 #pragma unroll
           for (int sub = 0; sub < kSub; ++sub) {
             if (sub < nsub) {
-              ptx::tma_load_3d(st + kRawOff + sub * kRawBytes, &tmap_w, &ctrl->full_raw[s], (kb0 + sub) * 32, n0, ti.e);
-              ptx::tma_load_2d(st + kAOff + sub * kABytes, &tmap_a, &ctrl->full_raw[s], (kb0 + sub) * 64, ti.row0);
+              ptx::tma_load_3d_s(st + kRawOff + sub * kRawBytes, &tmap_w, full, (kb0 + sub) * 32, n0, ti.e);
+              ptx::tma_load_2d_s(st + kAOff + sub * kABytes, &tmap_a, full, (kb0 + sub) * 64, ti.row0);
             }
           }
           if (++s == (uint32_t)stages) { s = 0; ph ^= 1; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    // (the whole warp runs the loop with the same values; one elected lane issues)
-    {
+    if (ptx::elect_one()) {
       uint32_t s = 0, ph = 0, acc_it = 0;
       int cursor = 0;
       bool ok = true;
-      const uint32_t smem_base = ptx::smem_u32(smem);
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full_op[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti);
         const uint32_t a = acc_it & 1;
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_empty[a], ((acc_it >> 1) & 1) ^ 1, abort_flag))) break;
+        if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, ((acc_it >> 1) & 1) ^ 1, abort_flag)) break;
         ptx::tc_fence_after();
         // a partly filled token tile multiplies only its valid columns (UMMA N in steps of 16)
         const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((uint32_t)(((ti.valid + 15) & ~15) >> 3) << 17);
         for (int si = 0; si < num_st; ++si) {
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->full_op[s], ph, abort_flag))) { ok = false; break; }
+          if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::tc_fence_after();
           // every operand descriptor of the stage = the first one + a compile-time offset
-          const uint64_t desc0 = ptx::make_smem_desc(smem_base + s * stage_bytes, 16, 1024);
+          const uint64_t desc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + s * stage_bytes, 16, 1024);
           const int kb0 = si * kSub;
 #pragma unroll
-          for (int sub = 0; sub < kSub; ++sub) {
-            if (kb0 + sub < p.num_kb) {
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                const uint64_t wdesc = desc0 + (uint64_t)((sub * kOpBytes + j * 32) >> 4);
-                const uint64_t adesc = desc0 + (uint64_t)((kAOff + sub * kABytes + j * 32) >> 4);
-                ptx::umma_elect<false>(tmem_base + a * BT, wdesc, adesc, idesc, (kb0 + sub > 0 || j > 0) ? 1u : 0u);
-              }
-            }
-          }
-          ptx::umma_commit_elect(&ctrl->empty[s]);
+          for (int sub = 0; sub < kSub; ++sub)
+            if (kb0 + sub < p.num_kb)
+              ptx::umma_block<false, 2, 2>(tmem_base + a * BT, desc0 + ((sub * kOpBytes) >> 4),
+                                           desc0 + ((kAOff + sub * kABytes) >> 4), idesc, kb0 + sub > 0 ? 1u : 0u);
+          ptx::umma_commit(empty0 + 8 * s);
           if (++s == (uint32_t)stages) { s = 0; ph ^= 1; }
         }
-        if (ok) { ptx::umma_commit_elect(&ctrl->acc_full[a]); ++acc_it; }
+        if (ok) { ptx::umma_commit(acc_full0 + 8 * a); ++acc_it; }
       }
     }
+    __syncwarp();
   } else if (warp < 2 + kDqConvWarps) {
     // ------------------------------ converters --------------------------------
     const int ct = (warp - 2) * 32 + lane;   // 0..255

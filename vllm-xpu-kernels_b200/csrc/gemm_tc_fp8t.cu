@@ -58,12 +58,6 @@ struct TParams {
   // token and 128 features in d_scale [M, n/256]
   float* d_scale;
   float clamp;            // >0: gate = min(gate, clamp), up = clamp(up, -clamp, clamp)
-  // 128 x 256 kernel: 4 stages and rows stored straight from the registers (few rows per expert:
-  // HBM-bound, bytes in flight matter, few rows to store), or 3 stages and the rows transposed
-  // through shared memory into whole 256-byte segments (many rows per expert: the store of a
-  // tile, which the promotion warps cannot overlap with anything, is 4 us as scattered 16-byte
-  // pieces and under 1 us as rows)
-  int stages;
 };
 
 struct TCtrl {
@@ -121,57 +115,57 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
-    if (lane == 0) {
-      uint32_t s = 0, ph = 0;
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 1;
       int cursor = 0;
       bool ok = true;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t st0 = ptx::smem_u32(smem);
+      uint32_t st = st0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
         const int n0 = ti.n_tile * kFeat;
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* wdst = smem + s * kTStageBytes;
-          ptx::mbar_expect_tx(&ctrl->full[s], kTStageBytes);
-          if (!kWKn) ptx::tma_load_3d(wdst, &tmap_w, &ctrl->full[s], kb * 128, n0, ti.e);
-          else ptx::tma_load_3d(wdst, &tmap_w, &ctrl->full[s], n0, kb * 128, ti.e);
-          ptx::tma_load_2d(wdst + 16384, &tmap_a, &ctrl->full[s], kb * 128, ti.row0);
-          if (++s == (uint32_t)kTStages) { s = 0; ph ^= 1; }
+          const uint32_t full = full0 + 8 * s;
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          ptx::mbar_expect_tx_s(full, kTStageBytes);
+          if (!kWKn) ptx::tma_load_3d_s(st, &tmap_w, full, kb * 128, n0, ti.e);
+          else ptx::tma_load_3d_s(st, &tmap_w, full, n0, kb * 128, ti.e);
+          ptx::tma_load_2d_s(st + 16384, &tmap_a, full, kb * 128, ti.row0);
+          st += kTStageBytes;
+          if (++s == (uint32_t)kTStages) { s = 0; ph ^= 1; st = st0; }
         }
       }
     }
+    __syncwarp();
   } else if (warp == 1) {
     // ------------------------------ MMA issuer --------------------------------
-    // (the whole warp runs the loop with the same values; one elected lane issues)
-    {
-      uint32_t s = 0, ph = 0, a = 0, aph = 0;
-      bool ok = true;
-      const uint32_t smem_base = ptx::smem_u32(smem);
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 0, a = 0, aph = 1;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
       // weights: K-major rows of 128 bytes, or (kWKn) the [K, N] tile read as an MN-major operand
-      constexpr uint32_t kWLbo = !kWKn ? 16u : 16384u;
-      constexpr uint32_t kWStep = !kWKn ? 32u : 4096u;   // bytes per 32-wide K step
+      const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kWKn ? 16384u : 16u, 1024);
+      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + 16384, 16, 1024);
+      uint64_t wdesc = wdesc0, adesc = adesc0;
       int my_tiles = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) ++my_tiles;
       const int64_t blocks = (int64_t)my_tiles * p.num_kb;   // every tile: same K loop, no tile state needed
-      for (int64_t i = 0; i < blocks && ok; ++i) {
-        bool go = ptx::mbar_wait(&ctrl->acc_empty[a], aph ^ 1, abort_flag);
-        if (go) go = ptx::mbar_wait(&ctrl->full[s], ph, abort_flag);
-        if (!__all_sync(0xffffffffu, go)) break;
+      for (int64_t i = 0; i < blocks; ++i) {
+        if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) break;
+        if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) break;
         ptx::tc_fence_after();
-        const uint32_t st_addr = smem_base + s * kTStageBytes;
-        const uint64_t wdesc0 = ptx::make_smem_desc(st_addr, kWLbo, 1024);
-        const uint64_t adesc0 = ptx::make_smem_desc(st_addr + 16384, 16, 1024);
-        const uint32_t d_tmem = tmem_base + a * 128;
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          ptx::umma_elect<true>(d_tmem, adesc0 + (uint64_t)((j * 32) >> 4), wdesc0 + (uint64_t)((j * kWStep) >> 4),
-                                p.idesc, j > 0 ? 1u : 0u);
-        ptx::umma_commit_elect(&ctrl->empty[s]);
-        ptx::umma_commit_elect(&ctrl->acc_full[a]);
-        if (++s == (uint32_t)kTStages) { s = 0; ph ^= 1; }
+        ptx::umma_block<true, 2, kWKn ? 4096 / 16 : 2>(tmem_base + a * 128, adesc, wdesc, p.idesc, 0u);
+        ptx::umma_commit(acc_full0 + 8 * a);
+        ptx::umma_commit(empty0 + 8 * s);
+        wdesc += kTStageBytes >> 4;
+        adesc += kTStageBytes >> 4;
+        if (++s == (uint32_t)kTStages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
         if (++a == (uint32_t)kTAcc) { a = 0; aph ^= 1; }
       }
     }
+    __syncwarp();
   } else {
     // ------------------------ promotion and epilogue --------------------------
     const int q = warp & 3;
@@ -199,6 +193,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
     };
     uint32_t a = 0, aph = 0;
+    const uint32_t acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
     int cursor = 0;
     bool ok = true;
     const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
@@ -238,7 +233,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
           ptx::tmem_wait_ld_tied(va, vb);
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&ctrl->acc_empty[a]);   // the stage is in registers
+          if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);   // the stage is in registers
           if (++a == (uint32_t)kTAcc) { a = 0; aph ^= 1; }
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
@@ -301,9 +296,13 @@ constexpr int kT2Threads = 384;
 // for, so the re-balanced total must fit what the CTA got at launch (threads x launch registers)
 constexpr int kT2LaunchRegs = 168, kT2LowRegs = 40, kT2HighRegs = 232;
 static_assert(128 * kT2LowRegs + 256 * kT2HighRegs <= kT2Threads * kT2LaunchRegs, "setmaxnreg budget");
-constexpr int kT2Stages = 4;          // ring of up to 4 stages (192 KB in flight per SM) ...
-constexpr int kT2StagesStaged = 3;    // ... or 3 with the fourth stage's room given to the store tiles
-constexpr int kT2RowPitch = 272;      // bytes per staged output row: 128 16-bit values + 16 (conflict-free 16-byte accesses)
+constexpr int kT2Stages = 4;          // ring: 192 KB in flight per SM
+// Finished rows leave through per-warp staging tiles of 32 rows x 32 values (64 bytes + 16, conflict-free
+// for 16-byte accesses), so that a store instruction writes whole 64-byte pieces of eight rows; straight
+// from the registers it would be 16 bytes of 32 rows (4 us per tile that nothing overlaps).  The tile is
+// that small so that the ring keeps four stages: with three and whole 256-byte rows the MMA thread
+// waited 400 of 1200 cycles per K block for data.
+constexpr int kT2RowPitch = 80;
 constexpr int kT2StageBytes = 49152;   // weights 2 x 16 KB, tokens 16 KB
 constexpr int kT2Acc = 2;
 
@@ -318,14 +317,10 @@ struct T2Ctrl {
   uint64_t xbar[4];        // ... and the barrier of each such pair of warps (one per lane quarter)
   alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
 };
-// store tiles (3-stage form): per epilogue warp its 32 token rows x 128 features in 16 bits
 constexpr size_t kT2XposeBytes = 8 * 32 * kT2RowPitch;
-constexpr size_t kT2Ring = (size_t)kT2Stages * kT2StageBytes;      // the ring's room either way
-constexpr size_t kT2Smem = 1024 + kT2Ring + ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
-static_assert(kT2XposeBytes <= kT2StageBytes + 24 * 1024, "store tiles must fit the fourth stage's room");
-constexpr size_t kT2SmemStaged = 1024 + (size_t)kT2StagesStaged * kT2StageBytes + kT2XposeBytes +
-                                 ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
-static_assert(kT2Smem <= kMaxSmem && kT2SmemStaged <= kMaxSmem, "shared memory");
+constexpr size_t kT2Smem = 1024 + (size_t)kT2Stages * kT2StageBytes + kT2XposeBytes +
+                           ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
+static_assert(kT2Smem <= kMaxSmem, "shared memory");
 
 //
 // kGated (the first grouped GEMM of a SiLU layer with block-scaled fp8 experts): a tile pairs the
@@ -343,9 +338,8 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             const __grid_constant__ CUtensorMap tmap_w, const TParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const uint32_t stages = (uint32_t)p.stages;
-  uint8_t* xpose_base = smem + stages * kT2StageBytes;     // used by the 3-stage form only
-  T2Ctrl* ctrl = reinterpret_cast<T2Ctrl*>(xpose_base + (stages == (uint32_t)kT2Stages ? 0 : kT2XposeBytes));
+  uint8_t* xpose_base = smem + kT2Stages * kT2StageBytes;
+  T2Ctrl* ctrl = reinterpret_cast<T2Ctrl*>(xpose_base + kT2XposeBytes);
   volatile int* abort_flag = &ctrl->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 256-feature tiles; gated: one tile per 128 gate features (p.n_tiles counts 128-feature blocks of n)
@@ -386,73 +380,59 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp < 4) {
     ptx::setmaxnreg_dec<kT2LowRegs>();
-    if (warp == 0 && lane == 0) {
+    const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+    if (warp == 0 && ptx::elect_one()) {
       // ------------------------------ TMA producer ------------------------------
-      uint32_t s = 0, ph = 0;
+      uint32_t s = 0, ph = 1;
       int cursor = 0;
       bool ok = true;
+      const uint32_t st0 = ptx::smem_u32(smem);
+      uint32_t st = st0;
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
         const int n0 = kGated ? ti.n_tile * 128 : ti.n_tile * 256;
         const int n1 = kGated ? (up_block0 + ti.n_tile) * 128 : n0 + 128;
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!ptx::mbar_wait(&ctrl->empty[s], ph ^ 1, abort_flag, true)) { ok = false; break; }
-          uint8_t* wdst = smem + s * kT2StageBytes;
-          ptx::mbar_expect_tx(&ctrl->full[s], kT2StageBytes);
+          const uint32_t full = full0 + 8 * s;
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          ptx::mbar_expect_tx_s(full, kT2StageBytes);
           // two 128-feature blocks (the second one is zero-filled past N)
           if (!kWKn) {
-            ptx::tma_load_3d(wdst, &tmap_w, &ctrl->full[s], kb * 128, n0, ti.e);
-            ptx::tma_load_3d(wdst + 16384, &tmap_w, &ctrl->full[s], kb * 128, n1, ti.e);
+            ptx::tma_load_3d_s(st, &tmap_w, full, kb * 128, n0, ti.e);
+            ptx::tma_load_3d_s(st + 16384, &tmap_w, full, kb * 128, n1, ti.e);
           } else {
-            ptx::tma_load_3d(wdst, &tmap_w, &ctrl->full[s], n0, kb * 128, ti.e);
-            ptx::tma_load_3d(wdst + 16384, &tmap_w, &ctrl->full[s], n1, kb * 128, ti.e);
+            ptx::tma_load_3d_s(st, &tmap_w, full, n0, kb * 128, ti.e);
+            ptx::tma_load_3d_s(st + 16384, &tmap_w, full, n1, kb * 128, ti.e);
           }
-          ptx::tma_load_2d(wdst + 32768, &tmap_a, &ctrl->full[s], kb * 128, ti.row0);
-          if (++s == stages) { s = 0; ph ^= 1; }
+          ptx::tma_load_2d_s(st + 32768, &tmap_a, full, kb * 128, ti.row0);
+          st += kT2StageBytes;
+          if (++s == (uint32_t)kT2Stages) { s = 0; ph ^= 1; st = st0; }
         }
       }
-    } else if (warp == 1) {
+    } else if (warp == 1 && ptx::elect_one()) {
       // ------------------------------ MMA issuer --------------------------------
-      // (the whole warp runs the loop with the same values; one elected lane issues)
-      uint32_t s = 0, ph = 0, a = 0, aph = 0;
-      const uint32_t smem_base = ptx::smem_u32(smem);
-      constexpr uint32_t kWLbo = !kWKn ? 16u : 16384u;
-      constexpr uint32_t kWStep = !kWKn ? 32u : 4096u;
+      // One thread; descriptors advance by additions.
+      uint32_t s = 0, ph = 0, a = 0, aph = 1;
+      const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
+      const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kWKn ? 16384u : 16u, 1024);
+      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + 32768, 16, 1024);
+      uint64_t wdesc = wdesc0, adesc = adesc0;
       int my_tiles = 0;
       for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) ++my_tiles;
-      const int64_t blocks = (int64_t)my_tiles * p.num_kb;
+      const int64_t blocks = (int64_t)my_tiles * p.num_kb;   // every tile: same K loop, no tile state needed
       const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((256u >> 3) << 17);
-      auto mma = [&](uint32_t d, uint64_t ad, uint64_t wd, uint32_t accumulate) {
-        ptx::umma_elect<true>(d, ad, wd, idesc, accumulate);
-      };
-      // The barriers of the next block are polled between this block's MMA issues, where
-      // the thread would otherwise only wait for room in the tensor pipe's queue.
-      bool full_ready = false, acc_ready = false;
       for (int64_t i = 0; i < blocks; ++i) {
-        // (spinning waits here and in the promotion warps: the hand-over of an accumulator stage
-        // is the kernel's critical loop, and a suspended try_wait wakes up late)
-        bool go = true;
-        if (!acc_ready) go = ptx::mbar_wait(&ctrl->acc_empty[a], aph ^ 1, abort_flag, true);
-        if (go && !full_ready) go = ptx::mbar_wait(&ctrl->full[s], ph, abort_flag, true);
-        if (!__all_sync(0xffffffffu, go)) break;
+        if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) break;
+        if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) break;
         ptx::tc_fence_after();
-        const uint32_t st_addr = smem_base + s * kT2StageBytes;
-        const uint64_t wdesc0 = ptx::make_smem_desc(st_addr, kWLbo, 1024);
-        const uint64_t adesc0 = ptx::make_smem_desc(st_addr + 32768, 16, 1024);
-        const uint32_t d_tmem = tmem_base + a * 256;
-        const uint32_t s1 = (s + 1 == stages) ? 0u : s + 1, ph1 = (s1 == 0u) ? ph ^ 1u : ph;
-        const uint32_t a1 = (a + 1 == (uint32_t)kT2Acc) ? 0u : a + 1, aph1 = (a1 == 0u) ? aph ^ 1u : aph;
-        const bool more = i + 1 < blocks;
-        mma(d_tmem, adesc0, wdesc0, 0u);
-        mma(d_tmem, adesc0 + (uint64_t)(32 >> 4), wdesc0 + (uint64_t)(kWStep >> 4), 1u);
-        full_ready = __all_sync(0xffffffffu, more && ptx::mbar_test_wait(&ctrl->full[s1], ph1));
-        mma(d_tmem, adesc0 + (uint64_t)(64 >> 4), wdesc0 + (uint64_t)((2 * kWStep) >> 4), 1u);
-        mma(d_tmem, adesc0 + (uint64_t)(96 >> 4), wdesc0 + (uint64_t)((3 * kWStep) >> 4), 1u);
-        ptx::umma_commit_elect(&ctrl->empty[s]);
-        ptx::umma_commit_elect(&ctrl->acc_full[a]);
-        acc_ready = __all_sync(0xffffffffu, more && ptx::mbar_test_wait(&ctrl->acc_empty[a1], aph1 ^ 1u));
-        s = s1; ph = ph1; a = a1; aph = aph1;
+        ptx::umma_block<true, 2, kWKn ? 4096 / 16 : 2>(tmem_base + a * 256, adesc, wdesc, idesc, 0u);
+        ptx::umma_commit(acc_full0 + 8 * a);
+        ptx::umma_commit(empty0 + 8 * s);
+        wdesc += kT2StageBytes >> 4;
+        adesc += kT2StageBytes >> 4;
+        if (++s == (uint32_t)kT2Stages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
+        if (++a == (uint32_t)kT2Acc) { a = 0; aph ^= 1; }
       }
     }
   } else {
@@ -494,6 +474,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
     };
     uint32_t a = 0, aph = 0, xpar = 0;
+    const uint32_t acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
     int cursor = 0;
     bool ok = true;
     const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
@@ -522,7 +503,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (g * kTGroup + jb >= p.num_kb) break;
           const float sc0 = cur.s0[jb];
           const float sc1 = kGated ? cur.s1[kGated ? jb : 0] : sc0;
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_full[a], aph, abort_flag, true))) {
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_full[a], aph, abort_flag))) {
             *abort_flag = 1; ok = false; break;
           }
           ptx::tc_fence_after();
@@ -538,7 +519,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
             if (pass == 1) {   // the whole stage is in registers
               ptx::tc_fence_before();
               __syncwarp();
-              if (lane == 0) ptx::mbar_arrive(&ctrl->acc_empty[a]);
+              if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);
               if (++a == (uint32_t)kT2Acc) { a = 0; aph ^= 1; }
             }
 #pragma unroll
@@ -589,7 +570,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (ok && r < ti.valid) {
           const float scale = fmaxf(__fdiv_rn(amax, 448.0f), 1.0f / (448.0f * 512.0f));
           // 64 codes of this thread's row into the warp's staging tile (rows of 64 + 16 bytes)
-          const uint32_t my_row = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch) + lane * 80;
+          const uint32_t my_row = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch) + lane * kT2RowPitch;
 #pragma unroll
           for (int c = 0; c < 64; c += 16) {
             uint32_t w[4];
@@ -615,7 +596,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
           for (int it = 0; it < 4; ++it) {
             const int rr = it * 8 + (lane >> 2);
             if (q * 32 + rr < ti.valid)
-              *reinterpret_cast<uint4*>(dbase + (int64_t)rr * half_n) = ptx::lds128(xp + rr * 80 + piece * 16);
+              *reinterpret_cast<uint4*>(dbase + (int64_t)rr * half_n) = ptx::lds128(xp + rr * kT2RowPitch + piece * 16);
           }
         }
         __syncwarp();
@@ -641,35 +622,25 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
             }
           }
         };
-        if (stages == (uint32_t)kT2Stages) {
-          if (r < ti.valid) {
-            uint16_t* drow = reinterpret_cast<uint16_t*>(p.d) + (int64_t)(ti.row0 + r) * p.n + f0;
+        const uint32_t xp = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch);
+        const int piece = lane & 3;
+        uint16_t* dbase = reinterpret_cast<uint16_t*>(p.d) + (int64_t)(ti.row0 + q * 32) * p.n + f0 + piece * 8;
 #pragma unroll
-            for (int c = 0; c < 128; c += 8) {
-              uint32_t w[4];
-              packed(c, w);
-              *reinterpret_cast<uint4*>(drow + c) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
-          }
-        } else {
-          // into the warp's staging tile ...
-          const uint32_t xp = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch);
-          const uint32_t my_row = xp + lane * kT2RowPitch;
+        for (int c0 = 0; c0 < 128; c0 += 32) {
+          // 32 values of this thread's row into the warp's staging tile ...
 #pragma unroll
-          for (int c = 0; c < 128; c += 8) {
+          for (int c = 0; c < 32; c += 8) {
             uint32_t w[4];
-            packed(c, w);
-            ptx::sts128(my_row + c * 2, make_uint4(w[0], w[1], w[2], w[3]));
+            packed(c0 + c, w);
+            ptx::sts128(xp + lane * kT2RowPitch + c * 2, make_uint4(w[0], w[1], w[2], w[3]));
           }
           __syncwarp();
-          // ... and out again two whole rows per store: 16 lanes cover the 256 bytes of a row
-          const int piece = lane & 15;
-          uint16_t* dbase = reinterpret_cast<uint16_t*>(p.d) + (int64_t)(ti.row0 + q * 32) * p.n + f0 + piece * 8;
+          // ... and out again eight rows per store: four lanes cover the 64 bytes of a row
 #pragma unroll
-          for (int it = 0; it < 16; ++it) {
-            const int rr = it * 2 + (lane >> 4);
+          for (int it = 0; it < 4; ++it) {
+            const int rr = it * 8 + (lane >> 2);
             if (q * 32 + rr < ti.valid)
-              *reinterpret_cast<uint4*>(dbase + (int64_t)rr * p.n) = ptx::lds128(xp + rr * kT2RowPitch + piece * 16);
+              *reinterpret_cast<uint4*>(dbase + (int64_t)rr * p.n + c0) = ptx::lds128(xp + rr * kT2RowPitch + piece * 16);
           }
           __syncwarp();
         }
@@ -692,9 +663,8 @@ template <bool kWKn, bool kGated>
 int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, const TParams& p, int grid, cudaStream_t st) {
   auto kern = grouped_gemm_fp8t256_kernel<kWKn, kGated>;
   static SmemConfig configured;
-  const size_t smem = p.stages == kT2Stages ? kT2Smem : kT2SmemStaged;
-  if (int rc = configured.ensure(kern, kT2SmemStaged > kT2Smem ? kT2SmemStaged : kT2Smem)) return rc;
-  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), smem, st, ta, tw, p));
+  if (int rc = configured.ensure(kern, kT2Smem)) return rc;
+  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), kT2Smem, st, ta, tw, p));
   return B200MOE_OK;
 }
 
@@ -742,10 +712,6 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   p.out_f16 = gated ? (a->mid_dtype == B200MOE_F16) : (a->d_dtype == B200MOE_F16);
   p.d_scale = reinterpret_cast<float*>(a->d_scale);
   p.clamp = a->clamp_limit;
-  {
-    const int64_t in_use = (a->rows_hint > 0 && a->rows_hint < a->m) ? a->rows_hint : a->m;
-    p.stages = (gated || in_use / a->num_experts >= 128) ? kT2StagesStaged : kT2Stages;
-  }
   // A operand = tokens (K-major), B operand = weights (K-major, or MN-major for [E,K,N])
   p.idesc = ptx::make_idesc(0u, 0u, 0u, kn ? 1u : 0u, kTTok, kFeat);
 

@@ -26,11 +26,6 @@ __device__ __forceinline__ void fence_barrier_init() {
 __device__ __forceinline__ void fence_proxy_async() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
@@ -50,35 +45,8 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // `kWaitBudgetCycles` clock cycles or until `*abort_flag` becomes non-zero.
 // Returns false (and raises the flag) when it gave up.
 constexpr long long kWaitBudgetCycles = 2000000000LL;  // roughly one second
-__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity,
-                                          volatile int* abort_flag, bool spin = false,
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           long long budget_cycles = kWaitBudgetCycles) {
-  if (spin) {
-    if (mbar_test_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    uint32_t spins = 0;
-    while (!mbar_test_wait(bar, parity)) {
-      if ((++spins & 0xfff) == 0) {
-        if (*abort_flag != 0) return false;
-        if (clock64() - t0 > budget_cycles) {
-          *abort_flag = 1;
-          return false;
-        }
-      }
-    }
-    return true;
-  }
   if (mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
   uint32_t spins = 0;
@@ -126,6 +94,9 @@ static __device__ __noinline__ bool mbar_wait_rest(uint32_t bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_try_wait_s(bar, parity) || mbar_wait_rest(bar, parity, abort_flag);
 }
+__device__ __forceinline__ void mbar_arrive_s(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -165,26 +136,7 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity,
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(m)) : "memory");
 }
-__device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int c0, int c1) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0),
-      "r"(c1)
-      : "memory");
-}
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c0),
-      "r"(c1), "r"(c2)
-      : "memory");
-}
-
-// The same with 32-bit shared addresses.
+// (Destination and barrier are 32-bit shared addresses.)
 __device__ __forceinline__ void tma_load_2d_s(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
@@ -284,20 +236,20 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t cluster_addr, float a, fl
 }
 // Tiled loads of a CTA pair: the data lands in the issuing CTA's shared memory, the bytes
 // are counted on `bar_cluster_addr`, which may be the other CTA's barrier.
-__device__ __forceinline__ void tma_load_2d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
                                                  int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1)
       : "memory");
 }
-__device__ __forceinline__ void tma_load_3d_pair(void* dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
+__device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
                                                  int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
+      ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
 
@@ -488,56 +440,58 @@ __device__ __forceinline__ void umma_mx_block(uint32_t tmem_d, uint64_t wdesc, u
 #undef B200_MX_MMA4
 #undef B200_MX_HEAD
 }
+// The four K = 32-byte instructions of one 128-byte-wide K block, issued by one thread (elect_one):
+// both descriptors advance by an addition, only the first instruction may overwrite D.  kAStep and
+// kBStep: 16-byte units between the K steps of the two operands.
+template <bool kFp8, int kAStep, int kBStep>
+__device__ __forceinline__ void umma_block(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                           uint32_t accumulate) {
+#define B200_UMMA4(KIND)                                                                                \
+  asm volatile(                                                                                          \
+      "{\n\t.reg .pred pa;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\tsetp.ne.b32 pa, %4, 0;\n\t"                \
+      "add.u64 a1, %1, %5;\n\tadd.u64 a2, %1, %6;\n\tadd.u64 a3, %1, %7;\n\t"                            \
+      "add.u64 b1, %2, %8;\n\tadd.u64 b2, %2, %9;\n\tadd.u64 b3, %2, %10;\n\t"                           \
+      "tcgen05.mma.cta_group::1.kind::" KIND " [%0], %1, %2, %3, pa;\n\t"                                \
+      "tcgen05.mma.cta_group::1.kind::" KIND " [%0], a1, b1, %3, 1;\n\t"                                 \
+      "tcgen05.mma.cta_group::1.kind::" KIND " [%0], a2, b2, %3, 1;\n\t"                                 \
+      "tcgen05.mma.cta_group::1.kind::" KIND " [%0], a3, b3, %3, 1;\n\t}"                                \
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(kAStep), "n"(2 * kAStep),  \
+        "n"(3 * kAStep), "n"(kBStep), "n"(2 * kBStep), "n"(3 * kBStep)                                    \
+      : "memory")
+  if (kFp8) B200_UMMA4("f8f6f4");
+  else B200_UMMA4("f16");
+#undef B200_UMMA4
+}
 // A commit makes the barrier receive one arrival when all tcgen05 operations issued so far by this
 // thread have completed.
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-// tcgen05.mma and tcgen05.commit for a warp that runs the issue loop convergently (all lanes
-// hold the same operands): one elected lane issues.
-template <bool kFp8>
-__device__ __forceinline__ void umma_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                           uint32_t idesc, uint32_t accumulate) {
-  if (kFp8) {
-    asm volatile(
-        "{\n\t.reg .pred pe, pa;\n\telect.sync _|pe, 0xffffffff;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
-        "@pe tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, pa;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  } else {
-    asm volatile(
-        "{\n\t.reg .pred pe, pa;\n\telect.sync _|pe, 0xffffffff;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
-        "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, pa;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-  }
-}
-__device__ __forceinline__ void umma_commit_elect(uint64_t* bar) {
+// kind::f16 issued by the even CTA of a pair for both: M = 256 (128 rows of A and of D per CTA), each
+// CTA holds N / 2 rows of B at the same shared-memory offsets, D at the same tensor-memory address in
+// both.  One K block as in umma_block.
+template <int kAStep, int kBStep>
+__device__ __forceinline__ void umma_f16_pair_block(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                                    uint32_t accumulate) {
   asm volatile(
-      "{\n\t.reg .pred pe;\n\telect.sync _|pe, 0xffffffff;\n\t"
-      "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
-      ::"r"(smem_u32(bar))
-      : "memory");
-}
-
-// kind::f16 issued by the even CTA of a pair for both (warp-uniform loop, one elected lane):
-// M = 256 (128 rows of A and of D per CTA), each CTA holds N / 2 rows of B at the same
-// shared-memory offsets, D at the same tensor-memory address in both.
-__device__ __forceinline__ void umma_f16_pair_elect(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc,
-                                                    uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred pe, pa;\n\telect.sync _|pe, 0xffffffff;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
-      "@pe tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, pa;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      "{\n\t.reg .pred pa;\n\t.reg .b64 a1, a2, a3, b1, b2, b3;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
+      "add.u64 a1, %1, %5;\n\tadd.u64 a2, %1, %6;\n\tadd.u64 a3, %1, %7;\n\t"
+      "add.u64 b1, %2, %8;\n\tadd.u64 b2, %2, %9;\n\tadd.u64 b3, %2, %10;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, pa;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a1, b1, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a2, b2, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], a3, b3, %3, 1;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "n"(kAStep), "n"(2 * kAStep),
+        "n"(3 * kAStep), "n"(kBStep), "n"(2 * kBStep), "n"(3 * kBStep)
       : "memory");
 }
 // One arrival on the barrier at `bar`'s offset in both CTAs of the pair once the pair's MMAs
 // issued so far have completed.
-__device__ __forceinline__ void umma_commit_pair_elect(uint64_t* bar) {
+__device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
   asm volatile(
-      "{\n\t.reg .pred pe;\n\t.reg .b16 m;\n\telect.sync _|pe, 0xffffffff;\n\tmov.b16 m, 3;\n\t"
-      "@pe tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
-      ::"r"(smem_u32(bar))
+      "{\n\t.reg .b16 m;\n\tmov.b16 m, 3;\n\t"
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], m;\n\t}"
+      ::"r"(bar)
       : "memory");
 }
 
