@@ -42,90 +42,59 @@ struct RowJob {
   int planes;            // mx: 1 or 2
 };
 
-__device__ __forceinline__ void copy_row(const RowJob& a, int64_t tok, const int* dest) {
-  const uint8_t* s = reinterpret_cast<const uint8_t*>(a.src) + tok * (int64_t)a.row_bytes;
-  uint8_t* dst = reinterpret_cast<uint8_t*>(a.dst);
-  const int nvec = a.row_bytes >> 4;
-  for (int j = threadIdx.x; j < nvec; j += blockDim.x) {
-    const vec16 v = ld16(s + (int64_t)j * 16);
-    for (int k = 0; k < a.K; ++k) {
-      const int r = dest[k];
-      if (r >= 0) st16(dst + (int64_t)r * a.row_bytes + (int64_t)j * 16, v);
-    }
-  }
-  if (a.src_s != nullptr) {
-    const uint8_t* ss = reinterpret_cast<const uint8_t*>(a.src_s) + tok * (int64_t)a.scale_row_bytes;
-    uint8_t* dst_s = reinterpret_cast<uint8_t*>(a.dst_s);
-    if ((a.scale_row_bytes & 3) == 0) {
-      for (int j = threadIdx.x; j < (a.scale_row_bytes >> 2); j += blockDim.x) {
-        const uint32_t v = reinterpret_cast<const uint32_t*>(ss)[j];
-        for (int k = 0; k < a.K; ++k) {
-          const int r = dest[k];
-          if (r >= 0) reinterpret_cast<uint32_t*>(dst_s + (int64_t)r * a.scale_row_bytes)[j] = v;
-        }
+__device__ __forceinline__ void copy_scales(const RowJob& a, int64_t tok, const int* dest) {
+  if (a.src_s == nullptr) return;
+  const uint8_t* ss = reinterpret_cast<const uint8_t*>(a.src_s) + tok * (int64_t)a.scale_row_bytes;
+  uint8_t* dst_s = reinterpret_cast<uint8_t*>(a.dst_s);
+  if ((a.scale_row_bytes & 3) == 0) {
+    for (int j = threadIdx.x; j < (a.scale_row_bytes >> 2); j += blockDim.x) {
+      const uint32_t v = reinterpret_cast<const uint32_t*>(ss)[j];
+      for (int k = 0; k < a.K; ++k) {
+        const int r = dest[k];
+        if (r >= 0) reinterpret_cast<uint32_t*>(dst_s + (int64_t)r * a.scale_row_bytes)[j] = v;
       }
-    } else {
-      for (int j = threadIdx.x; j < a.scale_row_bytes; j += blockDim.x) {
-        const uint8_t v = ss[j];
-        for (int k = 0; k < a.K; ++k) {
-          const int r = dest[k];
-          if (r >= 0) dst_s[(int64_t)r * a.scale_row_bytes + j] = v;
-        }
+    }
+  } else {
+    for (int j = threadIdx.x; j < a.scale_row_bytes; j += blockDim.x) {
+      const uint8_t v = ss[j];
+      for (int k = 0; k < a.K; ++k) {
+        const int r = dest[k];
+        if (r >= 0) dst_s[(int64_t)r * a.scale_row_bytes + j] = v;
       }
     }
   }
 }
 
-// Per-1x128 dynamic e4m3 quantisation.  A lane holds 8 consecutive elements, 16 lanes
-// cover one 128-wide group.
+// Per-1x128 dynamic e4m3 quantisation of piece j.  A lane holds 8 consecutive elements, 16 lanes
+// cover one 128-wide group; all lanes of the warp call it.
 template <typename T>
-__device__ __forceinline__ void quant_row_fp8(const RowJob& a, int64_t tok, const int* dest) {
+__device__ __forceinline__ void quant_piece_fp8(const RowJob& a, int j, bool in, const vec16& v, const int* dest) {
   const int H = a.H;
-  const T* s = reinterpret_cast<const T*>(a.src) + tok * (int64_t)H;
+  const T* e = reinterpret_cast<const T*>(&v);
+  float x[8];
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) { x[i] = in ? to_f32<T>(e[i]) : 0.f; amax = fmaxf(amax, fabsf(x[i])); }
+#pragma unroll
+  for (int mask = 8; mask > 0; mask >>= 1)
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, mask));
+  amax = fmaxf(amax, 1e-10f);
+  const float scale = fmaxf(__fdiv_rn(amax, 448.f), 1.0f / (448.f * 512.f));
+  const float inv = __fdiv_rn(1.0f, scale);
+  if (!in) return;
+  uint32_t c[2] = {0u, 0u};
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float q = fminf(fmaxf(__fmul_rn(x[i], inv), -448.f), 448.f);
+    c[i >> 2] |= (uint32_t)f32_to_e4m3(q) << (8 * (i & 3));
+  }
   uint8_t* dst_q = reinterpret_cast<uint8_t*>(a.dst);
   float* dst_s = reinterpret_cast<float*>(a.dst_s);
-  const int groups = H / 128;
-  const int nvec = H / 8;
-  // Full warps iterate together so the 16-lane shuffles stay converged.
-  for (int j0 = (threadIdx.x & ~31); j0 < nvec; j0 += blockDim.x) {
-    const int j = j0 + (threadIdx.x & 31);
-    float x[8];
-    float amax = 0.f;
-    if (j < nvec) {
-      const vec16 v = ld16(s + (int64_t)j * 8);
-      const T* e = reinterpret_cast<const T*>(&v);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) { x[i] = to_f32<T>(e[i]); amax = fmaxf(amax, fabsf(x[i])); }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) x[i] = 0.f;
-    }
-#pragma unroll
-    for (int mask = 8; mask > 0; mask >>= 1)
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, mask));
-    amax = fmaxf(amax, 1e-10f);
-    const float scale = fmaxf(__fdiv_rn(amax, 448.f), 1.0f / (448.f * 512.f));
-    const float inv = __fdiv_rn(1.0f, scale);
-    if (j < nvec) {
-      uint32_t lo = 0, hi = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float q = fminf(fmaxf(__fmul_rn(x[i], inv), -448.f), 448.f);
-        lo |= (uint32_t)f32_to_e4m3(q) << (8 * i);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float q = fminf(fmaxf(__fmul_rn(x[4 + i], inv), -448.f), 448.f);
-        hi |= (uint32_t)f32_to_e4m3(q) << (8 * i);
-      }
-      const int g = j / 16;
-      for (int k = 0; k < a.K; ++k) {
-        const int r = dest[k];
-        if (r >= 0) {
-          *reinterpret_cast<uint2*>(dst_q + (int64_t)r * H + (int64_t)j * 8) = make_uint2(lo, hi);
-          if ((j & 15) == 0) dst_s[(int64_t)r * groups + g] = scale;
-        }
-      }
+  for (int k = 0; k < a.K; ++k) {
+    const int r = dest[k];
+    if (r >= 0) {
+      *reinterpret_cast<uint2*>(dst_q + (int64_t)r * H + (int64_t)j * 8) = make_uint2(c[0], c[1]);
+      if ((j & 15) == 0) dst_s[(int64_t)r * (H / 128) + j / 16] = scale;
     }
   }
 }
@@ -133,43 +102,57 @@ __device__ __forceinline__ void quant_row_fp8(const RowJob& a, int64_t tok, cons
 // MXFP8 planes (mx_quant.cuh); sixteen lanes cover a 128-wide K block, whose first lane writes its
 // scale word.
 template <typename T>
-__device__ __forceinline__ void quant_row_mx(const RowJob& a, int64_t tok, const int* dest) {
-  const int H = a.H;
-  const T* s = reinterpret_cast<const T*>(a.src) + tok * (int64_t)H;
+__device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, const vec16& x, const int* dest) {
+  const int H = a.H, num_kb = (H + 127) / 128;
+  const T* e = reinterpret_cast<const T*>(&x);
   uint8_t* dst_q = reinterpret_cast<uint8_t*>(a.dst);
   uint32_t* dst_s = reinterpret_cast<uint32_t*>(a.dst_s);
-  const int nvec = H / 8, num_kb = (H + 127) / 128;
-  for (int j0 = (threadIdx.x & ~31); j0 < num_kb * 16; j0 += blockDim.x) {
-    const int j = j0 + (threadIdx.x & 31);
-    float v[8];
+  float v[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = 0.f;
-    if (j < nvec) {
-      const vec16 in = ld16(s + (int64_t)j * 8);
-      const T* e = reinterpret_cast<const T*>(&in);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = to_f32<T>(e[i]);
-    }
-    for (int p = 0; p < a.planes; ++p) {
-      uint2 codes;
-      const uint32_t word = mx_quant_lane(v, j < nvec, codes);
-      for (int k = 0; k < a.K; ++k) {
-        const int r = dest[k];
-        if (r >= 0) {
-          if (j < nvec) *reinterpret_cast<uint2*>(dst_q + (p * a.rows + r) * H + (int64_t)j * 8) = codes;
-          if ((j & 15) == 0 && j < num_kb * 16) dst_s[((int64_t)p * num_kb + (j >> 4)) * a.rows + r] = word;
-        }
+  for (int i = 0; i < 8; ++i) v[i] = in ? to_f32<T>(e[i]) : 0.f;
+#pragma unroll 1
+  for (int p = 0; p < a.planes; ++p) {
+    uint2 codes;
+    const uint32_t word = mx_quant_lane(v, in, codes);
+    for (int k = 0; k < a.K; ++k) {
+      const int r = dest[k];
+      if (r >= 0) {
+        if (in) *reinterpret_cast<uint2*>(dst_q + (p * a.rows + r) * H + (int64_t)j * 8) = codes;
+        if ((j & 15) == 0 && j < num_kb * 16) dst_s[((int64_t)p * num_kb + (j >> 4)) * a.rows + r] = word;
       }
     }
   }
 }
 
 enum RowForm { kRowCopy = 0, kRowFp8 = 1, kRowMx = 2 };
+// Piece j (16 bytes of the source row; `v` is read only for j < nvec) to its destinations.
+template <typename T, int kForm>
+__device__ __forceinline__ void place_piece(const RowJob& a, int j, int nvec, const vec16& v, const int* dest) {
+  if (kForm == kRowCopy) {
+    if (j >= nvec) return;
+    for (int k = 0; k < a.K; ++k) {
+      const int r = dest[k];
+      if (r >= 0) st16(reinterpret_cast<uint8_t*>(a.dst) + (int64_t)r * a.row_bytes + (int64_t)j * 16, v);
+    }
+  } else if (kForm == kRowFp8) {
+    quant_piece_fp8<T>(a, j, j < nvec, v, dest);
+  } else {
+    quant_piece_mx<T>(a, j, j < nvec, v, dest);
+  }
+}
 template <typename T, int kForm>
 __device__ __forceinline__ void place_row(const RowJob& a, int64_t tok, const int* dest) {
-  if (kForm == kRowCopy) copy_row(a, tok, dest);
-  else if (kForm == kRowFp8) quant_row_fp8<T>(a, tok, dest);
-  else quant_row_mx<T>(a, tok, dest);
+  const int nvec = kForm == kRowCopy ? a.row_bytes >> 4 : a.H / 8;
+  const int steps = kForm == kRowMx ? ((a.H + 127) / 128) * 16 : nvec;
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src) + tok * (int64_t)nvec * 16;
+  // full warps iterate together so that the shuffles stay converged
+  for (int j0 = (threadIdx.x & ~31); j0 < steps; j0 += blockDim.x) {
+    const int j = j0 + (threadIdx.x & 31);
+    vec16 v;
+    if (j < nvec) v = ld16(src + (int64_t)j * 16);
+    place_piece<T, kForm>(a, j, nvec, v, dest);
+  }
+  if (kForm == kRowCopy) copy_scales(a, tok, dest);
 }
 
 template <typename T, int kForm>
@@ -189,44 +172,58 @@ remap_rows_kernel(const RowJob a, const int32_t* __restrict__ row_map) {
 // plus the number of earlier slots with the same one, counted over all slots by the block's threads
 // (2048 slots x 8 are 64 comparisons a thread).  One more block counts the rows per expert.  The
 // separate sort, a single block that everything waited for, took 6 to 10 us of a decode step and
-// its launch; this form takes 3 us.  K up to kSmallK, else the sort.
+// its launch.  K up to kSmallK, else the sort.
+//
+// What remains is latency: the row's loads are issued before the counting, and the code is kept
+// small (a kernel that runs for 3 us runs from a cold instruction cache).
 constexpr int kSmallK = 8;
-template <typename T, int kForm>
+constexpr int kSmallPre = 4;   // 16-byte pieces of the row a thread holds while the positions are counted
+template <typename T, int kForm, typename Id>
 __global__ void __launch_bounds__(256)
-remap_small_kernel(const SortParams p, const RowJob a, int32_t* __restrict__ rows_per_expert,
-                   int32_t* __restrict__ row_map) {
-  __shared__ int dest[32];
+remap_small_kernel(const Id* __restrict__ ids, const int32_t* __restrict__ map, int numel, int id_limit, int n_buckets,
+                   const RowJob a, int32_t* __restrict__ rows_per_expert, int32_t* __restrict__ row_map) {
+  __shared__ int dest[kSmallK];
   __shared__ uint32_t part[8][kSmallK / 2];
   __shared__ int hist[kMaxBuckets];
   pdl_trigger();
   pdl_wait();
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const int numel = (int)p.numel, K = a.K;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, K = a.K;
+  auto bucket = [&](int i) {
+    const Id e = ids[i];
+    if (e < (Id)0 || e >= (Id)id_limit) return -1;
+    const int b = map != nullptr ? map[e] : (int)e;
+    return b < n_buckets ? b : -1;   // (a negative entry of the map stays negative)
+  };
   if (blockIdx.x == gridDim.x - 1) {
-    for (int e = t; e < p.n_buckets; e += 256) hist[e] = 0;
+    for (int e = t; e < n_buckets; e += 256) hist[e] = 0;
     __syncthreads();
     for (int i = t; i < numel; i += 256) {
-      const int b = bucket_of(p, i);
+      const int b = bucket(i);
       if (b >= 0) atomicAdd(&hist[b], 1);
     }
     __syncthreads();
-    for (int e = t; e < p.n_buckets; e += 256) rows_per_expert[e] = hist[e];
+    for (int e = t; e < n_buckets; e += 256) rows_per_expert[e] = hist[e];
     return;
   }
   const int64_t tok = blockIdx.x;
   const int slot0 = (int)tok * K;
+  // (the quantised forms walk whole 128-value groups)
+  const int nvec = kForm == kRowCopy ? a.row_bytes >> 4 : a.H / 8;
+  const uint8_t* src = reinterpret_cast<const uint8_t*>(a.src) + tok * (int64_t)nvec * 16;
+  vec16 pre[kSmallPre];
+#pragma unroll
+  for (int i = 0; i < kSmallPre; ++i)
+    if (t + 256 * i < nvec) pre[i] = ld16(src + (int64_t)(t + 256 * i) * 16);
   int own[kSmallK];
 #pragma unroll
-  for (int k = 0; k < kSmallK; ++k) own[k] = k < K ? bucket_of(p, slot0 + k) : -1;
-  uint32_t cnt[kSmallK / 2];   // two 16-bit counters a word
-#pragma unroll
-  for (int k = 0; k < kSmallK / 2; ++k) cnt[k] = 0;
+  for (int k = 0; k < kSmallK; ++k) own[k] = k < K ? bucket(slot0 + k) : -1;
+  uint32_t cnt[kSmallK / 2] = {};   // two 16-bit counters a word
+#pragma unroll 1
   for (int i = t; i < numel; i += 256) {
-    const int b = bucket_of(p, i);
-    if (b < 0) continue;
+    const int b = bucket(i);
 #pragma unroll
     for (int k = 0; k < kSmallK; ++k)
-      if (b < own[k] || (b == own[k] && i < slot0 + k)) cnt[k >> 1] += 1u << (16 * (k & 1));
+      if (b >= 0 && (b < own[k] || (b == own[k] && i < slot0 + k))) cnt[k >> 1] += 1u << (16 * (k & 1));
   }
 #pragma unroll
   for (int k = 0; k < kSmallK / 2; ++k) {
@@ -238,12 +235,20 @@ remap_small_kernel(const SortParams p, const RowJob a, int32_t* __restrict__ row
     uint32_t sum = 0;
 #pragma unroll
     for (int w = 0; w < 8; ++w) sum += part[w][t >> 1];
-    const int pos = bucket_of(p, slot0 + t) < 0 ? -1 : (int)((sum >> (16 * (t & 1))) & 0xffffu);
+    const int pos = bucket(slot0 + t) < 0 ? -1 : (int)((sum >> (16 * (t & 1))) & 0xffffu);
     dest[t] = pos;
     row_map[slot0 + t] = pos;
   }
   __syncthreads();
-  place_row<T, kForm>(a, tok, dest);
+  const int steps = kForm == kRowMx ? ((a.H + 127) / 128) * 16 : nvec;
+  if (steps <= 256 * kSmallPre) {
+#pragma unroll
+    for (int i = 0; i < kSmallPre; ++i)
+      if ((t & ~31) + 256 * i < steps) place_piece<T, kForm>(a, t + 256 * i, nvec, pre[i], dest);
+    if (kForm == kRowCopy) copy_scales(a, tok, dest);
+  } else {
+    place_row<T, kForm>(a, tok, dest);
+  }
 }
 
 __global__ void init_expert_map_kernel(int32_t* map, int n_local, int ep_rank, int total) {
@@ -284,8 +289,15 @@ int remap_rows(const SortParams& p, const RowJob& job, int32_t* rows_per_expert,
                void* workspace, size_t workspace_bytes, cudaStream_t st) {
   const bool early = p.numel <= kEarlyLaunchRows;
   if (p.numel > 0 && p.numel <= kBlockSlots && job.K <= kSmallK) {
-    B200_LAUNCHED("remap_small_kernel", launch_pdl(early, remap_small_kernel<T, kForm>, dim3((unsigned)num_rows + 1),
-                                                   dim3(256), 0, st, p, job, rows_per_expert, row_map));
+    const dim3 grid((unsigned)num_rows + 1);
+#define B200_REMAP_SMALL(ID)                                                                                          \
+  B200_LAUNCHED("remap_small_kernel", launch_pdl(early, remap_small_kernel<T, kForm, ID>, grid, dim3(256), 0, st,     \
+                                                 (const ID*)p.ids, p.map, (int)p.numel, p.id_limit, p.n_buckets, job, \
+                                                 rows_per_expert, row_map))
+    if (p.ids_dtype == B200MOE_I64) B200_REMAP_SMALL(int64_t);
+    else if (p.ids_dtype == B200MOE_U32) B200_REMAP_SMALL(uint32_t);
+    else B200_REMAP_SMALL(int32_t);
+#undef B200_REMAP_SMALL
     return B200MOE_OK;
   }
   AlignOut ao = {};
