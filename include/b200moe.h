@@ -35,7 +35,8 @@ typedef enum {
   B200MOE_FP4X2 = 8, /* float4_e2m1fn_x2: two e2m1 codes per byte, low nibble first */
   B200MOE_FP8_E4M3_X2 = 9, /* two float8_e4m3fn planes [2][rows][cols]: value =
                               plane 0 + plane 1 (MXFP8 activations + residual) */
-  B200MOE_I8 = 10 /* int8 */
+  B200MOE_I8 = 10, /* int8 */
+  B200MOE_FP8_E4M3_X3 = 11 /* three planes: a float16 exactly (int4 weights only) */
 } b200moe_dtype;
 
 /* Status codes. */
@@ -295,9 +296,11 @@ int b200moe_remap_quant_fp8(const void* hidden, b200moe_dtype dtype,
                             void* workspace, size_t workspace_bytes,
                             b200moe_stream stream);
 /* The same with MXFP8 planes (b200moe_quant_mxfp8) instead of fp8: codes
- * [planes][T*K,H], scale words [planes][ceil(H/128)][T*K]. */
+ * [planes][T*K,H], scale words [planes][ceil(H/128)][T*K]; with block_sums
+ * fp32 sums [ceil(H/128)][T*K] follow the words. */
 int b200moe_remap_quant_mxfp8(const void* hidden, b200moe_dtype dtype,
                               void* remapped_q, void* remapped_scales, int planes,
+                              int block_sums,
                               const int32_t* expert_map,
                               int32_t* rows_per_expert, int32_t* row_map,
                               const void* topk_ids, b200moe_dtype ids_dtype,
@@ -341,7 +344,7 @@ typedef struct {
   b200moe_dtype a_dtype;  /* BF16, F16, or FP8_E4M3 (with a_scale)                */
   const void* a_scale;    /* fp8 activations: block-fp8 weights: fp32 [M,K/128];
                              MXFP4 weights (MXFP8 activations, a_dtype FP8_E4M3
-                             or FP8_E4M3_X2): e8m0 bytes as 32-bit words
+                             or FP8_E4M3_X2, _X3): e8m0 bytes as 32-bit words
                              [planes][ceil(K/128)][M], the output of
                              b200moe_quant_mxfp8; else NULL                  */
   const void* w;          /* weights, layout per w_format                         */
@@ -514,6 +517,13 @@ int b200moe_silu_and_mul_quant(void* out, const void* in, b200moe_dtype dtype,
 int b200moe_quant_mxfp8(const void* x, b200moe_dtype dtype, void* q, void* s,
                         int64_t rows, int cols, int terms,
                         b200moe_stream stream);
+/* The same with up to three planes and, behind the scale words, fp32 sums
+ * [ceil(cols/128)][rows] of every 128-wide block (of what the planes hold): the
+ * activations of an int4 grouped GEMM.  With `gated` x is [rows, 2 * cols] and
+ * the values are silu(gate) * up as b200moe_silu_and_mul rounds them. */
+int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* q, void* s,
+                           int64_t rows, int cols, int terms, int block_sums,
+                           int gated, b200moe_stream stream);
 
 /* Replaces `moe_gather` (csrc/moe/moe_gather.cpp:161-204; schema
  * csrc/moe/torch_bindings.cpp:78-82).

@@ -1,0 +1,37 @@
+"""INT4 layers on the two kernels that take them, against the CPU oracle: the block-scaled one (few rows
+per expert, scales per 128 and 256 elements, two and three activation planes) and the one that expands
+the weights into tensor memory (more rows, or finer scales).  Token tiles and their remainders, several
+tiles per CTA, K down to half a block, feature tiles cut off by N."""
+import pytest
+import torch
+
+from gpu_utils import DEV
+from oracle import torch_oracle as to
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,H,I,group", [(1, 128, 128, 128), (9, 256, 384, 128), (33, 640, 256, 128), (70, 512, 512, 256),
+                                         (150, 256, 256, 256), (401, 384, 128, 128),
+                                         (3, 192, 320, 64), (70, 128, 192, 32), (640, 64, 2560, 64),
+                                         (900, 192, 1536, 64), (1100, 640, 768, 128)])
+def test_layer_int4(native, dtype, T, H, I, group):
+    E, K = 4, 2
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, H, generator=g).to(dtype)
+    w13 = torch.randint(0, 256, (E, 2 * I, H // 2), generator=g, dtype=torch.int32).to(torch.uint8)
+    w2 = torch.randint(0, 256, (E, H, I // 2), generator=g, dtype=torch.int32).to(torch.uint8)
+    s13 = (torch.rand(E, 2 * I, H // group, generator=g) * 0.4 + 0.1).mul(H ** -0.5).to(dtype)
+    s2 = (torch.rand(E, H, I // group, generator=g) * 0.4 + 0.1).mul(I ** -0.5).to(dtype)
+    b13 = torch.randn(E, 2 * I, generator=g).to(dtype)
+    b2 = torch.randn(E, H, generator=g).to(dtype)
+    tw, ids = torch.topk(torch.softmax(torch.randn(T, E, generator=g), -1), k=K, dim=-1)
+    ref = to.fused_moe_bf16(x, to.dequant_int4(w13, s13, group), b13, to.dequant_int4(w2, s2, group), b2, tw, ids.int(), E)
+    mv = lambda t: t.to(DEV)
+    layer = native.XpuFusedMoe(mv(w13), mv(s13), mv(b13), mv(w2), mv(s2), mv(b2), K, "silu", E)
+    out = torch.empty_like(x, device=DEV)
+    layer.apply(out, mv(x), mv(tw), mv(ids.int()))
+    torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=2e-2, atol=2e-2 * float(ref.float().abs().max()))
+    err = (out.cpu().float() - ref.float()).norm() / ref.float().norm()
+    assert err < (1e-2 if dtype == torch.bfloat16 else 2e-3), err

@@ -10,6 +10,8 @@
 #include "common.cuh"
 #include "mx_quant.cuh"
 
+#include <type_traits>
+
 namespace b200moe {
 namespace {
 
@@ -236,10 +238,10 @@ group_quant_fp8_scalar_kernel(const T* __restrict__ x, uint8_t* __restrict__ q,
 // (one block per row with a division per group and a byte store per scale ran at 1.9 TB/s:
 // 8192 x 2880 values in 50 us).
 constexpr int kMxQuantUnroll = 2;
-template <typename T>
+template <typename T, bool kGated>
 __global__ void __launch_bounds__(256)
 quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* __restrict__ s,
-                   int64_t rows, int cols, int terms) {
+                   int64_t rows, int cols, int terms, int sums) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
@@ -251,23 +253,41 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
   for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < total; w += (int64_t)gridDim.x * 8) {
     const int64_t r = w / steps;
     const int j0 = (int)(w - r * steps) * kMxQuantUnroll * 32 + lane;
-    const T* xr = x + r * (int64_t)cols;
-    vec16 in[kMxQuantUnroll];
+    const T* xr = x + r * (int64_t)cols * (kGated ? 2 : 1);
+    vec16 in[kMxQuantUnroll], up[kGated ? kMxQuantUnroll : 1];
 #pragma unroll
-    for (int u = 0; u < kMxQuantUnroll; ++u)
-      if (j0 + 32 * u < nvec) in[u] = ld16(xr + (int64_t)(j0 + 32 * u) * 8);
+    for (int u = 0; u < kMxQuantUnroll; ++u) {
+      if (j0 + 32 * u < nvec) {
+        in[u] = ld16(xr + (int64_t)(j0 + 32 * u) * 8);
+        if (kGated) up[kGated ? u : 0] = ld16(xr + cols + (int64_t)(j0 + 32 * u) * 8);
+      }
+    }
 #pragma unroll
     for (int u = 0; u < kMxQuantUnroll; ++u) {
       const int j = j0 + 32 * u;
       const T* e = reinterpret_cast<const T*>(&in[u]);
+      const T* ue = reinterpret_cast<const T*>(&up[kGated ? u : 0]);
       float v[8];
+      float total = 0.f;
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] = j < nvec ? to_f32<T>(e[i]) : 0.f;
+      for (int i = 0; i < 8; ++i) {
+        v[i] = j < nvec ? to_f32<T>(e[i]) : 0.f;
+        if (kGated && j < nvec)   // the two roundings of silu_and_mul
+          v[i] = to_f32<T>(from_f32<T>(to_f32<T>(from_f32<T>(silu_f32(v[i]))) * to_f32<T>(ue[i])));
+        total += v[i];
+      }
       for (int term = 0; term < terms; ++term) {
         uint2 codes;
         const uint32_t word = mx_quant_lane(v, j < nvec, codes);
         if (j < nvec) *reinterpret_cast<uint2*>(q + (term * rows + r) * cols + (int64_t)j * 8) = codes;
         if ((j & 15) == 0 && j < num_kb * 16) s[((int64_t)term * num_kb + (j >> 4)) * rows + r] = word;
+      }
+      if (sums) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) total -= v[i];
+        total = mx_block_sum(total);
+        if ((j & 15) == 0 && j < num_kb * 16)
+          reinterpret_cast<float*>(s)[((int64_t)terms * num_kb + (j >> 4)) * rows + r] = total;
       }
     }
   }
@@ -464,27 +484,34 @@ extern "C" int b200moe_moe_sum(void* out, const void* in, b200moe_dtype dtype, i
   return B200MOE_OK;
 }
 
-extern "C" int b200moe_quant_mxfp8(const void* x, b200moe_dtype dtype, void* q, void* s, int64_t rows,
-                                   int cols, int terms, b200moe_stream stream) {
+extern "C" int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* q, void* s, int64_t rows, int cols,
+                                      int terms, int block_sums, int gated, b200moe_stream stream) {
   B200_CHECK_ARG(dtype == B200MOE_BF16 || dtype == B200MOE_F16, "quant_mxfp8: input must be bfloat16 or float16");
   B200_CHECK_ARG(rows >= 0 && cols >= 0 && cols % 32 == 0, "quant_mxfp8: the row length must be a multiple of 32");
-  B200_CHECK_ARG(terms == 1 || terms == 2, "quant_mxfp8: terms must be 1 or 2");
+  B200_CHECK_ARG(terms >= 1 && terms <= 3, "quant_mxfp8: terms must be 1, 2 or 3");
   if (rows == 0 || cols == 0) return B200MOE_OK;
   B200_CHECK_ARG(x && q && s, "quant_mxfp8: null pointer");
-  B200_CHECK_ARG(aligned16(x) && (((uintptr_t)q & 7) == 0), "quant_mxfp8: buffers must be 16-byte aligned");
+  B200_CHECK_ARG(aligned16(x) && (((uintptr_t)q & 7) == 0) && (((uintptr_t)s & 3) == 0),
+                 "quant_mxfp8: buffers must be 16-byte aligned");
   const int64_t steps = ((cols + 255) / 256 + kMxQuantUnroll - 1) / kMxQuantUnroll;
   const int64_t blocks = (rows * steps + 7) / 8;
   const dim3 grid((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8));
-  const bool early = rows <= kEarlyLaunchRows;
+  auto run = [&](auto type, auto is_gated) {
+    using T = decltype(type);
+    return launch_pdl(rows <= kEarlyLaunchRows, quant_mxfp8_kernel<T, decltype(is_gated)::value>, grid, dim3(256), 0,
+                      as_stream(stream), (const T*)x, (uint8_t*)q, (uint32_t*)s, rows, cols, terms, block_sums);
+  };
   if (dtype == B200MOE_BF16)
-    B200_LAUNCHED("quant_mxfp8_kernel",
-                  launch_pdl(early, quant_mxfp8_kernel<__nv_bfloat16>, grid, dim3(256), 0, as_stream(stream),
-                             (const __nv_bfloat16*)x, (uint8_t*)q, (uint32_t*)s, rows, cols, terms));
+    B200_LAUNCHED("quant_mxfp8_kernel", gated ? run(__nv_bfloat16(), std::true_type()) : run(__nv_bfloat16(), std::false_type()));
   else
-    B200_LAUNCHED("quant_mxfp8_kernel",
-                  launch_pdl(early, quant_mxfp8_kernel<__half>, grid, dim3(256), 0, as_stream(stream),
-                             (const __half*)x, (uint8_t*)q, (uint32_t*)s, rows, cols, terms));
+    B200_LAUNCHED("quant_mxfp8_kernel", gated ? run(__half(), std::true_type()) : run(__half(), std::false_type()));
   return B200MOE_OK;
+}
+
+extern "C" int b200moe_quant_mxfp8(const void* x, b200moe_dtype dtype, void* q, void* s, int64_t rows,
+                                   int cols, int terms, b200moe_stream stream) {
+  B200_CHECK_ARG(terms == 1 || terms == 2, "quant_mxfp8: terms must be 1 or 2");
+  return b200moe_quant_mxfp8_ex(x, dtype, q, s, rows, cols, terms, 0, 0, stream);
 }
 
 namespace {

@@ -11,6 +11,7 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st);
 int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st);
 int grouped_gemm_tc_dq(const b200moe_gemm_args* a, cudaStream_t st);
 int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st);
+int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st);
 int grouped_gemm_check(const b200moe_gemm_args* a, cudaStream_t st);
 }  // namespace b200moe
 
@@ -32,7 +33,8 @@ extern "C" int b200moe_grouped_gemm(const b200moe_gemm_args* a, b200moe_stream s
                  "grouped_gemm: e4m3 output needs the SiLU epilogue, d_scale, a 16-bit mid_dtype, fp8 "
                  "activations and block-scaled fp8 weights");
   const bool a_x2 = a->a_dtype == B200MOE_FP8_E4M3_X2;
-  const bool a_fp8 = a->a_dtype == B200MOE_FP8_E4M3 || a_x2;
+  const bool a_x3 = a->a_dtype == B200MOE_FP8_E4M3_X3;
+  const bool a_fp8 = a->a_dtype == B200MOE_FP8_E4M3 || a_x2 || a_x3;
   B200_CHECK_ARG(a_fp8 || a->a_dtype == a->d_dtype,
                  "grouped_gemm: ptr_A must be fp8 (with scales) or have ptr_D's dtype");
   switch (a->w_format) {
@@ -75,14 +77,17 @@ extern "C" int b200moe_grouped_gemm(const b200moe_gemm_args* a, b200moe_stream s
       B200_CHECK_ARG(a->group_size == 32 || a->group_size == 64 || a->group_size == 128 || a->group_size == 256,
                      "group_size must be 32, 64, 128 or 256");
       B200_CHECK_ARG(a->k % a->group_size == 0, "ptr_scales.size(2) of int4 must be divisible by K");
-      B200_CHECK_ARG(!a_fp8, "grouped_gemm: int4 weights take 16-bit activations");
+      B200_CHECK_ARG(!a_fp8 || ((a_x2 || a_x3) && a->a_scale != nullptr),
+                     "grouped_gemm: int4 weights take 16-bit activations, or two or three planes of "
+                     "b200moe_quant_mxfp8_ex with their scale words and block sums");
       break;
     default:
       return fail(B200MOE_E_BADARG, "grouped_gemm: unknown weight format %d", (int)a->w_format);
   }
   const bool w_tensor8 = a->w_format == B200MOE_W_FP8_TENSOR_KN || a->w_format == B200MOE_W_FP8E5M2_TENSOR_KN ||
                          a->w_format == B200MOE_W_MXFP8_KN;
-  B200_CHECK_ARG(!a_x2 || a->w_format == B200MOE_W_MXFP4_NK || w_tensor8,
+  B200_CHECK_ARG(!a_x3 || a->w_format == B200MOE_W_INT4_NK, "grouped_gemm: three-plane activations need int4 weights");
+  B200_CHECK_ARG(!a_x2 || a->w_format == B200MOE_W_MXFP4_NK || a->w_format == B200MOE_W_INT4_NK || w_tensor8,
                  "grouped_gemm: two-plane fp8 activations need MXFP4, MXFP8 or per-tensor fp8 weights");
   const bool segmented = a->w_experts > 0 && a->w_experts != a->num_experts;
   B200_CHECK_ARG(a->w_experts >= 0 && (!segmented || a->num_experts % a->w_experts == 0),
@@ -97,6 +102,7 @@ extern "C" int b200moe_grouped_gemm(const b200moe_gemm_args* a, b200moe_stream s
   cudaStream_t st = as_stream(stream);
   // MXFP8 activations exist on the block-scaled tensor-core path only.
   if ((a->w_format == B200MOE_W_MXFP4_NK || w_tensor8) && a_fp8) return grouped_gemm_tc_mx(a, st);
+  if (a->w_format == B200MOE_W_INT4_NK && a_fp8) return grouped_gemm_tc_i4(a, st);
   if (d_quant) {
     B200_CHECK_ARG(a->impl != 2, "grouped_gemm: the checking kernel has no quantised output");
     return grouped_gemm_tc_fp8t(a, st);

@@ -1,0 +1,499 @@
+// INT4 x quantised activations on the block-scaled tensor-core instruction.
+//
+//   D[m, f] = sum_g scale[f, g] * sum_{k in g} (u[f, k] - 8) * a[m, k]  (+ bias),  u = nibble ^ 8
+//
+// Weights [E,N,K/2] are two's-complement nibbles with one 16-bit scale per row and 128 or 256 K
+// elements.  A nibble u in 0..15, put into a byte, IS the e4m3 number u * 2^-9 (the subnormals and
+// the first binade of e4m3 are linear), so unpacking is the whole conversion: five instructions per
+// eight weights, against seventeen for the 16-bit expansion of gemm_tc_dq.cu, whose integer pipe is the
+// bound when there are few tokens.  The activations are e4m3 planes with one power-of-two
+// scale per 32 values (mx_quant.cuh): two planes hold a bfloat16 exactly, three a float16 (values
+// 2^-14 of the group's largest and smaller excepted, whose error stays below 2^-21 of it), so
+// nothing is lost against 16-bit activations, and the weight is not rounded after its scale is applied.
+//
+// The zero point and the group scales are applied where a 128-wide K block's sum leaves tensor
+// memory: with features on the lanes the scale is one register per thread, and 8 * sum_k a[m, k] (kept
+// by the quantiser for every block) comes from shared memory, the same for all lanes.
+//
+// Roles (768 threads in warpgroups that re-balance registers, one persistent CTA per SM; tiles of
+// 128 features x BT tokens):
+//   warp 0       : TMA producer: per K block 128 x 64 packed bytes and the planes' BT x 128 bytes
+//   warp 1       : MMA issuer; copies the tokens' scale factors to tensor memory (tcgen05.cp); the
+//                  planes accumulate in the same columns, so the promotion reads BT columns only
+//   warps 2-3    : bring the tokens' scale words and sums, four K blocks at a time
+//   warps 4-15   : converters, three sets that take K blocks in turn (a set is one long chain of
+//                  latencies, 630 cycles per block): a thread unpacks a row's 64 bytes into 32 columns
+//                  of tensor memory, from where the MMA reads the weights (nothing goes back through
+//                  shared memory)
+//   warps 16-23  : promotion and epilogue; warp w owns lane quarter w & 3 and half of the columns
+// Waits are bounded as in the other kernels (sm100_ptx.cuh).
+#include "common.cuh"
+#include "gemm_tc_common.cuh"
+#include "sm100_ptx.cuh"
+
+namespace b200moe {
+namespace {
+
+constexpr int kI4RawBytes = 8192;    // 128 rows x 64 packed bytes
+constexpr int kI4Threads = 768;
+constexpr int kI4LaunchRegs = 80, kI4FeedRegs = 64, kI4ConvRegs = 56, kI4PromoRegs = 120;   // warpgroups 0, 1-3, 4-5
+static_assert(128 * kI4FeedRegs + 384 * kI4ConvRegs + 256 * kI4PromoRegs <= kI4Threads * kI4LaunchRegs, "setmaxnreg budget");
+constexpr int kI4MaxStages = 12;
+constexpr int kI4Group = 4;          // K blocks per hand-over of token scales
+constexpr int kI4Slots = 3;
+constexpr int kI4Sets = 3;           // converter sets
+constexpr int kI4Conv = 4;           // weight-operand stages in tensor memory (32 columns each)
+constexpr int kI4Acc = 4;            // accumulator stages
+
+struct I4Params {
+  const uint16_t* w_scale;   // [E, N, groups] in the activation type
+  const uint32_t* a_scale;   // [planes][num_kb][M] words of four e8m0 bytes, then float sums [num_kb][M]
+  const void* bias;
+  void* d;
+  const int32_t* rows_per_expert;
+  int32_t* status;
+  int64_t m;
+  int n, k, num_experts;
+  int n_tiles, num_kb;
+  int groups, kb_shift;      // scales per weight row; scale index = K block >> kb_shift
+  int stages;
+  uint32_t idesc;
+  int out_f16;
+};
+
+template <int BT, int kTerms>
+struct I4Shape {
+  static constexpr int kTokChunks = kTerms > 2 ? 2 : 1;       // scale chunks: two columns per plane
+  static constexpr int kABytes = kTerms * BT * 128;
+  static constexpr int kStageBytes = kI4RawBytes + kABytes;
+  static constexpr int kSfPer = 4 * kTokChunks;               // tokens' scale columns of a K block
+  static constexpr uint32_t kConvBase = kI4Acc * BT;
+  static constexpr uint32_t kSfBase = kConvBase + kI4Conv * 32;   // weights' scale columns (constant), then the tokens'
+  static constexpr uint32_t kCols = kSfBase + 8 + kI4Group * kSfPer;
+  static constexpr uint32_t kTmem = kCols <= 256 ? 256u : 512u;
+  static constexpr int kSlotBytes = kI4Group * (512 * kTokChunks + BT * 4);
+  static_assert(BT <= 32 && kCols <= 512, "tensor memory");
+};
+
+struct I4Ctrl {
+  uint64_t full[kI4MaxStages];
+  uint64_t empty[kI4MaxStages];      // the MMA has read the tokens and the converters the packed weights
+  uint64_t conv_full[kI4Conv];
+  uint64_t conv_empty[kI4Conv];
+  uint64_t acc_full[kI4Acc];
+  uint64_t acc_empty[kI4Acc];
+  uint64_t sf_full[kI4Slots];
+  uint64_t sf_empty[kI4Slots];       // the MMA thread and the promotion warps
+  uint32_t tmem_base;
+  int abort_flag;
+  alignas(16) uint16_t xpose[8][16 * 32];   // per promotion warp: output transpose tile
+};
+
+template <int BT, int kTerms>
+__global__ void __launch_bounds__(kI4Threads, 1)
+grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
+                       const I4Params p) {
+  using S = I4Shape<BT, kTerms>;
+  constexpr int kStageBytes = S::kStageBytes, kSlotBytes = S::kSlotBytes;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int stages = p.stages;
+  uint8_t* sf_ring = smem + stages * kStageBytes;
+  I4Ctrl* ctrl = reinterpret_cast<I4Ctrl*>(sf_ring + kI4Slots * kSlotBytes);
+  uint8_t* walk_mem = reinterpret_cast<uint8_t*>(ctrl) + ((sizeof(I4Ctrl) + 15) & ~(size_t)15);
+  volatile int* abort_flag = &ctrl->abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+  if (warp == 0) {
+    pdl_wait();
+    build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, walk_mem);
+    if (lane == 0) {
+      ptx::prefetch_tensormap(&tmap_a);
+      ptx::prefetch_tensormap(&tmap_w);
+    }
+  } else if (warp == 1) {
+    ptx::tmem_alloc(&ctrl->tmem_base, S::kTmem);
+    ptx::tmem_relinquish();
+  } else if (warp == 2 && lane == 0) {
+    for (int s = 0; s < kI4MaxStages; ++s) {
+      ptx::mbar_init(&ctrl->full[s], 1);
+      ptx::mbar_init(&ctrl->empty[s], 1 + 4);
+    }
+    for (int c = 0; c < kI4Conv; ++c) {
+      ptx::mbar_init(&ctrl->conv_full[c], 4);
+      ptx::mbar_init(&ctrl->conv_empty[c], 1);
+    }
+    for (int a = 0; a < kI4Acc; ++a) {
+      ptx::mbar_init(&ctrl->acc_full[a], 1);
+      ptx::mbar_init(&ctrl->acc_empty[a], 8);
+    }
+    for (int g = 0; g < kI4Slots; ++g) {
+      ptx::mbar_init(&ctrl->sf_full[g], 2);
+      ptx::mbar_init(&ctrl->sf_empty[g], 1 + 8);
+    }
+    ctrl->abort_flag = 0;
+    ptx::fence_barrier_init();
+  }
+  pdl_wait();
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = ctrl->tmem_base;
+  if (warp >= 4 && warp < 8) {
+    // the weights' scale factors: 2^9 everywhere, which makes the codes the integers 0..15
+    const uint32_t c9[4] = {0x88888888u, 0x88888888u, 0x88888888u, 0x88888888u};
+    ptx::tmem_st_32x4(tmem_base + S::kSfBase + ((uint32_t)((warp & 3) * 32) << 16), c9[0], c9[1], c9[2], c9[3]);
+    ptx::tmem_wait_st();
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::tc_fence_after();
+
+  const TileWalk walk = tile_walk_at(walk_mem, p.num_experts);
+  const int total_tiles = walk.total;
+  const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+  const uint32_t conv_full0 = ptx::smem_u32(&ctrl->conv_full[0]), conv_empty0 = ptx::smem_u32(&ctrl->conv_empty[0]);
+  const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
+  const uint32_t sf_full0 = ptx::smem_u32(&ctrl->sf_full[0]), sf_empty0 = ptx::smem_u32(&ctrl->sf_empty[0]);
+  int my_tiles = 0;
+  for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) ++my_tiles;
+
+  if (warp < 4) {
+    ptx::setmaxnreg_dec<kI4FeedRegs>();
+    if (warp == 0) {
+      // ------------------------------ TMA producer ------------------------------
+      if (ptx::elect_one()) {
+        uint32_t s = 0, ph = 1;
+        int cursor = 0;
+        bool ok = true;
+        const uint32_t st0 = ptx::smem_u32(smem);
+        uint32_t st = st0;
+        for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+          TileInfo ti;
+          locate_tile<BT>(walk, t, cursor, ti);
+          const int n0 = ti.n_tile * kFeat;
+          for (int kb = 0; kb < p.num_kb; ++kb) {
+            const uint32_t full = full0 + 8 * s;
+            if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+            ptx::mbar_expect_tx_s(full, kStageBytes);
+            ptx::tma_load_3d_s(st, &tmap_w, full, kb * 64, n0, ti.e);
+            ptx::tma_load_3d_s(st + kI4RawBytes, &tmap_a, full, kb * 128, ti.row0, 0);   // all planes
+            st += kStageBytes;
+            if (++s == (uint32_t)stages) { s = 0; ph ^= 1; st = st0; }
+          }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // ------------------------------ MMA issuer --------------------------------
+      if (ptx::elect_one()) {
+        uint32_t s = 0, ph = 0, c = 0, cph = 0, a = 0, aph = 1, slot = 0, slot_ph = 0;
+        int cursor = 0;
+        bool ok = true;
+        const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kI4RawBytes, 16, 1024);
+        const uint64_t sfdesc0 = ptx::make_smem_desc_plain(ptx::smem_u32(sf_ring), 128);
+        uint64_t adesc = adesc0, sfdesc = sfdesc0;
+        for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+          TileInfo ti;
+          locate_tile<BT>(walk, t, cursor, ti);
+          // a partly filled token tile multiplies only its valid columns (UMMA N in steps of 16)
+          const uint32_t n_eff = (uint32_t)((ti.valid + 15) & ~15);
+          const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((n_eff >> 3) << 17);
+          for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += kI4Group) {
+            if (!ptx::mbar_wait_s(sf_full0 + 8 * slot, slot_ph, abort_flag)) { ok = false; break; }
+  #pragma unroll
+            for (int u = 0; u < kI4Group; ++u) {
+              if (kb0 + u < p.num_kb) {
+                if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag) ||
+                    !ptx::mbar_wait_s(conv_full0 + 8 * c, cph, abort_flag) ||
+                    !ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) { ok = false; break; }
+                ptx::tc_fence_after();
+                const uint32_t sf = tmem_base + S::kSfBase, sfa = sf + 8 + u * S::kSfPer;
+                ptx::tmem_cp_scales(sfa, sfdesc + u * (S::kTokChunks * 32));
+                if (S::kTokChunks == 2) ptx::tmem_cp_scales(sfa + 4, sfdesc + u * (S::kTokChunks * 32) + 32);
+  #pragma unroll
+                for (int term = 0; term < kTerms; ++term)
+                  ptx::umma_mx_block_ts(tmem_base + a * BT, tmem_base + S::kConvBase + c * 32, adesc + term * (BT * 128 >> 4),
+                                        idesc, term > 0 ? 1u : 0u, sf, sfa + 2 * term);
+                ptx::umma_commit(acc_full0 + 8 * a);
+                ptx::umma_commit(conv_empty0 + 8 * c);
+                ptx::umma_commit(empty0 + 8 * s);
+                adesc += kStageBytes >> 4;
+                if (++s == (uint32_t)stages) { s = 0; ph ^= 1; adesc = adesc0; }
+                if (++c == kI4Conv) { c = 0; cph ^= 1; }
+                if (++a == kI4Acc) { a = 0; aph ^= 1; }
+              }
+            }
+            if (!ok) break;
+            ptx::umma_commit(sf_empty0 + 8 * slot);
+            sfdesc += kSlotBytes >> 4;
+            if (++slot == kI4Slots) { slot = 0; slot_ph ^= 1; sfdesc = sfdesc0; }
+          }
+        }
+      }
+      __syncwarp();
+    } else {
+      // ------------------------ tokens' scales and sums ---------------------------
+      const int ft = (warp - 2) * 32 + lane;            // 0..63
+      constexpr int kNT = kTerms * BT, kPer = kI4Group * kNT / 64, kPerSum = (kI4Group * BT + 63) / 64;
+      const int64_t plane_words = (int64_t)p.num_kb * p.m;
+      const float* sums = reinterpret_cast<const float*>(p.a_scale + kTerms * plane_words);
+      uint32_t slot = 0, slot_ph = 1;
+      int cursor = 0;
+      bool ok = true;
+      // (the ring is deep enough to hide the loads' latency)
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        TileInfo ti;
+        locate_tile<BT>(walk, t, cursor, ti);
+        for (int kb0 = 0; kb0 < p.num_kb; kb0 += kI4Group) {
+          uint32_t w[kPer];
+          float m[kPerSum];
+  #pragma unroll
+          for (int i = 0; i < kPer; ++i) {
+            const int x = ft + 64 * i, n = x % kNT, kb = kb0 + x / kNT, term = n / BT, tok = n % BT;
+            w[i] = (kb < p.num_kb && tok < ti.valid)
+                       ? __ldg(p.a_scale + term * plane_words + (int64_t)kb * p.m + ti.row0 + tok) : 0x7f7f7f7fu;
+          }
+  #pragma unroll
+          for (int i = 0; i < kPerSum; ++i) {
+            const int x = ft + 64 * i, tok = x % BT, kb = kb0 + x / BT;
+            m[i] = (x < kI4Group * BT && kb < p.num_kb && tok < ti.valid)
+                       ? -8.0f * __ldg(sums + (int64_t)kb * p.m + ti.row0 + tok) : 0.f;
+          }
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
+          const uint32_t ring = ptx::smem_u32(sf_ring) + slot * kSlotBytes;
+  #pragma unroll
+          for (int i = 0; i < kPer; ++i) {
+            // plane `term` takes the columns 2 * term and 2 * term + 1 (an MMA's scales start on an even one)
+            const int x = ft + 64 * i, n = x % kNT, u = x / kNT, term = n / BT, tok = n % BT;
+            ptx::sts32(ring + u * (S::kTokChunks * 512) + (term >> 1) * 512 + (tok & 31) * 16 + ((2 * term + (tok >> 5)) & 3) * 4,
+                       w[i]);
+          }
+  #pragma unroll
+          for (int i = 0; i < kPerSum; ++i)
+            if (ft + 64 * i < kI4Group * BT) ptx::sts32f(ring + kI4Group * 512 * S::kTokChunks + (ft + 64 * i) * 4, m[i]);
+          ptx::fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_s(sf_full0 + 8 * slot);
+          if (++slot == kI4Slots) { slot = 0; slot_ph ^= 1; }
+        }
+      }
+    }
+  } else if (warp < 16) {
+    ptx::setmaxnreg_dec<kI4ConvRegs>();
+    // ------------------------------ converters ------------------------------
+    const int row = (warp & 3) * 32 + lane, set = (warp - 4) >> 2;
+    const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
+    const uint32_t src0 = ptx::smem_u32(smem) + row * 64;
+    const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;      // 64-byte swizzle: chunk index xor row bits 1..2
+    uint32_t s = set, ph = 0;                                   // (at least kI4Sets stages)
+    const uint32_t blocks = (uint32_t)my_tiles * p.num_kb;      // every tile: the same K loop
+    for (uint32_t i = set; i < blocks; i += kI4Sets) {
+      const uint32_t c = i % kI4Conv;
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(full0 + 8 * s, ph, abort_flag))) break;
+      const uint32_t src = src0 + s * kStageBytes;
+      uint32_t o[32];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 v = ptx::lds128(src + ((uint32_t)(q * 16) ^ swz));
+        const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // nibbles of even and of odd k as bytes (sign bit flipped: 0..15), then in k order
+          const uint32_t e = (w[j] & 0x0f0f0f0fu) ^ 0x08080808u, d = ((w[j] >> 4) & 0x0f0f0f0fu) ^ 0x08080808u;
+          o[q * 8 + 2 * j] = __byte_perm(e, d, 0x5140);
+          o[q * 8 + 2 * j + 1] = __byte_perm(e, d, 0x7362);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_s(empty0 + 8 * s);
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(conv_empty0 + 8 * c, ((i / kI4Conv) & 1) ^ 1, abort_flag))) break;
+      ptx::tc_fence_after();
+      ptx::tmem_st_32x32(tmem_base + S::kConvBase + c * 32 + lane_sel, o);
+      ptx::tmem_wait_st();
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_s(conv_full0 + 8 * c);
+      s += kI4Sets;
+      if (s >= (uint32_t)stages) { s -= stages; ph ^= 1; }
+    }
+  } else {
+    ptx::setmaxnreg_inc<kI4PromoRegs>();
+    // ------------------------ promotion and epilogue --------------------------
+    constexpr int kHalf = BT / 2;                  // columns of this warp
+    const int q = warp & 3, half = (warp - 16) >> 2;
+    const int et = q * 32 + lane;
+    const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
+    const int col0 = half * kHalf;
+    uint32_t a = 0, aph = 0, slot = 0, slot_ph = 0;
+    int cursor = 0;
+    bool ok = true;
+    const bool vec4 = p.kb_shift == 0 && p.groups % 4 == 0 && (reinterpret_cast<uintptr_t>(p.w_scale) & 7) == 0;
+    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      TileInfo ti;
+      locate_tile<BT>(walk, t, cursor, ti);
+      const int feat = ti.n_tile * kFeat + et;
+      const bool feat_ok = feat < p.n;
+      const float bias_v = (p.bias != nullptr && feat_ok) ? load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + feat) : 0.f;
+      const uint16_t* srow = p.w_scale + ((int64_t)ti.e * p.n + (feat_ok ? feat : 0)) * p.groups;
+      const bool mine = col0 < ti.valid;           // any valid column in this warp's half
+      // the four scales of a group of K blocks (packed 16-bit), read one group ahead
+      auto scales_of = [&](int kb0) {
+        uint2 r = make_uint2(0u, 0u);
+        if (vec4) {
+          if (kb0 < p.groups) r = __ldg(reinterpret_cast<const uint2*>(srow + kb0));
+        } else {
+          uint32_t h[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int g = (kb0 + u) >> p.kb_shift;
+            h[u] = g < p.groups ? __ldg(srow + g) : 0;
+          }
+          r = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
+        }
+        return r;
+      };
+      float acc[kHalf];
+#pragma unroll
+      for (int i = 0; i < kHalf; ++i) acc[i] = 0.f;
+      uint2 nxt = scales_of(0);
+      for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += kI4Group) {
+        const uint2 cur = nxt;
+        nxt = scales_of(kb0 + kI4Group);
+        float sc[kI4Group];
+        if (p.out_f16) {
+          const float2 lo = __half22float2(*reinterpret_cast<const __half2*>(&cur.x));
+          const float2 hi = __half22float2(*reinterpret_cast<const __half2*>(&cur.y));
+          sc[0] = lo.x; sc[1] = lo.y; sc[2] = hi.x; sc[3] = hi.y;
+        } else {
+          sc[0] = __uint_as_float(cur.x << 16); sc[1] = __uint_as_float(cur.x & 0xffff0000u);
+          sc[2] = __uint_as_float(cur.y << 16); sc[3] = __uint_as_float(cur.y & 0xffff0000u);
+        }
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_full0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
+        const uint32_t sums = ptx::smem_u32(sf_ring) + slot * kSlotBytes + kI4Group * 512 * S::kTokChunks + col0 * 4;
+#pragma unroll
+        for (int u = 0; u < kI4Group; ++u) {
+          if (kb0 + u >= p.num_kb) break;
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(acc_full0 + 8 * a, aph, abort_flag))) { ok = false; break; }
+          ptx::tc_fence_after();
+          uint32_t v[kHalf];
+          if (mine) {
+            const uint32_t col = tmem_base + a * BT + col0 + lane_sel;
+            if (kHalf == 16) ptx::tmem_ld_32x16(col, reinterpret_cast<uint32_t(&)[16]>(v));
+            else ptx::tmem_ld_32x8(col, reinterpret_cast<uint32_t(&)[8]>(v));
+            ptx::tmem_wait_ld();
+            ptx::pin_registers(v);
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);   // the stage is in registers
+          if (++a == kI4Acc) { a = 0; aph ^= 1; }
+          if (mine) {
+#pragma unroll
+            for (int i = 0; i < kHalf; i += 4) {
+              const float4 m = ptx::lds128f(sums + (u * BT + i) * 4);   // -8 * the block's sum of the token
+              acc[i + 0] = fmaf(__uint_as_float(v[i + 0]) + m.x, sc[u], acc[i + 0]);
+              acc[i + 1] = fmaf(__uint_as_float(v[i + 1]) + m.y, sc[u], acc[i + 1]);
+              acc[i + 2] = fmaf(__uint_as_float(v[i + 2]) + m.z, sc[u], acc[i + 2]);
+              acc[i + 3] = fmaf(__uint_as_float(v[i + 3]) + m.w, sc[u], acc[i + 3]);
+            }
+          }
+        }
+        if (!ok) break;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_s(sf_empty0 + 8 * slot);
+        if (++slot == kI4Slots) { slot = 0; slot_ph ^= 1; }
+      }
+      if (!ok) break;
+      if (mine) {
+        constexpr int kChunk = kHalf < 16 ? kHalf : 16;
+#pragma unroll
+        for (int c0 = 0; c0 < kHalf; c0 += kChunk) {
+          if (col0 + c0 < ti.valid) {
+            float vals[kChunk];
+#pragma unroll
+            for (int i = 0; i < kChunk; ++i) vals[i] = acc[c0 + i] + bias_v;
+            store_block_transposed<kChunk, 32>(ctrl->xpose[warp - 16], vals, p.d, p.out_f16, (int64_t)ti.row0 + col0 + c0,
+                                               ti.valid - col0 - c0, p.m, p.n, ti.n_tile * kFeat + q * 32, lane);
+          }
+        }
+      }
+    }
+  }
+
+  pdl_trigger();
+  ptx::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    ptx::tc_fence_after();
+    if (*abort_flag != 0) __nanosleep(20000);
+    ptx::tmem_dealloc(tmem_base, S::kTmem);
+  }
+  if (tid == 0 && *abort_flag != 0) report_timeout(p.status);
+}
+
+template <int BT, int kTerms>
+int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
+  using S = I4Shape<BT, kTerms>;
+  auto kern = grouped_gemm_i4_kernel<BT, kTerms>;
+  p.idesc = ptx::make_idesc_mx(0u, 0u, kFeat, (uint32_t)BT);
+  CUtensorMap ta, tw;
+  {
+    cuuint64_t dims[3] = {(cuuint64_t)a->k, (cuuint64_t)a->m, (cuuint64_t)kTerms};
+    cuuint64_t strides[2] = {(cuuint64_t)a->k, (cuuint64_t)a->k * (cuuint64_t)a->m};
+    cuuint32_t box[3] = {128, (cuuint32_t)BT, (cuuint32_t)kTerms};
+    if (int rc = encode_map(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->a, dims, strides, box)) return rc;
+  }
+  {
+    cuuint64_t dims[3] = {(cuuint64_t)(a->k / 2), (cuuint64_t)a->n, (cuuint64_t)a->num_experts};
+    cuuint64_t strides[2] = {(cuuint64_t)(a->k / 2), (cuuint64_t)(a->k / 2) * a->n};
+    cuuint32_t box[3] = {64, (cuuint32_t)kFeat, 1};
+    if (int rc = encode_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B))
+      return rc;
+  }
+  const int fixed = 1024 + kI4Slots * S::kSlotBytes + (int)((sizeof(I4Ctrl) + 15) & ~(size_t)15) + tile_walk_bytes(p.num_experts);
+  p.stages = ((int)kMaxSmem - fixed) / S::kStageBytes;
+  if (p.stages > kI4MaxStages) p.stages = kI4MaxStages;
+  const size_t smem = (size_t)fixed + (size_t)p.stages * S::kStageBytes;
+  static SmemConfig configured;
+  if (int rc = configured.ensure(kern, smem)) return rc;
+  const int64_t tile_bound = ((a->m + BT - 1) / BT + a->num_experts) * (int64_t)p.n_tiles;
+  int grid = sm_count();
+  if (a->max_ctas > 0 && a->max_ctas < grid) grid = a->max_ctas;
+  if (tile_bound < grid) grid = (int)tile_bound;
+  B200_LAUNCHED("grouped_gemm_i4_kernel",
+                launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kI4Threads), smem, st, ta, tw, p));
+  return B200MOE_OK;
+}
+
+}  // namespace
+
+// INT4 weights x two (bfloat16 output) or three (float16 output) e4m3 planes: a codes [planes][M,K],
+// a_scale words [planes][K/128][M] and fp32 block sums [K/128][M] behind them (what
+// b200moe_quant_mxfp8_ex writes).  Returns B200MOE_E_UNSUPPORTED (no launch) for anything else.
+int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
+  const int planes = a->a_dtype == B200MOE_FP8_E4M3_X2 ? 2 : a->a_dtype == B200MOE_FP8_E4M3_X3 ? 3 : 0;
+  if (a->w_format != B200MOE_W_INT4_NK || planes == 0 || a->a_scale == nullptr || a->epilogue != B200MOE_EPI_NONE)
+    return fail(B200MOE_E_UNSUPPORTED, "int4 GEMM takes int4 weights and two or three e4m3 activation planes");
+  if (a->num_experts > kMaxExperts || a->k % 128 != 0 || (a->group_size != 128 && a->group_size != 256) || a->n % 8 != 0)
+    return fail(B200MOE_E_UNSUPPORTED, "int4 GEMM: K a multiple of 128, one scale per 128 or 256 of it");
+  if (((uintptr_t)a->a & 15) || ((uintptr_t)a->w & 15) || ((uintptr_t)a->d & 15) || ((uintptr_t)a->a_scale & 3))
+    return fail(B200MOE_E_BADARG, "int4 GEMM: A, W and D must be 16-byte aligned");
+  I4Params p;
+  p.w_scale = reinterpret_cast<const uint16_t*>(a->w_scale);
+  p.a_scale = reinterpret_cast<const uint32_t*>(a->a_scale);
+  p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
+  p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
+  p.n_tiles = (a->n + kFeat - 1) / kFeat;
+  p.num_kb = a->k / 128;
+  p.groups = a->k / a->group_size;
+  p.kb_shift = a->group_size == 256 ? 1 : 0;
+  p.out_f16 = a->d_dtype == B200MOE_F16;
+  const int64_t in_use = (a->rows_hint > 0 && a->rows_hint < a->m) ? a->rows_hint : a->m;
+  const int64_t avg = (in_use + a->num_experts - 1) / a->num_experts;
+  // (both the MMA and the promotion cost grow with the tile: it is what the average expert fills)
+  if (planes == 2) return avg <= 8 ? launch_i4<16, 2>(a, p, st) : launch_i4<32, 2>(a, p, st);
+  return avg <= 8 ? launch_i4<16, 3>(a, p, st) : launch_i4<32, 3>(a, p, st);
+}
+
+}  // namespace b200moe

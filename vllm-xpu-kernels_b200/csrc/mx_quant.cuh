@@ -40,5 +40,13 @@ __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, ui
   return word;
 }
 
+// Sum of a 128-wide block over its sixteen lanes: what the int4 GEMM needs to take its weights' zero
+// point out (x: the lane's values less what the planes left over).
+__device__ __forceinline__ float mx_block_sum(float x) {
+#pragma unroll
+  for (int d = 1; d < 16; d <<= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+  return x;
+}
+
 }  // namespace
 }  // namespace b200moe

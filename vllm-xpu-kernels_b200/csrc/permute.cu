@@ -39,7 +39,8 @@ struct RowJob {
   int H;                 // quantised forms: values per row
   int K;
   int64_t rows;          // mx: rows of a plane (T * K)
-  int planes;            // mx: 1 or 2
+  int planes;            // mx: 1 to 3
+  int sums;              // mx: fp32 block sums [ceil(H/128)][rows] follow the scale words
 };
 
 __device__ __forceinline__ void copy_scales(const RowJob& a, int64_t tok, const int* dest) {
@@ -108,8 +109,9 @@ __device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, 
   uint8_t* dst_q = reinterpret_cast<uint8_t*>(a.dst);
   uint32_t* dst_s = reinterpret_cast<uint32_t*>(a.dst_s);
   float v[8];
+  float total = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = in ? to_f32<T>(e[i]) : 0.f;
+  for (int i = 0; i < 8; ++i) { v[i] = in ? to_f32<T>(e[i]) : 0.f; total += v[i]; }
 #pragma unroll 1
   for (int p = 0; p < a.planes; ++p) {
     uint2 codes;
@@ -121,6 +123,15 @@ __device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, 
         if ((j & 15) == 0 && j < num_kb * 16) dst_s[((int64_t)p * num_kb + (j >> 4)) * a.rows + r] = word;
       }
     }
+  }
+  if (a.sums) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) total -= v[i];
+    total = mx_block_sum(total);
+    if ((j & 15) == 0 && j < num_kb * 16)
+      for (int k = 0; k < a.K; ++k)
+        if (dest[k] >= 0)
+          reinterpret_cast<float*>(dst_s)[((int64_t)a.planes * num_kb + (j >> 4)) * a.rows + dest[k]] = total;
   }
 }
 
@@ -677,7 +688,7 @@ extern "C" int b200moe_remap_quant_fp8(
 }
 
 extern "C" int b200moe_remap_quant_mxfp8(
-    const void* hidden, b200moe_dtype dtype, void* remapped_q, void* remapped_scales, int planes,
+    const void* hidden, b200moe_dtype dtype, void* remapped_q, void* remapped_scales, int planes, int block_sums,
     const int32_t* expert_map, int32_t* rows_per_expert, int32_t* row_map,
     const void* topk_ids, b200moe_dtype ids_dtype, int64_t num_rows, int hidden_size,
     int topk, int total_experts, int local_experts, void* workspace,
@@ -685,7 +696,7 @@ extern "C" int b200moe_remap_quant_mxfp8(
   B200_CHECK_ARG(dtype == B200MOE_BF16 || dtype == B200MOE_F16,
                  "remap_quant_mxfp8: activations must be bfloat16 or float16");
   B200_CHECK_ARG(hidden_size % 32 == 0, "remap_quant_mxfp8: hidden_size must be a multiple of 32");
-  B200_CHECK_ARG(planes == 1 || planes == 2, "remap_quant_mxfp8: one or two planes");
+  B200_CHECK_ARG(planes >= 1 && planes <= 3, "remap_quant_mxfp8: one to three planes");
   SortParams p;
   if (int rc = remap_params(p, expert_map, rows_per_expert, row_map, topk_ids, ids_dtype, num_rows, topk,
                             total_experts, local_experts)) return rc;
@@ -694,7 +705,7 @@ extern "C" int b200moe_remap_quant_mxfp8(
                  "remap_quant_mxfp8: buffers must be 16-byte aligned");
   RowJob job = {};
   job.src = hidden; job.dst = remapped_q; job.dst_s = remapped_scales; job.H = hidden_size; job.K = topk;
-  job.rows = num_rows * topk; job.planes = planes;
+  job.rows = num_rows * topk; job.planes = planes; job.sums = block_sums;
   auto run = dtype == B200MOE_BF16 ? remap_rows<__nv_bfloat16, kRowMx> : remap_rows<__half, kRowMx>;
   return run(p, job, rows_per_expert, row_map, num_rows, workspace, workspace_bytes, as_stream(stream));
 }

@@ -94,6 +94,23 @@ static __device__ __noinline__ bool mbar_wait_rest(uint32_t bar, uint32_t parity
 __device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   return mbar_try_wait_s(bar, parity) || mbar_wait_rest(bar, parity, abort_flag);
 }
+// The same without a call, for warps whose registers are full.
+__device__ __forceinline__ bool mbar_wait_inline_s(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
+  if (mbar_try_wait_s(bar, parity)) return true;
+  const long long t0 = clock64();
+  uint32_t spins = 0;
+#pragma unroll 1
+  while (!mbar_try_wait_s(bar, parity)) {
+    if ((++spins & 0xff) == 0) {
+      if (*abort_flag != 0) return false;
+      if (clock64() - t0 > kWaitBudgetCycles) {
+        *abort_flag = 1;
+        return false;
+      }
+    }
+  }
+  return true;
+}
 __device__ __forceinline__ void mbar_arrive_s(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -313,6 +330,20 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "memory");
 }
 
+// Registers filled by a tcgen05.ld, after its wait: no use of them is scheduled ahead of this point.
+template <int N>
+__device__ __forceinline__ void pin_registers(uint32_t (&r)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
+}
+__device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+      : "r"(taddr)
+      : "memory");
+}
+
 // tcgen05.wait::ld for loads that were issued earlier and whose destination
 // registers the code in between did not touch: the registers are operands of the
 // wait, so that no later use of them can be scheduled ahead of it.
@@ -356,6 +387,17 @@ __device__ __forceinline__ void tmem_st_32x8(uint32_t taddr, const uint32_t (&r)
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr),
                "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
                : "memory");
+}
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]),
+        "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]),
+        "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]),
+        "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -461,6 +503,40 @@ __device__ __forceinline__ void umma_block(uint32_t tmem_d, uint64_t adesc, uint
   if (kFp8) B200_UMMA4("f8f6f4");
   else B200_UMMA4("f16");
 #undef B200_UMMA4
+}
+// A 512-byte scale chunk from shared to tensor memory, as in umma_mx_block.
+__device__ __forceinline__ void tmem_cp_scales(uint32_t taddr, uint64_t desc) {
+  asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
+}
+// umma_mx_block's four instructions with the weights in tensor memory (eight columns per K step).
+__device__ __forceinline__ void umma_mx_block_ts(uint32_t tmem_d, uint32_t tmem_w, uint64_t adesc, uint32_t idesc,
+                                                 uint32_t accumulate, uint32_t sfw, uint32_t sfa) {
+  asm volatile(
+      "{\n\t.reg .pred pa;\n\t.reg .b32 w1, w2, w3, i1, i2, i3;\n\t.reg .b64 a1, a2, a3;\n\tsetp.ne.b32 pa, %6, 0;\n\t"
+      "add.u32 w1, %1, 8;\n\tadd.u32 w2, %1, 16;\n\tadd.u32 w3, %1, 24;\n\t"
+      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"
+      "or.b32 i1, %3, 0x20000010;\n\tor.b32 i2, %3, 0x40000020;\n\tor.b32 i3, %3, 0x60000030;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [%1], %2, %3, [%4], [%5], pa;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w1], a1, i1, [%4], [%5], 1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w2], a2, i2, [%4], [%5], 1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w3], a3, i3, [%4], [%5], 1;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_w), "l"(adesc), "r"(idesc), "r"(sfw), "r"(sfa), "r"(accumulate)
+      : "memory");
+}
+// umma_block's four kind::f16 instructions with the 128-row operand in tensor memory (eight columns per
+// K step, the other operand 32 bytes).
+__device__ __forceinline__ void umma_f16_block_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
+                                                  uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred pa;\n\t.reg .b32 a1, a2, a3;\n\t.reg .b64 b1, b2, b3;\n\tsetp.ne.b32 pa, %4, 0;\n\t"
+      "add.u32 a1, %1, 8;\n\tadd.u32 a2, %1, 16;\n\tadd.u32 a3, %1, 24;\n\t"
+      "add.u64 b1, %2, 2;\n\tadd.u64 b2, %2, 4;\n\tadd.u64 b3, %2, 6;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, pa;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], b2, %3, 1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [a3], b3, %3, 1;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 // A commit makes the barrier receive one arrival when all tcgen05 operations issued so far by this
 // thread have completed.

@@ -36,6 +36,13 @@ struct Plan {
   int64_t hidden = -1;
   at::ScalarType act_dtype = at::kFloat;
   WeightDesc d13{}, d2{};
+  bool i4 = false;            // int4 weights whose shapes the block-scaled kernel takes (gemm_tc_i4.cu)
+  // Up to this many rows per expert that kernel streams the weights faster than the one that expands
+  // them to 16 bits (gemm_tc_dq.cu), whose matrix work is the cheaper one from there on.  A layer of 8
+  // experts of 4096 x 14336, 2 a token: 104 against 121 us at 1 token, 244 against 289 at 33 (8 rows
+  // an expert), 483 against 313 at 128 (32 rows).
+  static constexpr int64_t kI4PlaneRows = 16;
+  bool i4_planes(int64_t rows, int64_t segments) const { return i4 && rows <= kI4PlaneRows * segments; }
 };
 const char* const kPlanName = "b200moe.layer_plan";
 
@@ -118,6 +125,10 @@ void describe(Plan& p, int64_t hidden, at::ScalarType out_dtype) {
     TORCH_CHECK((*b)->size(1) == (b == &p.b13 ? 2 * p.inter : hidden), "ptr_bias.size(1) must match N");
     TORCH_CHECK((*b)->scalar_type() == out_dtype, "ptr_bias must have ptr_D's dtype");
   }
+  auto i4_ok = [](const WeightDesc& d, int64_t k) {
+    return d.format == B200MOE_W_INT4_NK && (d.group == 128 || d.group == 256) && k % 128 == 0;
+  };
+  p.i4 = i4_ok(p.d13, hidden) && i4_ok(p.d2, p.inter * p.inter_scale);
   p.hidden = hidden;
   p.act_dtype = out_dtype;
 }
@@ -147,6 +158,9 @@ struct Experts {
   int device;
   b200moe_stream stream;
   bool a_fp8;                 // gemm1's rows are e4m3 with 1x128 scales
+  bool planes_in;             // ... or e4m3 planes with one scale per 32 values
+  int planes;
+  bool sums;                  // ... and the sums of their 128-wide blocks behind the scales (int4 weights)
   int64_t inter2() const { return p.inter * p.inter_scale; }
   // offsets
   size_t g1 = 0, act = 0, act_q = 0, act_s = 0;
@@ -157,15 +171,17 @@ struct Experts {
   void lay_out_second(Layout& l) {
     const int64_t I = p.inter, I2 = o.form == kUnfused ? inter2() : I;
     const bool direct_fp8 = p.block_fp8 && (o.form == kFp8 || (p.act == kSilu && I % 128 == 0));
-    if (!direct_fp8) act = l.take(M * I2 * 2);
+    if (!direct_fp8 && !gated_quant()) act = l.take(M * I2 * 2);
     if (p.block_fp8) {
       act_q = l.take(M * I2);
       act_s = l.take(M * (I2 / 128) * 4);
-    } else if (p.mx) {
-      act_q = l.take((size_t)p.planes * M * I2);
-      act_s = l.take((size_t)p.planes * ((I2 + 127) / 128) * M * 4);
+    } else if (planes_in) {
+      act_q = l.take((size_t)planes * M * I2);
+      act_s = l.take((size_t)(planes + (sums ? 1 : 0)) * ((I2 + 127) / 128) * M * 4);
     }
   }
+  // SiLU, multiply and the planes of gemm2's input in one pass
+  bool gated_quant() const { return planes_in && o.form == kUnfused && p.act == kSilu && p.inter % 32 == 0; }
 
   void gemm(bool first, const void* a, b200moe_dtype a_dtype, const void* a_scale, void* d, b200moe_dtype d_dtype,
             void* d_scale, const int32_t* rows, b200moe_epilogue epi) const {
@@ -193,9 +209,9 @@ struct Experts {
 
   void run(uint8_t* ws, const void* a, const void* a_scale, const int32_t* rows, void* d) const {
     const int64_t I = p.inter, I2 = inter2();
-    const b200moe_dtype mx_dtype = p.planes == 2 ? B200MOE_FP8_E4M3_X2 : B200MOE_FP8_E4M3;
-    const b200moe_dtype a_dtype = a_fp8 ? B200MOE_FP8_E4M3 : p.mx ? mx_dtype : out;
-    bool fp8_ready = false;
+    const b200moe_dtype mx_dtype = planes == 3 ? B200MOE_FP8_E4M3_X3 : planes == 2 ? B200MOE_FP8_E4M3_X2 : B200MOE_FP8_E4M3;
+    const b200moe_dtype a_dtype = a_fp8 ? B200MOE_FP8_E4M3 : planes_in ? mx_dtype : out;
+    bool fp8_ready = false, planes_ready = false;
     if (o.form == kFp8) {
       gemm(true, a, a_dtype, a_scale, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, rows, B200MOE_EPI_SILU_MUL);
       mark(o, "gemm1");
@@ -219,6 +235,9 @@ struct Experts {
         check_status(b200moe_silu_and_mul_per_block_quant_ragged(ws + act_q, (float*)(ws + act_s), ws + g1, out, M,
                                                                  (int)I, rows, segments, stream));
         fp8_ready = true;
+      } else if (gated_quant()) {
+        check_status(b200moe_quant_mxfp8_ex(ws + g1, out, ws + act_q, ws + act_s, M, (int)I, planes, sums, 1, stream));
+        planes_ready = true;
       } else {
         void *to = ws + act, *from = ws + g1;
         switch (p.act) {
@@ -238,8 +257,9 @@ struct Experts {
         check_status(b200moe_per_token_group_fp8_quant(ws + act, out, ws + act_q, (float*)(ws + act_s), M, (int)I2, 128,
                                                        1e-10f, 0, I2 / 128, 1, stream));
       gemm(false, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, d, out, nullptr, rows, B200MOE_EPI_NONE);
-    } else if (p.mx) {
-      check_status(b200moe_quant_mxfp8(ws + act, out, ws + act_q, ws + act_s, M, (int)I2, p.planes, stream));
+    } else if (planes_in) {
+      if (!planes_ready)
+        check_status(b200moe_quant_mxfp8_ex(ws + act, out, ws + act_q, ws + act_s, M, (int)I2, planes, sums, 0, stream));
       gemm(false, ws + act_q, mx_dtype, ws + act_s, d, out, nullptr, rows, B200MOE_EPI_NONE);
     } else {
       gemm(false, ws + act, out, nullptr, d, out, nullptr, rows, B200MOE_EPI_NONE);
@@ -357,11 +377,14 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   mark(o, "routing");
 
   const bool quant_fp8 = p.block_fp8 && !a1q.has_value();
+  const bool i4 = p.i4_planes(o.rows_hint > 0 && o.rows_hint < M ? o.rows_hint : M, p.experts);
+  const bool planes_in = p.mx || i4;
+  const int planes = i4 ? (od == at::kHalf ? 3 : 2) : p.planes;   // exact for the 16-bit type
   if (!p.mx && !p.block_fp8)
     TORCH_CHECK(x.scalar_type() == od, "ptr_A and ptr_D must have the same dtype");
   // (16-bit rows with caller-made scales: the scales are permuted and left unused)
   const bool a_fp8 = quant_fp8 || (p.block_fp8 && x.scalar_type() == at::kFloat8_e4m3fn);
-  Experts e{p, o, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8};
+  Experts e{p, o, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8, planes_in, planes, i4};
   Layout l;
   const size_t rows_at = l.take(p.experts * 4), map_at = l.take(M * 4);
   const size_t sort_bytes = b200moe_sort_workspace_bytes(M, (int)p.experts);
@@ -371,9 +394,9 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (quant_fp8) {
     l.take(M * H);
     as_at = l.take(M * (H / 128) * 4);
-  } else if (p.mx) {
-    l.take((size_t)p.planes * M * H);
-    as_at = l.take((size_t)p.planes * ((H + 127) / 128) * M * 4);
+  } else if (planes_in) {
+    l.take((size_t)planes * M * H);
+    as_at = l.take((size_t)(planes + (i4 ? 1 : 0)) * ((H + 127) / 128) * M * 4);
   } else {
     l.take(M * H * x.element_size());
     if (a1q.has_value()) as_at = l.take(M * a1q->size(1) * a1q->element_size());
@@ -392,9 +415,9 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                          (float*)(ws + as_at), emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T,
                                          (int)H, (int)K, (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes,
                                          st));
-  else if (p.mx)
+  else if (planes_in)
     check_status(b200moe_remap_quant_mxfp8(x.data_ptr(), float_dtype(x, "hidden_states"), ws + a_at, ws + as_at,
-                                           p.planes, emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T, (int)H,
+                                           planes, i4, emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T, (int)H,
                                            (int)K, (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes, st));
   else
     check_status(b200moe_remap_hidden_states(
@@ -403,7 +426,7 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
         a1q.has_value() ? (int)a1q->size(1) : 0, a1q.has_value() ? (int)a1q->element_size() : 0, (int)K,
         (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes, st));
   mark(o, "permute");
-  e.run(ws, ws + a_at, (a_fp8 || p.mx) ? ws + as_at : nullptr, rows, ws + d_at);
+  e.run(ws, ws + a_at, (a_fp8 || planes_in) ? ws + as_at : nullptr, rows, ws + d_at);
   if (gather) {
     const at::Tensor& y = THPVariable_Unpack(a[2]);
     const at::Tensor& w = THPVariable_Unpack(a[4]);
@@ -453,7 +476,7 @@ PyObject* layer_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   describe(p, H, y.scalar_type());
   raise_if_timed_out(device_status_word(x.get_device()));
   Experts e{p, o, out, y.scalar_type(), M, H, (int)segments, (int)x.get_device(), (b200moe_stream)stream.stream(),
-            p.block_fp8};
+            p.block_fp8, false, 0};
   Layout l;
   e.lay_out(l);
   e.lay_out_second(l);
