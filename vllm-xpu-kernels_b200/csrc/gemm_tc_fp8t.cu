@@ -58,6 +58,7 @@ struct TParams {
   // token and 128 features in d_scale [M, n/256]
   float* d_scale;
   float clamp;            // >0: gate = min(gate, clamp), up = clamp(up, -clamp, clamp)
+  int stages;             // 128 x 256 kernel: pipeline stages
 };
 
 struct TCtrl {
@@ -287,16 +288,26 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
 // twice the work (the issuing thread, not the tensor pipe, bounds the 128-feature tile).
 // A thread then owns 128 accumulators, more than the even register split of 384 threads
 // allows: the warps are laid out in warpgroups and re-balance registers with setmaxnreg
-//   warps 0-3  : producer (warp 0), MMA issuer (warp 1), two idle warps; 40 registers
-//   warps 4-11 : promotion + epilogue, 232 registers; warp w reads lane quarter w & 3 and
+//   warps 0-3  : producer (warp 0), MMA issuer (warp 1), scale preparers (warps 2 and 3); 56 registers
+//   warps 4-11 : promotion + epilogue, 224 registers; warp w reads lane quarter w & 3 and
 //                the 128 columns of feature block (w - 4) / 4, in two passes of 64
 // Tensor memory holds two accumulator stages of 256 columns.
+//
+// The promotion sets the rate: a K block's MMAs take 512 cycles, the additions of two warps on a
+// scheduler 256 to 300, but a warp that waits for the stage, loads, adds, and reads its scales from
+// global memory one after the other took 917 to 1000.  So everything that is not a load or an addition
+// is kept off its path: scales (already multiplied, four K blocks per hand-over) and tile coordinates come
+// from the preparers through shared memory; a chunk's tensor-memory load is in flight while the chunk
+// before it is added up, also from one K block to the next; the next K block's barriers are looked at once,
+// before the additions that hide the look, and nothing else in the loop branches.  128 experts of 188 rows,
+// N 2048, K 768: 140 -> 110 us; 256 experts of 256 rows on average, N 4096, K 7168: 3.06 -> 2.85 ms.
 constexpr int kT2Threads = 384;
 // setmaxnreg.inc waits - without any limit - until the CTA's register pool holds what it asks
 // for, so the re-balanced total must fit what the CTA got at launch (threads x launch registers)
-constexpr int kT2LaunchRegs = 168, kT2LowRegs = 40, kT2HighRegs = 232;
+constexpr int kT2LaunchRegs = 168, kT2LowRegs = 56, kT2HighRegs = 224;
 static_assert(128 * kT2LowRegs + 256 * kT2HighRegs <= kT2Threads * kT2LaunchRegs, "setmaxnreg budget");
-constexpr int kT2Stages = 4;          // ring: 192 KB in flight per SM
+constexpr int kT2Stages = 4;          // ring: 192 KB in flight per SM (one less beside a walk of many hundred experts)
+constexpr int kT2Slots = 2;           // scale groups handed over ahead
 // Finished rows leave through per-warp staging tiles of 32 rows x 32 values (64 bytes + 16, conflict-free
 // for 16-byte accesses), so that a store instruction writes whole 64-byte pieces of eight rows; straight
 // from the registers it would be 16 bytes of 32 rows (4 us per tile that nothing overlaps).  The tile is
@@ -306,21 +317,30 @@ constexpr int kT2RowPitch = 80;
 constexpr int kT2StageBytes = 49152;   // weights 2 x 16 KB, tokens 16 KB
 constexpr int kT2Acc = 2;
 
+// A group of K blocks' scales as the promotion warps read them.
+struct alignas(16) T2Slot {
+  float s[2][kTGroup][128];  // [feature block of the tile][K block][token row]: a_scale * w_scale
+};
 struct T2Ctrl {
   uint64_t full[kT2Stages];
   uint64_t empty[kT2Stages];
   uint64_t acc_full[kT2Acc];
   uint64_t acc_empty[kT2Acc];
+  uint64_t sf_full[kT2Slots];
+  uint64_t sf_empty[kT2Slots];
   uint32_t tmem_base;
   int abort_flag;
   float xchg[2][2][128];   // gated epilogue: group maxima exchanged between the two warps of a token row
   uint64_t xbar[4];        // ... and the barrier of each such pair of warps (one per lane quarter)
-  alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
+  alignas(16) T2Slot slot[kT2Slots];
+  // The CTA's tile i (first row, valid rows, feature tile, expert) at i % 4, written with its first
+  // group of scales: by then every warp has read a group of tile i - 2 or later, so it has finished i - 4.
+  int4 tile[4];
 };
 constexpr size_t kT2XposeBytes = 8 * 32 * kT2RowPitch;
-constexpr size_t kT2Smem = 1024 + (size_t)kT2Stages * kT2StageBytes + kT2XposeBytes +
-                           ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
-static_assert(kT2Smem <= kMaxSmem, "shared memory");
+// shared memory: the ring, the staging tiles, T2Ctrl, the tile walk
+constexpr size_t kT2Fixed = 1024 + kT2XposeBytes + ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
+static_assert(kT2Fixed + 3 * (size_t)kT2StageBytes + tile_walk_bytes(kMaxExperts) <= kMaxSmem, "shared memory");
 
 //
 // kGated (the first grouped GEMM of a SiLU layer with block-scaled fp8 experts): a tile pairs the
@@ -338,8 +358,10 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
                             const __grid_constant__ CUtensorMap tmap_w, const TParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint8_t* xpose_base = smem + kT2Stages * kT2StageBytes;
+  const int stages = p.stages;
+  uint8_t* xpose_base = smem + stages * kT2StageBytes;
   T2Ctrl* ctrl = reinterpret_cast<T2Ctrl*>(xpose_base + kT2XposeBytes);
+  uint8_t* walk_mem = reinterpret_cast<uint8_t*>(ctrl) + ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
   volatile int* abort_flag = &ctrl->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   // 256-feature tiles; gated: one tile per 128 gate features (p.n_tiles counts 128-feature blocks of n)
@@ -348,7 +370,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
 
   if (warp == 0) {
     pdl_wait();
-    build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, n_tiles2, ctrl->walk);
+    build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, n_tiles2, walk_mem);
     if (lane == 0) {
       ptx::prefetch_tensormap(&tmap_a);
       ptx::prefetch_tensormap(&tmap_w);
@@ -365,6 +387,10 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       ptx::mbar_init(&ctrl->acc_full[a], 1);
       ptx::mbar_init(&ctrl->acc_empty[a], 8);
     }
+    for (int g = 0; g < kT2Slots; ++g) {
+      ptx::mbar_init(&ctrl->sf_full[g], 2);
+      ptx::mbar_init(&ctrl->sf_empty[g], 8);
+    }
     for (int x = 0; x < 4; ++x) ptx::mbar_init(&ctrl->xbar[x], 2);
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
@@ -375,8 +401,10 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
   ptx::tc_fence_after();
 
   const uint32_t tmem_base = ctrl->tmem_base;
-  const TileWalk walk = tile_walk_at(ctrl->walk, p.num_experts);
+  const TileWalk walk = tile_walk_at(walk_mem, p.num_experts);
   const int total_tiles = walk.total;
+  const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
+  const uint32_t sf_full0 = ptx::smem_u32(&ctrl->sf_full[0]), sf_empty0 = ptx::smem_u32(&ctrl->sf_empty[0]);
 
   if (warp < 4) {
     ptx::setmaxnreg_dec<kT2LowRegs>();
@@ -407,7 +435,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
           }
           ptx::tma_load_2d_s(st + 32768, &tmap_a, full, kb * 128, ti.row0);
           st += kT2StageBytes;
-          if (++s == (uint32_t)kT2Stages) { s = 0; ph ^= 1; st = st0; }
+          if (++s == (uint32_t)stages) { s = 0; ph ^= 1; st = st0; }
         }
       }
     } else if (warp == 1 && ptx::elect_one()) {
@@ -431,8 +459,62 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
         ptx::umma_commit(empty0 + 8 * s);
         wdesc += kT2StageBytes >> 4;
         adesc += kT2StageBytes >> 4;
-        if (++s == (uint32_t)kT2Stages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
+        if (++s == (uint32_t)stages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
         if (++a == (uint32_t)kT2Acc) { a = 0; aph ^= 1; }
+      }
+    } else if (warp >= 2) {
+      // ------------------------------ scale preparers ---------------------------
+      const int ft = tid - 64, kbs = p.num_kb;            // 0..63: rows ft and ft + 64
+      const bool vec4_ok = (kbs % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.a_scale) & 15) == 0);
+      uint32_t slot = 0, ph = 1, seq = 0;
+      int cursor = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++seq) {
+        TileInfo ti;
+        locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
+        const int nb0 = kGated ? ti.n_tile : ti.n_tile * 2, nb1 = kGated ? ti.n_tile + up_block0 : nb0 + 1;
+        const float* w0 = p.w_scale + ((int64_t)ti.e * p.n_tiles + nb0) * kbs;
+        const float* w1 = w0 + (nb1 < p.n_tiles ? (int64_t)(nb1 - nb0) * kbs : 0);   // past N: any scale, the block's values are zero
+        for (int g = 0; g < n_groups; ++g) {
+          const int kb0 = g * kTGroup;
+          float4 av[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int row = ft + 64 * i;
+            const bool live = row < ti.valid;
+            const float* src = p.a_scale + (int64_t)(ti.row0 + row) * kbs + kb0;
+            if (vec4_ok) {
+              av[i] = live ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            } else {
+              av[i].x = live ? __ldg(src) : 0.f;
+              av[i].y = live && kb0 + 1 < kbs ? __ldg(src + 1) : 0.f;
+              av[i].z = live && kb0 + 2 < kbs ? __ldg(src + 2) : 0.f;
+              av[i].w = live && kb0 + 3 < kbs ? __ldg(src + 3) : 0.f;
+            }
+          }
+          float wv[2][kTGroup];
+#pragma unroll
+          for (int j = 0; j < kTGroup; ++j) {
+            const int kl = min(kb0 + j, kbs - 1);
+            wv[0][j] = __ldg(w0 + kl);
+            wv[1][j] = __ldg(w1 + kl);
+          }
+          if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, ph, abort_flag))) { ok = false; break; }
+          T2Slot* out = &ctrl->slot[slot];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const float rv[kTGroup] = {av[i].x, av[i].y, av[i].z, av[i].w};
+#pragma unroll
+            for (int j = 0; j < kTGroup; ++j) {
+              out->s[0][j][ft + 64 * i] = rv[j] * wv[0][j];
+              out->s[1][j][ft + 64 * i] = rv[j] * wv[1][j];
+            }
+          }
+          if (ft == 0 && g == 0) ctrl->tile[seq & 3] = make_int4(ti.row0, ti.valid, ti.n_tile, ti.e);
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_s(sf_full0 + 8 * slot);
+          if (++slot == kT2Slots) { slot = 0; ph ^= 1; }
+        }
       }
     }
   } else {
@@ -442,105 +524,88 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int r = q * 32 + lane;
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
     const int half = (warp - 4) >> 2;                  // which 128-feature block of the tile (gated: which 64 features of both)
-    const int kbs = p.num_kb;
-    const bool vec4_ok = (kbs % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.a_scale) & 15) == 0);
-    // combined scales a_scale[row, kb] * w_scale[block, kb] of a group of K blocks: s0 for this warp's
-    // (first) feature block, s1 (gated) for the up block
-    struct ScaleRegs { float s0[kTGroup]; float s1[kGated ? kTGroup : 1]; };
-    ScaleRegs cur, pre;
-    bool pre_valid = false;
-    auto fetch_group = [&](const TileInfo& tt, int g, ScaleRegs& sr) {
-      const int kb0 = g * kTGroup;
-      const int nb = kGated ? tt.n_tile : tt.n_tile * 2 + half;
-      const int64_t wsb = ((int64_t)tt.e * p.n_tiles + nb) * kbs + kb0;
-      float av[kTGroup];
-      const bool live = r < tt.valid;
-      const float* src = p.a_scale + (int64_t)(tt.row0 + r) * kbs + kb0;
-      if (live && vec4_ok) {
-        const float4 q4 = *reinterpret_cast<const float4*>(src);
-        av[0] = q4.x; av[1] = q4.y; av[2] = q4.z; av[3] = q4.w;
-      } else {
-#pragma unroll
-        for (int jb = 0; jb < kTGroup; ++jb) av[jb] = (live && kb0 + jb < kbs) ? src[jb] : 0.f;
-      }
-#pragma unroll
-      for (int jb = 0; jb < kTGroup; ++jb)
-        sr.s0[jb] = av[jb] * ((nb < p.n_tiles && kb0 + jb < kbs) ? p.w_scale[wsb + jb] : 0.f);
-      if (kGated) {
-        const int64_t wsb2 = ((int64_t)tt.e * p.n_tiles + up_block0 + tt.n_tile) * kbs + kb0;
-#pragma unroll
-        for (int jb = 0; jb < kTGroup; ++jb)
-          sr.s1[kGated ? jb : 0] = av[jb] * ((kb0 + jb < kbs) ? p.w_scale[wsb2 + jb] : 0.f);
-      }
-    };
-    uint32_t a = 0, aph = 0, xpar = 0;
-    const uint32_t acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
-    int cursor = 0;
+    uint32_t a = 0, aph = 0, slot = 0, sph = 0, xpar = 0;
+    // one shared address, the rest are constants from there (registers are full)
+    const uint32_t cs = ptx::smem_u32(ctrl);
+    constexpr uint32_t kAccFull = offsetof(T2Ctrl, acc_full), kAccEmpty = offsetof(T2Ctrl, acc_empty);
+    constexpr uint32_t kSfFull = offsetof(T2Ctrl, sf_full), kSfEmpty = offsetof(T2Ctrl, sf_empty), kSlot = offsetof(T2Ctrl, slot);
     bool ok = true;
-    const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-      TileInfo ti;
-      locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
-      float acc[128];
+    const int my_tiles = (int)blockIdx.x < total_tiles ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    // A K block's scales are read when its first chunk is asked for, without a branch.
+    float sc0 = 0.f, sc1 = 0.f;
+    uint32_t jb = 0;                                   // position in the slot
+    const uint32_t my_scales = cs + kSlot + (kGated ? 0 : half * kTGroup * 512) + r * 4;
+    auto read_scales = [&](bool last) {                // `last`: the tile's last K block
+      const uint32_t at = my_scales + slot * (uint32_t)sizeof(T2Slot) + jb * 512;
+      sc0 = ptx::lds32f(at);
+      if (kGated) sc1 = ptx::lds32f(at + kTGroup * 512);
+      const bool done = jb == kTGroup - 1 || last;
+      ptx::mbar_arrive_if(cs + kSfEmpty + 8 * slot, done && lane == 0);   // (the warp is converged: its reads come first)
+      jb = done ? 0u : jb + 1;
+      slot ^= done ? 1u : 0u;
+      sph ^= done && slot == 0 ? 1u : 0u;
+    };
+    static_assert(kT2Slots == 2, "slot parity");
+    auto wait_block = [&]() {                          // the stage and the scales of the next K block
+      return __all_sync(0xffffffffu, ptx::mbar_wait_inline_s(cs + kAccFull + 8 * a, aph, abort_flag) &&
+                                         ptx::mbar_wait_inline_s(cs + kSfFull + 8 * slot, sph, abort_flag));
+    };
+    // Chunks of 32 columns (chunk c of a stage -> acc[16 c ..]).  plain: the 128 columns of this warp's
+    // block; gated: 64 gate columns, then the 64 up columns of the same features.
+    const uint32_t col_base = tmem_base + (kGated ? half * 64 : half * 128) + lane_sel;
+    constexpr uint32_t kSecond = kGated ? 128 : 64;
+    for (int tile = 0; tile < my_tiles && ok; ++tile) {
+      float2 acc[64];
 #pragma unroll
-      for (int i = 0; i < 128; ++i) acc[i] = 0.f;
+      for (int i = 0; i < 64; ++i) acc[i] = make_float2(0.f, 0.f);
       uint32_t va[32], vb[32];
-      if (!pre_valid) fetch_group(ti, 0, cur);
-      else cur = pre;
-      pre_valid = false;
-      for (int g = 0; g < n_groups && ok; ++g) {
-        if (g + 1 < n_groups) {
-          fetch_group(ti, g + 1, pre);
-        } else if (t + (int)gridDim.x < total_tiles) {
-          int cursor2 = cursor;
-          TileInfo tn;
-          locate_tile<kTTok>(walk, t + gridDim.x, cursor2, tn, p.w_experts);
-          fetch_group(tn, 0, pre);
-          pre_valid = true;
-        }
-#pragma unroll
-        for (int jb = 0; jb < kTGroup; ++jb) {
-          if (g * kTGroup + jb >= p.num_kb) break;
-          const float sc0 = cur.s0[jb];
-          const float sc1 = kGated ? cur.s1[kGated ? jb : 0] : sc0;
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->acc_full[a], aph, abort_flag))) {
-            *abort_flag = 1; ok = false; break;
-          }
+      if (!wait_block()) { ok = false; break; }
+      ptx::tc_fence_after();
+      ptx::tmem_ld_32x32(col_base + a * 256, va);
+      read_scales(p.num_kb == 1);
+#pragma unroll 1
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        const uint32_t col = col_base + a * 256, empty = cs + kAccEmpty + 8 * a;
+        const bool more = kb + 1 < p.num_kb;
+        const float c0 = sc0, c1 = kGated ? sc1 : sc0;
+        if (++a == (uint32_t)kT2Acc) { a = 0; aph ^= 1; }
+        ptx::tmem_wait_ld_one(va);
+        ptx::tmem_ld_32x32(col + 32, vb);
+        ptx::fma_f32x2(acc, va, c0);
+        ptx::tmem_wait_ld_one(vb);
+        ptx::tmem_ld_32x32(col + kSecond, va);
+        ptx::fma_f32x2(acc + 16, vb, c0);
+        ptx::tmem_wait_ld_one(va);
+        ptx::tmem_ld_32x32(col + kSecond + 32, vb);
+        const bool ready = ptx::mbar_test_wait_s(cs + kAccFull + 8 * a, aph) & ptx::mbar_test_wait_s(cs + kSfFull + 8 * slot, sph);
+        ptx::fma_f32x2(acc + 32, va, c1);
+        ptx::tmem_wait_ld_one(vb);
+        ptx::tc_fence_before();   // the whole stage is in registers
+        __syncwarp();
+        ptx::mbar_arrive_if(empty, lane == 0);
+        if (more) {
+          if (!__all_sync(0xffffffffu, ready) && !wait_block()) { ok = false; break; }
           ptx::tc_fence_after();
-          // plain: the 128 columns of this warp's block in two passes; gated: 64 gate columns, then
-          // the 64 up columns of the same features
-          const uint32_t col = tmem_base + a * 256 + (kGated ? half * 64 : half * 128) + lane_sel;
-#pragma unroll
-          for (int pass = 0; pass < 2; ++pass) {
-            const float sc = pass == 0 ? sc0 : sc1;
-            ptx::tmem_ld_32x32(col + pass * (kGated ? 128 : 64), va);
-            ptx::tmem_ld_32x32(col + pass * (kGated ? 128 : 64) + 32, vb);
-            ptx::tmem_wait_ld_tied(va, vb);
-            if (pass == 1) {   // the whole stage is in registers
-              ptx::tc_fence_before();
-              __syncwarp();
-              if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);
-              if (++a == (uint32_t)kT2Acc) { a = 0; aph ^= 1; }
-            }
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              acc[pass * 64 + i] = fmaf(__uint_as_float(va[i]), sc, acc[pass * 64 + i]);
-              acc[pass * 64 + 32 + i] = fmaf(__uint_as_float(vb[i]), sc, acc[pass * 64 + 32 + i]);
-            }
-          }
+          ptx::tmem_ld_32x32(col_base + a * 256, va);
+          read_scales(kb + 2 == p.num_kb);
         }
-        if (g + 1 < n_groups) cur = pre;
+        ptx::fma_f32x2(acc + 48, vb, c1);
       }
+      if (!ok) { ptx::tmem_wait_ld(); break; }
+      const int4 here = ctrl->tile[tile & 3];
+      TileInfo ti;
+      ti.row0 = here.x; ti.valid = here.y; ti.n_tile = here.z; ti.e = here.w;
+      auto value = [&](int i) -> float& { return (i & 1) ? acc[i >> 1].y : acc[i >> 1].x; };
       if (kGated) {
-        // acc[0..64) = gate, acc[64..128) = up of features j0 + half * 64 ..
+        // values 0..63 = gate, 64..127 = up of features j0 + half * 64 ..
         const int half_n = p.n >> 1;
         const int j0 = ti.n_tile * 128 + half * 64;
         float amax = 0.f;
-        // acc[i] becomes the activated value of feature j0 + i (the up half is consumed)
+        // value(i) becomes the activated value of feature j0 + i (the up half is consumed)
         auto activate = [&](auto round16) {
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
-            float g = acc[i], u = acc[64 + i];
+            float g = value(i), u = value(64 + i);
             if (p.bias != nullptr) {
               g += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + j0 + i);
               u += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + half_n + j0 + i);
@@ -552,8 +617,8 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
               g = round16(fminf(g, p.clamp));
               u = round16(fminf(fmaxf(u, -p.clamp), p.clamp));
             }
-            acc[i] = __fmul_rn(__fdividef(g, 1.0f + __expf(-g)), u);
-            amax = fmaxf(amax, fabsf(acc[i]));
+            value(i) = __fmul_rn(__fdividef(g, 1.0f + __expf(-g)), u);
+            amax = fmaxf(amax, fabsf(value(i)));
           }
         };
         if (p.out_f16) activate([](float x) { return __half2float(__float2half_rn(x)); });
@@ -579,7 +644,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
               uint32_t x = 0;
 #pragma unroll
               for (int b = 0; b < 4; ++b)
-                x |= (uint32_t)f32_to_e4m3(fmaxf(-448.0f, fminf(__fdividef(acc[c + i + b], scale), 448.0f))) << (8 * b);
+                x |= (uint32_t)f32_to_e4m3(fmaxf(-448.0f, fminf(__fdividef(value(c + i + b), scale), 448.0f))) << (8 * b);
               w[i >> 2] = x;
             }
             ptx::sts128(my_row + c, make_uint4(w[0], w[1], w[2], w[3]));
@@ -608,7 +673,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
         auto packed = [&](int c, uint32_t (&w)[4]) {
 #pragma unroll
           for (int i = 0; i < 8; i += 2) {
-            float x0 = acc[c + i], x1 = acc[c + i + 1];
+            float x0 = value(c + i), x1 = value(c + i + 1);
             if (p.bias != nullptr) {
               x0 += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + f0 + c + i);
               x1 += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + f0 + c + i + 1);
@@ -660,11 +725,14 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 template <bool kWKn, bool kGated>
-int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, const TParams& p, int grid, cudaStream_t st) {
+int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, TParams& p, int grid, cudaStream_t st) {
   auto kern = grouped_gemm_fp8t256_kernel<kWKn, kGated>;
+  const size_t fixed = kT2Fixed + tile_walk_bytes(p.num_experts);
+  p.stages = fixed + kT2Stages * (size_t)kT2StageBytes <= kMaxSmem ? kT2Stages : 3;
+  const size_t smem = fixed + p.stages * (size_t)kT2StageBytes;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, kT2Smem)) return rc;
-  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), kT2Smem, st, ta, tw, p));
+  if (int rc = configured.ensure(kern, smem)) return rc;
+  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), smem, st, ta, tw, p));
   return B200MOE_OK;
 }
 

@@ -77,6 +77,18 @@ __device__ __forceinline__ bool mbar_try_wait_s(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// One look, without the suspension a try_wait may take.
+__device__ __forceinline__ bool mbar_test_wait_s(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 static __device__ __noinline__ bool mbar_wait_rest(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   const long long t0 = clock64();
   uint32_t spins = 0;
@@ -113,6 +125,12 @@ __device__ __forceinline__ bool mbar_wait_inline_s(uint32_t bar, uint32_t parity
 }
 __device__ __forceinline__ void mbar_arrive_s(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// ... by the lanes for which `p` holds, without a branch
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool p) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar),
+               "r"((uint32_t)p)
+               : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
@@ -168,13 +186,6 @@ __device__ __forceinline__ void tma_load_3d_s(uint32_t dst, const CUtensorMap* m
       " [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
-}
-
-// Brings a tile into L2 only.
-__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];"
-               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
 }
 
 // ---- CTA pairs (a cluster of two CTAs working on one tcgen05.mma tile) ----------------
@@ -523,6 +534,26 @@ __device__ __forceinline__ void umma_mx_block_ts(uint32_t tmem_d, uint32_t tmem_
       ::"r"(tmem_d), "r"(tmem_w), "l"(adesc), "r"(idesc), "r"(sfw), "r"(sfa), "r"(accumulate)
       : "memory");
 }
+// Waits for this thread's tcgen05.ld and makes `r` depend on it.
+__device__ __forceinline__ void tmem_wait_ld_one(uint32_t (&r)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
+                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15]),
+                 "+r"(r[16]), "+r"(r[17]), "+r"(r[18]), "+r"(r[19]), "+r"(r[20]), "+r"(r[21]), "+r"(r[22]),
+                 "+r"(r[23]), "+r"(r[24]), "+r"(r[25]), "+r"(r[26]), "+r"(r[27]), "+r"(r[28]), "+r"(r[29]),
+                 "+r"(r[30]), "+r"(r[31])
+               :
+               : "memory");
+}
+// acc[i] += v[i] * s for 32 values, two per instruction (each rounded as fmaf rounds it).
+__device__ __forceinline__ void fma_f32x2(float2* acc, const uint32_t (&v)[32], float s) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i)
+    asm volatile("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%0, %1};\n\t"
+        "fma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "+f"(acc[i].x), "+f"(acc[i].y)
+        : "r"(v[2 * i]), "r"(v[2 * i + 1]), "f"(s));
+}
 // umma_block's four kind::f16 instructions with the 128-row operand in tensor memory (eight columns per
 // K step, the other operand 32 bytes).
 __device__ __forceinline__ void umma_f16_block_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
@@ -595,6 +626,11 @@ __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
 }
 __device__ __forceinline__ void sts32f(uint32_t addr, float v) {
   asm volatile("st.shared.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
+}
+__device__ __forceinline__ float lds32f(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
 }
 __device__ __forceinline__ float4 lds128f(uint32_t addr) {
   float4 v;
