@@ -540,7 +540,8 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       sc0 = ptx::lds32f(at);
       if (kGated) sc1 = ptx::lds32f(at + kTGroup * 512);
       const bool done = jb == kTGroup - 1 || last;
-      ptx::mbar_arrive_if(cs + kSfEmpty + 8 * slot, done && lane == 0);   // (the warp is converged: its reads come first)
+      __syncwarp();   // lane 0's arrival hands the slot back for all lanes: their reads come first
+      ptx::mbar_arrive_if(cs + kSfEmpty + 8 * slot, done && lane == 0);
       jb = done ? 0u : jb + 1;
       slot ^= done ? 1u : 0u;
       sph ^= done && slot == 0 ? 1u : 0u;
