@@ -286,7 +286,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t src0 = ptx::smem_u32(smem) + row * 64;
     const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;      // 64-byte swizzle: chunk index xor row bits 1..2
-    uint32_t s = set, ph = 0;                                   // (at least kI4Sets stages)
+    uint32_t s = set, ph = 0;
     const uint32_t blocks = (uint32_t)my_tiles * p.num_kb;      // every tile: the same K loop
     for (uint32_t i = set; i < blocks; i += kI4Sets) {
       const uint32_t c = i % kI4Conv;
@@ -451,7 +451,11 @@ int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
     if (int rc = encode_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B))
       return rc;
   }
-  const int fixed = 1024 + kI4Slots * S::kSlotBytes + (int)((sizeof(I4Ctrl) + 15) & ~(size_t)15) + tile_walk_bytes(p.num_experts);
+  constexpr int kFixed = 1024 + kI4Slots * S::kSlotBytes + (int)((sizeof(I4Ctrl) + 15) & ~(size_t)15);
+  constexpr int kLeast = ((int)kMaxSmem - kFixed - tile_walk_bytes(kMaxExperts)) / S::kStageBytes;
+  constexpr int kDepth = converter_ring_depth(kI4Sets, kI4Conv);
+  static_assert(kLeast >= kDepth && kI4MaxStages >= kDepth && kI4Sets <= kI4Conv, "ring depth that the converters' waits need");
+  const int fixed = kFixed + tile_walk_bytes(p.num_experts);
   p.stages = ((int)kMaxSmem - fixed) / S::kStageBytes;
   if (p.stages > kI4MaxStages) p.stages = kI4MaxStages;
   const size_t smem = (size_t)fixed + (size_t)p.stages * S::kStageBytes;
