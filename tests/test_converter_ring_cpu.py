@@ -63,6 +63,7 @@ def test_ring_depth_that_parity_waits_need(sets, operands):
 
 @pytest.mark.parametrize("source,planted", [
     ("gemm_tc_i4.cu", ("constexpr int kI4MaxStages = 12;", "constexpr int kI4MaxStages = 6;")),
+    ("gemm_tc_dq.cu", ("kDqMaxRaw = 12,", "kDqMaxRaw = 8,")),
 ])
 def test_kernels_with_a_shorter_ring_do_not_compile(tmp_path, source, planted):
     nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"

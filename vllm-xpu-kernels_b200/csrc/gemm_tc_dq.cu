@@ -372,7 +372,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
     if (t < total_tiles) { enter_tile(); settle(); }
     Scales nxt;
     if (t < total_tiles) nxt = load_scales();
-    uint32_t s = set, ph = 0;                       // (at least kSets raw stages)
+    uint32_t s = set, ph = 0;
     uint32_t c = (set * kHalves) % kSlots, cph = 1 ^ (((set * kHalves) / kSlots) & 1);
     while (t < total_tiles) {
       const Scales cur = nxt;
@@ -523,12 +523,15 @@ int launch_dq(const b200moe_gemm_args* a, DqParams& p, cudaStream_t st) {
   }
   // Shared memory: the weights of small tiles stream at HBM's rate and get most of it, the tokens of
   // large ones (32 KB per 64 K) what four raw stages leave.
-  const int room = (int)kMaxSmem - 1024 - (int)((sizeof(DqCtrl) + 15) & ~(size_t)15);
-  p.tok_stages = BT > 64 ? (room - 4 * kDqRawBytes) / S::kTokBytes : 6;
-  if (p.tok_stages > kDqMaxTok) p.tok_stages = kDqMaxTok;
-  p.raw_stages = (room - p.tok_stages * S::kTokBytes) / kDqRawBytes;
-  if (p.raw_stages > kDqMaxRaw) p.raw_stages = kDqMaxRaw;
-  const size_t smem = kMaxSmem - room + (size_t)p.tok_stages * S::kTokBytes + (size_t)p.raw_stages * kDqRawBytes;
+  constexpr int kRoom = (int)kMaxSmem - 1024 - (int)((sizeof(DqCtrl) + 15) & ~(size_t)15);
+  constexpr int kTokFit = BT > 64 ? (kRoom - 4 * kDqRawBytes) / S::kTokBytes : 6;
+  constexpr int kTok = kTokFit < kDqMaxTok ? kTokFit : kDqMaxTok;
+  constexpr int kRawFit = (kRoom - kTok * S::kTokBytes) / kDqRawBytes;
+  constexpr int kRaw = kRawFit < kDqMaxRaw ? kRawFit : kDqMaxRaw;
+  static_assert(kRaw >= converter_ring_depth(S::kSets, S::kSlots / S::kHalves), "ring depth that the converters' waits need");
+  p.tok_stages = kTok;
+  p.raw_stages = kRaw;
+  constexpr size_t smem = kMaxSmem - kRoom + (size_t)kTok * S::kTokBytes + (size_t)kRaw * kDqRawBytes;
   static SmemConfig configured;
   if (int rc = configured.ensure(kern, smem)) return rc;
   const int64_t tile_bound = ((a->m + BT - 1) / BT + a->num_experts) * (int64_t)p.n_tiles;
