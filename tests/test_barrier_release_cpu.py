@@ -28,3 +28,13 @@ def test_lane_0_arrives_for_its_warp_after_a_warp_barrier(path):
             assert before == "__syncwarp();", f"{path.name}:{i}: {code}"
         before = code
     assert arrivals > 0
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_tensor_memory_waits_name_the_registers_they_wait_for(path):
+    """A tcgen05.ld fills its registers after the statement; only a wait that takes them as operands keeps
+    the compiler from using them earlier.  (A wait without any is for leaving: nothing is used.)"""
+    loads = [code for _, code in _statements(path) if "tmem_ld_32x" in code]
+    waits = [code for _, code in _statements(path) if re.search(r"tmem_wait_ld\w*\(", code)]
+    assert loads and waits
+    assert not [w for w in waits if "tmem_wait_ld()" in w and "break;" not in w]

@@ -312,7 +312,8 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
               if (kChunk == 32) ptx::tmem_ld_32x32(col + BT, reinterpret_cast<uint32_t(&)[32]>(vu));
               else ptx::tmem_ld_32x16(col + BT, reinterpret_cast<uint32_t(&)[16]>(vu));
             }
-            ptx::tmem_wait_ld();
+            if (kGated) ptx::tmem_wait_ld(v, vu);
+            else ptx::tmem_wait_ld(v);
             float vals[kChunk];
 #pragma unroll
             for (int i = 0; i < kChunk; ++i) {
@@ -396,7 +397,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
               if (col0 + c0 < ti.valid) {
                 if (kChunk == 32) ptx::tmem_ld_32x32(tmem_base + a * BT + col0 + c0 + lane_sel, reinterpret_cast<uint32_t(&)[32]>(v));
                 else ptx::tmem_ld_32x16(tmem_base + a * BT + col0 + c0 + lane_sel, reinterpret_cast<uint32_t(&)[16]>(v));
-                ptx::tmem_wait_ld();
+                ptx::tmem_wait_ld(v);
               }
               if (last_chunk) {  // the stage is free as soon as its last column is in registers
                 ptx::tc_fence_before();
@@ -643,7 +644,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         if (c0 < ti.valid) {
           uint32_t v[kChunk];
           ptx::tmem_ld_32x32(tmem_base + a * kPairTok + c0 + lane_sel, v);
-          ptx::tmem_wait_ld();
+          ptx::tmem_wait_ld(v);
           float vals[kChunk];
 #pragma unroll
           for (int i = 0; i < kChunk; ++i) vals[i] = __uint_as_float(v[i]) + bias_v;

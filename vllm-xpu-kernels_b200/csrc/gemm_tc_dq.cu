@@ -448,8 +448,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
             uint32_t v[kChunk];
             if (kChunk == 32) ptx::tmem_ld_32x32(tmem_base + a * kUnit + c0 + lane_sel, reinterpret_cast<uint32_t(&)[32]>(v));
             else ptx::tmem_ld_32x16(tmem_base + a * kUnit + c0 + lane_sel, reinterpret_cast<uint32_t(&)[16]>(v));
-            ptx::tmem_wait_ld();
-            ptx::pin_registers(v);
+            ptx::tmem_wait_ld(v);
             float vals[kChunk];
 #pragma unroll
             for (int i = 0; i < kChunk; ++i) vals[i] = __uint_as_float(v[i]) + bias_v;

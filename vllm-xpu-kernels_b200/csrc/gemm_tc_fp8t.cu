@@ -231,7 +231,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
           // both halves in flight together, one wait: tcgen05.wait::ld covers every load before it
           ptx::tmem_ld_32x32(tmem_base + a * 128 + col0 + lane_sel, va);
           ptx::tmem_ld_32x32(tmem_base + a * 128 + col0 + 32 + lane_sel, vb);
-          ptx::tmem_wait_ld_tied(va, vb);
+          ptx::tmem_wait_ld(va, vb);
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);   // the stage is in registers

@@ -381,8 +381,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             const uint32_t col = tmem_base + a * BT + col0 + lane_sel;
             if (kHalf == 16) ptx::tmem_ld_32x16(col, reinterpret_cast<uint32_t(&)[16]>(v));
             else ptx::tmem_ld_32x8(col, reinterpret_cast<uint32_t(&)[8]>(v));
-            ptx::tmem_wait_ld();
-            ptx::pin_registers(v);
+            ptx::tmem_wait_ld(v);
           }
           ptx::tc_fence_before();
           __syncwarp();

@@ -543,7 +543,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
             const uint32_t col = tmem_base + a * kNT + term * BT + c0 + lane_sel;
             if (kChunk == 32) ptx::tmem_ld_32x32(col, reinterpret_cast<uint32_t(&)[32]>(v));
             else ptx::tmem_ld_32x16(col, reinterpret_cast<uint32_t(&)[16]>(v));
-            ptx::tmem_wait_ld();
+            ptx::tmem_wait_ld(v);
 #pragma unroll
             for (int i = 0; i < kChunk; ++i) acc[i] += __uint_as_float(v[i]);
           }

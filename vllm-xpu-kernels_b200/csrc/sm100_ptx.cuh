@@ -313,9 +313,6 @@ __device__ __forceinline__ void tc_fence_before() {
 __device__ __forceinline__ void tc_fence_after() {
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 }
-__device__ __forceinline__ void tmem_wait_ld() {
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
 // 32 lanes x 32 consecutive 32-bit columns: thread i gets lane (base lane + i).
 __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
@@ -341,12 +338,6 @@ __device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16])
       : "memory");
 }
 
-// Registers filled by a tcgen05.ld, after its wait: no use of them is scheduled ahead of this point.
-template <int N>
-__device__ __forceinline__ void pin_registers(uint32_t (&r)[N]) {
-#pragma unroll
-  for (int i = 0; i < N; ++i) asm volatile("" : "+r"(r[i]));
-}
 __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -355,25 +346,17 @@ __device__ __forceinline__ void tmem_ld_32x8(uint32_t taddr, uint32_t (&r)[8]) {
       : "memory");
 }
 
-// tcgen05.wait::ld for loads that were issued earlier and whose destination
-// registers the code in between did not touch: the registers are operands of the
-// wait, so that no later use of them can be scheduled ahead of it.
-__device__ __forceinline__ void tmem_wait_ld_tied(uint32_t (&r)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]),
-                 "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]),
-                 "+r"(r[15])
-               :
-               : "memory");
-}
-// The same for two 32-register loads in flight together.  The second statement emits
-// nothing; it only makes every later use of the second array depend on a point after
-// the wait (volatile asm statements keep their order).
-__device__ __forceinline__ void tmem_wait_ld_tied(uint32_t (&r)[32], uint32_t (&q)[32]) {
-#define B200_R8(a, i) "+r"(a[i]), "+r"(a[i + 1]), "+r"(a[i + 2]), "+r"(a[i + 3]), "+r"(a[i + 4]), "+r"(a[i + 5]), "+r"(a[i + 6]), "+r"(a[i + 7])
-  asm volatile("tcgen05.wait::ld.sync.aligned;" : B200_R8(r, 0), B200_R8(r, 8), B200_R8(r, 16), B200_R8(r, 24) : : "memory");
-  asm volatile("" : B200_R8(q, 0), B200_R8(q, 8), B200_R8(q, 16), B200_R8(q, 24) : : "memory");
-#undef B200_R8
+// Waits for all of this thread's tcgen05.ld.  The registers they filled are operands of a statement behind
+// the wait (it emits nothing; volatile asm statements keep their order), so that no use of them is scheduled
+// ahead of it.
+template <int... N>
+__device__ __forceinline__ void tmem_wait_ld(uint32_t (&...r)[N]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+  auto pin = [](auto& a) {
+#pragma unroll
+    for (uint32_t& x : a) asm volatile("" : "+r"(x));
+  };
+  (pin(r), ...);
 }
 // Register re-balancing between the warpgroups of a CTA (every warp of a warpgroup
 // executes the same one): dec gives registers back to the CTA's pool, inc waits until
