@@ -884,7 +884,10 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
                          : (kn ? launch_tc_pair<true, false>(ta_half, tw, p, max_pairs, st)
                                : launch_tc_pair<false, false>(ta_half, tw, p, max_pairs, st));
     if (rc != B200MOE_E_UNSUPPORTED) return rc;
-    if (gated) bt = 128;   // no clusters on this device: the single-CTA gated tile
+    // no clusters on this device: the single-CTA form, from the start (its gated tile has other boxes)
+    b200moe_gemm_args single = *a;
+    single.impl = 3;
+    return grouped_gemm_tc(&single, st);
   }
 
   if (tile_bound < grid) grid = (int)tile_bound;
