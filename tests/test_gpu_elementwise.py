@@ -1,9 +1,11 @@
 """GPU parity: gated activations, dynamic per-group fp8 quantisation, moe_gather
 and moe_sum against the torch oracle, with the reference's tolerances."""
+import ctypes
+
 import pytest
 import torch
 
-from conftest import load_golden
+from conftest import PKG_DIR, load_golden
 from gpu_utils import DEV
 from oracle import torch_oracle as to
 
@@ -126,3 +128,18 @@ def test_moe_sum_input_validation(native):
     with pytest.raises(RuntimeError, match="expert_map must be int32"):
         torch.ops._moe_C.moe_sum(x, out, torch.zeros(4, 2, dtype=torch.int32, device=DEV),
                                  torch.zeros(4, dtype=torch.int64, device=DEV))
+
+
+def test_a_refused_launch_is_reported_once(native):
+    """A launch that the runtime refuses (more rows than a grid has blocks; nothing runs) fails by itself and
+    leaves no error behind that a later, good call would report."""
+    lib = ctypes.CDLL(str(PKG_DIR / "vllm_xpu_kernels" / "libb200moe.so"))
+    lib.b200moe_last_error.restype = ctypes.c_char_p
+    x = torch.zeros(16, dtype=torch.bfloat16, device=DEV)
+    status = torch.zeros(1, dtype=torch.int32, device=DEV)
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    rc = lib.b200moe_silu_and_mul(p(x), p(x), 2, ctypes.c_int64(1 << 31), 8, None)
+    assert rc == -3 and b"launch of silu_and_mul_kernel failed" in lib.b200moe_last_error()
+    rc = lib.b200moe_selftest_bounded_wait(p(status), ctypes.c_int64(1000000), None)
+    assert rc == 0, lib.b200moe_last_error()
+    torch.cuda.synchronize()

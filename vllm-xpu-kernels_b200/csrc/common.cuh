@@ -23,12 +23,16 @@ int fail(int code, const char* fmt, ...);
     if (!(cond)) return ::b200moe::fail(B200MOE_E_BADARG, __VA_ARGS__); \
   } while (0)
 
+// An error that a call returns also stays behind as the thread's last error, which the next
+// B200_LAUNCH_OK would take for its own: it is cleared where it is reported.
 #define B200_CUDA_OK(expr)                                                     \
   do {                                                                         \
     cudaError_t e__ = (expr);                                                  \
-    if (e__ != cudaSuccess)                                                    \
+    if (e__ != cudaSuccess) {                                                  \
+      (void)cudaGetLastError();                                                \
       return ::b200moe::fail(B200MOE_E_CUDA, "%s failed: %s", #expr,          \
                              cudaGetErrorString(e__));                         \
+    }                                                                          \
   } while (0)
 
 #define B200_LAUNCH_OK(name)                                                   \
@@ -66,9 +70,11 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
 #define B200_LAUNCHED(name, ...)                                               \
   do {                                                                         \
     cudaError_t e__ = (__VA_ARGS__);                                           \
-    if (e__ != cudaSuccess)                                                    \
+    if (e__ != cudaSuccess) {                                                  \
+      (void)cudaGetLastError();                                                \
       return ::b200moe::fail(B200MOE_E_CUDA, "launch of %s failed: %s", name, \
                              cudaGetErrorString(e__));                         \
+    }                                                                          \
   } while (0)
 
 inline cudaStream_t as_stream(b200moe_stream s) { return (cudaStream_t)s; }
