@@ -1,0 +1,73 @@
+"""The layer calls' workspaces: one per stream, given back, never shared by calls that may run at the same
+time.  Results are compared bit for bit with the same call made alone (the layer is deterministic)."""
+import gc
+
+import pytest
+import torch
+
+from gpu_utils import DEV
+
+pytestmark = pytest.mark.gpu
+
+E, K, H, I = 8, 2, 512, 256
+SIZES = [1, 7, 40, 130, 400]
+
+
+def _layer(native, seed=0, **kw):
+    g = torch.Generator().manual_seed(seed)
+    w13 = (torch.randn(E, H, 2 * I, generator=g) * H ** -0.5).to(torch.bfloat16).to(DEV)
+    w2 = (torch.randn(E, I, H, generator=g) * I ** -0.5).to(torch.bfloat16).to(DEV)
+    return native.XpuFusedMoe(w13, None, None, w2, None, None, K, "silu", E, **kw)
+
+
+def _call(T, seed=0):
+    """(output, hidden states, routing weights, ids) of a call with T tokens."""
+    g = torch.Generator().manual_seed(1000 * seed + T)
+    w, ids = torch.topk(torch.softmax(torch.randn(T, E, generator=g), -1), k=K, dim=-1)
+    return (torch.empty(T, H, dtype=torch.bfloat16, device=DEV),
+            torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV), w.to(DEV), ids.int().to(DEV))
+
+
+def _alone(native, layer, call):
+    out = torch.empty_like(call[0])
+    layer.apply(out, *call[1:])
+    torch.cuda.synchronize()
+    return out
+
+
+def _in_use():
+    gc.collect()
+    torch.cuda.synchronize()
+    return torch.cuda.memory_allocated()
+
+
+def test_graphs_replay_beside_other_calls_and_give_their_memory_back(native):
+    """Two graphs captured on one stream and replayed at the same time on two others, beside calls made on
+    the stream of the capture; their intermediates go with them."""
+    layer = _layer(native)
+    calls = [_call(T) for T in (400, 130, 40)]
+    want = [_alone(native, layer, c) for c in calls]
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        layer.apply(*calls[2])
+    before = _in_use()
+    graphs = [torch.cuda.CUDAGraph() for _ in range(2)]
+    for graph, call in zip(graphs, calls):
+        with torch.cuda.graph(graph, stream=side):
+            layer.apply(*call)
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for _ in range(20):
+        for c in calls:
+            c[0].fill_(float("nan"))
+        torch.cuda.synchronize()
+        for _ in range(5):
+            for graph, stream in zip(graphs, streams):
+                with torch.cuda.stream(stream):
+                    graph.replay()
+            with torch.cuda.stream(side):
+                layer.apply(*calls[2])
+        torch.cuda.synchronize()
+        for c, ref in zip(calls, want):
+            assert torch.equal(c[0], ref)
+    del graphs, graph
+    assert _in_use() == before

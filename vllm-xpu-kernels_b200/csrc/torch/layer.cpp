@@ -17,7 +17,6 @@
 #include <memory>
 #include <mutex>
 #include <utility>
-#include <vector>
 
 namespace b200shim {
 namespace {
@@ -50,47 +49,41 @@ const char* const kPlanName = "b200moe.layer_plan";
 // One grow-only buffer per (device, stream), shared by all layers: the calls of a stream run one
 // after the other, so the next one may overwrite what the previous one left.  At most kMaxSlabs
 // streams keep one (the least recently used is given back).  All are given back with the last layer
-// object, but for buffers that a CUDA graph has captured, which stay until workspace_clear().
+// object.  A call under stream capture takes its memory from the graph's pool instead: a graph is
+// replayed on any stream, beside later calls on the one it was captured on and beside other graphs,
+// and what it uses has to live as long as it does.
 constexpr size_t kMaxSlabs = 8;
 struct Slab {
   at::Tensor mem;
   uint64_t used = 0;
-  bool captured = false;
 };
 std::mutex g_mutex;
 auto& g_slabs = *new std::map<std::pair<int, int64_t>, Slab>();   // (never destroyed: CUDA may be gone at exit)
-auto& g_captured = *new std::vector<at::Tensor>();
 uint64_t g_tick = 0;
 int64_t g_plans = 0;
 
-void clear_slabs(bool captured_too) {
+void clear_slabs() {
   std::lock_guard<std::mutex> lock(g_mutex);
-  for (auto it = g_slabs.begin(); it != g_slabs.end();)
-    it = (captured_too || !it->second.captured) ? g_slabs.erase(it) : std::next(it);
-  if (captured_too) g_captured.clear();
+  g_slabs.clear();
 }
 
 at::Tensor workspace(const c10::cuda::CUDAStream& stream, size_t bytes, bool persistent) {
   const auto options = at::TensorOptions().dtype(at::kByte).device(stream.device());
-  if (!persistent) return at::empty({(int64_t)bytes}, options);
+  if (!persistent || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
+    return at::empty({(int64_t)bytes}, options);
   std::lock_guard<std::mutex> lock(g_mutex);
   const std::pair<int, int64_t> key(stream.device_index(), (int64_t)stream.id());
   Slab& slab = g_slabs[key];
   if (!slab.mem.defined() || (size_t)slab.mem.numel() < bytes) {
-    if (slab.captured) g_captured.push_back(slab.mem);
-    slab.captured = false;
     slab.mem = at::Tensor();
     slab.mem = at::empty({(int64_t)((bytes + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1))}, options);
     while (g_slabs.size() > kMaxSlabs) {
       auto oldest = g_slabs.end();
       for (auto it = g_slabs.begin(); it != g_slabs.end(); ++it)
         if (it->first != key && (oldest == g_slabs.end() || it->second.used < oldest->second.used)) oldest = it;
-      if (oldest->second.captured) g_captured.push_back(oldest->second.mem);
       g_slabs.erase(oldest);
     }
   }
-  if (!slab.captured && c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-    slab.captured = true;
   slab.used = ++g_tick;
   return slab.mem;
 }
@@ -294,7 +287,7 @@ void free_plan(PyObject* capsule) {
   delete (Plan*)PyCapsule_GetPointer(capsule, kPlanName);
   bool last;
   { std::lock_guard<std::mutex> lock(g_mutex); last = --g_plans == 0; }
-  if (last) clear_slabs(false);
+  if (last) clear_slabs();
 }
 
 // layer_plan(w13, s13, b13, w2, s2, b2, inter, topk, experts, total_experts, act, inter_scale,
@@ -489,7 +482,7 @@ PyObject* layer_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
 
 PyObject* workspace_clear(PyObject*, PyObject*) {
   HANDLE_TH_ERRORS
-  clear_slabs(true);
+  clear_slabs();
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }

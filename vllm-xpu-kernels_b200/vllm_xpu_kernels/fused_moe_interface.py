@@ -121,8 +121,9 @@ def compute_num_tokens_per_block(num_tokens, num_experts_per_node):
 # Intermediates of a layer call (permuted rows, the two GEMM outputs, scales, index maps) live
 # in one grow-only workspace per device and stream, shared by all layer objects: layers of a model
 # run one after the other on a stream, so the next call may overwrite what the previous one left
-# (csrc/torch/layer.cpp; given back with the last layer object).  ``persistent_workspace=False``
-# takes a fresh torch allocation per call instead, as the reference does.
+# (csrc/torch/layer.cpp; given back with the last layer object).  Under stream capture they come
+# from the graph's pool.  ``persistent_workspace=False`` takes a fresh torch allocation per call
+# instead, as the reference does.
 class _Workspace:
     """The workspaces as a whole; ``clear()`` gives them back."""
 
