@@ -1,6 +1,8 @@
 """The layer calls' workspaces: one per stream, given back, never shared by calls that may run at the same
 time.  Results are compared bit for bit with the same call made alone (the layer is deterministic)."""
 import gc
+import threading
+import time
 
 import pytest
 import torch
@@ -71,3 +73,80 @@ def test_graphs_replay_beside_other_calls_and_give_their_memory_back(native):
             assert torch.equal(c[0], ref)
     del graphs, graph
     assert _in_use() == before
+
+
+def test_other_threads_run_while_a_launch_waits(native):
+    """Calls behind a sleeping stream fill its launch queue: the call that then waits for a place must not
+    hold the interpreter (what the stream waits for may need it)."""
+    layer, call = _layer(native), _call(7)
+    layer.apply(*call)
+    torch.cuda.synchronize()
+    ticks, done = [], threading.Event()
+
+    def tick():
+        while not done.is_set():
+            ticks.append(time.monotonic())
+            time.sleep(0.002)
+
+    other = threading.Thread(target=tick)
+    other.start()
+    torch.cuda._sleep(10 ** 9)            # cycles: half a second
+    for _ in range(500):
+        layer.apply(*call)                # several launches each, more than a queue holds
+    done.set()
+    other.join()
+    torch.cuda.synchronize()
+    assert max(b - a for a, b in zip(ticks, ticks[1:])) < 0.15
+
+
+@pytest.mark.parametrize("streams", [1, 3])
+def test_threads_and_streams_do_not_meet(native, streams):
+    """Threads that call layers of different sizes at the same time, on one stream or on one each."""
+    layer = _layer(native)
+    calls = [_call(T) for T in SIZES[-3:]]
+    want = [_alone(native, layer, c) for c in calls]
+    own = [torch.cuda.Stream() for _ in range(streams)]
+    failed = []
+
+    def work(i):
+        with torch.cuda.stream(own[i % streams]):
+            for _ in range(60):
+                calls[i][0].fill_(float("nan"))
+                layer.apply(*calls[i])
+                same = torch.equal(calls[i][0], want[i])
+                if not same:
+                    failed.append(i)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failed
+
+
+def test_a_stage_hook_may_call_a_layer(native):
+    layer, inner, call, other = _layer(native), _layer(native, seed=1), _call(40), _call(400)
+    want, want_inner = _alone(native, layer, call), _alone(native, inner, other)
+    stages = []
+
+    def hook(stage):
+        stages.append(stage)
+        inner.apply(*other)
+
+    layer.stage_hook = hook
+    layer.apply(*call)
+    torch.cuda.synchronize()
+    assert stages == ["routing", "permute", "gemm1", "activation", "gemm2", "gather"]
+    assert torch.equal(call[0], want) and torch.equal(other[0], want_inner)
+
+    def fail(stage):
+        raise ValueError(stage)
+
+    layer.stage_hook = fail
+    with pytest.raises(ValueError, match="routing"):
+        layer.apply(*call)
+    layer.stage_hook = None
+    assert torch.equal(_alone(native, layer, call), want)

@@ -47,10 +47,12 @@ const char* const kPlanName = "b200moe.layer_plan";
 
 // ------------------------------- workspace ------------------------------------
 // One grow-only buffer per (device, stream), shared by all layers: the calls of a stream run one
-// after the other, so the next one may overwrite what the previous one left.  At most kMaxSlabs
-// streams keep one (the least recently used is given back).  All are given back with the last layer
-// object.  A call under stream capture takes its memory from the graph's pool instead: a graph is
-// replayed on any stream, beside later calls on the one it was captured on and beside other graphs,
+// after the other, so the next one may overwrite what the previous one left.  A call has the buffer
+// to itself while it launches and puts it back when it returns; one that launches on the same stream
+// meanwhile (from another thread, or from a stage hook) finds none and takes its own.  At most
+// kMaxSlabs streams keep one (the least recently used is given back), all are given back with the last
+// layer object.  A call under stream capture takes its memory from the graph's pool instead: a graph
+// is replayed on any stream, beside later calls on the one it was captured on and beside other graphs,
 // and what it uses has to live as long as it does.
 constexpr size_t kMaxSlabs = 8;
 struct Slab {
@@ -63,30 +65,70 @@ uint64_t g_tick = 0;
 int64_t g_plans = 0;
 
 void clear_slabs() {
+  std::map<std::pair<int, int64_t>, Slab> old;   // (freed behind the lock)
   std::lock_guard<std::mutex> lock(g_mutex);
-  g_slabs.clear();
+  g_slabs.swap(old);
 }
 
-at::Tensor workspace(const c10::cuda::CUDAStream& stream, size_t bytes, bool persistent) {
-  const auto options = at::TensorOptions().dtype(at::kByte).device(stream.device());
-  if (!persistent || c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None)
-    return at::empty({(int64_t)bytes}, options);
-  std::lock_guard<std::mutex> lock(g_mutex);
-  const std::pair<int, int64_t> key(stream.device_index(), (int64_t)stream.id());
-  Slab& slab = g_slabs[key];
-  if (!slab.mem.defined() || (size_t)slab.mem.numel() < bytes) {
-    slab.mem = at::Tensor();
-    slab.mem = at::empty({(int64_t)((bytes + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1))}, options);
-    while (g_slabs.size() > kMaxSlabs) {
-      auto oldest = g_slabs.end();
+class Workspace {
+ public:
+  Workspace(const c10::cuda::CUDAStream& stream, size_t bytes, bool persistent)
+      : key_(stream.device_index(), (int64_t)stream.id()),
+        keep_(persistent && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None) {
+    if (keep_) {
+      std::lock_guard<std::mutex> lock(g_mutex);
+      auto it = g_slabs.find(key_);
+      if (it != g_slabs.end()) {
+        mem = std::move(it->second.mem);
+        g_slabs.erase(it);
+      }
+    }
+    if (mem.defined() && (size_t)mem.numel() >= bytes) return;
+    mem = at::Tensor();
+    if (keep_) bytes = (bytes + ((size_t)1 << 20)) & ~(((size_t)1 << 20) - 1);
+    mem = at::empty({(int64_t)bytes}, at::TensorOptions().dtype(at::kByte).device(stream.device()));
+  }
+  ~Workspace() {
+    if (!keep_ || !mem.defined()) return;
+    at::Tensor old;                       // (freed behind the lock)
+    std::lock_guard<std::mutex> lock(g_mutex);
+    Slab& slab = g_slabs[key_];
+    if (!slab.mem.defined() || slab.mem.numel() < mem.numel()) {
+      old = std::move(slab.mem);
+      slab.mem = mem;
+    }
+    slab.used = ++g_tick;
+    if (g_slabs.size() > kMaxSlabs) {
+      auto oldest = g_slabs.begin();
       for (auto it = g_slabs.begin(); it != g_slabs.end(); ++it)
-        if (it->first != key && (oldest == g_slabs.end() || it->second.used < oldest->second.used)) oldest = it;
+        if (it->second.used < oldest->second.used) oldest = it;
+      old = std::move(oldest->second.mem);
       g_slabs.erase(oldest);
     }
   }
-  slab.used = ++g_tick;
-  return slab.mem;
-}
+  Workspace(const Workspace&) = delete;
+  at::Tensor mem;
+
+ private:
+  const std::pair<int, int64_t> key_;
+  const bool keep_;
+};
+
+// Other Python threads run while a call launches (a launch waits when the stream's queue is full, and what
+// it waits for may need a Python thread); back in for a hook, for Python objects and when an error leaves.
+class WithoutGil {
+ public:
+  WithoutGil() : state_(PyEval_SaveThread()) {}
+  ~WithoutGil() { end(); }
+  void end() {
+    if (state_ != nullptr) PyEval_RestoreThread(state_);
+    state_ = nullptr;
+  }
+  void begin() { state_ = PyEval_SaveThread(); }
+
+ private:
+  PyThreadState* state_;
+};
 
 // Offsets into a workspace whose size is known once everything has been laid out.
 struct Layout {
@@ -133,17 +175,21 @@ struct CallOptions {
   int max_ctas = 0;
   PyObject* hook = nullptr;   // called with a stage's name after it has been launched
 };
-void mark(const CallOptions& o, const char* stage) {
+void mark(const CallOptions& o, WithoutGil& gil, const char* stage) {
   if (o.hook == nullptr) return;
+  gil.end();
   PyObject* r = PyObject_CallFunction(o.hook, "s", stage);
   if (r == nullptr) throw python_error();
   Py_DECREF(r);
+  gil.begin();
 }
 
 // gemm1 (+ activation) and gemm2 on expert-major rows.
 struct Experts {
   const Plan& p;
+  const WeightDesc d13, d2;   // (the plan's own change with a call of another hidden size or type)
   const CallOptions& o;
+  WithoutGil& gil;
   b200moe_dtype out;          // 16-bit type between the stages
   at::ScalarType out_scalar;
   int64_t M, hidden;
@@ -179,7 +225,7 @@ struct Experts {
   void gemm(bool first, const void* a, b200moe_dtype a_dtype, const void* a_scale, void* d, b200moe_dtype d_dtype,
             void* d_scale, const int32_t* rows, b200moe_epilogue epi) const {
     b200moe_gemm_args g = {};
-    const WeightDesc& w = first ? p.d13 : p.d2;
+    const WeightDesc& w = first ? d13 : d2;
     const at::Tensor& wt = first ? p.w13 : p.w2;
     const auto& sc = first ? p.s13 : p.s2;
     const auto& bias = first ? p.b13 : p.b2;
@@ -207,15 +253,15 @@ struct Experts {
     bool fp8_ready = false, planes_ready = false;
     if (o.form == kFp8) {
       gemm(true, a, a_dtype, a_scale, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, rows, B200MOE_EPI_SILU_MUL);
-      mark(o, "gemm1");
+      mark(o, gil, "gemm1");
       fp8_ready = true;
     } else if (o.form == kEpilogue) {
       gemm(true, a, a_dtype, a_scale, ws + act, out, nullptr, rows,
            p.act == kSilu ? B200MOE_EPI_SILU_MUL : B200MOE_EPI_SWIGLUOAI);
-      mark(o, "gemm1");
+      mark(o, gil, "gemm1");
     } else {
       gemm(true, a, a_dtype, a_scale, ws + g1, out, nullptr, rows, B200MOE_EPI_NONE);
-      mark(o, "gemm1");
+      mark(o, gil, "gemm1");
       if (p.clamp > 0) {
         at::Tensor t = at::from_blob(ws + g1, {M, 2 * I},
                                      at::TensorOptions().dtype(out_scalar).device(at::kCUDA, device));
@@ -244,7 +290,7 @@ struct Experts {
         }
       }
     }
-    mark(o, "activation");
+    mark(o, gil, "activation");
     if (p.block_fp8) {
       if (!fp8_ready)
         check_status(b200moe_per_token_group_fp8_quant(ws + act, out, ws + act_q, (float*)(ws + act_s), M, (int)I2, 128,
@@ -257,7 +303,7 @@ struct Experts {
     } else {
       gemm(false, ws + act, out, nullptr, d, out, nullptr, rows, B200MOE_EPI_NONE);
     }
-    mark(o, "gemm2");
+    mark(o, gil, "gemm2");
   }
 };
 
@@ -367,8 +413,6 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   raise_if_timed_out(device_status_word(x.get_device()));   // an earlier call on this device gave up a wait
   if (o.rows_hint == 0 && map.has_value() && p.total_experts > p.experts)
     o.rows_hint = std::max<int64_t>(1, M * p.experts / p.total_experts);   // the other ranks' share is masked
-  mark(o, "routing");
-
   const bool quant_fp8 = p.block_fp8 && !a1q.has_value();
   const bool i4 = p.i4_planes(o.rows_hint > 0 && o.rows_hint < M ? o.rows_hint : M, p.experts);
   const bool planes_in = p.mx || i4;
@@ -377,7 +421,11 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
     TORCH_CHECK(x.scalar_type() == od, "ptr_A and ptr_D must have the same dtype");
   // (16-bit rows with caller-made scales: the scales are permuted and left unused)
   const bool a_fp8 = quant_fp8 || (p.block_fp8 && x.scalar_type() == at::kFloat8_e4m3fn);
-  Experts e{p, o, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8, planes_in, planes, i4};
+  const at::Tensor* y = gather ? &THPVariable_Unpack(a[2]) : nullptr;
+  const at::Tensor* w = gather ? &THPVariable_Unpack(a[4]) : nullptr;
+  WithoutGil gil;
+  mark(o, gil, "routing");
+  Experts e{p, p.d13, p.d2, o, gil, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8, planes_in, planes, i4};
   Layout l;
   const size_t rows_at = l.take(p.experts * 4), map_at = l.take(M * 4);
   const size_t sort_bytes = b200moe_sort_workspace_bytes(M, (int)p.experts);
@@ -399,8 +447,8 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   size_t d_at = a_at;
   if (l.end - a_at < (size_t)M * H * 2) d_at = l.take(M * H * 2);
   e.lay_out_second(l);
-  at::Tensor mem = workspace(stream, l.end, a[10] == Py_True);
-  uint8_t* ws = mem.data_ptr<uint8_t>();
+  const Workspace workspace(stream, l.end, a[10] == Py_True);
+  uint8_t* ws = workspace.mem.data_ptr<uint8_t>();
   int32_t *rows = (int32_t*)(ws + rows_at), *row_map = (int32_t*)(ws + map_at);
   const int32_t* emap = map.has_value() ? map->data_ptr<int32_t>() : nullptr;
   if (quant_fp8)
@@ -418,21 +466,21 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
         emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T, (int)H, (int)x.element_size(),
         a1q.has_value() ? (int)a1q->size(1) : 0, a1q.has_value() ? (int)a1q->element_size() : 0, (int)K,
         (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes, st));
-  mark(o, "permute");
+  mark(o, gil, "permute");
   e.run(ws, ws + a_at, (a_fp8 || planes_in) ? ws + as_at : nullptr, rows, ws + d_at);
   if (gather) {
-    const at::Tensor& y = THPVariable_Unpack(a[2]);
-    const at::Tensor& w = THPVariable_Unpack(a[4]);
-    check_status(b200moe_moe_gather(y.data_ptr(), ws + d_at, w.data_ptr<float>(), row_map, out, T, (int)H, (int)K, st));
-    mark(o, "gather");
+    check_status(b200moe_moe_gather(y->data_ptr(), ws + d_at, w->data_ptr<float>(), row_map, out, T, (int)H, (int)K, st));
+    mark(o, gil, "gather");
+    gil.end();
     Py_RETURN_NONE;
   }
+  gil.end();
   auto view = [&](size_t at, int64_t r, int64_t c, at::ScalarType t) {
-    return mem.narrow(0, (int64_t)at, r * c * (int64_t)c10::elementSize(t)).view(t).view({r, c});
+    return workspace.mem.narrow(0, (int64_t)at, r * c * (int64_t)c10::elementSize(t)).view(t).view({r, c});
   };
-  PyObject* y = THPVariable_Wrap(view(d_at, M, H, od));
-  PyObject* m = THPVariable_Wrap(view(map_at, T, K, at::kInt));
-  return Py_BuildValue("(NN)", y, m);
+  PyObject* rows_out = THPVariable_Wrap(view(d_at, M, H, od));
+  PyObject* map_out = THPVariable_Wrap(view(map_at, T, K, at::kInt));
+  return Py_BuildValue("(NN)", rows_out, map_out);
   END_HANDLE_TH_ERRORS
 }
 
@@ -468,14 +516,16 @@ PyObject* layer_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const auto stream = at::cuda::getCurrentCUDAStream();
   describe(p, H, y.scalar_type());
   raise_if_timed_out(device_status_word(x.get_device()));
-  Experts e{p, o, out, y.scalar_type(), M, H, (int)segments, (int)x.get_device(), (b200moe_stream)stream.stream(),
-            p.block_fp8, false, 0};
+  WithoutGil gil;
+  Experts e{p, p.d13, p.d2, o, gil, out, y.scalar_type(), M, H, (int)segments, (int)x.get_device(),
+            (b200moe_stream)stream.stream(), p.block_fp8, false, 0};
   Layout l;
   e.lay_out(l);
   e.lay_out_second(l);
-  at::Tensor mem = workspace(stream, l.end, a[8] == Py_True);
-  e.run(mem.data_ptr<uint8_t>(), x.data_ptr(), scale.has_value() ? scale->data_ptr() : nullptr,
+  const Workspace workspace(stream, l.end, a[8] == Py_True);
+  e.run(workspace.mem.data_ptr<uint8_t>(), x.data_ptr(), scale.has_value() ? scale->data_ptr() : nullptr,
         rows.data_ptr<int32_t>(), y.data_ptr());
+  gil.end();
   Py_RETURN_NONE;
   END_HANDLE_TH_ERRORS
 }
