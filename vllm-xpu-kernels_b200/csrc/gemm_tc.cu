@@ -454,7 +454,7 @@ int launch_tc(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams& p, i
   auto kern = grouped_gemm_tc_kernel<BT, kFp8, kWKn, kGated>;
   static_assert(smem_bytes<BT, kFp8, kGated>() <= kMaxSmem, "shared memory");
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, smem_bytes<BT, kFp8, kGated>())) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   B200_LAUNCHED("grouped_gemm_tc_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kTcThreads), smem_bytes<BT, kFp8, kGated>(), st, ta, tw, p));
   return B200MOE_OK;
 }
@@ -741,7 +741,7 @@ int launch_tc_pair(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams&
   auto kern = grouped_gemm_tc_pair_kernel<kWKn, kGated>;
   constexpr size_t kSmem = kGated ? kPairGatedSmem : kPairSmem;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, kSmem)) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -202,15 +202,13 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn get_encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (fn == nullptr) {
+  static const EncodeTiledFn fn = [] {   // (threads that come first together wait for one look-up)
     void* ptr = nullptr;
     cudaDriverEntryPointQueryResult qres;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) ==
-            cudaSuccess &&
-        qres == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &qres) == cudaSuccess &&
+                       qres == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<EncodeTiledFn>(ptr) : nullptr;
+  }();
   return fn;
 }
 
@@ -249,22 +247,22 @@ int sm_count() {
   return v;
 }
 
-// cudaFuncAttributeMaxDynamicSharedMemorySize belongs to a (kernel, device) pair: the
-// largest size set so far is remembered per device, so a process that drives several GPUs
-// configures the kernel on each of them.  One static instance per kernel instantiation.
+// cudaFuncAttributeMaxDynamicSharedMemorySize belongs to a (kernel, device) pair, so a process that
+// drives several GPUs sets it on each of them.  It is always set to the most a CTA may have, not to what
+// the call needs: threads that come first together with different needs set the same.  One static
+// instance per kernel instantiation.
 struct SmemConfig {
-  std::atomic<size_t> bytes[kMaxDevices];
+  std::atomic<bool> done[kMaxDevices];
   template <typename Kern>
-  int ensure(Kern kern, size_t need) {
+  int ensure(Kern kern) {
     const int dev = current_device();
-    if (bytes[dev].load(std::memory_order_acquire) < need) {
-      B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
-      bytes[dev].store(need, std::memory_order_release);
+    if (!done[dev].load(std::memory_order_acquire)) {
+      B200_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
+      done[dev].store(true, std::memory_order_release);
     }
     return B200MOE_OK;
   }
 };
-
 
 }  // namespace
 }  // namespace b200moe

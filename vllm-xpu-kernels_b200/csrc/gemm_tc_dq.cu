@@ -532,7 +532,7 @@ int launch_dq(const b200moe_gemm_args* a, DqParams& p, cudaStream_t st) {
   p.raw_stages = kRaw;
   constexpr size_t smem = kMaxSmem - kRoom + (size_t)kTok * S::kTokBytes + (size_t)kRaw * kDqRawBytes;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, smem)) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   const int64_t tile_bound = ((a->m + BT - 1) / BT + a->num_experts) * (int64_t)p.n_tiles;
   int grid = sm_count();
   if (a->max_ctas > 0 && a->max_ctas < grid) grid = a->max_ctas;

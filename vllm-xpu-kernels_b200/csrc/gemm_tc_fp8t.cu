@@ -732,7 +732,7 @@ int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, TParams& p, int
   p.stages = fixed + kT2Stages * (size_t)kT2StageBytes <= kMaxSmem ? kT2Stages : 3;
   const size_t smem = fixed + p.stages * (size_t)kT2StageBytes;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, smem)) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), smem, st, ta, tw, p));
   return B200MOE_OK;
 }
@@ -741,7 +741,7 @@ template <bool kWKn>
 int launch_fp8t(const CUtensorMap& ta, const CUtensorMap& tw, const TParams& p, int grid, cudaStream_t st) {
   auto kern = grouped_gemm_fp8t_kernel<kWKn>;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, kTSmem)) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   B200_LAUNCHED("grouped_gemm_fp8t_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kTThreads), kTSmem, st, ta, tw, p));
   return B200MOE_OK;
 }

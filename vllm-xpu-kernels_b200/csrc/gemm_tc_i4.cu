@@ -459,7 +459,7 @@ int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
   if (p.stages > kI4MaxStages) p.stages = kI4MaxStages;
   const size_t smem = (size_t)fixed + (size_t)p.stages * S::kStageBytes;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, smem)) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   const int64_t tile_bound = ((a->m + BT - 1) / BT + a->num_experts) * (int64_t)p.n_tiles;
   int grid = sm_count();
   if (a->max_ctas > 0 && a->max_ctas < grid) grid = a->max_ctas;

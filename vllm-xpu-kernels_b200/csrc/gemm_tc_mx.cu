@@ -609,7 +609,7 @@ int launch_mx(const CUtensorMap& ta, const CUtensorMap& tw, MxParams& p, int gri
   if (p.stages < 2) return fail(B200MOE_E_UNSUPPORTED, "block-scaled GEMM: tile does not fit shared memory");
   const size_t smem = (size_t)fixed + (size_t)p.stages * body;
   static SmemConfig configured;
-  if (int rc = configured.ensure(kern, smem)) return rc;
+  if (int rc = configured.ensure(kern)) return rc;
   B200_LAUNCHED("grouped_gemm_mx_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kMxThreads), smem, st, ta, tw, p));
   return B200MOE_OK;
 }
