@@ -278,7 +278,7 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
       }
       for (int term = 0; term < terms; ++term) {
         uint2 codes;
-        const uint32_t word = mx_quant_lane(v, j < nvec, codes);
+        const uint32_t word = mx_quant_lane(v, j < nvec, codes, sums ? kMxLeastExact : kMxLeast);
         if (j < nvec) *reinterpret_cast<uint2*>(q + (term * rows + r) * cols + (int64_t)j * 8) = codes;
         if ((j & 15) == 0 && j < num_kb * 16) s[((int64_t)term * num_kb + (j >> 4)) * rows + r] = word;
       }

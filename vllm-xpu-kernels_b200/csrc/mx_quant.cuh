@@ -15,7 +15,12 @@ namespace {
 //
 // amax / 448 <= 2^e is amax <= 1.75 * 2^(e + 8), a comparison of exponent and mantissa; scale and
 // inverse are then exact powers of two (the divisions this replaces gave the same bits).
-__device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes) {
+//
+// `least`: biased exponent of the smallest scale.  The MXFP8 format's is 2^-33, below which values
+// lose bits and then vanish.  Planes that stand for 16-bit activations (an int4 layer's) go down to
+// 2^-100: what they leave of a bfloat16 is below 2^-109, and nothing gets near fp32's subnormals.
+constexpr int kMxLeast = 127 - 33, kMxLeastExact = 127 - 100;
+__device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes, int least) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
@@ -23,7 +28,7 @@ __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, ui
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
   const uint32_t bits = __float_as_uint(amax);
   int e = (int)(bits >> 23) - 8 + ((bits & 0x007fffffu) > 0x00600000u ? 1 : 0);   // biased exponent of the scale
-  e = e < 94 ? 94 : e;
+  e = e < least ? least : e;
   if (bits >= 0x7f800000u) e = 255;   // an infinity in the group: the scale byte is NaN
   const float sc = __uint_as_float((uint32_t)e << 23), inv = e == 255 ? 0.f : __uint_as_float((uint32_t)(254 - e) << 23);
   uint32_t c[2] = {0u, 0u};
