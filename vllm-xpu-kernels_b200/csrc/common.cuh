@@ -9,6 +9,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
 #include <utility>
 
 #include "../../include/b200moe.h"
@@ -76,6 +77,27 @@ __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.lau
                              cudaGetErrorString(e__));                         \
     }                                                                          \
   } while (0)
+
+constexpr int kMaxDevices = 64;
+
+inline int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return (dev >= 0 && dev < kMaxDevices) ? dev : 0;
+}
+
+// SM count of the current device (cached per device: a process may drive several).
+inline int sm_count() {
+  static std::atomic<int> n[kMaxDevices];
+  const int dev = current_device();
+  int v = n[dev].load(std::memory_order_relaxed);
+  if (v == 0) {
+    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
+    if (v <= 0) v = 148;
+    n[dev].store(v, std::memory_order_relaxed);
+  }
+  return v;
+}
 
 inline cudaStream_t as_stream(b200moe_stream s) { return (cudaStream_t)s; }
 

@@ -495,7 +495,8 @@ extern "C" int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* 
                  "quant_mxfp8: buffers must be 16-byte aligned");
   const int64_t steps = ((cols + 255) / 256 + kMxQuantUnroll - 1) / kMxQuantUnroll;
   const int64_t blocks = (rows * steps + 7) / 8;
-  const dim3 grid((unsigned)(blocks < 148 * 8 ? blocks : 148 * 8));
+  const int64_t most = (int64_t)sm_count() * 8;
+  const dim3 grid((unsigned)(blocks < most ? blocks : most));
   auto run = [&](auto type, auto is_gated) {
     using T = decltype(type);
     return launch_pdl(rows <= kEarlyLaunchRows, quant_mxfp8_kernel<T, decltype(is_gated)::value>, grid, dim3(256), 0,

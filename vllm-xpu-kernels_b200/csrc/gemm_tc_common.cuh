@@ -226,27 +226,6 @@ int encode_map(CUtensorMap* map, CUtensorMapDataType dt, int rank, const void* b
   return B200MOE_OK;
 }
 
-constexpr int kMaxDevices = 64;
-
-inline int current_device() {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  return (dev >= 0 && dev < kMaxDevices) ? dev : 0;
-}
-
-// SM count of the current device (cached per device: a process may drive several).
-int sm_count() {
-  static std::atomic<int> n[kMaxDevices];
-  const int dev = current_device();
-  int v = n[dev].load(std::memory_order_relaxed);
-  if (v == 0) {
-    cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev);
-    if (v <= 0) v = 148;
-    n[dev].store(v, std::memory_order_relaxed);
-  }
-  return v;
-}
-
 // cudaFuncAttributeMaxDynamicSharedMemorySize belongs to a (kernel, device) pair, so a process that
 // drives several GPUs sets it on each of them.  It is always set to the most a CTA may have, not to what
 // the call needs: threads that come first together with different needs set the same.  One static

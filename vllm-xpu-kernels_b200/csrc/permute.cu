@@ -529,7 +529,8 @@ extern "C" int b200moe_fused_moe_prologue(
   a.first_token_offset = reinterpret_cast<int64_t*>(ws + off[6]);
   a.num_tokens = num_rows; a.topk = topk; a.experts = num_experts_on_rank;
   const int64_t want = (int64_t)n < 1 ? 1 : (int64_t)n;
-  const int grid = (int)(want < 148 * 8 ? want : 148 * 8);
+  const int64_t most = (int64_t)sm_count() * 8;
+  const int grid = (int)(want < most ? want : most);
   B200_LAUNCHED("prologue_expand_kernel", launch_pdl(n <= kEarlyLaunchRows, prologue_expand_kernel, dim3(grid), dim3(kBlockThreads), 0, st,
       a));
   return B200MOE_OK;
@@ -728,7 +729,6 @@ namespace {
 constexpr size_t kNoAllocScratchBytes = 1u << 20;  // 1 MiB
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
-constexpr int kMaxDevices = 64;
 // device address of the array per device ordinal; written once, read by any thread
 std::atomic<void*> g_noalloc_ptr[kMaxDevices];
 }  // namespace
