@@ -81,10 +81,6 @@ __device__ __forceinline__ void locate_tile(const TileWalk& w, int t, int& curso
   ti.valid = left < BT ? left : BT;
 }
 
-__device__ __forceinline__ void store_out(void* d, int out_f16, int64_t idx, float v) {
-  if (out_f16) reinterpret_cast<__half*>(d)[idx] = __float2half_rn(v);
-  else reinterpret_cast<__nv_bfloat16*>(d)[idx] = __float2bfloat16_rn(v);
-}
 // A bounded wait gave up: tell the caller through its status word.  A plain store, so the
 // word may live in device memory or in mapped host memory that the host polls without a
 // synchronisation.

@@ -308,7 +308,7 @@ class XpuFusedMoe:
             # fused where the tensor-core kernel of this recipe has the epilogue
             fuse_activation = self.is_mxfp4 and self._act_kind == "swigluoai"
         if is_block_fp8:
-            fuse_activation = False     # (the fp8 form is chosen per call, see _experts)
+            fuse_activation = False     # (the fp8 form is chosen per call: fuses_activation)
         self.fuse_activation = fuse_activation
         if mxfp4_activations is None:
             # the mxfp8 recipe is defined with MXFP8 activations (reference moe_utils.py:198-200)
@@ -379,16 +379,6 @@ class XpuFusedMoe:
               expert_map=None, a1q_scale=None):
         self._apply_kernel(output, hidden_states, topk_weights, topk_ids,
                            expert_map, a1q_scale)
-
-    def _quant_mx(self, x):
-        """[rows, cols] 16-bit -> (e4m3 codes [planes * rows, cols], int32 scale words
-        [planes, ceil(cols / 128), rows]); planes = 2 adds the residual plane."""
-        rows, cols = x.shape
-        planes = self.mx_planes
-        q = torch.empty((planes * rows, cols), dtype=torch.float8_e4m3fn, device=x.device)
-        s = torch.empty((planes, (cols + 127) // 128, rows), dtype=torch.int32, device=x.device)
-        torch.ops._C.b200_quant_mxfp8(x, q, s)
-        return q, s
 
     # The stages are the reference's eight steps (:328-419), launched from native code; what
     # differs is inside the kernels and, for block fp8, that activations really are quantised

@@ -2,8 +2,9 @@
 """Quantisation helpers of the fused-MoE layer.
 
 Mirrors the helper surface of ``vllm_xpu_kernels/moe_utils.py`` in
-vllm-xpu-kernels that the layer itself uses (``quant_fp8_block_act`` :150-166,
-``quant_act_xpu`` :405-411) plus the pure-tensor dequantisers (:29-68,
+vllm-xpu-kernels for callers of these helpers: the activation quantisers
+(``quant_fp8_block_act`` :150-166, ``quant_act_xpu`` :405-411; the layer itself
+quantises in its native call) and the pure-tensor dequantisers (:29-68,
 :134-148).  The eager qdq simulation ``ref_fused_moe`` of the reference is not
 part of this build: only the CUDA kernels run.
 """
