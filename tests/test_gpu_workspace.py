@@ -150,3 +150,70 @@ def test_a_stage_hook_may_call_a_layer(native):
         layer.apply(*call)
     layer.stage_hook = None
     assert torch.equal(_alone(native, layer, call), want)
+
+
+def test_more_streams_than_workspaces(native):
+    """Twelve streams take turns: eight keep a buffer, the least recently used one is given back while its
+    stream may still be at work."""
+    layer = _layer(native)
+    streams = [torch.cuda.Stream() for _ in range(12)]
+    calls = [_call(T, seed=i) for i, T in enumerate((SIZES * 3)[:12])]
+    want = [_alone(native, layer, c) for c in calls]
+    native._WORKSPACE.clear()
+    before = _in_use()
+    with torch.cuda.stream(streams[0]):
+        layer.apply(*calls[0])
+    one = _in_use() - before
+    assert one > 0
+    for _ in range(10):
+        for c in calls:
+            c[0].fill_(float("nan"))
+        torch.cuda.synchronize()
+        for _ in range(3):
+            for s, c in zip(streams, calls):
+                with torch.cuda.stream(s):
+                    layer.apply(*c)
+        torch.cuda.synchronize()
+        for c, ref in zip(calls, want):
+            assert torch.equal(c[0], ref)
+    kept = _in_use() - before
+    native._WORKSPACE.clear()
+    assert _in_use() == before
+    for s in streams:                     # equal sizes: eight buffers of the twelve streams
+        with torch.cuda.stream(s):
+            layer.apply(*calls[0])
+    assert _in_use() - before == 8 * one and kept > 0
+    native._WORKSPACE.clear()
+
+
+def test_the_last_layer_gives_the_workspaces_back(native):
+    call = _call(40)
+    gc.collect()
+    native._WORKSPACE.clear()
+    before = _in_use()
+    layers = [_layer(native, seed=s) for s in range(2)]
+    weights = _in_use() - before
+    for layer in layers:
+        layer.apply(*call)
+    assert _in_use() > before + weights
+    del layer
+    layers.pop()
+    assert _in_use() > before + weights // 2       # the other layer's call may come next
+    layers.pop()
+    assert _in_use() == before
+
+
+def test_setting_an_attribute_of_the_plan_counts_from_the_next_call(native):
+    call = _call(40)
+    layer, other = _layer(native), _layer(native, seed=1)
+    first = _alone(native, layer, call)
+    g = torch.Generator().manual_seed(3)
+    bias = torch.randn(E, H, generator=g).to(torch.bfloat16).to(DEV)
+    for name, value in (("w2", other.w2), ("w2_bias", bias), ("gemm1_clamp_limit", 0.25)):
+        fresh = _layer(native)
+        setattr(fresh, name, value)               # before its first call: there is no plan yet
+        setattr(layer, name, value)
+        got = _alone(native, layer, call)
+        assert not torch.equal(got, first) and torch.equal(got, _alone(native, fresh, call))
+        setattr(layer, name, getattr(_layer(native), name))
+        assert torch.equal(_alone(native, layer, call), first)
