@@ -377,6 +377,29 @@ def test_prequantised_hidden_states_are_refused_for_other_recipes(native):
                     a1q_scale=sc)
 
 
+def test_wrong_prequantised_inputs_are_refused(native):
+    """Scales of another type or width than gemm1 reads, fewer than there are rows, and hidden states that
+    are neither e4m3 nor of the output's type (nothing is launched for any of them)."""
+    cfg = wl.scaled(wl.CONFIGS["cfg3_qwen3_fp8"], H=512, I=256, E=8)
+    w13, s13, w2, s2 = wl.to_op_layout(cfg, wl.make_weights(cfg, seed=6))
+    layer = native.XpuFusedMoe(w13.to(DEV), s13.to(DEV), None, w2.to(DEV), s2.to(DEV), None, 2, cfg.activation, cfg.E)
+    T, H = 6, cfg.H
+    q = torch.zeros(T, H, dtype=torch.float8_e4m3fn, device=DEV)
+    sc = torch.ones(T, H // 128, device=DEV)
+    tw, ids = torch.ones(T, 2, device=DEV), torch.zeros(T, 2, dtype=torch.int32, device=DEV)
+    out = torch.empty(T, H, dtype=torch.bfloat16, device=DEV)
+    for scales in (sc.bfloat16(), sc.double(), torch.ones(T, H // 256, device=DEV), torch.ones(T, H // 32, device=DEV)):
+        with pytest.raises(RuntimeError, match="ptr_A_scale must be float32"):
+            layer.apply(out, q, tw, ids, a1q_scale=scales)
+    with pytest.raises(RuntimeError, match="hidden_states_scales must be"):
+        layer.apply(out, q, tw, ids, a1q_scale=sc[:T - 1].contiguous())
+    for x in (q.view(torch.float8_e5m2), q.half(), q.float()):
+        with pytest.raises(RuntimeError, match="ptr_A and ptr_D must have the same dtype"):
+            layer.apply(out, x, tw, ids, a1q_scale=sc)
+    layer.apply(out, q, tw, ids, a1q_scale=torch.ones(T + 3, H // 128, device=DEV))   # (more rows: the first T count)
+    assert not out.isnan().any()
+
+
 def test_a_bounded_wait_that_runs_out_reaches_the_caller(native):
     """The failure path of the tensor-core kernels, made on purpose without faulting anything: a
     small kernel waits with the kernels' own bounded wait, and a budget of about a millisecond,

@@ -395,8 +395,14 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   TORCH_CHECK(ids.dim() == 2 && ids.size(0) == T && ids.size(1) == K, "topk_ids must be [num_rows, TopK]");
   TORCH_CHECK(x.is_contiguous() && ids.is_contiguous(), "remap_hidden_states expects contiguous tensors");
   if (p.experts > 1024) throw std::runtime_error("local_experts_num exceeds the maximum supported number");
-  if (a1q.has_value())
+  if (a1q.has_value()) {
     TORCH_CHECK(a1q->is_contiguous() && a1q->dim() == 2, "remap_hidden_states expects contiguous scales");
+    TORCH_CHECK(a1q->size(0) >= T, "hidden_states_scales must be [num_rows, hidden_size // block_k]");
+    const bool rows_fp8 = p.block_fp8 && x.scalar_type() == at::kFloat8_e4m3fn;   // gemm1 reads the scales as they are
+    TORCH_CHECK(!rows_fp8 || (a1q->scalar_type() == at::kFloat && a1q->size(1) == H / 128),
+                "ptr_A_scale must be float32 [Total_M, K / 128]");
+    TORCH_CHECK(rows_fp8 || x.scalar_type() == od, "ptr_A and ptr_D must have the same dtype");
+  }
   if (gather) {
     const at::Tensor& y = tensor_arg(a[2], "output");
     const at::Tensor& w = tensor_arg(a[4], "topk_weights");
