@@ -217,3 +217,23 @@ def test_setting_an_attribute_of_the_plan_counts_from_the_next_call(native):
         assert not torch.equal(got, first) and torch.equal(got, _alone(native, fresh, call))
         setattr(layer, name, getattr(_layer(native), name))
         assert torch.equal(_alone(native, layer, call), first)
+
+
+def test_a_call_looks_at_the_weights_as_they_are(native):
+    """Weights that get other memory in place (a reload) are used from the next call on, ones that no longer
+    fit are refused."""
+    call = _call(40)
+    layer = _layer(native)
+    first = _alone(native, layer, call)
+    w2 = layer.w2.clone()
+    layer.w2.data = w2 * 2
+    got = _alone(native, layer, call)
+    fresh = _layer(native)
+    fresh.w2 = w2 * 2
+    assert not torch.equal(got, first) and torch.equal(got, _alone(native, fresh, call))
+    for wrong in (w2[:, :, :-8].contiguous(), w2[:-1].contiguous(), w2.half(), w2.transpose(1, 2).contiguous().transpose(1, 2)):
+        layer.w2.data = wrong
+        with pytest.raises(RuntimeError, match="ptr_B|weights of the activation dtype"):
+            layer.apply(*call)
+    layer.w2.data = w2
+    assert torch.equal(_alone(native, layer, call), first)

@@ -31,17 +31,11 @@ struct Plan {
   int topk = 0, act = 0, inter_scale = 1, planes = 1;
   bool block_fp8 = false, mx = false;
   double clamp = 0.0;
-  // the weights as described for the last (hidden size, activation type): the checks run once
-  int64_t hidden = -1;
-  at::ScalarType act_dtype = at::kFloat;
-  WeightDesc d13{}, d2{};
-  bool i4 = false;            // int4 weights whose shapes the block-scaled kernel takes (gemm_tc_i4.cu)
   // Up to this many rows per expert that kernel streams the weights faster than the one that expands
   // them to 16 bits (gemm_tc_dq.cu), whose matrix work is the cheaper one from there on.  A layer of 8
   // experts of 4096 x 14336, 2 a token: 104 against 121 us at 1 token, 244 against 289 at 33 (8 rows
   // an expert), 483 against 313 at 128 (32 rows).
   static constexpr int64_t kI4PlaneRows = 16;
-  bool i4_planes(int64_t rows, int64_t segments) const { return i4 && rows <= kI4PlaneRows * segments; }
 };
 const char* const kPlanName = "b200moe.layer_plan";
 
@@ -147,11 +141,18 @@ b200moe_dtype dtype16(at::ScalarType t, const char* what) {
   return B200MOE_BF16;
 }
 
-void describe(Plan& p, int64_t hidden, at::ScalarType out_dtype) {
-  if (p.hidden == hidden && p.act_dtype == out_dtype) return;
+// A layer's weights as the library reads them.  Checked by every call: a tensor of the plan may have got
+// other contents, sizes or memory meanwhile.
+struct Weights {
+  WeightDesc d13, d2;
+  bool i4;                    // int4 weights whose shapes the block-scaled kernel takes (gemm_tc_i4.cu)
+};
+Weights describe(const Plan& p, int64_t hidden, at::ScalarType out_dtype) {
   const at::ScalarType a = (p.block_fp8 || p.mx) ? at::kFloat8_e4m3fn : out_dtype;
-  p.d13 = describe_weights(p.w13, p.s13, 2 * p.inter, hidden, p.experts, 0, a);
-  p.d2 = describe_weights(p.w2, p.s2, hidden, p.inter * p.inter_scale, p.experts, 0, a);
+  const int64_t k2 = p.inter * p.inter_scale;
+  Weights w;
+  w.d13 = describe_weights(p.w13, p.s13, 2 * p.inter, hidden, p.experts, 0, a);
+  w.d2 = describe_weights(p.w2, p.s2, hidden, k2, p.experts, 0, a);
   for (const auto* b : {&p.b13, &p.b2}) {
     if (!b->has_value()) continue;
     TORCH_CHECK((*b)->dim() == 2, "ptr_bias must be 2D [num_experts, N]");
@@ -163,9 +164,8 @@ void describe(Plan& p, int64_t hidden, at::ScalarType out_dtype) {
   auto i4_ok = [](const WeightDesc& d, int64_t k) {
     return d.format == B200MOE_W_INT4_NK && (d.group == 128 || d.group == 256) && k % 128 == 0;
   };
-  p.i4 = i4_ok(p.d13, hidden) && i4_ok(p.d2, p.inter * p.inter_scale);
-  p.hidden = hidden;
-  p.act_dtype = out_dtype;
+  w.i4 = i4_ok(w.d13, hidden) && i4_ok(w.d2, k2);
+  return w;
 }
 
 // What a call brings along besides its tensors.
@@ -187,7 +187,7 @@ void mark(const CallOptions& o, WithoutGil& gil, const char* stage) {
 // gemm1 (+ activation) and gemm2 on expert-major rows.
 struct Experts {
   const Plan& p;
-  const WeightDesc d13, d2;   // (the plan's own change with a call of another hidden size or type)
+  const Weights& weights;
   const CallOptions& o;
   WithoutGil& gil;
   b200moe_dtype out;          // 16-bit type between the stages
@@ -225,7 +225,7 @@ struct Experts {
   void gemm(bool first, const void* a, b200moe_dtype a_dtype, const void* a_scale, void* d, b200moe_dtype d_dtype,
             void* d_scale, const int32_t* rows, b200moe_epilogue epi) const {
     b200moe_gemm_args g = {};
-    const WeightDesc& w = first ? d13 : d2;
+    const WeightDesc& w = first ? weights.d13 : weights.d2;
     const at::Tensor& wt = first ? p.w13 : p.w2;
     const auto& sc = first ? p.s13 : p.s2;
     const auto& bias = first ? p.b13 : p.b2;
@@ -365,7 +365,7 @@ PyObject* layer_plan(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 13, "layer_run takes 13 arguments");
-  Plan& p = *plan_arg(a[0]);
+  const Plan& p = *plan_arg(a[0]);
   CallOptions o;
   o.form = (int)int_arg(a[1]);
   o.rows_hint = int_arg(a[8]);
@@ -415,12 +415,12 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
   const b200moe_stream st = (b200moe_stream)stream.stream();
-  describe(p, H, od);
+  const Weights weights = describe(p, H, od);
   raise_if_timed_out(device_status_word(x.get_device()));   // an earlier call on this device gave up a wait
   if (o.rows_hint == 0 && map.has_value() && p.total_experts > p.experts)
     o.rows_hint = std::max<int64_t>(1, M * p.experts / p.total_experts);   // the other ranks' share is masked
   const bool quant_fp8 = p.block_fp8 && !a1q.has_value();
-  const bool i4 = p.i4_planes(o.rows_hint > 0 && o.rows_hint < M ? o.rows_hint : M, p.experts);
+  const bool i4 = weights.i4 && (o.rows_hint > 0 && o.rows_hint < M ? o.rows_hint : M) <= Plan::kI4PlaneRows * p.experts;
   const bool planes_in = p.mx || i4;
   const int planes = i4 ? (od == at::kHalf ? 3 : 2) : p.planes;   // exact for the 16-bit type
   if (!p.mx && !p.block_fp8)
@@ -431,7 +431,7 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* w = gather ? &THPVariable_Unpack(a[4]) : nullptr;
   WithoutGil gil;
   mark(o, gil, "routing");
-  Experts e{p, p.d13, p.d2, o, gil, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8, planes_in, planes, i4};
+  Experts e{p, weights, o, gil, out, od, M, H, (int)p.experts, (int)x.get_device(), st, a_fp8, planes_in, planes, i4};
   Layout l;
   const size_t rows_at = l.take(p.experts * 4), map_at = l.take(M * 4);
   const size_t sort_bytes = b200moe_sort_workspace_bytes(M, (int)p.experts);
@@ -495,7 +495,7 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
 PyObject* layer_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   HANDLE_TH_ERRORS
   TORCH_CHECK(n == 10, "layer_experts takes 10 arguments");
-  Plan& p = *plan_arg(a[0]);
+  const Plan& p = *plan_arg(a[0]);
   CallOptions o;
   o.form = (int)int_arg(a[1]);
   o.rows_hint = int_arg(a[6]);
@@ -520,10 +520,10 @@ PyObject* layer_experts(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   const c10::cuda::CUDAGuard guard(x.device());
   const auto stream = at::cuda::getCurrentCUDAStream();
-  describe(p, H, y.scalar_type());
+  const Weights weights = describe(p, H, y.scalar_type());
   raise_if_timed_out(device_status_word(x.get_device()));
   WithoutGil gil;
-  Experts e{p, p.d13, p.d2, o, gil, out, y.scalar_type(), M, H, (int)segments, (int)x.get_device(),
+  Experts e{p, weights, o, gil, out, y.scalar_type(), M, H, (int)segments, (int)x.get_device(),
             (b200moe_stream)stream.stream(), p.block_fp8, false, 0};
   Layout l;
   e.lay_out(l);
