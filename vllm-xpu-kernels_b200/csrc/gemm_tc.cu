@@ -813,21 +813,27 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   // even, so leave headroom before a second token tile re-reads the weights).
   int bt;
   if (a_fp8) {
-    // fp8 pays a hand-over per 128-wide K block, so wider tiles win earlier (measured on the
-    // DeepSeek and Qwen3 shapes: 8 rows per expert 0.72 / 0.88 / 0.84 of the copy rate at
-    // 16 / 64 / 128 tokens, 32 rows 0.32 / 0.69 / 0.82)
+    // fp8 pays a hand-over per 128-wide K block, so wide tiles win early.  Measured at 16 / 64 / 128
+    // tokens, 128 experts: N 4096, K 7168: 4 rows per expert 605 / 661 / 628 us, 8 rows 767 / 849 / 685,
+    // 16 rows 914 / 761 / 638; N 2048, K 768: 4 rows 59 / 64 / 50 us, 8 rows 61 / 66 / 51, 16 rows
+    // 76 / 66 / 52.  The line at 4 rows is where K decides between 16 and 128 tokens; the 64-token tile
+    // was the better one up to 12 rows before the 128-token kernel's promotion loop was shortened and is
+    // 5 to 30 % behind it now.
     bt = avg <= 4 ? 16 : (avg < 12 ? 64 : 128);
-  } else if (avg <= 8) bt = 16;
-  else if (avg <= 40) bt = 64;
-  else if (avg <= 96) bt = 128;   // measured on skewed routing: 128 rows per expert are 13 % faster at 256
-  else bt = 256;
-  // two accumulators per stage: tensor memory holds the gated form up to 128-token tiles; beyond,
-  // a CTA pair splits gate and up between its two CTAs (whole 128-feature tiles only)
-  // (whole 128-feature tiles only).  The pair's epilogue passes the up half through the other
-  // CTA's shared memory chunk by chunk, which a tile's MMAs hide from K = 4096 on; with 256-token
-  // tiles it also wants segments that fill them.  Measured, gemm1 of the Mixtral shape: 1024 rows
-  // per expert 1.33 ms against 1.59 (single-CTA gated tile) and 1.42 (plain pair + silu_and_mul),
-  // 128 rows per expert 0.39 against 0.31; N=2816, K=2048, 1024 rows: 0.120 against 0.096.
+  } else {
+    // Measured at 16 / 64 / 128 / 256 tokens (a CTA pair), 8 experts, N 28672, K 4096: 8 rows per expert
+    // 289 / 285 / 295 / 340 us, 32 rows 336 / 291 / 301 / 342, 64 rows 539 / 320 / 307 / 344, 96 rows
+    // - / 348 / 316 / 353, 128 rows - / 427 / 386 / 357, 256 rows - / 732 / 585 / 529.
+    bt = avg <= 8 ? 16 : avg <= 40 ? 64 : avg <= 96 ? 128 : 256;
+  }
+  // Two accumulators per stage: tensor memory holds the gated form up to 128-token tiles; beyond, a CTA
+  // pair splits gate and up between its two CTAs (whole 128-feature tiles only).  The pair's epilogue
+  // passes the up half through the other CTA's shared memory chunk by chunk, which a tile's MMAs hide
+  // from K = 4096 on; with 256-token tiles it also wants segments that fill them.  Measured, single-CTA
+  // gated tile / pair / plain pair + silu_and_mul, N 28672, K 4096: 128 rows per expert 389 / 430 / 455
+  // us, 192 rows 470 / 441 / 485, 256 rows (half of the experts need a second tile) 545 / 577 / 618, 512
+  // rows 921 / 895 / 1051, 1024 rows 1656 / 1602 / 1890, 2048 rows 3109 / 2925 / 3339; N 2816, K 2048:
+  // 1024 rows 88 / 132 / 111.
   // (impl 4 forces the pair form, impl 3 the single-CTA forms.)
   const bool gated_pair = gated && !a_fp8 && a->impl != 3 && (a->n / 2) % kFeat == 0 &&
                           (a->impl == 4 || (avg > 192 && a->k >= 4096));

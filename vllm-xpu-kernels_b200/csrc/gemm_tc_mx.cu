@@ -683,8 +683,14 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   // both planes' accumulators share tensor memory: two planes of 96 tokens are one MMA of
   // N = 192 (enough work per instruction to keep the tensor pipe busy), two stages of them
   // and the scale columns fill the 512 columns
-  if (x2 && bt > 64) bt = avg > 48 ? 96 : 64;   // measured: 64 rows per expert -22 %, 32 rows +8 %
+  if (x2 && bt > 64) bt = avg > 48 ? 96 : 64;
   if (!x2 && avg > 128) bt = 192;               // one plane: the same N = 192 instruction
+  // Measured, 128 experts, N 5760, K 2880.  Two planes at 16 / 64 / 96 tokens: 8 rows per expert 238 / 305
+  // / 373 us, 16 rows 305 / 309 / 373, 48 rows 670 / 356 / 426, 64 rows - / 469 / 430; one plane at 16 / 64
+  // / 128 / 192: 8 rows 232 / 283 / 301 / 347, 16 rows 313 / 285 / 300 / 350, 40 rows 549 / 318 / 322 / 367,
+  // 64 rows - / 416 / 330 / 385, 128 rows - / 635 / 811 / 562.  Segments around a multiple of the tile
+  // cost a second tile: at 96 rows two planes take 667 us with 64 tokens and 842 with 96 (K 2880, N 2880:
+  // 313 and 293), at 192 rows 1178 and 1381 (534 and 498).
   // weights: e2m1 K-major, or e4m3 / e5m2 MN-major; activations e4m3 K-major
   const uint32_t a_fmt = w4 ? 5u : (a->w_format == B200MOE_W_FP8E5M2_TENSOR_KN ? 1u : 0u);
   p.idesc = ptx::make_idesc_mx(a_fmt, 0u, kFeat, (uint32_t)(bt * p.terms)) | (w8 ? (1u << 15) : 0u);

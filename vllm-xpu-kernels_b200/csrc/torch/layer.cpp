@@ -31,10 +31,12 @@ struct Plan {
   int topk = 0, act = 0, inter_scale = 1, planes = 1;
   bool block_fp8 = false, mx = false;
   double clamp = 0.0;
-  // Up to this many rows per expert that kernel streams the weights faster than the one that expands
-  // them to 16 bits (gemm_tc_dq.cu), whose matrix work is the cheaper one from there on.  A layer of 8
-  // experts of 4096 x 14336, 2 a token: 104 against 121 us at 1 token, 244 against 289 at 33 (8 rows
-  // an expert), 483 against 313 at 128 (32 rows).
+  // Up to this many rows per expert the block-scaled int4 kernel (gemm_tc_i4.cu) takes the layer: it
+  // streams the weights faster than the one that expands them to 16 bits (gemm_tc_dq.cu), until experts
+  // need a second of its tiles of 32 tokens.  A layer of 8 experts of 4096 x 14336, 2 a token, bfloat16
+  // (float16, three planes): 106 (117) against 125 us at 1 token, 256 (285) against 305 at 8 rows an
+  // expert, 264 (287) against 307 at 12, 266 (295) against 311 at 16, 279 (306) against 315 at 20, 297
+  // (393) against 317 at 24, 373 (465) against 320 at 32.  Half a tile leaves room for uneven routing.
   static constexpr int64_t kI4PlaneRows = 16;
 };
 const char* const kPlanName = "b200moe.layer_plan";

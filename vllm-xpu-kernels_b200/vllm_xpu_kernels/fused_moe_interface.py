@@ -284,10 +284,12 @@ class XpuFusedMoe:
         # block-scaled fp8 with SiLU: the token-major tensor-core kernel can apply the activation and the
         # 1x128 e4m3 quantisation of gemm2's input in its epilogue (same values as the two-kernel form).
         # The epilogue runs on the warps that also promote the K blocks' partial sums, the kernel's
-        # bottleneck, so it pays only where a weight tile is reused by many token tiles; measured on
-        # B200 (gemm1 of the DeepSeek-V3 shape, 65536 rows): 2048 rows per expert 2.61 ms fused against
-        # 2.62 + 0.21 ms, 256 rows per expert 2.80 against 2.51 + 0.20 ms.  Taken per call from
-        # FP8_FUSED_MIN_ROWS routed rows per expert on; fuse_activation=True / False force it.
+        # bottleneck, so short K loops lose by it and long ones break even; from FP8_FUSED_MIN_ROWS
+        # routed rows per expert on the two forms are within 2 % of each other on both shapes, and the
+        # fused one saves the [rows, 2I] intermediate.  Fused against two kernels, the two in turn: gemm1 of
+        # N 4096, K 7168 (65536 rows) 3.65 against 3.86 ms at 256 rows per expert, 3.07 / 3.10 at 512, 2.75
+        # / 2.77 at 1024, 2.65 / 2.65 at 2048; N 1536, K 2048 253 against 229 us at 256, 422 / 416 at 512,
+        # 393 / 387 at 1024, 377 / 376 at 2048.  fuse_activation=True / False force it.
         self._fp8_fused_ok = (is_block_fp8 and self._act_kind == "silu" and self.inter_size % FP8_BLOCK_SIZE == 0
                               and fuse_activation is not False)
         self._fp8_fused_min_rows = 12 if fuse_activation else FP8_FUSED_MIN_ROWS
