@@ -58,3 +58,33 @@ def test_layer_int4_keeps_small_activations(native, T, size):
     assert float(ref.abs().max()) > 0
     err = (out.cpu().double() - ref.double()).norm() / ref.double().norm()
     assert err < 1e-2, err
+
+
+@pytest.mark.parametrize("dtype,bar", [(torch.bfloat16, 6e-3), (torch.float16, 8e-4)])
+def test_int4_tokens_in_a_small_and_a_large_batch(native, dtype, bar):
+    """Up to 16 rows per expert a group's scale multiplies the block's sum, above every weight is rounded
+    after its scale: the same tokens come out differently, both as close to exact arithmetic as 16-bit rows
+    between the stages allow (bar: sqrt(5) roundings of about 2^-9 resp. 2^-12 of their size)."""
+    E, K, H, I, group, T = 4, 2, 512, 384, 128, 16
+    g = torch.Generator().manual_seed(5)
+    x = torch.randn(40 * T, H, generator=g).to(dtype)
+    codes = [torch.randint(0, 256, s, generator=g, dtype=torch.int32).to(torch.uint8) for s in ((E, 2 * I, H // 2), (E, H, I // 2))]
+    scales = [(torch.rand(E, n, k // group, generator=g) * 0.2 + 0.1).mul(k ** -0.5).to(dtype) for n, k in ((2 * I, H), (H, I))]
+    tw, ids = torch.topk(torch.softmax(torch.randn(40 * T, E, generator=g), -1), k=K, dim=-1)
+    layer = native.XpuFusedMoe(codes[0].to(DEV), scales[0].to(DEV), None, codes[1].to(DEV), scales[1].to(DEV), None, K, "silu", E)
+    outs = []
+    for n in (T, 40 * T):
+        out = torch.empty(n, H, dtype=dtype, device=DEV)
+        layer.apply(out, x[:n].to(DEV), tw[:n].to(DEV), ids[:n].int().to(DEV))
+        outs.append(out[:T].cpu().double())
+    w13, w2 = (torch.stack((c & 15, c >> 4), -1).flatten(-2).double().sub(8).mul(s.double().repeat_interleave(group, -1))
+               for c, s in zip(codes, scales))
+    exact = torch.zeros(T, H, dtype=torch.float64)
+    for t in range(T):
+        for k in range(K):
+            h = w13[ids[t, k]] @ x[t].double()
+            exact[t] += tw[t, k].double() * (w2[ids[t, k]] @ (torch.nn.functional.silu(h[:I]) * h[I:]))
+    few, many = ((o - exact).norm() / exact.norm() for o in outs)
+    apart = (outs[0] - outs[1]).norm() / exact.norm()
+    print(f"{dtype}: few rows {few:.2e}, many rows {many:.2e}, apart {apart:.2e}")
+    assert few < bar and many < bar and 0 < apart < 2 * bar
