@@ -1,5 +1,8 @@
 """CPU: host-side decisions of the layer object (no kernel runs: the object is built around CPU
 tensors and only asked which form a call of a given size would take)."""
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -43,3 +46,13 @@ def test_recipes_that_cannot_take_prequantised_inputs_say_so(native):
     with pytest.raises(NotImplementedError):
         bf16.apply(torch.empty_like(x), x, torch.ones(2, 2), torch.zeros(2, 2, dtype=torch.int32),
                    a1q_scale=torch.ones(2, 2))
+
+
+def test_a_used_layer_can_be_copied_and_saved(native):
+    """The native plan of a layer that has been called stays behind: a copy makes its own, from its own tensors."""
+    _, layer = _layer(native, "cfg1_small_bf16", dict(H=256, I=256, E=4))
+    plan = layer._plan()
+    for other in (copy.copy(layer), copy.deepcopy(layer), pickle.loads(pickle.dumps(layer))):
+        assert layer._native_plan is plan
+        assert other._native_plan is None and other._plan() is not plan
+        assert torch.equal(other.w13, layer.w13) and other.recipe == layer.recipe

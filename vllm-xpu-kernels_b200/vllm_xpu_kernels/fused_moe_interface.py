@@ -366,6 +366,10 @@ class XpuFusedMoe:
         if name in _PLAN_FIELDS:
             object.__setattr__(self, "_native_plan", None)
 
+    def __getstate__(self):
+        """What a copy takes along: everything but the native plan, which it makes anew from its own tensors."""
+        return {**self.__dict__, "_native_plan": None}
+
     def _plan(self):
         """The layer as csrc/torch/layer.cpp sees it (tensors, sizes, recipe); made on first use."""
         if self._native_plan is None:
