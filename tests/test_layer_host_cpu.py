@@ -56,3 +56,10 @@ def test_a_used_layer_can_be_copied_and_saved(native):
         assert layer._native_plan is plan
         assert other._native_plan is None and other._plan() is not plan
         assert torch.equal(other.w13, layer.w13) and other.recipe == layer.recipe
+
+
+def test_a_layer_names_its_activation_op(native):
+    _, layer = _layer(native, "cfg1_small_bf16", dict(H=256, I=256, E=4))
+    assert layer.act_func is torch.ops._C.silu_and_mul
+    with pytest.raises(AttributeError):
+        layer.act_func = torch.ops._C.gelu_and_mul

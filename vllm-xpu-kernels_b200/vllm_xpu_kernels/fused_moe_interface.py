@@ -370,6 +370,12 @@ class XpuFusedMoe:
         """What a copy takes along: everything but the native plan, which it makes anew from its own tensors."""
         return {**self.__dict__, "_native_plan": None}
 
+    @property
+    def act_func(self):
+        """The activation op ``act(out, gemm1_output)`` of this layer (reference :239-254).  To be called, not
+        set: layer calls launch it, or a fused form of it, from native code."""
+        return _activation_op(self._act_kind)
+
     def _plan(self):
         """The layer as csrc/torch/layer.cpp sees it (tensors, sizes, recipe); made on first use."""
         if self._native_plan is None:
