@@ -519,7 +519,8 @@ int b200moe_quant_mxfp8(const void* x, b200moe_dtype dtype, void* q, void* s,
                         b200moe_stream stream);
 /* The same with up to three planes and, behind the scale words, fp32 sums
  * [ceil(cols/128)][rows] of every 128-wide block (of what the planes hold): the
- * activations of an int4 grouped GEMM.  With `gated` x is [rows, 2 * cols] and
+ * activations of an int4 grouped GEMM, whose scales go down to 2^-100 (so that
+ * small values keep their bits).  With `gated` x is [rows, 2 * cols] and
  * the values are silu(gate) * up as b200moe_silu_and_mul rounds them. */
 int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* q, void* s,
                            int64_t rows, int cols, int terms, int block_sums,
