@@ -422,7 +422,9 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (o.rows_hint == 0 && map.has_value() && p.total_experts > p.experts)
     o.rows_hint = std::max<int64_t>(1, M * p.experts / p.total_experts);   // the other ranks' share is masked
   const bool quant_fp8 = p.block_fp8 && !a1q.has_value();
-  const bool i4 = weights.i4 && (o.rows_hint > 0 && o.rows_hint < M ? o.rows_hint : M) <= Plan::kI4PlaneRows * p.experts;
+  // (the block-scaled int4 kernel has no activation in its epilogue)
+  const bool i4 = weights.i4 && o.form == kUnfused &&
+                  (o.rows_hint > 0 && o.rows_hint < M ? o.rows_hint : M) <= Plan::kI4PlaneRows * p.experts;
   const bool planes_in = p.mx || i4;
   const int planes = i4 ? (od == at::kHalf ? 3 : 2) : p.planes;   // exact for the 16-bit type
   if (!p.mx && !p.block_fp8)
