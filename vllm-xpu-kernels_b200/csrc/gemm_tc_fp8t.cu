@@ -59,6 +59,7 @@ struct TParams {
   float* d_scale;
   float clamp;            // >0: gate = min(gate, clamp), up = clamp(up, -clamp, clamp)
   int stages;             // 128 x 256 kernel: pipeline stages
+  int d_aligned32;        // 128 x 256 kernel: rows of D begin on 32-byte boundaries
 };
 
 struct TCtrl {
@@ -291,35 +292,44 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
 //   warps 0-3  : producer (warp 0), MMA issuer (warp 1), scale preparers (warps 2 and 3); 56 registers
 //   warps 4-11 : promotion + epilogue, 224 registers; warp w reads lane quarter w & 3 and
 //                the 128 columns of feature block (w - 4) / 4, in two passes of 64
-// Tensor memory holds two accumulator stages of 256 columns.
+// Tensor memory holds two accumulator stages of 256 columns.  A CTA's K blocks are one stream over all its
+// tiles: every role counts them, and stages, scale slots and parities follow from the count.
 //
-// The promotion sets the rate: a K block's MMAs take 512 cycles, the additions of two warps on a
-// scheduler 256 to 300, but a warp that waits for the stage, loads, adds, and reads its scales from
-// global memory one after the other took 917 to 1000.  So everything that is not a load or an addition
-// is kept off its path: scales (already multiplied, four K blocks per hand-over) and tile coordinates come
-// from the preparers through shared memory; a chunk's tensor-memory load is in flight while the chunk
-// before it is added up, also from one K block to the next; the next K block's barriers are looked at once,
-// before the additions that hide the look, and nothing else in the loop branches.  128 experts of 188 rows,
-// N 2048, K 768: 140 -> 110 us; 256 experts of 256 rows on average, N 4096, K 7168: 3.06 -> 2.85 ms.
+// What bounds a K block: its MMAs take 512 cycles; their operands and the loads that bring the next ones
+// pass 96 KB through shared memory (768 cycles at 128 bytes a cycle); a promotion warp's own path is about
+// 600 cycles (clock64, MMAs and loads left out), of which loads and additions are 380 and the rest is
+// hand-overs: a wait for a barrier that is complete already costs a warp 100 cycles or more, and two warps a
+// scheduler cannot hide it.  So the warp waits once per K block, for the accumulator alone: the issuer has
+// seen the block's scales before it issues, and the accumulator of the next block is looked at before the
+// last additions.  (The same warp with waits for scales and stage and its two arrivals apart: 850 cycles.
+// Loads that ran ahead of the wait, 64-bit accumulators and scalar additions all cost registers or moves:
+// slower.)  Under load about 850 cycles a K block remain, at 1.3 to 1.4 GHz under the power cap where the
+// same loop on zeros runs at 1.85.
+//
+// Finished 16-bit rows leave by TMA: a warp puts its 32 rows x 128 features into shared memory and goes on.
+// Storing from the registers (32 bytes of 32 rows an instruction) cost every warp about 3600 cycles per tile
+// that nothing overlapped, staging through a smaller tile and storing 64-byte pieces 4000; now about 2500,
+// most of it the additional passes through shared memory.  The last, partly filled 32 rows of an expert are
+// stored from the registers, because the rows behind them belong to another tile.  The buffer takes the room
+// of one ring stage; three stages are as fast as four were.
+//
+// Before / after, 64 experts x 256 rows, N 4096, K 7168: 570 -> 528 us; N 7168, K 2048: 309 -> 287;
+// 128 experts of 188 rows, N 1536, K 2048: 140 -> 126; N 2048, K 768: 94 -> 78; 64 experts x 140 rows,
+// N 4096, K 7168: 622 -> 519; 32 experts of 32 rows on average: 175 -> 170.
 constexpr int kT2Threads = 384;
 // setmaxnreg.inc waits - without any limit - until the CTA's register pool holds what it asks
 // for, so the re-balanced total must fit what the CTA got at launch (threads x launch registers)
 constexpr int kT2LaunchRegs = 168, kT2LowRegs = 56, kT2HighRegs = 224;
 static_assert(128 * kT2LowRegs + 256 * kT2HighRegs <= kT2Threads * kT2LaunchRegs, "setmaxnreg budget");
-constexpr int kT2Stages = 4;          // ring: 192 KB in flight per SM (one less beside a walk of many hundred experts)
+constexpr int kT2Stages = 3;          // ring: 144 KB in flight per SM (one stage less beside a walk of many hundred experts)
 constexpr int kT2Slots = 2;           // scale groups handed over ahead
-// Finished rows leave through per-warp staging tiles of 32 rows x 32 values (64 bytes + 16, conflict-free
-// for 16-byte accesses), so that a store instruction writes whole 64-byte pieces of eight rows; straight
-// from the registers it would be 16 bytes of 32 rows (4 us per tile that nothing overlaps).  The tile is
-// that small so that the ring keeps four stages: with three and whole 256-byte rows the MMA thread
-// waited 400 of 1200 cycles per K block for data.
-constexpr int kT2RowPitch = 80;
+constexpr int kT2Tiles = 16;          // tile coordinates handed over ahead
 constexpr int kT2StageBytes = 49152;   // weights 2 x 16 KB, tokens 16 KB
 constexpr int kT2Acc = 2;
 
 // A group of K blocks' scales as the promotion warps read them.
 struct alignas(16) T2Slot {
-  float s[2][kTGroup][128];  // [feature block of the tile][K block][token row]: a_scale * w_scale
+  float s[kTGroup][2][128];  // [K block][feature block of the tile][token row]: a_scale * w_scale
 };
 struct T2Ctrl {
   uint64_t full[kT2Stages];
@@ -333,14 +343,15 @@ struct T2Ctrl {
   float xchg[2][2][128];   // gated epilogue: group maxima exchanged between the two warps of a token row
   uint64_t xbar[4];        // ... and the barrier of each such pair of warps (one per lane quarter)
   alignas(16) T2Slot slot[kT2Slots];
-  // The CTA's tile i (first row, valid rows, feature tile, expert) at i % 4, written with its first
-  // group of scales: by then every warp has read a group of tile i - 2 or later, so it has finished i - 4.
-  int4 tile[4];
+  // The CTA's tile i (first row, valid rows, feature tile, expert) at i % kT2Tiles, written before the group of
+  // scales in which it begins, that is when every warp has read the last block of the third group before
+  // that one: the tiles in use span at most 13 blocks, and a block begins at most one tile.
+  int4 tile[kT2Tiles];
 };
-constexpr size_t kT2XposeBytes = 8 * 32 * kT2RowPitch;
-// shared memory: the ring, the staging tiles, T2Ctrl, the tile walk
-constexpr size_t kT2Fixed = 1024 + kT2XposeBytes + ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
-static_assert(kT2Fixed + 3 * (size_t)kT2StageBytes + tile_walk_bytes(kMaxExperts) <= kMaxSmem, "shared memory");
+// shared memory: the ring, (not gated) the finished tile, T2Ctrl, the tile walk
+constexpr int kT2OutBytes = 8 * 8192;   // 32 rows x 128 features of 16 bits a promotion warp
+constexpr size_t kT2Fixed = 1024 + ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
+static_assert(kT2Fixed + 2 * (size_t)kT2StageBytes + kT2OutBytes + tile_walk_bytes(kMaxExperts) <= kMaxSmem, "shared memory");
 
 //
 // kGated (the first grouped GEMM of a SiLU layer with block-scaled fp8 experts): a tile pairs the
@@ -352,15 +363,25 @@ static_assert(kT2Fixed + 3 * (size_t)kT2StageBytes + tile_walk_bytes(kMaxExperts
 // the two warps) and stores e4m3 codes and the group's fp32 scale: the arithmetic of
 // silu_and_mul_per_block_quant on the unfused output, value for value, without the [M, n]
 // round trip through HBM.
+// (D's rows begin on 16-byte boundaries; on 32-byte ones unless the caller's buffer does not)
+__device__ __forceinline__ void store32(void* to, const uint32_t (&w)[8], int aligned32) {
+  if (aligned32) ptx::stg256(to, w);
+  else {
+    reinterpret_cast<uint4*>(to)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    reinterpret_cast<uint4*>(to)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  }
+}
+
 template <bool kWKn, bool kGated>
 __global__ void __launch_bounds__(kT2Threads, 1)
 grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
-                            const __grid_constant__ CUtensorMap tmap_w, const TParams p) {
+                            const __grid_constant__ CUtensorMap tmap_w,
+                            const __grid_constant__ CUtensorMap tmap_d, const TParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int stages = p.stages;
-  uint8_t* xpose_base = smem + stages * kT2StageBytes;
-  T2Ctrl* ctrl = reinterpret_cast<T2Ctrl*>(xpose_base + kT2XposeBytes);
+  uint8_t* out_base = smem + stages * kT2StageBytes;
+  T2Ctrl* ctrl = reinterpret_cast<T2Ctrl*>(out_base + (kGated ? 0 : kT2OutBytes));
   uint8_t* walk_mem = reinterpret_cast<uint8_t*>(ctrl) + ((sizeof(T2Ctrl) + 15) & ~(size_t)15);
   volatile int* abort_flag = &ctrl->abort_flag;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -403,7 +424,10 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const uint32_t tmem_base = ctrl->tmem_base;
   const TileWalk walk = tile_walk_at(walk_mem, p.num_experts);
   const int total_tiles = walk.total;
-  const int n_groups = (p.num_kb + kTGroup - 1) / kTGroup;
+  const int my_tiles = (int)blockIdx.x < total_tiles ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+  // The CTA's K blocks are one stream over all its tiles: every role counts them, stages, slots and
+  // parities follow from the count.
+  const uint32_t blocks = (uint32_t)my_tiles * (uint32_t)p.num_kb;
   const uint32_t sf_full0 = ptx::smem_u32(&ctrl->sf_full[0]), sf_empty0 = ptx::smem_u32(&ctrl->sf_empty[0]);
 
   if (warp < 4) {
@@ -446,11 +470,10 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kWKn ? 16384u : 16u, 1024);
       const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + 32768, 16, 1024);
       uint64_t wdesc = wdesc0, adesc = adesc0;
-      int my_tiles = 0;
-      for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) ++my_tiles;
-      const int64_t blocks = (int64_t)my_tiles * p.num_kb;   // every tile: same K loop, no tile state needed
       const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((256u >> 3) << 17);
-      for (int64_t i = 0; i < blocks; ++i) {
+      for (uint32_t i = 0; i < blocks; ++i) {
+        // (the block's scales: so that acc_full stands for them too)
+        if (i % kTGroup == 0 && !ptx::mbar_wait_s(sf_full0 + 8 * ((i >> 2) & 1), (i >> 3) & 1, abort_flag)) break;
         if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) break;
         if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) break;
         ptx::tc_fence_after();
@@ -465,56 +488,59 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
     } else if (warp >= 2) {
       // ------------------------------ scale preparers ---------------------------
       const int ft = tid - 64, kbs = p.num_kb;            // 0..63: rows ft and ft + 64
-      const bool vec4_ok = (kbs % 4 == 0) && ((reinterpret_cast<uintptr_t>(p.a_scale) & 15) == 0);
-      uint32_t slot = 0, ph = 1, seq = 0;
-      int cursor = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++seq) {
-        TileInfo ti;
-        locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
-        const int nb0 = kGated ? ti.n_tile : ti.n_tile * 2, nb1 = kGated ? ti.n_tile + up_block0 : nb0 + 1;
-        const float* w0 = p.w_scale + ((int64_t)ti.e * p.n_tiles + nb0) * kbs;
-        const float* w1 = w0 + (nb1 < p.n_tiles ? (int64_t)(nb1 - nb0) * kbs : 0);   // past N: any scale, the block's values are zero
-        for (int g = 0; g < n_groups; ++g) {
-          const int kb0 = g * kTGroup;
-          float4 av[2];
+      const bool whole = kbs % kTGroup == 0;              // no group spans two tiles
+      const bool vec4 = whole && (reinterpret_cast<uintptr_t>(p.a_scale) & 15) == 0;
+      int cursor = 0, kb = kbs, t = (int)blockIdx.x - (int)gridDim.x;
+      uint32_t seq = 0;
+      const float *a0 = nullptr, *w0 = nullptr;
+      int64_t w1 = 0;
+      bool live[2] = {false, false};
+      for (uint32_t b = 0; b < blocks; b += kTGroup) {
+        const uint32_t slot = (b / kTGroup) % kT2Slots;
+        float av[2][kTGroup], wv[2][kTGroup];
+#pragma unroll
+        for (int j = 0; j < kTGroup; ++j) {
+          if (kb == kbs && b + j < blocks) {
+            TileInfo ti;
+            t += gridDim.x;
+            locate_tile<kTTok>(walk, t, cursor, ti, p.w_experts);
+            const int nb0 = kGated ? ti.n_tile : ti.n_tile * 2, nb1 = kGated ? ti.n_tile + up_block0 : nb0 + 1;
+            w0 = p.w_scale + ((int64_t)ti.e * p.n_tiles + nb0) * kbs;
+            w1 = nb1 < p.n_tiles ? (int64_t)(nb1 - nb0) * kbs : 0;   // past N: any scale, the block's values are zero
+            a0 = p.a_scale + (int64_t)(ti.row0 + ft) * kbs;
+            live[0] = ft < ti.valid;
+            live[1] = ft + 64 < ti.valid;
+            if (ft == 0) ctrl->tile[seq % kT2Tiles] = make_int4(ti.row0, ti.valid, ti.n_tile, ti.e);
+            ++seq;
+            kb = 0;
+          }
+          const bool in = b + j < blocks;
+          wv[0][j] = in ? __ldg(w0 + kb) : 0.f;
+          wv[1][j] = in ? __ldg(w0 + w1 + kb) : 0.f;
 #pragma unroll
           for (int i = 0; i < 2; ++i) {
-            const int row = ft + 64 * i;
-            const bool live = row < ti.valid;
-            const float* src = p.a_scale + (int64_t)(ti.row0 + row) * kbs + kb0;
-            if (vec4_ok) {
-              av[i] = live ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
-            } else {
-              av[i].x = live ? __ldg(src) : 0.f;
-              av[i].y = live && kb0 + 1 < kbs ? __ldg(src + 1) : 0.f;
-              av[i].z = live && kb0 + 2 < kbs ? __ldg(src + 2) : 0.f;
-              av[i].w = live && kb0 + 3 < kbs ? __ldg(src + 3) : 0.f;
+            const float* src = a0 + (int64_t)(64 * i) * kbs + kb;
+            if (!vec4) {
+              av[i][j] = in && live[i] ? __ldg(src) : 0.f;
+            } else if (j == 0) {
+              const float4 v = live[i] ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
             }
           }
-          float wv[2][kTGroup];
-#pragma unroll
-          for (int j = 0; j < kTGroup; ++j) {
-            const int kl = min(kb0 + j, kbs - 1);
-            wv[0][j] = __ldg(w0 + kl);
-            wv[1][j] = __ldg(w1 + kl);
-          }
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, ph, abort_flag))) { ok = false; break; }
-          T2Slot* out = &ctrl->slot[slot];
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const float rv[kTGroup] = {av[i].x, av[i].y, av[i].z, av[i].w};
-#pragma unroll
-            for (int j = 0; j < kTGroup; ++j) {
-              out->s[0][j][ft + 64 * i] = rv[j] * wv[0][j];
-              out->s[1][j][ft + 64 * i] = rv[j] * wv[1][j];
-            }
-          }
-          if (ft == 0 && g == 0) ctrl->tile[seq & 3] = make_int4(ti.row0, ti.valid, ti.n_tile, ti.e);
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_s(sf_full0 + 8 * slot);
-          if (++slot == kT2Slots) { slot = 0; ph ^= 1; }
+          if (in) ++kb;
         }
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, ((b / (kTGroup * kT2Slots)) & 1) ^ 1, abort_flag))) break;
+        T2Slot* out = &ctrl->slot[slot];
+#pragma unroll
+        for (int j = 0; j < kTGroup; ++j) {
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            out->s[j][0][ft + 64 * i] = av[i][j] * wv[0][j];
+            out->s[j][1][ft + 64 * i] = av[i][j] * wv[1][j];
+          }
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_s(sf_full0 + 8 * slot);
       }
     }
   } else {
@@ -524,89 +550,62 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
     const int r = q * 32 + lane;
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
     const int half = (warp - 4) >> 2;                  // which 128-feature block of the tile (gated: which 64 features of both)
-    uint32_t a = 0, aph = 0, slot = 0, sph = 0, xpar = 0;
     // one shared address, the rest are constants from there (registers are full)
     const uint32_t cs = ptx::smem_u32(ctrl);
-    constexpr uint32_t kAccFull = offsetof(T2Ctrl, acc_full), kAccEmpty = offsetof(T2Ctrl, acc_empty);
+    constexpr uint32_t kAccFull = offsetof(T2Ctrl, acc_full), kAccEmpty = offsetof(T2Ctrl, acc_empty), kAbort = offsetof(T2Ctrl, abort_flag);
     constexpr uint32_t kSfFull = offsetof(T2Ctrl, sf_full), kSfEmpty = offsetof(T2Ctrl, sf_empty), kSlot = offsetof(T2Ctrl, slot);
-    bool ok = true;
-    const int my_tiles = (int)blockIdx.x < total_tiles ? (total_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    // A K block's scales are read when its first chunk is asked for, without a branch.
-    float sc0 = 0.f, sc1 = 0.f;
-    uint32_t jb = 0;                                   // position in the slot
-    const uint32_t my_scales = cs + kSlot + (kGated ? 0 : half * kTGroup * 512) + r * 4;
-    auto read_scales = [&](bool last) {                // `last`: the tile's last K block
-      const uint32_t at = my_scales + slot * (uint32_t)sizeof(T2Slot) + jb * 512;
-      sc0 = ptx::lds32f(at);
-      if (kGated) sc1 = ptx::lds32f(at + kTGroup * 512);
-      const bool done = jb == kTGroup - 1 || last;
-      __syncwarp();   // lane 0's arrival hands the slot back for all lanes: their reads come first
-      ptx::mbar_arrive_if(cs + kSfEmpty + 8 * slot, done && lane == 0);
-      jb = done ? 0u : jb + 1;
-      slot ^= done ? 1u : 0u;
-      sph ^= done && slot == 0 ? 1u : 0u;
-    };
-    static_assert(kT2Slots == 2, "slot parity");
-    auto wait_block = [&]() {                          // the stage and the scales of the next K block
-      return __all_sync(0xffffffffu, ptx::mbar_wait_inline_s(cs + kAccFull + 8 * a, aph, abort_flag) &&
-                                         ptx::mbar_wait_inline_s(cs + kSfFull + 8 * slot, sph, abort_flag));
-    };
+    static_assert(kT2Slots * kTGroup == 8 && kT2Acc == 2 && sizeof(T2Slot) == kTGroup * 1024, "parities of the block count");
+    const uint32_t my_scales = cs + kSlot + (kGated ? 0 : half * 512) + r * 4;
     // Chunks of 32 columns (chunk c of a stage -> acc[16 c ..]).  plain: the 128 columns of this warp's
     // block; gated: 64 gate columns, then the 64 up columns of the same features.
     const uint32_t col_base = tmem_base + (kGated ? half * 64 : half * 128) + lane_sel;
     constexpr uint32_t kSecond = kGated ? 128 : 64;
-    for (int tile = 0; tile < my_tiles && ok; ++tile) {
+    uint32_t b = 0, xpar = 0;
+    bool ok = true, seen = false;   // seen: the next block's accumulator was there when last looked at
+    for (int tile = 0; tile < my_tiles; ++tile) {
       float2 acc[64];
 #pragma unroll
       for (int i = 0; i < 64; ++i) acc[i] = make_float2(0.f, 0.f);
-      uint32_t va[32], vb[32];
-      if (!wait_block()) { ok = false; break; }
-      ptx::tc_fence_after();
-      ptx::tmem_ld_32x32(col_base + a * 256, va);
-      read_scales(p.num_kb == 1);
 #pragma unroll 1
-      for (int kb = 0; kb < p.num_kb; ++kb) {
-        const uint32_t col = col_base + a * 256, empty = cs + kAccEmpty + 8 * a;
-        const bool more = kb + 1 < p.num_kb;
-        const float c0 = sc0, c1 = kGated ? sc1 : sc0;
-        if (++a == (uint32_t)kT2Acc) { a = 0; aph ^= 1; }
-        ptx::tmem_wait_ld_one(va);
-        ptx::tmem_ld_32x32(col + 32, vb);
-        ptx::fma_f32x2(acc, va, c0);
-        ptx::tmem_wait_ld_one(vb);
-        ptx::tmem_ld_32x32(col + kSecond, va);
-        ptx::fma_f32x2(acc + 16, vb, c0);
-        ptx::tmem_wait_ld_one(va);
-        ptx::tmem_ld_32x32(col + kSecond + 32, vb);
-        const bool ready = ptx::mbar_test_wait_s(cs + kAccFull + 8 * a, aph) & ptx::mbar_test_wait_s(cs + kSfFull + 8 * slot, sph);
-        ptx::fma_f32x2(acc + 32, va, c1);
-        ptx::tmem_wait_ld_one(vb);
-        ptx::tc_fence_before();   // the whole stage is in registers
-        __syncwarp();
-        ptx::mbar_arrive_if(empty, lane == 0);
-        if (more) {
-          if (!__all_sync(0xffffffffu, ready) && !wait_block()) { ok = false; break; }
-          ptx::tc_fence_after();
-          ptx::tmem_ld_32x32(col_base + a * 256, va);
-          read_scales(kb + 2 == p.num_kb);
+      for (int left = p.num_kb; left > 0; --left, ++b) {
+        if (!__all_sync(0xffffffffu, seen)) {
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait_lean(cs + kAccFull + 8 * (b & 1), (b >> 1) & 1, cs + kAbort));
+          if (!ok) break;
         }
+        ptx::tc_fence_after();
+        const uint32_t col = col_base + (b & 1) * 256;
+        uint32_t va[32], vb[32];
+        ptx::tmem_ld_32x32(col, va);
+        ptx::tmem_ld_32x32(col + 32, vb);
+        const float c0 = ptx::lds32f(my_scales + (b & 7) * 1024);
+        const float c1 = kGated ? ptx::lds32f(my_scales + (b & 7) * 1024 + 512) : c0;
+        ptx::tmem_wait_ld(va, vb);
+        ptx::fma_f32x2(acc, va, c0);
+        ptx::fma_f32x2(acc + 16, vb, c0);
+        ptx::tmem_ld_32x32(col + kSecond, va);
+        ptx::tmem_ld_32x32(col + kSecond + 32, vb);
+        ptx::tmem_wait_ld(va, vb);
+        ptx::tc_fence_before();   // the whole stage is in registers
+        __syncwarp();             // ... of all lanes, which have also read the block's scales
+        ptx::mbar_arrive_if(cs + kAccEmpty + 8 * (b & 1), lane == 0, cs + kSfEmpty + 8 * ((b >> 2) & 1), (b & 3) == 3);
+        seen = ptx::mbar_test_wait_s(cs + kAccFull + 8 * ((b + 1) & 1), ((b + 1) >> 1) & 1);
+        ptx::fma_f32x2(acc + 32, va, c1);
         ptx::fma_f32x2(acc + 48, vb, c1);
       }
-      if (!ok) { ptx::tmem_wait_ld(); break; }
-      const int4 here = ctrl->tile[tile & 3];
+      if (!ok) break;
+      const int4 here = ctrl->tile[tile % kT2Tiles];
       TileInfo ti;
       ti.row0 = here.x; ti.valid = here.y; ti.n_tile = here.z; ti.e = here.w;
-      auto value = [&](int i) -> float& { return (i & 1) ? acc[i >> 1].y : acc[i >> 1].x; };
       if (kGated) {
         // values 0..63 = gate, 64..127 = up of features j0 + half * 64 ..
         const int half_n = p.n >> 1;
         const int j0 = ti.n_tile * 128 + half * 64;
         float amax = 0.f;
-        // value(i) becomes the activated value of feature j0 + i (the up half is consumed)
+        // the first half of acc becomes the activated values of features j0 ..
         auto activate = [&](auto round16) {
 #pragma unroll
           for (int i = 0; i < 64; ++i) {
-            float g = value(i), u = value(64 + i);
+            float g = (i & 1) ? acc[i >> 1].y : acc[i >> 1].x, u = (i & 1) ? acc[32 + (i >> 1)].y : acc[32 + (i >> 1)].x;
             if (p.bias != nullptr) {
               g += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + j0 + i);
               u += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + half_n + j0 + i);
@@ -618,8 +617,10 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
               g = round16(fminf(g, p.clamp));
               u = round16(fminf(fmaxf(u, -p.clamp), p.clamp));
             }
-            value(i) = __fmul_rn(__fdividef(g, 1.0f + __expf(-g)), u);
-            amax = fmaxf(amax, fabsf(value(i)));
+            const float v = __fmul_rn(__fdividef(g, 1.0f + __expf(-g)), u);
+            amax = fmaxf(amax, fabsf(v));
+            if (i & 1) acc[i >> 1].y = v;
+            else acc[i >> 1].x = v;
           }
         };
         if (p.out_f16) activate([](float x) { return __half2float(__float2half_rn(x)); });
@@ -635,83 +636,82 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
         xpar ^= 1u;
         if (ok && r < ti.valid) {
           const float scale = fmaxf(__fdiv_rn(amax, 448.0f), 1.0f / (448.0f * 512.0f));
-          // 64 codes of this thread's row into the warp's staging tile (rows of 64 + 16 bytes)
-          const uint32_t my_row = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch) + lane * kT2RowPitch;
+          uint8_t* drow = reinterpret_cast<uint8_t*>(p.d) + (int64_t)(ti.row0 + r) * half_n + j0;
 #pragma unroll
-          for (int c = 0; c < 64; c += 16) {
-            uint32_t w[4];
+          for (int c = 0; c < 64; c += 32) {
+            uint32_t w[8];
 #pragma unroll
-            for (int i = 0; i < 16; i += 4) {
+            for (int i = 0; i < 32; i += 4) {
               uint32_t x = 0;
 #pragma unroll
-              for (int b = 0; b < 4; ++b)
-                x |= (uint32_t)f32_to_e4m3(fmaxf(-448.0f, fminf(__fdividef(value(c + i + b), scale), 448.0f))) << (8 * b);
+              for (int b4 = 0; b4 < 4; ++b4)
+              {
+                const float2 v2 = acc[(c + i + b4) >> 1];
+                x |= (uint32_t)f32_to_e4m3(fmaxf(-448.0f, fminf(__fdividef((b4 & 1) ? v2.y : v2.x, scale), 448.0f))) << (8 * b4);
+              }
               w[i >> 2] = x;
             }
-            ptx::sts128(my_row + c, make_uint4(w[0], w[1], w[2], w[3]));
+            store32(drow + c, w, p.d_aligned32);
           }
           if (half == 0) p.d_scale[(int64_t)(ti.row0 + r) * (half_n >> 7) + ti.n_tile] = scale;
         }
         __syncwarp();
-        if (ok) {
-          // eight rows per store: four lanes cover the 64 bytes of a row
-          const uint32_t xp = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch);
-          const int piece = lane & 3;
-          uint8_t* dbase = reinterpret_cast<uint8_t*>(p.d) + (int64_t)(ti.row0 + q * 32) * half_n + j0 + piece * 16;
+      } else {
+        const int f0 = ti.n_tile * 256 + half * 128;
+        if (p.bias != nullptr && f0 < p.n) {
+          const int64_t at = (int64_t)ti.e * p.n + f0;
 #pragma unroll
-          for (int it = 0; it < 4; ++it) {
-            const int rr = it * 8 + (lane >> 2);
-            if (q * 32 + rr < ti.valid)
-              *reinterpret_cast<uint4*>(dbase + (int64_t)rr * half_n) = ptx::lds128(xp + rr * kT2RowPitch + piece * 16);
+          for (int c = 0; c < 64; c += 8) {
+#pragma unroll
+            for (int i = c; i < c + 8; ++i) {
+              acc[i].x += load_bias(p.bias, p.out_f16, at + 2 * i);
+              acc[i].y += load_bias(p.bias, p.out_f16, at + 2 * i + 1);
+            }
+            asm volatile("" ::: "memory");   // a few loads at a time: registers are full
+          }
+        }
+        uint32_t w[64];
+        if (p.out_f16) {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) {
+            const __half2 h = __floats2half2_rn(acc[i].x, acc[i].y);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < 64; ++i) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(acc[i].x, acc[i].y);
+            w[i] = *reinterpret_cast<const uint32_t*>(&h);
+          }
+        }
+        const bool whole = f0 < p.n && q * 32 + 32 <= ti.valid;   // the warp's 32 rows: by TMA
+        const uint32_t out = ptx::smem_u32(out_base) + (warp - 4) * 8192;
+        if (whole) {
+          if (lane == 0) ptx::bulk_wait_read();   // the tile before has left the buffer
+          __syncwarp();
+          // two boxes of 32 rows x 64 features, 128-byte swizzle
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            ptx::sts128(out + (j >> 3) * 4096 + lane * 128 + (((j & 7) ^ (lane & 7)) << 4),
+                        make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]));
+        } else if (f0 < p.n && r < ti.valid) {
+          uint16_t* drow = reinterpret_cast<uint16_t*>(p.d) + (int64_t)(ti.row0 + r) * p.n + f0;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) store32(drow + 16 * j, reinterpret_cast<uint32_t(&)[8]>(w[8 * j]), p.d_aligned32);
+        }
+        if (whole) {
+          ptx::fence_proxy_async();
+          __syncwarp();
+          if (lane == 0) {
+            ptx::tma_store_2d(&tmap_d, out, f0, ti.row0 + q * 32);
+            ptx::tma_store_2d(&tmap_d, out + 4096, f0 + 64, ti.row0 + q * 32);
+            ptx::bulk_commit();
           }
         }
         __syncwarp();
-        continue;
-      }
-      const int f0 = ti.n_tile * 256 + half * 128;
-      if (ok && f0 < p.n) {
-        // the 128 finished values of this thread's row, bias added and rounded, as 16 x 16 bytes
-        auto packed = [&](int c, uint32_t (&w)[4]) {
-#pragma unroll
-          for (int i = 0; i < 8; i += 2) {
-            float x0 = value(c + i), x1 = value(c + i + 1);
-            if (p.bias != nullptr) {
-              x0 += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + f0 + c + i);
-              x1 += load_bias(p.bias, p.out_f16, (int64_t)ti.e * p.n + f0 + c + i + 1);
-            }
-            if (p.out_f16) {
-              const __half2 h = __floats2half2_rn(x0, x1);
-              w[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-            } else {
-              const __nv_bfloat162 h = __floats2bfloat162_rn(x0, x1);
-              w[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-            }
-          }
-        };
-        const uint32_t xp = ptx::smem_u32(xpose_base + (warp - 4) * 32 * kT2RowPitch);
-        const int piece = lane & 3;
-        uint16_t* dbase = reinterpret_cast<uint16_t*>(p.d) + (int64_t)(ti.row0 + q * 32) * p.n + f0 + piece * 8;
-#pragma unroll
-        for (int c0 = 0; c0 < 128; c0 += 32) {
-          // 32 values of this thread's row into the warp's staging tile ...
-#pragma unroll
-          for (int c = 0; c < 32; c += 8) {
-            uint32_t w[4];
-            packed(c0 + c, w);
-            ptx::sts128(xp + lane * kT2RowPitch + c * 2, make_uint4(w[0], w[1], w[2], w[3]));
-          }
-          __syncwarp();
-          // ... and out again eight rows per store: four lanes cover the 64 bytes of a row
-#pragma unroll
-          for (int it = 0; it < 4; ++it) {
-            const int rr = it * 8 + (lane >> 2);
-            if (q * 32 + rr < ti.valid)
-              *reinterpret_cast<uint4*>(dbase + (int64_t)rr * p.n + c0) = ptx::lds128(xp + rr * kT2RowPitch + piece * 16);
-          }
-          __syncwarp();
-        }
       }
     }
+    if (!kGated && lane == 0) ptx::bulk_wait();
   }
 
   pdl_trigger();
@@ -726,14 +726,14 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 template <bool kWKn, bool kGated>
-int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, TParams& p, int grid, cudaStream_t st) {
+int launch_fp8t256(const CUtensorMap& ta, const CUtensorMap& tw, const CUtensorMap& td, TParams& p, int grid, cudaStream_t st) {
   auto kern = grouped_gemm_fp8t256_kernel<kWKn, kGated>;
-  const size_t fixed = kT2Fixed + tile_walk_bytes(p.num_experts);
-  p.stages = fixed + kT2Stages * (size_t)kT2StageBytes <= kMaxSmem ? kT2Stages : 3;
+  const size_t fixed = kT2Fixed + (kGated ? 0 : kT2OutBytes) + tile_walk_bytes(p.num_experts);
+  p.stages = fixed + kT2Stages * (size_t)kT2StageBytes <= kMaxSmem ? kT2Stages : 2;
   const size_t smem = fixed + p.stages * (size_t)kT2StageBytes;
   static SmemConfig configured;
   if (int rc = configured.ensure(kern)) return rc;
-  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), smem, st, ta, tw, p));
+  B200_LAUNCHED("grouped_gemm_fp8t256_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kT2Threads), smem, st, ta, tw, td, p));
   return B200MOE_OK;
 }
 
@@ -781,10 +781,11 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   p.out_f16 = gated ? (a->mid_dtype == B200MOE_F16) : (a->d_dtype == B200MOE_F16);
   p.d_scale = reinterpret_cast<float*>(a->d_scale);
   p.clamp = a->clamp_limit;
+  p.d_aligned32 = ((uintptr_t)a->d & 31) == 0;   // (the row pitch is a multiple of 128 bytes)
   // A operand = tokens (K-major), B operand = weights (K-major, or MN-major for [E,K,N])
   p.idesc = ptx::make_idesc(0u, 0u, 0u, kn ? 1u : 0u, kTTok, kFeat);
 
-  CUtensorMap ta, tw;
+  CUtensorMap ta, tw, td;
   {
     cuuint64_t dims[2] = {(cuuint64_t)a->k, (cuuint64_t)a->m};
     cuuint64_t strides[1] = {(cuuint64_t)a->k};
@@ -811,8 +812,16 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   const int64_t tile_bound = ((a->m + kTTok - 1) / kTTok + a->num_experts) * (int64_t)(wide ? (p.n_tiles + 1) / 2 : p.n_tiles);
   if (tile_bound < grid) grid = (int)tile_bound;
   if (grid < 1) grid = 1;
-  if (gated) return kn ? launch_fp8t256<true, true>(ta, tw, p, grid, st) : launch_fp8t256<false, true>(ta, tw, p, grid, st);
-  if (wide) return kn ? launch_fp8t256<true, false>(ta, tw, p, grid, st) : launch_fp8t256<false, false>(ta, tw, p, grid, st);
+  if (gated) return kn ? launch_fp8t256<true, true>(ta, tw, ta, p, grid, st) : launch_fp8t256<false, true>(ta, tw, ta, p, grid, st);
+  if (wide) {
+    cuuint64_t dims[2] = {(cuuint64_t)a->n, (cuuint64_t)a->m};
+    cuuint64_t strides[1] = {(cuuint64_t)a->n * 2};
+    cuuint32_t box[2] = {64, 32};
+    const int rc = encode_map(&td, p.out_f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, a->d, dims,
+                              strides, box);
+    if (rc) return rc;
+    return kn ? launch_fp8t256<true, false>(ta, tw, td, p, grid, st) : launch_fp8t256<false, false>(ta, tw, td, p, grid, st);
+  }
   return kn ? launch_fp8t<true>(ta, tw, p, grid, st) : launch_fp8t<false>(ta, tw, p, grid, st);
 }
 

@@ -123,6 +123,25 @@ __device__ __forceinline__ bool mbar_wait_inline_s(uint32_t bar, uint32_t parity
   }
   return true;
 }
+// The same without a call and for warps whose registers are full: one register for the time, the abort flag
+// by its shared address.
+__device__ __forceinline__ bool mbar_wait_lean(uint32_t bar, uint32_t parity, uint32_t abort_flag) {
+  if (mbar_try_wait_s(bar, parity)) return true;
+  const uint32_t t0 = (uint32_t)clock();
+  uint32_t spins = 0;
+#pragma unroll 1
+  while (!mbar_try_wait_s(bar, parity)) {
+    if ((++spins & 0xff) != 0) continue;
+    uint32_t aborted;
+    asm volatile("ld.volatile.shared.u32 %0, [%1];" : "=r"(aborted) : "r"(abort_flag) : "memory");
+    if (aborted != 0) return false;
+    if ((uint32_t)clock() - t0 > (uint32_t)kWaitBudgetCycles) {
+      asm volatile("st.volatile.shared.u32 [%0], %1;" ::"r"(abort_flag), "r"(1) : "memory");
+      return false;
+    }
+  }
+  return true;
+}
 __device__ __forceinline__ void mbar_arrive_s(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
@@ -130,6 +149,13 @@ __device__ __forceinline__ void mbar_arrive_s(uint32_t bar) {
 __device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool p) {
   asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %1, 0;\n\t@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(bar),
                "r"((uint32_t)p)
+               : "memory");
+}
+// ... and, where `also` holds too, on a second barrier
+__device__ __forceinline__ void mbar_arrive_if(uint32_t bar, bool p, uint32_t second, bool also) {
+  asm volatile("{\n\t.reg .pred q, t;\n\tsetp.ne.u32 q, %2, 0;\n\tsetp.ne.and.u32 t, %3, 0, q;\n\t"
+               "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t@t mbarrier.arrive.shared::cta.b64 _, [%1];\n\t}" ::"r"(bar),
+               "r"(second), "r"((uint32_t)p), "r"((uint32_t)also)
                : "memory");
 }
 __device__ __forceinline__ void mbar_expect_tx_s(uint32_t bar, uint32_t bytes) {
@@ -187,6 +213,18 @@ __device__ __forceinline__ void tma_load_3d_s(uint32_t dst, const CUtensorMap* m
       ::"r"(dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
+
+// Tiled store from this CTA's shared memory; the rows the box covers all belong to the caller.  The thread
+// that issues it commits a group, and waits for it before the memory is written again or the CTA ends.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(src), "r"(c0), "r"(c1)
+               : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// All groups of this thread have read their shared memory / are complete.
+__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void bulk_wait() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---- CTA pairs (a cluster of two CTAs working on one tcgen05.mma tile) ----------------
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -390,6 +428,13 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r
 }
 __device__ __forceinline__ void tmem_wait_st() {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// 32 bytes of one thread to a 32-byte aligned global address.
+__device__ __forceinline__ void stg256(void* to, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(to), "r"(w[0]), "r"(w[1]), "r"(w[2]),
+               "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
 }
 
 // ---- UMMA ------------------------------------------------------------------------
