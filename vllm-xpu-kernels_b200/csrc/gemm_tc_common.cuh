@@ -104,20 +104,8 @@ __device__ __forceinline__ float load_bias(const void* b, int out_f16, int64_t i
 // kFeat/8 lanes cover one token row, 256/kFeat rows per store instruction.
 // kFeat = 32 (one value per lane) or 16 (values on the even lanes only).
 template <int kTok, int kFeatW>
-__device__ __forceinline__ void store_block_transposed(uint16_t* xp, const float (&vals)[kTok],
-                                                       void* d, int out_f16, int64_t row0,
-                                                       int tok_valid, int64_t m_limit, int n_out,
-                                                       int feat0, int lane) {
-  const int col = (kFeatW == 32) ? lane : (lane >> 1);
-  const bool writer = (kFeatW == 32) || !(lane & 1);
-  const uint32_t xp_s = ptx::smem_u32(xp);
-#pragma unroll
-  for (int i = 0; i < kTok; ++i) {
-    uint16_t bits;
-    if (out_f16) { const __half h = __float2half_rn(vals[i]); bits = *reinterpret_cast<const uint16_t*>(&h); }
-    else { const __nv_bfloat16 h = __float2bfloat16_rn(vals[i]); bits = *reinterpret_cast<const uint16_t*>(&h); }
-    if (writer) ptx::sts16(xp_s + (i * kFeatW + col) * 2, bits);
-  }
+__device__ __forceinline__ void store_tile_rows(uint32_t xp_s, void* d, int64_t row0, int tok_valid, int64_t m_limit, int n_out,
+                                                int feat0, int lane) {
   __syncwarp();
   constexpr int kLanesPerRow = kFeatW / 8;          // 16-byte pieces per token row
   constexpr int kRowsPerIter = 32 / kLanesPerRow;
@@ -132,6 +120,37 @@ __device__ __forceinline__ void store_block_transposed(uint16_t* xp, const float
     }
   }
   __syncwarp();
+}
+__device__ __forceinline__ uint16_t bits16(float x, int out_f16) {
+  if (out_f16) { const __half h = __float2half_rn(x); return *reinterpret_cast<const uint16_t*>(&h); }
+  const __nv_bfloat16 h = __float2bfloat16_rn(x);
+  return *reinterpret_cast<const uint16_t*>(&h);
+}
+// The same for gated outputs shared out over lane pairs: vals[j] = D(token 2 j + (lane & 1), feature lane / 2).
+template <int kHalfTok>
+__device__ __forceinline__ void store_pairs_transposed(uint16_t* xp, const float (&vals)[kHalfTok], void* d, int out_f16,
+                                                       int64_t row0, int tok_valid, int64_t m_limit, int n_out, int feat0,
+                                                       int lane) {
+  const uint32_t xp_s = ptx::smem_u32(xp);
+  const uint32_t at = xp_s + ((lane & 1) * 16 + (lane >> 1)) * 2;
+#pragma unroll
+  for (int j = 0; j < kHalfTok; ++j) ptx::sts16(at + j * 64, bits16(vals[j], out_f16));
+  store_tile_rows<2 * kHalfTok, 16>(xp_s, d, row0, tok_valid, m_limit, n_out, feat0, lane);
+}
+template <int kTok, int kFeatW>
+__device__ __forceinline__ void store_block_transposed(uint16_t* xp, const float (&vals)[kTok],
+                                                       void* d, int out_f16, int64_t row0,
+                                                       int tok_valid, int64_t m_limit, int n_out,
+                                                       int feat0, int lane) {
+  const int col = (kFeatW == 32) ? lane : (lane >> 1);
+  const bool writer = (kFeatW == 32) || !(lane & 1);
+  const uint32_t xp_s = ptx::smem_u32(xp);
+#pragma unroll
+  for (int i = 0; i < kTok; ++i) {
+    const uint16_t bits = bits16(vals[i], out_f16);
+    if (writer) ptx::sts16(xp_s + (i * kFeatW + col) * 2, bits);
+  }
+  store_tile_rows<kTok, kFeatW>(xp_s, d, row0, tok_valid, m_limit, n_out, feat0, lane);
 }
 
 // Fills the tile walk at `mem` (tiles of expert e = ceil(rows_e / BT) * n_tiles).  Called by one

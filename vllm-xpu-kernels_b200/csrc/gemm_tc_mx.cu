@@ -11,10 +11,10 @@
 //
 // Same orientation, tile walk and epilogue as the other tensor-core kernels
 // (weights' output features on the 128-row M side, tokens on the N side).  Roles:
-//   warp 0    : TMA producer.  Weight tile of 128 rows x 128 codes, fetched with
+//   warp 0    : weight producer.  Weight tile of 128 rows x 128 codes, fetched by TMA with
 //               the 16U4_ALIGN16B tensor-map type, which spreads every 8 packed
 //               bytes into a 16-byte slot (the operand format the MMA reads),
-//               128-byte swizzle; activation tile BT rows x 128 bytes.
+//               128-byte swizzle; asks for blocks further on to be brought into L2.
 //   warp 1    : MMA issuer, owns tensor memory; also copies the scale factors of each
 //               K block from shared to tensor memory (tcgen05.cp, which replicates them
 //               over the four lane quarters as the MMA wants them)
@@ -24,6 +24,7 @@
 //               coalesced 32-bit word per token and K block) a group of K blocks
 //               ahead, and write both to a ring of groups in the layout tcgen05.cp
 //               reads
+//   warp 10   : token producer: the tile's rows (rounded up to 16) x 128 bytes of every plane
 //   warps 6-9 : epilogue.  When K is not a multiple of 128 (the weights' tensor-map type
 //               needs it) they also bring and spread the last, partial block of a tile.
 //
@@ -36,6 +37,13 @@
 // e8m0 scale per 32 K rows, [E,K/32,N]: the reference's "mxfp8" recipe,
 // vllm_xpu_kernels/moe_utils.py:76-78, 236-403) take the same path with their real
 // scale factors, staged from the transposed scale tensor.
+//
+// What bounds it (128 experts, two planes): shared memory.  A K block writes 16 KB of spread weights and 256
+// bytes a token row, and its MMAs read the same again: 64 KB or 512 cycles at 128 bytes a cycle with 64 rows,
+// where the MMAs themselves take 320; with loads left out a K block takes 360 to 410 cycles, with them about
+// 660.  With few rows it is 320 cycles and DRAM (about 370 at the copy rate); measured about 400.  So a tile brings
+// and multiplies only the rows it has, and the second plane follows directly (both planes in boxes of 96 rows and
+// N = 96 + rows before: 430 -> 396 us at 64 rows per expert, N 5760, K 2880).
 //
 // Numerics: products of e2m1 and e4m3 codes are exact, scaling by powers of two is
 // exact, accumulation is fp32; the difference from the reference's w4a16 path
@@ -51,8 +59,14 @@ namespace {
 
 constexpr int kMxWBytes = 16384;    // 128 rows x 128 codes in 16-byte slots of 16
 constexpr int kMxWTx = 8192;        // the spreading load reports the packed bytes it read to its barrier
-constexpr int kMxThreads = 320;
+constexpr int kMxThreads = 352;
 constexpr int kMxMaxStages = 8;
+// K blocks the weights are asked for into L2 ahead of their load.  A row's piece of a K block is 64 bytes and L2
+// fetches 256, so every fourth block comes from DRAM, and the ring is too short for that latency (stamps: 1500 to
+// 1900 cycles for that block, 750 for the others).  128 experts, N 5760, K 2880, gated, with / without: 4 rows per
+// expert 204 / 217 us, 16 rows 262 / 283, 64 rows 385 / 393; 4, 8 and 10 blocks ahead, or on into the next tile, are
+// slower.
+constexpr int kMxAhead = 6;
 constexpr int kMxGroup = 4;         // K blocks per scale group (one hand-over from the scale preparers)
 constexpr int kMxSlots = 4;         // scale groups in the ring, at most
 constexpr int kMxSfwCap = 24576 + 32;    // largest weight-scale piece (128 rows x K/32 bytes) staged in shared memory
@@ -148,12 +162,19 @@ __device__ __forceinline__ bool stage_w_scales_kn(const MxParams& p, MxCtrl* ctr
   return true;
 }
 
+// Maps of the activation planes with boxes of 16, 32, ... BT rows: a tile brings and multiplies its rows
+// rounded up to 16, the second plane's directly behind the first one's.
+template <int BT>
+struct MxTokenMaps {
+  CUtensorMap rows[BT / 16];
+};
+
 // BT tokens per tile, kTerms activation planes, kSub 128-wide K blocks per
 // pipeline stage (one barrier hand-over per stage: with small token tiles the
 // roles' fixed cost per hand-over, not the data, bounds the rate).
 template <int BT, int kTerms, int kSub, bool kW8>
 __global__ void __launch_bounds__(kMxThreads, 1)
-grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
+grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
                        const __grid_constant__ CUtensorMap tmap_w, const MxParams p) {
   static_assert(kMxGroup % kSub == 0, "a scale group is a whole number of stages");
   constexpr int kChunk = BT >= 32 ? 32 : 16;
@@ -182,7 +203,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
     pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, after);
     if (lane == 0) {
-      ptx::prefetch_tensormap(&tmap_a);
+      ptx::prefetch_tensormap(&tmap_a.rows[BT / 16 - 1]);
       ptx::prefetch_tensormap(&tmap_w);
     }
   } else if (warp == 1) {
@@ -190,7 +211,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
     ptx::tmem_relinquish();
   } else if (warp == 2 && lane == 0) {
     for (int s = 0; s < kMxMaxStages; ++s) {
-      ptx::mbar_init(&ctrl->full[s], 1);
+      ptx::mbar_init(&ctrl->full[s], 2);
       ptx::mbar_init(&ctrl->empty[s], 1);
     }
     for (int g = 0; g < kMxSlots; ++g) {
@@ -220,7 +241,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int n_groups = (p.num_kb + kMxGroup - 1) / kMxGroup;
 
   if (warp == 0) {
-    // ------------------------------ TMA producer ------------------------------
+    // ------------------------------ weight producer ---------------------------
     if (ptx::elect_one()) {
       uint32_t s = 0, ph = 1;
       int cursor = 0;
@@ -228,6 +249,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
       const uint32_t st0 = ptx::smem_u32(smem);
       uint32_t st = st0;
+      const int whole_kb = tail_kb >= 0 ? tail_kb : p.num_kb;   // the partial block does not come this way
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti);
@@ -235,27 +257,45 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
         for (int kb0 = 0; kb0 < p.num_kb; kb0 += kSub) {
           if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           const uint32_t full = full0 + 8 * s;
-          const bool whole = kb0 + kSub < p.num_kb || (tail_kb < 0 && kb0 + kSub == p.num_kb);
-          if (whole) {
-            ptx::mbar_expect_tx_s(full, kSub * (kWTx + kABytes));
+          ptx::mbar_expect_tx_s(full, max(0, min(kSub, whole_kb - kb0)) * kWTx);
 #pragma unroll
-            for (int sub = 0; sub < kSub; ++sub) {
+          for (int sub = 0; sub < kSub; ++sub) {
+            if (kb0 + sub < whole_kb) {
               // kW8: 128 K rows x 128 features, one byte each; rows past K are zero-filled
               if (kW8) ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, n0, (kb0 + sub) * 128, ti.e);
               else ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, (kb0 + sub) * 128, n0, ti.e);
-              ptx::tma_load_3d_s(st + kAOff + sub * kABytes, &tmap_a, full, (kb0 + sub) * 128, ti.row0, 0);   // all planes
-            }
-          } else {
-            // a tile's last stage: fewer K blocks, or the partial one (only its tokens come this way)
-            const int nsub = p.num_kb - kb0;
-            ptx::mbar_expect_tx_s(full, nsub * (kWTx + kABytes) - (tail_kb >= 0 ? kWTx : 0));
-            for (int sub = 0; sub < nsub; ++sub) {
-              const int kb = kb0 + sub;
-              if (kW8) ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, n0, kb * 128, ti.e);
-              else if (kb != tail_kb) ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, kb * 128, n0, ti.e);
-              ptx::tma_load_3d_s(st + kAOff + sub * kABytes, &tmap_a, full, kb * 128, ti.row0, 0);
             }
           }
+          if (!kW8 && kb0 + kMxAhead < whole_kb) ptx::tma_prefetch_3d(&tmap_w, (kb0 + kMxAhead) * 128, n0, ti.e);
+          st += kStageBytes;
+          if (++s == (uint32_t)stages) { s = 0; ph ^= 1; st = st0; }
+        }
+      }
+    }
+    __syncwarp();
+  } else if (warp == 10) {
+    // ------------------------------ token producer ----------------------------
+    // (a thread of its own: a TMA instruction occupies the thread that issues it for about 130 cycles)
+    if (ptx::elect_one()) {
+      uint32_t s = 0, ph = 1;
+      int cursor = 0;
+      bool ok = true;
+      const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
+      const uint32_t st0 = ptx::smem_u32(smem) + kAOff;
+      uint32_t st = st0;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        TileInfo ti;
+        locate_tile<BT>(walk, t, cursor, ti);
+        const CUtensorMap* tok_map = &tmap_a.rows[BT == 16 ? 0 : (ti.valid - 1) >> 4];
+        const int tok_bytes = BT == 16 ? kABytes : ((ti.valid + 15) & ~15) * (kTerms * 128);
+        for (int kb0 = 0; kb0 < p.num_kb; kb0 += kSub) {
+          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          const uint32_t full = full0 + 8 * s;
+          ptx::mbar_expect_tx_s(full, min(kSub, p.num_kb - kb0) * tok_bytes);
+#pragma unroll
+          for (int sub = 0; sub < kSub; ++sub)
+            if (kb0 + sub < p.num_kb)
+              ptx::tma_load_3d_s(st + sub * kABytes, tok_map, full, (kb0 + sub) * 128, ti.row0, 0);   // all planes
           st += kStageBytes;
           if (++s == (uint32_t)stages) { s = 0; ph ^= 1; st = st0; }
         }
@@ -275,20 +315,25 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
       const uint32_t sf_full0 = ptx::smem_u32(&ctrl->sf_full[0]), sf_empty0 = ptx::smem_u32(&ctrl->sf_empty[0]);
       const uint32_t tail_full = ptx::smem_u32(&ctrl->tail_full);
       const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
-      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kAOff, 16, 1024);
-      const uint64_t wdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), kW8 ? 16384 : 16, 1024);
-      const uint64_t tdesc = ptx::make_smem_desc(ptx::smem_u32(tail_w), 16, 1024);
-      const uint64_t sfdesc0 = ptx::make_smem_desc_plain(ptx::smem_u32(sf_ring), 128);
-      uint64_t wdesc = wdesc0, adesc = adesc0, sfdesc = sfdesc0;
+      // descriptors: the upper halves do not change, the lower ones hold the address
+      const uint64_t adesc_at0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kAOff, 16, 1024);
+      const uint64_t wdesc_at0 = ptx::make_smem_desc(ptx::smem_u32(smem), kW8 ? 16384 : 16, 1024);
+      const uint64_t sfdesc_at0 = ptx::make_smem_desc_plain(ptx::smem_u32(sf_ring), 128);
+      const uint32_t a_hi = (uint32_t)(adesc_at0 >> 32), w_hi = (uint32_t)(wdesc_at0 >> 32), sf_hi = (uint32_t)(sfdesc_at0 >> 32);
+      const uint32_t adesc0 = (uint32_t)adesc_at0, wdesc0 = (uint32_t)wdesc_at0, sfdesc0 = (uint32_t)sfdesc_at0;
+      const uint32_t tdesc = (uint32_t)ptx::make_smem_desc(ptx::smem_u32(tail_w), 16, 1024);
+      uint32_t wdesc = wdesc0, adesc = adesc0, sfdesc = sfdesc0;
       const int whole_kb = tail_kb >= 0 ? tail_kb : p.num_kb;   // K blocks before the partial one
-      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+      // A partly filled token tile multiplies only up to its last valid row (UMMA N in steps of 16).
+      auto instruction = [&](int t) {
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti);
+        return (p.idesc & ~(0x3fu << 17)) | ((uint32_t)(kTerms * ((ti.valid + 15) & ~15)) >> 3 << 17);
+      };
+      uint32_t idesc_next = (int)blockIdx.x < total_tiles ? instruction(blockIdx.x) : 0u;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         const uint32_t a = acc_it & 1;
-        // A partly filled token tile multiplies only up to its last valid column (UMMA N in
-        // steps of 16; with two planes the second one's columns follow the first one's BT).
-        const uint32_t n_eff = (uint32_t)((kTerms - 1) * BT + ((ti.valid + 15) & ~15));
-        const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((n_eff >> 3) << 17);
+        const uint32_t idesc = idesc_next;
         const uint32_t d_tmem = tmem_base + a * kNT;
         if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, ((acc_it >> 1) & 1) ^ 1, abort_flag)) break;
         ptx::tc_fence_after();
@@ -298,10 +343,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
           return go;
         };
         // scales first: tcgen05.cp and tcgen05.mma of one thread execute in issue order
-        auto issue = [&](int u, uint64_t w, uint32_t accumulate) {
+        auto issue = [&](int u, uint32_t w, uint32_t accumulate) {
           ptx::umma_mx_block<kTokChunks, kW8 ? 4096 / 16 : 32 / 16>(
-              d_tmem, w, adesc + (u % kSub) * (kABytes >> 4), idesc, accumulate,
-              tmem_base + kSfBase + u * kSfPer, sfdesc + u * 32, sfdesc + kMxGroup * 32 + u * (kTokChunks * 32));
+              d_tmem, w, w_hi, adesc + (u % kSub) * (kABytes >> 4), a_hi, idesc, accumulate, tmem_base + kSfBase + u * kSfPer,
+              sfdesc + u * 32, sfdesc + kMxGroup * 32 + u * (kTokChunks * 32), sf_hi);
         };
         auto release_stage = [&]() {
           ptx::umma_commit(empty0 + 8 * s);
@@ -310,7 +355,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (++s == (uint32_t)stages) { s = 0; ph ^= 1; wdesc = wdesc0; adesc = adesc0; }
         };
         for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += kMxGroup) {
+          // the next tile's, while the pipe has work (not between two tiles)
+          if (kb0 + kMxGroup >= p.num_kb && t + (int)gridDim.x < total_tiles) idesc_next = instruction(t + gridDim.x);
           if (!ptx::mbar_wait_s(sf_full0 + 8 * slot, slot_ph, abort_flag)) { ok = false; break; }
+          ptx::fence_proxy_async();
           if (kb0 + kMxGroup <= whole_kb) {
 #pragma unroll
             for (int u = 0; u < kMxGroup; ++u) {
@@ -355,21 +403,23 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
     int cursor = 0, cursor_next = 0, cursor_la = 0;
     bool ok = true;
 
-    // Token scales of one group: word [plane][kb][row], coalesced over the lanes, read one group
-    // ahead of their use by a look-ahead position (la_*) that runs over the same sequence.
-    // (Two register sets that change roles: a move from one to the other would wait for the loads.)
+    // Token scales of one group: thread ft takes words ft + 128 i of [K block][plane][token], coalesced over
+    // the lanes, read one group ahead of their use by a look-ahead position (la_*) that runs over the same
+    // sequence.  (Two register sets that change roles: a move from one to the other would wait for the loads.)
+    auto word_u = [&](int i) { return (ft + 128 * i) / kNT; };
+    auto word_tok = [&](int i) { return (ft + 128 * i) % BT; };
+    auto word_term = [&](int i) { return (ft + 128 * i) % kNT / BT; };
     uint32_t tok_a[kPer], tok_b[kPer];
+    int64_t src[kPer];                                   // word of K block u, row 0
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) src[i] = word_term(i) * plane_words + (int64_t)word_u(i) * p.m + word_tok(i);
     bool odd = false;
     auto fetch_b = [&](const TileInfo& ti, int g, uint32_t (&db)[kPer]) {
+      const uint32_t* base = p.a_scale + (int64_t)(g * kMxGroup) * p.m + ti.row0;
 #pragma unroll
-      for (int i = 0; i < kPer; ++i) {
-        const int x = ft + 128 * i;
-        const int n = x % kNT;                      // row of the side-by-side token operand
-        const int kb = g * kMxGroup + x / kNT;
-        const int term = n / BT, tok = n % BT;
-        db[i] = (x < kMxGroup * kNT && kb < p.num_kb && tok < ti.valid)
-                    ? __ldg(p.a_scale + term * plane_words + (int64_t)kb * p.m + ti.row0 + tok) : 0x7f7f7f7fu;
-      }
+      for (int i = 0; i < kPer; ++i)
+        db[i] = (ft + 128 * i < kMxGroup * kNT && word_u(i) < p.num_kb - g * kMxGroup && word_tok(i) < ti.valid) ? __ldg(base + src[i])
+                                                                                                              : 0x7f7f7f7fu;
     };
     int la_t = blockIdx.x, la_g = 0;
     TileInfo la_ti;
@@ -405,6 +455,15 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
       }
       const uint32_t sfw_s = ptx::smem_u32(sfw + b * p.sfw_bytes);
       const bool row_ok = ti.n_tile * kFeat + wrow < p.n;
+      // Where the token words go: row n of the side-by-side token operand (planes of v16 rows) in the layout
+      // tcgen05.cp reads.
+      const int v16 = (ti.valid + 15) & ~15;
+      uint32_t dst[kPer];
+#pragma unroll
+      for (int i = 0; i < kPer; ++i) {
+        const int n = word_term(i) * v16 + word_tok(i);
+        dst[i] = kMxGroup * 512 + word_u(i) * (kTokChunks * 512) + (n >> 7) * 512 + (n & 31) * 16 + ((n >> 5) & 3) * 4;
+      }
       auto group = [&](int g, const uint32_t (&use)[kPer], uint32_t (&fill)[kPer]) {
         if (++la_g == n_groups) {
           la_g = 0;
@@ -434,12 +493,16 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
               if (4 * u + q < left) wa[u] |= ptx::lds8(sfw_s + (16 * g + 4 * u + q) * 128 + wrow) << (8 * q);
           }
         }
+        if (!staged || !row_ok) {   // per-tensor scale: applied in the epilogue
 #pragma unroll
-        for (int u = 0; u < kMxGroup; ++u) {
-          const int lu = left - 4 * u;
-          const uint32_t keep = lu >= 4 ? 0xffffffffu : (lu <= 0 ? 0u : ((1u << (8 * lu)) - 1u));
-          if (!staged || !row_ok) wa[u] = 0x7f7f7f7fu;   // per-tensor scale: applied in the epilogue
-          else wa[u] = (wa[u] & keep) | (0x7f7f7f7fu & ~keep);
+          for (int u = 0; u < kMxGroup; ++u) wa[u] = 0x7f7f7f7fu;
+        } else if (left < 4 * kMxGroup) {
+#pragma unroll
+          for (int u = 0; u < kMxGroup; ++u) {
+            const int lu = left - 4 * u;
+            const uint32_t keep = lu >= 4 ? 0xffffffffu : (lu <= 0 ? 0u : ((1u << (8 * lu)) - 1u));
+            wa[u] = (wa[u] & keep) | (0x7f7f7f7fu & ~keep);
+          }
         }
         // the ring slot's previous group has been copied to tensor memory
         if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->sf_empty[slot], slot_ph ^ 1, abort_flag))) {
@@ -450,14 +513,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
 #pragma unroll
         for (int u = 0; u < kMxGroup; ++u) ptx::sts32(ring + u * 512 + (wrow & 31) * 16 + (wrow >> 5) * 4, wa[u]);
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-          const int x = ft + 128 * i;
-          const int n = x % kNT, u = x / kNT;
-          if (x < kMxGroup * kNT)
-            ptx::sts32(ring + kMxGroup * 512 + u * (kTokChunks * 512) + (n >> 7) * 512 + (n & 31) * 16 +
-                       ((n >> 5) & 3) * 4, use[i]);
-        }
-        ptx::fence_proxy_async();
+        for (int i = 0; i < kPer; ++i)
+          if (ft + 128 * i < kMxGroup * kNT && word_tok(i) < v16) ptx::sts32(ring + dst[i], use[i]);
+        // (the issuer's proxy fence stands between these writes and its tcgen05.cp: one here would wait for the
+        // loads of the next group as well)
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&ctrl->sf_full[slot]);
         if (++slot == kSlots) { slot = 0; slot_ph ^= 1; }
@@ -531,51 +590,52 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
       // wait does not take issue slots from the feeder warp on the same scheduler
       if (!ptx::mbar_wait_warp(&ctrl->acc_full[a], (acc_it >> 1) & 1, abort_flag, 128)) { ok = false; break; }
       ptx::tc_fence_after();
+      const uint32_t second = (uint32_t)((ti.valid + 15) & ~15);   // the second plane's first column
 #pragma unroll
       for (int c0 = 0; c0 < BT; c0 += kChunk) {
         if (c0 < ti.valid) {
-          uint32_t v[kChunk];
-          float acc[kChunk];
+          uint32_t v[kTerms][kChunk];
 #pragma unroll
-          for (int i = 0; i < kChunk; ++i) acc[i] = 0.f;
-#pragma unroll
-          for (int term = 0; term < kTerms; ++term) {   // the planes' partial results add up
-            const uint32_t col = tmem_base + a * kNT + term * BT + c0 + lane_sel;
-            if (kChunk == 32) ptx::tmem_ld_32x32(col, reinterpret_cast<uint32_t(&)[32]>(v));
-            else ptx::tmem_ld_32x16(col, reinterpret_cast<uint32_t(&)[16]>(v));
-            ptx::tmem_wait_ld(v);
-#pragma unroll
-            for (int i = 0; i < kChunk; ++i) acc[i] += __uint_as_float(v[i]);
+          for (int term = 0; term < kTerms; ++term) {
+            const uint32_t col = tmem_base + a * kNT + term * second + c0 + lane_sel;
+            if (kChunk == 32) ptx::tmem_ld_32x32(col, reinterpret_cast<uint32_t(&)[32]>(v[term]));
+            else ptx::tmem_ld_32x16(col, reinterpret_cast<uint32_t(&)[16]>(v[term]));
           }
+          ptx::tmem_wait_ld(v[0], v[kTerms - 1]);
           float vals[kChunk];
 #pragma unroll
-          for (int i = 0; i < kChunk; ++i) vals[i] = kW8 ? fmaf(acc[i], w_mul, bias_v) : acc[i] + bias_v;
+          for (int i = 0; i < kChunk; ++i) {
+            float acc = 0.f + __uint_as_float(v[0][i]);
+            if (kTerms == 2) acc += __uint_as_float(v[kTerms - 1][i]);   // the planes' partial results add up
+            vals[i] = kW8 ? fmaf(acc, w_mul, bias_v) : acc + bias_v;
+          }
           if (p.swiglu) {
+            // Gate sits on even features, up on the next odd one: neighbours in the warp.  Of two tokens the even
+            // lane takes the first and the odd lane the second, so a pair computes each output once.
             // One branch around the whole block: the unrolled body stays straight-line code, so
-            // the 32 shuffle / exp / divide chains overlap instead of running one after another.
+            // the shuffle / exp / divide chains overlap instead of running one after another.
             const float c_lim = p.clamp_limit > 0.f ? p.clamp_limit : INFINITY;
+            const bool odd = lane & 1;
+            float out[kChunk / 2];
 #pragma unroll
-            for (int i = 0; i < kChunk; ++i) {
-              // gate sits on even features, up on the next odd one: neighbours in the warp
-              const float x = vals[i];
-              const float other = __shfl_xor_sync(0xffffffffu, x, 1);
-              float gate = (lane & 1) ? other : x;
-              float up = (lane & 1) ? x : other;
+            for (int j = 0; j < kChunk / 2; ++j) {
+              const float mine = odd ? vals[2 * j + 1] : vals[2 * j];
+              const float other = __shfl_xor_sync(0xffffffffu, odd ? vals[2 * j] : vals[2 * j + 1], 1);
+              float gate = odd ? other : mine;
+              float up = odd ? mine : other;
               gate = fminf(gate, c_lim);
               up = fminf(fmaxf(up, -c_lim), c_lim);
               gate = fminf(gate, p.limit);
               up = fminf(fmaxf(up, -p.limit), p.limit);
-              vals[i] = (up + 1.0f) * gate * __fdividef(1.0f, 1.0f + __expf(-gate * p.alpha));
+              out[j] = (up + 1.0f) * gate * __fdividef(1.0f, 1.0f + __expf(-gate * p.alpha));
             }
-          }
-          if (p.swiglu)
-            store_block_transposed<kChunk, 16>(ctrl->xpose[warp - 6], vals, p.d, p.out_f16,
-                                               (int64_t)ti.row0 + c0, ti.valid - c0, p.m, n_out,
-                                               (ti.n_tile * kFeat + q * 32) >> 1, lane);
-          else
+            store_pairs_transposed(ctrl->xpose[warp - 6], out, p.d, p.out_f16, (int64_t)ti.row0 + c0, ti.valid - c0, p.m,
+                                   n_out, (ti.n_tile * kFeat + q * 32) >> 1, lane);
+          } else {
             store_block_transposed<kChunk, 32>(ctrl->xpose[warp - 6], vals, p.d, p.out_f16,
                                                (int64_t)ti.row0 + c0, ti.valid - c0, p.m, n_out,
                                                ti.n_tile * kFeat + q * 32, lane);
+          }
         }
       }
       ptx::tc_fence_before();
@@ -597,7 +657,14 @@ grouped_gemm_mx_kernel(const __grid_constant__ CUtensorMap tmap_a,
 }
 
 template <int BT, int kTerms, int kSub, bool kW8>
-int launch_mx(const CUtensorMap& ta, const CUtensorMap& tw, MxParams& p, int grid, cudaStream_t st) {
+int launch_mx(const b200moe_gemm_args* a, const CUtensorMap& tw, MxParams& p, int grid, cudaStream_t st) {
+  MxTokenMaps<BT> ta;
+  for (int i = 0; i < BT / 16; ++i) {
+    cuuint64_t dims[3] = {(cuuint64_t)a->k, (cuuint64_t)a->m, (cuuint64_t)kTerms};
+    cuuint64_t strides[2] = {(cuuint64_t)a->k, (cuuint64_t)a->k * (cuuint64_t)a->m};
+    cuuint32_t box[3] = {128, (cuuint32_t)(16 * (i + 1)), (cuuint32_t)kTerms};
+    if (int rc = encode_map(&ta.rows[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->a, dims, strides, box)) return rc;
+  }
   auto kern = grouped_gemm_mx_kernel<BT, kTerms, kSub, kW8>;
   const uint32_t need = 2 * kTerms * BT + kMxGroup * (kTerms * BT > 128 ? 16 : 8);
   p.tmem_cols = need <= 128 ? 128u : (need <= 256 ? 256u : 512u);
@@ -695,14 +762,7 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   const uint32_t a_fmt = w4 ? 5u : (a->w_format == B200MOE_W_FP8E5M2_TENSOR_KN ? 1u : 0u);
   p.idesc = ptx::make_idesc_mx(a_fmt, 0u, kFeat, (uint32_t)(bt * p.terms)) | (w8 ? (1u << 15) : 0u);
 
-  CUtensorMap ta, tw;
-  {
-    cuuint64_t dims[3] = {(cuuint64_t)a->k, (cuuint64_t)a->m, (cuuint64_t)p.terms};
-    cuuint64_t strides[2] = {(cuuint64_t)a->k, (cuuint64_t)a->k * (cuuint64_t)a->m};
-    cuuint32_t box[3] = {128, (cuuint32_t)bt, (cuuint32_t)p.terms};
-    int rc = encode_map(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->a, dims, strides, box);
-    if (rc) return rc;
-  }
+  CUtensorMap tw;
   if (w8) {
     cuuint64_t dims[3] = {(cuuint64_t)a->n, (cuuint64_t)a->k, (cuuint64_t)a->num_experts};
     cuuint64_t strides[2] = {(cuuint64_t)a->n, (cuuint64_t)a->k * a->n};
@@ -728,14 +788,14 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   // Small token tiles move two K blocks per pipeline stage.
 #define B200_MX_CASES(W8)                                                              \
   if (x2) {                                                                            \
-    if (bt == 16) return launch_mx<16, 2, 2, W8>(ta, tw, p, grid, st);                 \
-    if (bt == 96) return launch_mx<96, 2, 1, W8>(ta, tw, p, grid, st);                 \
-    return launch_mx<64, 2, 1, W8>(ta, tw, p, grid, st);                               \
+    if (bt == 16) return launch_mx<16, 2, 2, W8>(a, tw, p, grid, st);                 \
+    if (bt == 96) return launch_mx<96, 2, 1, W8>(a, tw, p, grid, st);                 \
+    return launch_mx<64, 2, 1, W8>(a, tw, p, grid, st);                               \
   }                                                                                    \
-  if (bt == 192) return launch_mx<192, 1, 1, W8>(ta, tw, p, grid, st);                 \
-  if (bt == 16) return launch_mx<16, 1, 2, W8>(ta, tw, p, grid, st);                   \
-  if (bt == 64) return launch_mx<64, 1, 2, W8>(ta, tw, p, grid, st);                   \
-  return launch_mx<128, 1, 1, W8>(ta, tw, p, grid, st);
+  if (bt == 192) return launch_mx<192, 1, 1, W8>(a, tw, p, grid, st);                 \
+  if (bt == 16) return launch_mx<16, 1, 2, W8>(a, tw, p, grid, st);                   \
+  if (bt == 64) return launch_mx<64, 1, 2, W8>(a, tw, p, grid, st);                   \
+  return launch_mx<128, 1, 1, W8>(a, tw, p, grid, st);
   if (w8) { B200_MX_CASES(true) }
   B200_MX_CASES(false)
 #undef B200_MX_CASES

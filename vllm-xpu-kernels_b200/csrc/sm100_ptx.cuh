@@ -214,6 +214,13 @@ __device__ __forceinline__ void tma_load_3d_s(uint32_t dst, const CUtensorMap* m
       : "memory");
 }
 
+// Brings the box into L2 only.
+__device__ __forceinline__ void tma_prefetch_3d(const CUtensorMap* map, int c0, int c1, int c2) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global [%0, {%1, %2, %3}];" ::"l"(reinterpret_cast<uint64_t>(map)), "r"(c0),
+               "r"(c1), "r"(c2)
+               : "memory");
+}
+
 // Tiled store from this CTA's shared memory; the rows the box covers all belong to the caller.  The thread
 // that issues it commits a group, and waits for it before the memory is written again or the CTA ends.
 __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int c0, int c1) {
@@ -483,34 +490,41 @@ __host__ __device__ constexpr uint32_t make_idesc_mx(uint32_t a_fmt, uint32_t b_
 // lane quarters; the weight rows' to column sf, the tokens' kTokChunks chunks to the columns after
 // them), then the four K = 32 instructions run on scale bytes 0..3 of those columns.  kWStep:
 // 16-byte units between the K steps of the weight operand (the tokens' are 32 bytes apart).
+// Descriptors come as halves, of which only the lower ones (addresses) differ between blocks: 64-bit
+// additions cost the issuing thread 20 cycles a K block.
 template <int kTokChunks, int kWStep>
-__device__ __forceinline__ void umma_mx_block(uint32_t tmem_d, uint64_t wdesc, uint64_t adesc, uint32_t idesc,
-                                                    uint32_t accumulate, uint32_t sf, uint64_t sfw_desc,
-                                                    uint64_t sfa_desc) {
-#define B200_MX_MMA4                                                                                             \
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [t], pa;\n\t"             \
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w1, a1, i1, [%5], [t], 1;\n\t"              \
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w2, a2, i2, [%5], [t], 1;\n\t"              \
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w3, a3, i3, [%5], [t], 1;\n\t}"
-#define B200_MX_HEAD                                                                                             \
-      "{\n\t.reg .pred pa;\n\t.reg .b32 t, i1, i2, i3;\n\t.reg .b64 w1, w2, w3, a1, a2, a3;\n\t"              \
-      "setp.ne.b32 pa, %4, 0;\n\tadd.u32 t, %5, 4;\n\t"                                                          \
-      "add.u64 w1, %1, %8;\n\tadd.u64 w2, %1, %9;\n\tadd.u64 w3, %1, %10;\n\t"                                   \
-      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"                                       \
-      "or.b32 i1, %3, 0x20000010;\n\tor.b32 i2, %3, 0x40000020;\n\tor.b32 i3, %3, 0x60000030;\n\t"               \
-      "tcgen05.cp.cta_group::1.32x128b.warpx4 [%5], %6;\n\t"                                                 \
-      "tcgen05.cp.cta_group::1.32x128b.warpx4 [t], %7;\n\t"
+__device__ __forceinline__ void umma_mx_block(uint32_t tmem_d, uint32_t wdesc, uint32_t w_hi, uint32_t adesc, uint32_t a_hi,
+                                              uint32_t idesc, uint32_t accumulate, uint32_t sf, uint32_t sfw_desc,
+                                              uint32_t sfa_desc, uint32_t sf_hi) {
+#define B200_MX_MMA4                                                                                                   \
+      "mov.b64 w0, {%1, %2};\n\tmov.b64 a0, {%3, %4};\n\t"                                                             \
+      "add.u32 x1, %1, %11;\n\tadd.u32 x2, %1, %12;\n\tadd.u32 x3, %1, %13;\n\t"                                      \
+      "add.u32 y1, %3, 2;\n\tadd.u32 y2, %3, 4;\n\tadd.u32 y3, %3, 6;\n\t"                                            \
+      "mov.b64 w1, {x1, %2};\n\tmov.b64 w2, {x2, %2};\n\tmov.b64 w3, {x3, %2};\n\t"                                   \
+      "mov.b64 a1, {y1, %4};\n\tmov.b64 a2, {y2, %4};\n\tmov.b64 a3, {y3, %4};\n\t"                                   \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w0, a0, %5, [%7], [t], pa;\n\t"                       \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w1, a1, i1, [%7], [t], 1;\n\t"                        \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w2, a2, i2, [%7], [t], 1;\n\t"                        \
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], w3, a3, i3, [%7], [t], 1;\n\t}"
+#define B200_MX_HEAD                                                                                                   \
+      "{\n\t.reg .pred pa;\n\t.reg .b32 t, t2, c2, i1, i2, i3, x1, x2, x3, y1, y2, y3;\n\t"                           \
+      ".reg .b64 s0, s1, s2, w0, w1, w2, w3, a0, a1, a2, a3;\n\t"                                                      \
+      "setp.ne.b32 pa, %6, 0;\n\tadd.u32 t, %7, 4;\n\t"                                                                \
+      "or.b32 i1, %5, 0x20000010;\n\tor.b32 i2, %5, 0x40000020;\n\tor.b32 i3, %5, 0x60000030;\n\t"                    \
+      "mov.b64 s0, {%8, %10};\n\tmov.b64 s1, {%9, %10};\n\t"                                                          \
+      "tcgen05.cp.cta_group::1.32x128b.warpx4 [%7], s0;\n\t"                                                           \
+      "tcgen05.cp.cta_group::1.32x128b.warpx4 [t], s1;\n\t"
   if (kTokChunks == 1) {
     asm volatile(B200_MX_HEAD B200_MX_MMA4
-                 ::"r"(tmem_d), "l"(wdesc), "l"(adesc), "r"(idesc), "r"(accumulate), "r"(sf), "l"(sfw_desc),
-                 "l"(sfa_desc), "n"(kWStep), "n"(2 * kWStep), "n"(3 * kWStep)
+                 ::"r"(tmem_d), "r"(wdesc), "r"(w_hi), "r"(adesc), "r"(a_hi), "r"(idesc), "r"(accumulate), "r"(sf),
+                 "r"(sfw_desc), "r"(sfa_desc), "r"(sf_hi), "n"(kWStep), "n"(2 * kWStep), "n"(3 * kWStep)
                  : "memory");
   } else {
     asm volatile(B200_MX_HEAD
-                 "{\n\t.reg .b32 t2;\n\t.reg .b64 c2;\n\tadd.u32 t2, %5, 8;\n\tadd.u64 c2, %7, 32;\n\t"
-                 "tcgen05.cp.cta_group::1.32x128b.warpx4 [t2], c2;\n\t}\n\t" B200_MX_MMA4
-                 ::"r"(tmem_d), "l"(wdesc), "l"(adesc), "r"(idesc), "r"(accumulate), "r"(sf), "l"(sfw_desc),
-                 "l"(sfa_desc), "n"(kWStep), "n"(2 * kWStep), "n"(3 * kWStep)
+                 "add.u32 t2, %7, 8;\n\tadd.u32 c2, %9, 32;\n\tmov.b64 s2, {c2, %10};\n\t"
+                 "tcgen05.cp.cta_group::1.32x128b.warpx4 [t2], s2;\n\t" B200_MX_MMA4
+                 ::"r"(tmem_d), "r"(wdesc), "r"(w_hi), "r"(adesc), "r"(a_hi), "r"(idesc), "r"(accumulate), "r"(sf),
+                 "r"(sfw_desc), "r"(sfa_desc), "r"(sf_hi), "n"(kWStep), "n"(2 * kWStep), "n"(3 * kWStep)
                  : "memory");
   }
 #undef B200_MX_MMA4
