@@ -11,6 +11,8 @@
 // Behaviour follows csrc/moe/topk.cpp:395-583 (gating),
 // csrc/moe/topk_softplus_sqrt_kernels.cpp:205-400 (sqrt-softplus gating) and
 // csrc/moe/grouped_topk.cpp:404-447, 525-678 (grouped) of vllm-xpu-kernels.
+#include <limits.h>
+
 #include "common.cuh"
 #include "det_math.h"
 
@@ -351,6 +353,143 @@ grouped_topk_kernel(const T* __restrict__ scores, const T* __restrict__ swb,
   }
 }
 
+// The same for 32 * VPT experts in a power-of-two number of groups: a lane owns VPT consecutive columns, so a
+// group is the columns of 32 / n_group neighbouring lanes, all groups are scored at once, ids ascend with the
+// lanes, and a round of the selection is one integer maximum over the warp (redux) and a ballot.  Instructions bound
+// it: the general kernel tests every column against every group (an integer division each) and needs ten shuffles
+// with their comparisons per round.  256 experts in 8 groups, top 8: 8192 tokens 45 -> 12 us, 1024 tokens 14 -> 6.
+template <int VPT>
+struct OwnColumns {
+  // Columns lane * VPT .. of a row that begins on a 16-byte boundary.
+  template <typename T>
+  static __device__ __forceinline__ void load(const T* row, int lane, float (&v)[VPT]) {
+    constexpr int kBytes = VPT * (int)sizeof(T);
+    const T* from = row + lane * VPT;
+    if (kBytes % 16 == 0) {
+#pragma unroll
+      for (int j = 0; j < kBytes / 16; ++j) {
+        const vec16 q = ld16(from + j * (16 / (int)sizeof(T)));
+        const T* e = reinterpret_cast<const T*>(&q);
+#pragma unroll
+        for (int i = 0; i < 16 / (int)sizeof(T); ++i) v[j * (16 / (int)sizeof(T)) + i] = to_f32<T>(e[i]);
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i) v[i] = to_f32<T>(from[i]);
+    }
+  }
+};
+// Integers in the order of the floats (-0 and +0 alike); INT_MIN is below all of them.
+__device__ __forceinline__ int order_of(float x) {
+  const int b = __float_as_int(x + 0.0f);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float from_order(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+template <typename T, int VPT>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+grouped_topk_aligned_kernel(const T* __restrict__ scores, const T* __restrict__ swb, T* __restrict__ out_val,
+                            int32_t* __restrict__ out_idx, int64_t num_tokens, int n_group, int topk_group, int K,
+                            bool renorm, double rsf) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr uint32_t kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int64_t tok = (int64_t)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  if (tok >= num_tokens) return;  // whole warp leaves together
+  const int lanes = 32 / n_group;   // of a group
+  const T* sc = scores + tok * (int64_t)(32 * VPT);
+  float v[VPT];
+  OwnColumns<VPT>::load(swb + tok * (int64_t)(32 * VPT), lane, v);
+
+  // Group scores: sum of the two largest, rounded through T as the reference stores it.
+  float m1 = -INFINITY, m2 = -INFINITY;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) {
+    if (v[i] > m1) { m2 = m1; m1 = v[i]; }
+    else if (v[i] > m2) { m2 = v[i]; }
+  }
+  for (int mask = 1; mask < lanes; mask <<= 1) {
+    const float o1 = __shfl_xor_sync(kAll, m1, mask);
+    const float o2 = __shfl_xor_sync(kAll, m2, mask);
+    const float n2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
+    m1 = fmaxf(m1, o1);
+    m2 = n2;
+  }
+  const float gs = to_f32<T>(from_f32<T>(__fadd_rn(m1, m2)));
+  // lane g keeps group g's
+  const float of_lane = __shfl_sync(kAll, gs, (lane * lanes) & 31);
+  const float my_gs = lane < n_group ? of_lane : -INFINITY;
+
+  // Threshold search as in the general kernel.
+  float value = (lane < n_group && isfinite(my_gs)) ? my_gs : -INFINITY;
+  const int target = 32 - n_group + topk_group;
+  int count = 32 - n_group;
+  int pre_count = 0;
+  float thr = -INFINITY;
+  for (int it = 0; it < 32 && count < target; ++it) {
+    thr = from_order(__reduce_max_sync(kAll, order_of(value)));
+    if (value == thr) value = -INFINITY;
+    pre_count = count;
+    count = __popc(__ballot_sync(kAll, value == -INFINITY));
+  }
+  if (thr == -INFINITY) {
+    for (int i = lane; i < K; i += 32) {
+      out_idx[tok * K + i] = i;
+      out_val[tok * K + i] = from_f32<T>(1.0f / (float)K);
+    }
+    return;
+  }
+  const uint32_t gt = __ballot_sync(kAll, lane < n_group && my_gs > thr);
+  const uint32_t eq = __ballot_sync(kAll, lane < n_group && my_gs == thr);
+  // of the groups at the threshold the first target - pre_count
+  const bool kept_lane = ((gt >> lane) & 1u) || (((eq >> lane) & 1u) && __popc(eq & ((1u << lane) - 1u)) < target - pre_count);
+  const uint32_t keep_mask = __ballot_sync(kAll, kept_lane);
+  const bool kept = (keep_mask >> (lane / lanes)) & 1u;
+
+  // K rounds of arg-max, ties to the lower expert id: a lane's best is the first of its largest
+  // columns that are left, the warp's the lowest lane's.
+  int key[VPT];
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) key[i] = order_of(kept && isfinite(v[i]) ? v[i] : -INFINITY);
+  int best = INT_MIN, best_i = 0;
+  auto find = [&]() {
+    best = INT_MIN;
+#pragma unroll
+    for (int i = 0; i < VPT; ++i)
+      if (key[i] > best) { best = key[i]; best_i = i; }
+  };
+  find();
+  int my_id = 0;  // lane k keeps the k-th id
+  for (int k = 0; k < K; ++k) {
+    const int top = __reduce_max_sync(kAll, best);
+    const int winner = __ffs(__ballot_sync(kAll, best == top)) - 1;
+    const int id = __shfl_sync(kAll, lane * VPT + best_i, winner);
+    if (lane == k) my_id = id;
+    if (lane == winner) {
+#pragma unroll
+      for (int i = 0; i < VPT; ++i)
+        if (i == best_i) key[i] = INT_MIN;
+      find();
+    }
+  }
+
+  float w = 0.f;
+  if (lane < K) w = to_f32<T>(sc[my_id]);
+  float s = w;
+#pragma unroll
+  for (int mask = 16; mask > 0; mask >>= 1)
+    s = __fadd_rn(s, __shfl_xor_sync(kAll, s, mask));
+  const float topk_sum = __fadd_rn(1e-20f, s);
+  if (lane < K) {
+    float r;
+    if (renorm) r = (float)((double)__fdiv_rn(w, topk_sum) * rsf);
+    else r = (float)((double)w * rsf);
+    out_idx[tok * K + lane] = my_id;
+    out_val[tok * K + lane] = from_f32<T>(r);
+  }
+}
+
 }  // namespace
 }  // namespace b200moe
 
@@ -418,8 +557,19 @@ extern "C" int b200moe_grouped_topk(void* topk_values, int32_t* topk_indices,
       return fail(B200MOE_E_BADARG,
                   "Invalid dtype, only supports float16, float32, and bfloat16");
   }
+  // 64 to 512 experts (a power of two of them) in a power-of-two number of groups: see the kernel
+  const bool aligned = num_experts >= 64 && num_experts <= 512 && (num_experts & (num_experts - 1)) == 0 &&
+                       (n_group & (n_group - 1)) == 0 && (((uintptr_t)scores_with_bias) & 15) == 0;
+#define B200_GT_ALIGNED(VPT_)                                                  \
+  B200_LAUNCHED("grouped_topk_aligned_kernel", launch_pdl(num_tokens * topk <= kEarlyLaunchRows, grouped_topk_aligned_kernel<scalar_t, VPT_>, \
+      dim3(grid), dim3(kWarpsPerBlock * 32), 0, st, \
+      (const scalar_t*)scores, (const scalar_t*)scores_with_bias, (scalar_t*)topk_values, topk_indices, num_tokens, n_group, topk_group, topk, renormalize != 0, routed_scaling_factor))
   B200_DISPATCH_FLOAT(dtype, "grouped_topk", {
-    if (num_experts <= 32) B200_GT_CASE(1);
+    if (aligned && num_experts == 64) B200_GT_ALIGNED(2);
+    else if (aligned && num_experts == 128) B200_GT_ALIGNED(4);
+    else if (aligned && num_experts == 256) B200_GT_ALIGNED(8);
+    else if (aligned && num_experts == 512) B200_GT_ALIGNED(16);
+    else if (num_experts <= 32) B200_GT_CASE(1);
     else if (num_experts <= 64) B200_GT_CASE(2);
     else if (num_experts <= 128) B200_GT_CASE(4);
     else if (num_experts <= 256) B200_GT_CASE(8);
@@ -427,6 +577,7 @@ extern "C" int b200moe_grouped_topk(void* topk_values, int32_t* topk_indices,
     else B200_GT_CASE(32);
   });
 #undef B200_GT_CASE
+#undef B200_GT_ALIGNED
   return B200MOE_OK;
 }
 
