@@ -761,7 +761,7 @@ extern "C" int b200moe_moe_align_block_size_noalloc(
     g_noalloc_ptr[dev].store(scratch, std::memory_order_release);
   }
   // Nothing in the buffer has to start at zero: the count pass overwrites every
-  // histogram cell it later reads and the scan pass writes the prefix array.
+  // histogram cell it later reads and the scan pass writes the sizes.
   return b200moe_moe_align_block_size(topk_ids, ids_dtype, numel, num_experts, block_size,
                                       sorted_token_ids, sorted_len, expert_ids, expert_ids_len,
                                       num_tokens_post_pad, expert_map, scratch,
