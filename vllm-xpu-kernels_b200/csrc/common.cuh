@@ -125,6 +125,14 @@ template <> __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(flo
 __device__ __forceinline__ uint8_t f32_to_e4m3(float v) {
   return (uint8_t)__nv_cvt_float_to_fp8(v, __NV_SATFINITE, __NV_E4M3);
 }
+// Two at once (one conversion instruction), x in the low byte.
+__device__ __forceinline__ uint32_t f32x2_to_e4m3x2(float x, float y) {
+  return __nv_cvt_float2_to_fp8x2(make_float2(x, y), __NV_SATFINITE, __NV_E4M3);
+}
+__device__ __forceinline__ float2 e4m3x2_to_f32x2(uint32_t v) {
+  const __half2_raw h = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)v, __NV_E4M3);
+  return __half22float2(*reinterpret_cast<const __half2*>(&h));
+}
 __device__ __forceinline__ float e4m3_to_f32(uint8_t v) {
   __half_raw h = __nv_cvt_fp8_to_halfraw(v, __NV_E4M3);
   return __half2float(*reinterpret_cast<__half*>(&h));

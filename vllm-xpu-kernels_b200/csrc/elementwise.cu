@@ -251,7 +251,7 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
   const int steps = (pieces + kMxQuantUnroll - 1) / kMxQuantUnroll;
   const int64_t total = rows * steps;
   for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < total; w += (int64_t)gridDim.x * 8) {
-    const int64_t r = w / steps;
+    const int64_t r = total <= 0xffffffffll ? (int64_t)((uint32_t)w / (uint32_t)steps) : w / steps;
     const int j0 = (int)(w - r * steps) * kMxQuantUnroll * 32 + lane;
     const T* xr = x + r * (int64_t)cols * (kGated ? 2 : 1);
     vec16 in[kMxQuantUnroll], up[kGated ? kMxQuantUnroll : 1];
@@ -278,7 +278,7 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
       }
       for (int term = 0; term < terms; ++term) {
         uint2 codes;
-        const uint32_t word = mx_quant_lane(v, j < nvec, codes, sums ? kMxLeastExact : kMxLeast);
+        const uint32_t word = mx_quant_lane(v, j < nvec, codes, sums ? kMxLeastExact : kMxLeast, sums || term + 1 < terms);
         if (j < nvec) *reinterpret_cast<uint2*>(q + (term * rows + r) * cols + (int64_t)j * 8) = codes;
         if ((j & 15) == 0 && j < num_kb * 16) s[((int64_t)term * num_kb + (j >> 4)) * rows + r] = word;
       }

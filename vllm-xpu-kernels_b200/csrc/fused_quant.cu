@@ -73,7 +73,6 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
   pdl_trigger();
   pdl_wait();
   constexpr int N = Vec16<T>::N;
-  const int64_t r0 = (int64_t)blockIdx.x * kRows;
   if (a.rows_per_segment != nullptr) {
     __shared__ int64_t in_use;
     if (threadIdx.x < 32) {
@@ -85,13 +84,13 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
     }
     __syncthreads();
     if (in_use < rows) rows = in_use;
-    if (r0 >= rows) return;
   }
   const int lanes_per_group = a.group / N;
   const int nvec = a.hidden / N;
   const int64_t in_pitch = (int64_t)a.hidden * (kGated ? 2 : 1);
   const T* in0 = reinterpret_cast<const T*>(a.in);
   const int lane = threadIdx.x & 31;
+  for (int64_t r0 = (int64_t)blockIdx.x * kRows; r0 < rows; r0 += (int64_t)gridDim.x * kRows)
   for (int base = 0; base < nvec; base += blockDim.x) {
     const int c = base + threadIdx.x;
     vec16 gq[kRows], uq[kRows];
@@ -157,11 +156,17 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
           else *reinterpret_cast<uint16_t*>(dst) = *reinterpret_cast<const uint16_t*>(o);
         } else {
           alignas(8) uint8_t o[N];
+          const float inv = __fdividef(1.0f, scale);   // the group's, once: v * inv is __fdividef(v, scale)
 #pragma unroll
-          for (int i = 0; i < N; ++i) {
-            const float q = __fdividef(v[i], scale);
-            if (kFmt == kOutI8) o[i] = (uint8_t)f32_to_i8_rn(q);
-            else o[i] = f32_to_e4m3(fmaxf(-448.0f, fminf(q, 448.0f)));
+          for (int i = 0; i < N; i += 2) {
+            const float q0 = __fmul_rn(v[i], inv), q1 = __fmul_rn(v[i + 1], inv);
+            if (kFmt == kOutI8) {
+              o[i] = (uint8_t)f32_to_i8_rn(q0);
+              o[i + 1] = (uint8_t)f32_to_i8_rn(q1);
+            } else {
+              // (the conversion saturates; the minimum makes 448 of a NaN)
+              *reinterpret_cast<uint16_t*>(o + i) = (uint16_t)f32x2_to_e4m3x2(fminf(q0, 448.0f), fminf(q1, 448.0f));
+            }
           }
           uint8_t* dst = reinterpret_cast<uint8_t*>(a.out) + r * (int64_t)a.hidden + (int64_t)c * N;
           if (N == 8) *reinterpret_cast<uint2*>(dst) = *reinterpret_cast<const uint2*>(o);
@@ -217,19 +222,18 @@ silu_mul_static_quant_kernel(uint8_t* __restrict__ out, const T* __restrict__ in
 template <bool kGated, int kFmt>
 int launch_group_quant(b200moe_dtype dtype, const GroupQuantArgs& a, int64_t rows, cudaStream_t st,
                        const char* name) {
-  if (dtype == B200MOE_BF16) {
-    B200_LAUNCHED("group_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<__nv_bfloat16, kGated, kFmt>,
-        dim3((unsigned)((rows + kRows - 1) / kRows)), dim3(threads_for(a.hidden / 8)), 0, st,
-        a, rows));
-  } else if (dtype == B200MOE_F16) {
-    B200_LAUNCHED("group_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<__half, kGated, kFmt>,
-        dim3((unsigned)((rows + kRows - 1) / kRows)), dim3(threads_for(a.hidden / 8)), 0, st,
-        a, rows));
-  } else {
-    B200_LAUNCHED("group_quant_kernel", launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<float, kGated, kFmt>,
-        dim3((unsigned)((rows + kRows - 1) / kRows)), dim3(threads_for(a.hidden / 4)), 0, st,
-        a, rows));
-  }
+  const int threads = threads_for(a.hidden / (dtype == B200MOE_F32 ? 4 : 8));
+  // As many blocks as are resident together: each sums the segments once and walks over its rows.  Instructions
+  // bound the kernel (issue slots 79 % in use, DRAM 43 %): the reciprocal of a group's scale once, two values a
+  // conversion, 65536 x 2048 values with SiLU 189 -> 174 us.
+  const int64_t blocks = (rows + kRows - 1) / kRows, most = (int64_t)sm_count() * (2048 / threads);
+  const dim3 grid((unsigned)(blocks < most ? blocks : most));
+  auto run = [&](auto type) {
+    return launch_pdl(rows <= kEarlyLaunchRows, group_quant_kernel<decltype(type), kGated, kFmt>, grid, dim3(threads), 0, st, a, rows);
+  };
+  if (dtype == B200MOE_BF16) B200_LAUNCHED("group_quant_kernel", run(__nv_bfloat16()));
+  else if (dtype == B200MOE_F16) B200_LAUNCHED("group_quant_kernel", run(__half()));
+  else B200_LAUNCHED("group_quant_kernel", run(0.f));
   return B200MOE_OK;
 }
 

@@ -10,8 +10,8 @@ namespace {
 
 // A lane holds 8 values, four lanes one group of 32, sixteen lanes (aligned in the warp) one
 // 128-wide block; all lanes of the warp call it.  Writes the codes, leaves the residual
-// v - code * scale in v (what a second plane quantises) and returns the block's scale word: byte g
-// of it is group g's scale, 0x7f (2^0) for groups whose lanes are not `active`.
+// v - code * scale in v if it is asked for (what a second plane quantises) and returns the block's scale word:
+// byte g of it is group g's scale, 0x7f (2^0) for groups whose lanes are not `active`.
 //
 // amax / 448 <= 2^e is amax <= 1.75 * 2^(e + 8), a comparison of exponent and mantissa; scale and
 // inverse are then exact powers of two (the divisions this replaces gave the same bits).
@@ -20,7 +20,7 @@ namespace {
 // lose bits and then vanish.  Planes that stand for 16-bit activations (an int4 layer's) go down to
 // 2^-100: what they leave of a bfloat16 is below 2^-109, and nothing gets near fp32's subnormals.
 constexpr int kMxLeast = 127 - 33, kMxLeastExact = 127 - 100;
-__device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes, int least) {
+__device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes, int least, bool residual) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
@@ -31,12 +31,26 @@ __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, ui
   e = e < least ? least : e;
   if (bits >= 0x7f800000u) e = 255;   // an infinity in the group: the scale byte is NaN
   const float sc = __uint_as_float((uint32_t)e << 23), inv = e == 255 ? 0.f : __uint_as_float((uint32_t)(254 - e) << 23);
-  uint32_t c[2] = {0u, 0u};
+  // Instructions bound the quantisers (ALU pipe 69 %, DRAM 29 %): two values a conversion, one comparison a value,
+  // no residual behind the last plane, and as code * scale is exact the residual is one fused operation.
+  // 8192 x 2880 values with the launch: two planes 52 -> 42 us, one 33 -> 28.
+  uint32_t c[2];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const uint32_t o = f32_to_e4m3(fminf(fmaxf(__fmul_rn(v[i], inv), -448.f), 448.f));
-    c[i >> 2] |= o << (8 * (i & 3));
-    v[i] = __fsub_rn(v[i], __fmul_rn(e4m3_to_f32((uint8_t)o), sc));
+  for (int i = 0; i < 8; i += 4) {
+    uint32_t o[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      o[j] = f32x2_to_e4m3x2(fmaxf(__fmul_rn(v[i + 2 * j], inv), -448.f),   // saturates; the maximum makes -448 of a NaN
+                             fmaxf(__fmul_rn(v[i + 2 * j + 1], inv), -448.f));
+    c[i >> 2] = o[0] | (o[1] << 16);
+    if (residual) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float2 d = e4m3x2_to_f32x2(o[j]);
+        v[i + 2 * j] = fmaf(-d.x, sc, v[i + 2 * j]);
+        v[i + 2 * j + 1] = fmaf(-d.y, sc, v[i + 2 * j + 1]);
+      }
+    }
   }
   codes = make_uint2(c[0], c[1]);
   const uint32_t byte = (active ? (uint32_t)e : 0x7fu) << (8 * ((threadIdx.x >> 2) & 3));

@@ -115,7 +115,7 @@ __device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, 
 #pragma unroll 1
   for (int p = 0; p < a.planes; ++p) {
     uint2 codes;
-    const uint32_t word = mx_quant_lane(v, in, codes, a.sums ? kMxLeastExact : kMxLeast);
+    const uint32_t word = mx_quant_lane(v, in, codes, a.sums ? kMxLeastExact : kMxLeast, a.sums || p + 1 < a.planes);
     for (int k = 0; k < a.K; ++k) {
       const int r = dest[k];
       if (r >= 0) {
