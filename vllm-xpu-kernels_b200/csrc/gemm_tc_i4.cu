@@ -18,14 +18,23 @@
 // Roles (768 threads in warpgroups that re-balance registers, one persistent CTA per SM; tiles of
 // 128 features x BT tokens):
 //   warp 0       : TMA producer: per K block 128 x 64 packed bytes and the planes' BT x 128 bytes
-//   warp 1       : MMA issuer; copies the tokens' scale factors to tensor memory (tcgen05.cp); the
-//                  planes accumulate in the same columns, so the promotion reads BT columns only
-//   warps 2-3    : bring the tokens' scale words and sums, four K blocks at a time
+//   warps 1-2    : MMA issuers, a thread each, which take K blocks in turn; they copy the tokens' scale
+//                  factors to tensor memory (tcgen05.cp); the planes accumulate in the same columns, so the
+//                  promotion reads BT columns only
+//   warp 3       : brings the tokens' scale words and sums, four K blocks at a time
 //   warps 4-15   : converters, three sets that take K blocks in turn (a set is one long chain of
 //                  latencies, 630 cycles per block): a thread unpacks a row's 64 bytes into 32 columns
 //                  of tensor memory, from where the MMA reads the weights (nothing goes back through
 //                  shared memory)
 //   warps 16-23  : promotion and epilogue; warp w owns lane quarter w & 3 and half of the columns
+// What bounds it is none of the units but the chain of hand-overs of a K block: a look at an mbarrier that is
+// already complete costs its warp about 100 cycles, an arrival as much, and one issuer that waited for the stage,
+// the operand, the accumulator and the scales needed 620 cycles a block.  So there are two issuers, and each
+// hand-over stands for all that it implies: the converters' arrival for the stage's tokens (they waited for the
+// same stage), an accumulator's completion for its operand columns and for the group's scales, and a stage is
+// released with the arrival of the block kI4Conv further on, which waited for the MMAs of the one before.
+// 33 tokens x top-2 of 8 experts, 28672 x 4096 and 4096 x 14336: 144 -> 135 and 97 -> 94.5 us; the next in the
+// row are the promotion warps (540 cycles a block).
 // Waits are bounded as in the other kernels (sm100_ptx.cuh).
 #include "common.cuh"
 #include "gemm_tc_common.cuh"
@@ -42,8 +51,12 @@ constexpr int kI4MaxStages = 12;
 constexpr int kI4Group = 4;          // K blocks per hand-over of token scales
 constexpr int kI4Slots = 3;
 constexpr int kI4Sets = 3;           // converter sets
-constexpr int kI4Conv = 4;           // weight-operand stages in tensor memory (32 columns each)
-constexpr int kI4Acc = 4;            // accumulator stages
+constexpr int kI4Issuers = 2;        // threads that issue MMAs
+// Blocks in tensor memory: operand (32 columns), token scales and accumulator of block i are slot i % kI4Conv.
+constexpr int kI4Conv = 6;
+// A slot stays with one issuer, whose instructions execute in order, and with one converter set, which has seen
+// the slot's block before the last complete when it waits for the last by parity.
+static_assert(kI4Conv % kI4Issuers == 0 && kI4Conv % kI4Sets == 0, "slots");
 
 struct I4Params {
   const uint16_t* w_scale;   // [E, N, groups] in the activation type
@@ -67,9 +80,9 @@ struct I4Shape {
   static constexpr int kABytes = kTerms * BT * 128;
   static constexpr int kStageBytes = kI4RawBytes + kABytes;
   static constexpr int kSfPer = 4 * kTokChunks;               // tokens' scale columns of a K block
-  static constexpr uint32_t kConvBase = kI4Acc * BT;
+  static constexpr uint32_t kConvBase = kI4Conv * BT;
   static constexpr uint32_t kSfBase = kConvBase + kI4Conv * 32;   // weights' scale columns (constant), then the tokens'
-  static constexpr uint32_t kCols = kSfBase + 8 + kI4Group * kSfPer;
+  static constexpr uint32_t kCols = kSfBase + 8 + kI4Conv * kSfPer;
   static constexpr uint32_t kTmem = kCols <= 256 ? 256u : 512u;
   static constexpr int kSlotBytes = kI4Group * (512 * kTokChunks + BT * 4);
   static_assert(BT <= 32 && kCols <= 512, "tensor memory");
@@ -77,13 +90,12 @@ struct I4Shape {
 
 struct I4Ctrl {
   uint64_t full[kI4MaxStages];
-  uint64_t empty[kI4MaxStages];      // the MMA has read the tokens and the converters the packed weights
+  uint64_t empty[kI4MaxStages];      // the converters, which have read the packed weights, and one of them for the MMA
   uint64_t conv_full[kI4Conv];
-  uint64_t conv_empty[kI4Conv];
-  uint64_t acc_full[kI4Acc];
-  uint64_t acc_empty[kI4Acc];
+  uint64_t acc_full[kI4Conv];        // the block's MMAs are complete (its operand columns are free, too)
+  uint64_t acc_empty[kI4Conv];
   uint64_t sf_full[kI4Slots];
-  uint64_t sf_empty[kI4Slots];       // the MMA thread and the promotion warps
+  uint64_t sf_empty[kI4Slots];       // the promotion warps, which have seen the group's MMAs complete
   uint32_t tmem_base;
   int abort_flag;
   alignas(16) uint16_t xpose[8][16 * 32];   // per promotion warp: output transpose tile
@@ -121,15 +133,14 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
     for (int c = 0; c < kI4Conv; ++c) {
       ptx::mbar_init(&ctrl->conv_full[c], 4);
-      ptx::mbar_init(&ctrl->conv_empty[c], 1);
     }
-    for (int a = 0; a < kI4Acc; ++a) {
+    for (int a = 0; a < kI4Conv; ++a) {
       ptx::mbar_init(&ctrl->acc_full[a], 1);
       ptx::mbar_init(&ctrl->acc_empty[a], 8);
     }
     for (int g = 0; g < kI4Slots; ++g) {
-      ptx::mbar_init(&ctrl->sf_full[g], 2);
-      ptx::mbar_init(&ctrl->sf_empty[g], 1 + 8);
+      ptx::mbar_init(&ctrl->sf_full[g], 1);
+      ptx::mbar_init(&ctrl->sf_empty[g], 8);
     }
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
@@ -152,7 +163,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   const TileWalk walk = tile_walk_at(walk_mem, p.num_experts);
   const int total_tiles = walk.total;
   const uint32_t full0 = ptx::smem_u32(&ctrl->full[0]), empty0 = ptx::smem_u32(&ctrl->empty[0]);
-  const uint32_t conv_full0 = ptx::smem_u32(&ctrl->conv_full[0]), conv_empty0 = ptx::smem_u32(&ctrl->conv_empty[0]);
+  const uint32_t conv_full0 = ptx::smem_u32(&ctrl->conv_full[0]);
   const uint32_t acc_full0 = ptx::smem_u32(&ctrl->acc_full[0]), acc_empty0 = ptx::smem_u32(&ctrl->acc_empty[0]);
   const uint32_t sf_full0 = ptx::smem_u32(&ctrl->sf_full[0]), sf_empty0 = ptx::smem_u32(&ctrl->sf_empty[0]);
   int my_tiles = 0;
@@ -184,58 +195,58 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         }
       }
       __syncwarp();
-    } else if (warp == 1) {
-      // ------------------------------ MMA issuer --------------------------------
+    } else if (warp <= kI4Issuers) {
+      // ------------------------------ MMA issuers -------------------------------
+      // Every kI4Issuers-th block each: blocks have accumulators of their own, so their order does not matter.
       if (ptx::elect_one()) {
-        uint32_t s = 0, ph = 0, c = 0, cph = 0, a = 0, aph = 1, slot = 0, slot_ph = 0;
+        const uint32_t mine = warp - 1;
+        uint32_t turn = 0, c = 0, cph = 0, s = 0;      // whose block, its slot, its ring stage
+        uint32_t u = 0, slot = 0, slot_ph = 0;         // its place in the group of scales, the group's
         int cursor = 0;
         bool ok = true;
-        const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kI4RawBytes, 16, 1024);
+        const uint64_t adesc_at0 = ptx::make_smem_desc(ptx::smem_u32(smem) + kI4RawBytes, 16, 1024);
+        const uint32_t adesc0 = (uint32_t)adesc_at0, a_hi = (uint32_t)(adesc_at0 >> 32);
         const uint64_t sfdesc0 = ptx::make_smem_desc_plain(ptx::smem_u32(sf_ring), 128);
-        uint64_t adesc = adesc0, sfdesc = sfdesc0;
+        const uint32_t sf = tmem_base + S::kSfBase;
         for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
           TileInfo ti;
           locate_tile<BT>(walk, t, cursor, ti);
           // a partly filled token tile multiplies only its valid columns (UMMA N in steps of 16)
           const uint32_t n_eff = (uint32_t)((ti.valid + 15) & ~15);
           const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((n_eff >> 3) << 17);
-          for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += kI4Group) {
-            if (!ptx::mbar_wait_s(sf_full0 + 8 * slot, slot_ph, abort_flag)) { ok = false; break; }
-  #pragma unroll
-            for (int u = 0; u < kI4Group; ++u) {
-              if (kb0 + u < p.num_kb) {
-                if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag) ||
-                    !ptx::mbar_wait_s(conv_full0 + 8 * c, cph, abort_flag) ||
-                    !ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) { ok = false; break; }
-                ptx::tc_fence_after();
-                const uint32_t sf = tmem_base + S::kSfBase, sfa = sf + 8 + u * S::kSfPer;
-                ptx::tmem_cp_scales(sfa, sfdesc + u * (S::kTokChunks * 32));
-                if (S::kTokChunks == 2) ptx::tmem_cp_scales(sfa + 4, sfdesc + u * (S::kTokChunks * 32) + 32);
-  #pragma unroll
-                for (int term = 0; term < kTerms; ++term)
-                  ptx::umma_mx_block_ts(tmem_base + a * BT, tmem_base + S::kConvBase + c * 32, adesc + term * (BT * 128 >> 4),
-                                        idesc, term > 0 ? 1u : 0u, sf, sfa + 2 * term);
-                ptx::umma_commit(acc_full0 + 8 * a);
-                ptx::umma_commit(conv_empty0 + 8 * c);
-                ptx::umma_commit(empty0 + 8 * s);
-                adesc += kStageBytes >> 4;
-                if (++s == (uint32_t)stages) { s = 0; ph ^= 1; adesc = adesc0; }
-                if (++c == kI4Conv) { c = 0; cph ^= 1; }
-                if (++a == kI4Acc) { a = 0; aph ^= 1; }
-              }
+#pragma unroll 1
+          for (int kb = 0; kb < p.num_kb; ++kb) {
+            if (turn == mine) {
+              // (the converters have seen the block's loads land, the tokens' among them)
+              if ((u < kI4Issuers && !ptx::mbar_wait_s(sf_full0 + 8 * slot, slot_ph, abort_flag)) ||
+                  !ptx::mbar_wait_s(conv_full0 + 8 * c, cph, abort_flag) ||
+                  !ptx::mbar_wait_s(acc_empty0 + 8 * c, cph ^ 1, abort_flag)) { ok = false; break; }
+              ptx::tc_fence_after();
+              const uint32_t sfa = sf + 8 + c * S::kSfPer, adesc = adesc0 + s * (kStageBytes >> 4);
+              const uint64_t sfd = sfdesc0 + slot * (kSlotBytes >> 4) + u * (S::kTokChunks * 32);
+              ptx::tmem_cp_scales(sfa, sfd);
+              if (S::kTokChunks == 2) ptx::tmem_cp_scales(sfa + 4, sfd + 32);
+#pragma unroll
+              for (int term = 0; term < kTerms; ++term)
+                ptx::umma_mx_block_ts(tmem_base + c * BT, tmem_base + S::kConvBase + c * 32, adesc + term * (BT * 128 >> 4), a_hi,
+                                      idesc, term > 0 ? 1u : 0u, sf, sfa + 2 * term);
+              ptx::umma_commit(acc_full0 + 8 * c);
             }
-            if (!ok) break;
-            ptx::umma_commit(sf_empty0 + 8 * slot);
-            sfdesc += kSlotBytes >> 4;
-            if (++slot == kI4Slots) { slot = 0; slot_ph ^= 1; sfdesc = sfdesc0; }
+            if (++turn == kI4Issuers) turn = 0;
+            if (++c == kI4Conv) { c = 0; cph ^= 1; }
+            if (++s == (uint32_t)stages) s = 0;
+            if (++u == kI4Group || kb + 1 == p.num_kb) {
+              u = 0;
+              if (++slot == kI4Slots) { slot = 0; slot_ph ^= 1; }
+            }
           }
         }
       }
       __syncwarp();
     } else {
       // ------------------------ tokens' scales and sums ---------------------------
-      const int ft = (warp - 2) * 32 + lane;            // 0..63
-      constexpr int kNT = kTerms * BT, kPer = kI4Group * kNT / 64, kPerSum = (kI4Group * BT + 63) / 64;
+      const int ft = lane;
+      constexpr int kNT = kTerms * BT, kPer = kI4Group * kNT / 32, kPerSum = kI4Group * BT / 32;
       const int64_t plane_words = (int64_t)p.num_kb * p.m;
       const float* sums = reinterpret_cast<const float*>(p.a_scale + kTerms * plane_words);
       uint32_t slot = 0, slot_ph = 1;
@@ -250,14 +261,14 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           float m[kPerSum];
   #pragma unroll
           for (int i = 0; i < kPer; ++i) {
-            const int x = ft + 64 * i, n = x % kNT, kb = kb0 + x / kNT, term = n / BT, tok = n % BT;
+            const int x = ft + 32 * i, n = x % kNT, kb = kb0 + x / kNT, term = n / BT, tok = n % BT;
             w[i] = (kb < p.num_kb && tok < ti.valid)
                        ? __ldg(p.a_scale + term * plane_words + (int64_t)kb * p.m + ti.row0 + tok) : 0x7f7f7f7fu;
           }
   #pragma unroll
           for (int i = 0; i < kPerSum; ++i) {
-            const int x = ft + 64 * i, tok = x % BT, kb = kb0 + x / BT;
-            m[i] = (x < kI4Group * BT && kb < p.num_kb && tok < ti.valid)
+            const int x = ft + 32 * i, tok = x % BT, kb = kb0 + x / BT;
+            m[i] = (kb < p.num_kb && tok < ti.valid)
                        ? -8.0f * __ldg(sums + (int64_t)kb * p.m + ti.row0 + tok) : 0.f;
           }
           if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
@@ -265,13 +276,13 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   #pragma unroll
           for (int i = 0; i < kPer; ++i) {
             // plane `term` takes the columns 2 * term and 2 * term + 1 (an MMA's scales start on an even one)
-            const int x = ft + 64 * i, n = x % kNT, u = x / kNT, term = n / BT, tok = n % BT;
+            const int x = ft + 32 * i, n = x % kNT, u = x / kNT, term = n / BT, tok = n % BT;
             ptx::sts32(ring + u * (S::kTokChunks * 512) + (term >> 1) * 512 + (tok & 31) * 16 + ((2 * term + (tok >> 5)) & 3) * 4,
                        w[i]);
           }
   #pragma unroll
           for (int i = 0; i < kPerSum; ++i)
-            if (ft + 64 * i < kI4Group * BT) ptx::sts32f(ring + kI4Group * 512 * S::kTokChunks + (ft + 64 * i) * 4, m[i]);
+            ptx::sts32f(ring + kI4Group * 512 * S::kTokChunks + (ft + 32 * i) * 4, m[i]);
           ptx::fence_proxy_async();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive_s(sf_full0 + 8 * slot);
@@ -286,10 +297,9 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const uint32_t lane_sel = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t src0 = ptx::smem_u32(smem) + row * 64;
     const uint32_t swz = (uint32_t)((row >> 1) & 3) << 4;      // 64-byte swizzle: chunk index xor row bits 1..2
-    uint32_t s = set, ph = 0;
+    uint32_t s = set, ph = 0, c = set, cph = 0;
     const uint32_t blocks = (uint32_t)my_tiles * p.num_kb;      // every tile: the same K loop
     for (uint32_t i = set; i < blocks; i += kI4Sets) {
-      const uint32_t c = i % kI4Conv;
       if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(full0 + 8 * s, ph, abort_flag))) break;
       const uint32_t src = src0 + s * kStageBytes;
       uint32_t o[32];
@@ -307,13 +317,18 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_s(empty0 + 8 * s);
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(conv_empty0 + 8 * c, ((i / kI4Conv) & 1) ^ 1, abort_flag))) break;
+      // the operand columns are free when the MMAs of the slot's block before are complete: its accumulator is full
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(acc_full0 + 8 * c, cph ^ 1, abort_flag))) break;
       ptx::tc_fence_after();
       ptx::tmem_st_32x32(tmem_base + S::kConvBase + c * 32 + lane_sel, o);
       ptx::tmem_wait_st();
       ptx::tc_fence_before();
+      // ... and the MMAs of block i - kI4Conv are done with their stage's tokens
+      const uint32_t old = s >= kI4Conv ? s - kI4Conv : s + stages - kI4Conv;
       __syncwarp();
-      if (lane == 0) ptx::mbar_arrive_s(conv_full0 + 8 * c);
+      ptx::mbar_arrive_if(conv_full0 + 8 * c, lane == 0, empty0 + 8 * old, (warp & 3) == 0 && i >= kI4Conv);
+      c += kI4Sets;
+      if (c >= kI4Conv) { c -= kI4Conv; cph ^= 1; }
       s += kI4Sets;
       if (s >= (uint32_t)stages) { s -= stages; ph ^= 1; }
     }
@@ -325,7 +340,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     const int et = q * 32 + lane;
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
     const int col0 = half * kHalf;
-    uint32_t a = 0, aph = 0, slot = 0, slot_ph = 0;
+    uint32_t a = 0, aph = 0, slot = 0;
     int cursor = 0;
     bool ok = true;
     const bool vec4 = p.kb_shift == 0 && p.groups % 4 == 0 && (reinterpret_cast<uintptr_t>(p.w_scale) & 7) == 0;
@@ -369,7 +384,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           sc[0] = __uint_as_float(cur.x << 16); sc[1] = __uint_as_float(cur.x & 0xffff0000u);
           sc[2] = __uint_as_float(cur.y << 16); sc[3] = __uint_as_float(cur.y & 0xffff0000u);
         }
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_full0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
+        // (the group's sums are there when its first accumulator is: the issuer has waited for them)
         const uint32_t sums = ptx::smem_u32(sf_ring) + slot * kSlotBytes + kI4Group * 512 * S::kTokChunks + col0 * 4;
 #pragma unroll
         for (int u = 0; u < kI4Group; ++u) {
@@ -385,8 +400,8 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           }
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);   // the stage is in registers
-          if (++a == kI4Acc) { a = 0; aph ^= 1; }
+          if (lane == 0) ptx::mbar_arrive_s(acc_empty0 + 8 * a);   // the accumulator is in registers
+          if (++a == kI4Conv) { a = 0; aph ^= 1; }
           if (mine) {
 #pragma unroll
             for (int i = 0; i < kHalf; i += 4) {
@@ -401,7 +416,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         if (!ok) break;
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_s(sf_empty0 + 8 * slot);
-        if (++slot == kI4Slots) { slot = 0; slot_ph ^= 1; }
+        if (++slot == kI4Slots) slot = 0;
       }
       if (!ok) break;
       if (mine) {
@@ -451,11 +466,15 @@ int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
       return rc;
   }
   constexpr int kFixed = 1024 + kI4Slots * S::kSlotBytes + (int)((sizeof(I4Ctrl) + 15) & ~(size_t)15);
+  // A multiple of the converter sets: then a stage is always read by the same set, which has seen the fill before
+  // the one that it waits for by parity (the issuers finish blocks out of order).  And deeper than the slots: a
+  // stage is released when the block kI4Conv further on is stored.
   constexpr int kLeast = ((int)kMaxSmem - kFixed - tile_walk_bytes(kMaxExperts)) / S::kStageBytes;
   constexpr int kDepth = converter_ring_depth(kI4Sets, kI4Conv);
-  static_assert(kLeast >= kDepth && kI4MaxStages >= kDepth && kI4Sets <= kI4Conv, "ring depth that the converters' waits need");
+  static_assert(kLeast / kI4Sets * kI4Sets >= kDepth && kI4MaxStages >= kDepth && kI4MaxStages % kI4Sets == 0,
+                "ring depth that the converters' waits need");
   const int fixed = kFixed + tile_walk_bytes(p.num_experts);
-  p.stages = ((int)kMaxSmem - fixed) / S::kStageBytes;
+  p.stages = ((int)kMaxSmem - fixed) / S::kStageBytes / kI4Sets * kI4Sets;
   if (p.stages > kI4MaxStages) p.stages = kI4MaxStages;
   const size_t smem = (size_t)fixed + (size_t)p.stages * S::kStageBytes;
   static SmemConfig configured;

@@ -557,18 +557,20 @@ __device__ __forceinline__ void tmem_cp_scales(uint32_t taddr, uint64_t desc) {
   asm volatile("tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(desc) : "memory");
 }
 // umma_mx_block's four instructions with the weights in tensor memory (eight columns per K step).
-__device__ __forceinline__ void umma_mx_block_ts(uint32_t tmem_d, uint32_t tmem_w, uint64_t adesc, uint32_t idesc,
-                                                 uint32_t accumulate, uint32_t sfw, uint32_t sfa) {
+__device__ __forceinline__ void umma_mx_block_ts(uint32_t tmem_d, uint32_t tmem_w, uint32_t adesc, uint32_t a_hi,
+                                                 uint32_t idesc, uint32_t accumulate, uint32_t sfw, uint32_t sfa) {
   asm volatile(
-      "{\n\t.reg .pred pa;\n\t.reg .b32 w1, w2, w3, i1, i2, i3;\n\t.reg .b64 a1, a2, a3;\n\tsetp.ne.b32 pa, %6, 0;\n\t"
+      "{\n\t.reg .pred pa;\n\t.reg .b32 w1, w2, w3, i1, i2, i3, y1, y2, y3;\n\t.reg .b64 a0, a1, a2, a3;\n\t"
+      "setp.ne.b32 pa, %7, 0;\n\t"
       "add.u32 w1, %1, 8;\n\tadd.u32 w2, %1, 16;\n\tadd.u32 w3, %1, 24;\n\t"
-      "add.u64 a1, %2, 2;\n\tadd.u64 a2, %2, 4;\n\tadd.u64 a3, %2, 6;\n\t"
-      "or.b32 i1, %3, 0x20000010;\n\tor.b32 i2, %3, 0x40000020;\n\tor.b32 i3, %3, 0x60000030;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [%1], %2, %3, [%4], [%5], pa;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w1], a1, i1, [%4], [%5], 1;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w2], a2, i2, [%4], [%5], 1;\n\t"
-      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w3], a3, i3, [%4], [%5], 1;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_w), "l"(adesc), "r"(idesc), "r"(sfw), "r"(sfa), "r"(accumulate)
+      "add.u32 y1, %2, 2;\n\tadd.u32 y2, %2, 4;\n\tadd.u32 y3, %2, 6;\n\t"
+      "mov.b64 a0, {%2, %3};\n\tmov.b64 a1, {y1, %3};\n\tmov.b64 a2, {y2, %3};\n\tmov.b64 a3, {y3, %3};\n\t"
+      "or.b32 i1, %4, 0x20000010;\n\tor.b32 i2, %4, 0x40000020;\n\tor.b32 i3, %4, 0x60000030;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [%1], a0, %4, [%5], [%6], pa;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w1], a1, i1, [%5], [%6], 1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w2], a2, i2, [%5], [%6], 1;\n\t"
+      "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], [w3], a3, i3, [%5], [%6], 1;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_w), "r"(adesc), "r"(a_hi), "r"(idesc), "r"(sfw), "r"(sfa), "r"(accumulate)
       : "memory");
 }
 // Waits for this thread's tcgen05.ld and makes `r` depend on it.
