@@ -104,7 +104,19 @@ topk_gating_kernel(const T* __restrict__ gating, float* __restrict__ out_w,
     }
   }
 
-  float sum_val = 0.f;
+  // With a NaN in a row the comparisons below leave the lanes with different picks; lane 0's count.
+  bool odd = false;
+#pragma unroll
+  for (int i = 0; i < VPT; ++i) odd |= v[i] != v[i];
+  odd = __any_sync(0xffffffffu, odd);
+
+  // A chain of K dependent picks is what bounds the kernel.  Lane j keeps picks j, j + R, ..: a chunk of R goes
+  // out together, with its final weights if it is the last (lane 0 alone used to store every pick and to read
+  // the weights back for the scale).  16 tokens x 128 experts, top-8: 3.9 -> 2.85 us; 8192 x 256: 18.2 -> 11.8;
+  // one token x 8, top-2: 1.8 -> 1.5.
+  float sum_val = 0.f, my_p = 0.f;
+  int my_e = 0;
+#pragma unroll 1
   for (int k = 0; k < K; ++k) {
     float best_v = v[0];
     float best_p = p[0];
@@ -115,34 +127,50 @@ topk_gating_kernel(const T* __restrict__ gating, float* __restrict__ out_w,
     }
     const int local_e = sub + best_i * R;
     int e = local_e;
+    if (R == 32 && !odd) {
+      // Largest value, then the lowest column that has it: two warp-wide reductions on integers that order
+      // as the floats do (zeros of both signs are one value).
+      const uint32_t bits = __float_as_uint(__fadd_rn(best_v, 0.f));
+      const uint32_t key = (bits & 0x80000000u) ? ~bits : bits | 0x80000000u;
+      const uint32_t top = __reduce_max_sync(0xffffffffu, key);
+      e = (int)__reduce_min_sync(0xffffffffu, key == top ? (uint32_t)e : 0xffffffffu);
+      best_p = __shfl_sync(0xffffffffu, best_p, e & 31);
+      if (kMode == 2) best_v = __shfl_sync(0xffffffffu, best_v, e & 31);
+    } else {
 #pragma unroll
-    for (int mask = R / 2; mask > 0; mask >>= 1) {
-      const float ov = __shfl_xor_sync(0xffffffffu, best_v, mask);
-      const float op = __shfl_xor_sync(0xffffffffu, best_p, mask);
-      const int oe = __shfl_xor_sync(0xffffffffu, e, mask);
-      if (ov > best_v || (ov == best_v && oe < e)) { best_v = ov; best_p = op; e = oe; }
+      for (int mask = R / 2; mask > 0; mask >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best_v, mask);
+        const float op = __shfl_xor_sync(0xffffffffu, best_p, mask);
+        const int oe = __shfl_xor_sync(0xffffffffu, e, mask);
+        if (ov > best_v || (ov == best_v && oe < e)) { best_v = ov; best_p = op; e = oe; }
+      }
     }
     if (kMode == 2 && bias != nullptr) best_p = __fsub_rn(best_v, bias[e]);
-    sum_val = __fadd_rn(sum_val, best_p);
-    if (live && sub == 0) {
-      const int64_t pos = row * K + k;
-      store_index(out_idx, idx_dtype, pos, e);
-      out_src[pos] = (int32_t)((int64_t)k * num_rows + row);
-      out_w[pos] = best_p;  // rescaled below
-    }
     if (e == local_e) {
 #pragma unroll
       for (int i = 0; i < VPT; ++i)
         if (i == best_i) v[i] = -10000.f;
     }
+    if (odd) {
+      e = __shfl_sync(0xffffffffu, e, 0, R);
+      best_p = __shfl_sync(0xffffffffu, best_p, 0, R);
+    }
+    sum_val = __fadd_rn(sum_val, best_p);
+    if (sub == k % R) { my_e = e; my_p = best_p; }
+    if (live && (k % R == R - 1 || k == K - 1) && sub <= k % R) {
+      const int mine = k / R * R + sub;
+      const int64_t pos = row * K + mine;
+      store_index(out_idx, idx_dtype, pos, my_e);
+      out_src[pos] = (int32_t)((int64_t)mine * num_rows + row);
+      out_w[pos] = my_p;   // of all chunks but the last: rescaled below
+    }
   }
-  if (live && sub == 0) {
+  if (live) {
     float scale = rsf;
     if (renorm) scale = __fdiv_rn(scale, sum_val > 0.f ? sum_val : 1.f);
-    for (int k = 0; k < K; ++k) {
-      const int64_t pos = row * K + k;
-      out_w[pos] = __fmul_rn(out_w[pos], scale);
-    }
+    const int last = (K - 1) / R * R;
+    for (int k = sub; k < last; k += R) out_w[row * K + k] = __fmul_rn(out_w[row * K + k], scale);
+    if (last + sub < K) out_w[row * K + last + sub] = __fmul_rn(my_p, scale);
   }
 }
 
