@@ -49,9 +49,12 @@ int fail(int code, const char* fmt, ...);
 // stream still runs, so that its set-up (and the launch itself) is off the critical path; the wait
 // ends when every earlier kernel of the stream has completed (each of them waited for its own
 // predecessor) and its writes are visible.  A decode step is a chain of few-microsecond kernels and
-// gains 0.5 to 1 us per launch.  Kernels of many waves lose: measured on 65536 routed rows, the
-// layer is 5 % slower with it (blocks that wait take the place of blocks that work).
-constexpr int64_t kEarlyLaunchRows = 2048;   // routed rows up to which a layer's kernels launch early
+// gains 0.5 to 1 us per launch, a chain of nine at a few thousand rows as much.  Kernels of many waves lose
+// (blocks that wait take the place of blocks that work).  Layer calls without / with, us: qwen3 fp8 4096 routed
+// rows 176 / 166, 8192 rows 192 / 181, 32768 rows 353 / 351; one of 8 DeepSeek ranks at 4096 rows 303 / 295, 8192
+// rows 278 / 274; gpt-oss MXFP4 16384 rows 1520 / 1613; DeepSeek 8192 rows no difference, 32768 rows 3279 / 3410,
+// 65536 rows 5 % slower.  The line lies where none of them loses.
+constexpr int64_t kEarlyLaunchRows = 8192;   // routed rows up to which a layer's kernels launch early
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(bool early, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem,
                               cudaStream_t st, Args&&... args) {
