@@ -389,6 +389,11 @@ typedef struct {
                              pre-activation values (and the bias) have: they are
                              rounded to it before the activation, as the unfused
                              GEMM's output would be                                */
+  int rows_ready;         /* 1: rows_per_expert was complete before the kernel ahead
+                             of this call in the stream could let it start (a layer's
+                             second GEMM: the first has waited for it).  The kernel
+                             then brings weights of its first tiles to L2 while it
+                             waits.  Never changes the result.                     */
   int64_t rows_hint;      /* 0, or the number of rows expected to be in use when `m`
                              is only a loose upper bound (buffers sized for the worst
                              case): tile sizes are picked for rows_hint / num_experts

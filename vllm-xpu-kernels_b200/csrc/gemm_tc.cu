@@ -49,6 +49,7 @@ struct TcParams {
   int64_t m;
   int n, k, num_experts;
   int w_experts;  // >0: segment s uses weight set s % w_experts
+  int rows_ready; // 1: prefetch_first_tiles
   int n_tiles;  // ceil(n / 128)
   int num_kb;   // K blocks of 128 bytes
   uint32_t idesc;
@@ -125,6 +126,15 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
+    if (!kGated && p.rows_ready) {
+      prefetch_first_tiles<BT>(p.rows_per_expert, p.num_experts, p.w_experts, p.n_tiles, p.num_kb, kPreBytes / kWTileBytes,
+                               ctrl->walk, [&](const TileInfo& ti, int kb) {
+        const int k0 = kb * kElemsPerKb, n0 = ti.n_tile * kFeat;
+        if (!kWKn) ptx::tma_prefetch_3d(&tmap_w, k0, n0, ti.e);
+        else ptx::tma_prefetch_3d(&tmap_w, n0, k0, ti.e);
+        if (kWKn && !kFp8) ptx::tma_prefetch_3d(&tmap_w, n0 + 64, k0, ti.e);
+      });
+    }
     pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, ctrl->walk);
     if (lane == 0) {
@@ -799,6 +809,7 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   p.a_scale = reinterpret_cast<const float*>(a->a_scale); p.w_scale = reinterpret_cast<const float*>(a->w_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
+  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
   const int w_sets = (a->w_experts > 0 && a->w_experts != a->num_experts) ? a->w_experts : a->num_experts;
   p.w_experts = w_sets != a->num_experts ? w_sets : 0;
   p.n_tiles = ((gated ? a->n / 2 : a->n) + kFeat - 1) / kFeat;

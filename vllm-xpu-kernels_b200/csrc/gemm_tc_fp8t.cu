@@ -58,6 +58,7 @@ struct TParams {
   // token and 128 features in d_scale [M, n/256]
   float* d_scale;
   float clamp;            // >0: gate = min(gate, clamp), up = clamp(up, -clamp, clamp)
+  int rows_ready;         // 128 x 256 kernel, 1: prefetch_first_tiles
   int stages;             // 128 x 256 kernel: pipeline stages
   int d_aligned32;        // 128 x 256 kernel: rows of D begin on 32-byte boundaries
 };
@@ -390,6 +391,19 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
   const int up_block0 = p.n_tiles / 2;        // gated: first 128-feature block of the up half
 
   if (warp == 0) {
+    if (!kGated && p.rows_ready) {
+      prefetch_first_tiles<kTTok>(p.rows_per_expert, p.num_experts, p.w_experts, n_tiles2, p.num_kb, kPreBytes / 32768,
+                                  walk_mem, [&](const TileInfo& ti, int kb) {
+        const int n0 = ti.n_tile * 256;
+        if (!kWKn) {
+          ptx::tma_prefetch_3d(&tmap_w, kb * 128, n0, ti.e);
+          ptx::tma_prefetch_3d(&tmap_w, kb * 128, n0 + 128, ti.e);
+        } else {
+          ptx::tma_prefetch_3d(&tmap_w, n0, kb * 128, ti.e);
+          ptx::tma_prefetch_3d(&tmap_w, n0 + 128, kb * 128, ti.e);
+        }
+      });
+    }
     pdl_wait();
     build_tile_walk<kTTok>(p.rows_per_expert, p.num_experts, n_tiles2, walk_mem);
     if (lane == 0) {
@@ -774,6 +788,7 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   p.w_scale = reinterpret_cast<const float*>(a->w_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
+  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
   const int w_sets = (a->w_experts > 0 && a->w_experts != a->num_experts) ? a->w_experts : a->num_experts;
   p.w_experts = w_sets != a->num_experts ? w_sets : 0;
   p.n_tiles = a->n / kFeat;

@@ -70,6 +70,7 @@ struct I4Params {
   int n_tiles, num_kb;
   int groups, kb_shift;      // scales per weight row; scale index = K block >> kb_shift
   int stages;
+  int rows_ready;            // 1: prefetch_first_tiles
   uint32_t idesc;
   int out_f16;
 };
@@ -117,6 +118,9 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
+    if (p.rows_ready)
+      prefetch_first_tiles<BT>(p.rows_per_expert, p.num_experts, 0, p.n_tiles, p.num_kb, kPreBytes / kI4RawBytes, walk_mem,
+                               [&](const TileInfo& ti, int kb) { ptx::tma_prefetch_3d(&tmap_w, kb * 64, ti.n_tile * kFeat, ti.e); });
     pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, walk_mem);
     if (lane == 0) {
@@ -505,6 +509,7 @@ int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
   p.w_scale = reinterpret_cast<const uint16_t*>(a->w_scale);
   p.a_scale = reinterpret_cast<const uint32_t*>(a->a_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
+  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
   p.n_tiles = (a->n + kFeat - 1) / kFeat;
   p.num_kb = a->k / 128;

@@ -87,6 +87,7 @@ struct MxParams {
   int terms;       // activation planes (1 or 2)
   int tail;        // 1: the last K block is partial, its weights are brought by the epilogue warps
   int stages;
+  int rows_ready;  // 1: prefetch_first_tiles
   int sfw_bytes;   // bytes of one staged weight-scale buffer
   uint32_t tmem_cols;
   uint32_t idesc;
@@ -200,6 +201,10 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
+    if (!kW8 && p.rows_ready)
+      prefetch_first_tiles<BT>(p.rows_per_expert, p.num_experts, 0, p.n_tiles, p.tail ? p.num_kb - 1 : p.num_kb,
+                               kPreBytes / kMxWTx, after,
+                               [&](const TileInfo& ti, int kb) { ptx::tma_prefetch_3d(&tmap_w, kb * 128, ti.n_tile * kFeat, ti.e); });
     pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, after);
     if (lane == 0) {
@@ -715,6 +720,7 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   p.w_tensor_scale = reinterpret_cast<const float*>(a->w_scale);
   p.a_scale = reinterpret_cast<const uint32_t*>(a->a_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
+  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
   p.n_tiles = (a->n + kFeat - 1) / kFeat;
   p.num_kb = (a->k + 127) / 128;

@@ -245,6 +245,7 @@ struct Experts {
     g.clamp_limit = epi != B200MOE_EPI_NONE && p.clamp > 0 ? (float)p.clamp : 0.f;
     g.status = device_status_word(device);
     g.max_ctas = o.max_ctas; g.rows_hint = o.rows_hint;
+    g.rows_ready = !first;   // gemm1 has waited for them
     check_status(b200moe_grouped_gemm(&g, stream));
   }
 
