@@ -824,13 +824,13 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   // even, so leave headroom before a second token tile re-reads the weights).
   int bt;
   if (a_fp8) {
-    // fp8 pays a hand-over per 128-wide K block, so wide tiles win early.  Measured at 16 / 64 / 128
-    // tokens, 128 experts: N 4096, K 7168: 4 rows per expert 605 / 661 / 628 us, 8 rows 767 / 849 / 685,
-    // 16 rows 914 / 761 / 638; N 2048, K 768: 4 rows 59 / 64 / 50 us, 8 rows 61 / 66 / 51, 16 rows
-    // 76 / 66 / 52.  The line at 4 rows is where K decides between 16 and 128 tokens; the 64-token tile
-    // was the better one up to 12 rows before the 128-token kernel's promotion loop was shortened and is
-    // 5 to 30 % behind it now.
-    bt = avg <= 4 ? 16 : (avg < 12 ? 64 : 128);
+    // fp8 pays a hand-over per 128-wide K block, so wide tiles win early.  Layer calls with tiles of 16 / 64 /
+    // 128 tokens, us: 128 experts, N 1536, K 2048: 4 rows per expert 140 / 155 / 140, 6 rows 142 / 160 / 142,
+    // 8 rows 143 / 161 / 142, 12 rows 153 / 164 / 146; 256 experts, N 4096, K 7168: 4 rows 1176 / 1248 / 1311,
+    // 5 rows 1255 / 1301 / 1338, 6 rows 1224 / 1195 / 1206, 8 rows 1361 / 1298 / 1308, 12 rows 1697 / 1437 /
+    // 1370; 32 of those experts: 6 rows 205 / 206 / 215, 8 rows 232 / 233 / 225, 12 rows 327 / 253 / 243.
+    // Nowhere is 64 the best by more than 1 %, so there is no such tile.
+    bt = avg <= 6 ? 16 : 128;
   } else {
     // Measured at 16 / 64 / 128 / 256 tokens (a CTA pair), 8 experts, N 28672, K 4096: 8 rows per expert
     // 289 / 285 / 295 / 340 us, 32 rows 336 / 291 / 301 / 342, 64 rows 539 / 320 / 307 / 344, 96 rows
@@ -910,12 +910,9 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   if (tile_bound < grid) grid = (int)tile_bound;
   if (grid < 1) grid = 1;
 
+  if (a_fp8) return kn ? launch_tc<16, true, true>(ta, tw, p, grid, st) : launch_tc<16, true, false>(ta, tw, p, grid, st);
 #define B200_TC_CASE(BT_)                                                         \
   if (bt == BT_) {                                                                \
-    if (a_fp8) {                                                                  \
-      if (kn) return launch_tc<(BT_ > 64 ? 64 : BT_), true, true>(ta, tw, p, grid, st);  \
-      return launch_tc<(BT_ > 64 ? 64 : BT_), true, false>(ta, tw, p, grid, st);         \
-    }                                                                             \
     if (kn) return launch_tc<BT_, false, true>(ta, tw, p, grid, st);              \
     return launch_tc<BT_, false, false>(ta, tw, p, grid, st);                     \
   }

@@ -283,13 +283,12 @@ class XpuFusedMoe:
         self._use_ref = False
         # block-scaled fp8 with SiLU: the token-major tensor-core kernel can apply the activation and the
         # 1x128 e4m3 quantisation of gemm2's input in its epilogue (same values as the two-kernel form).
-        # The epilogue runs on the warps that also promote the K blocks' partial sums, the kernel's
-        # bottleneck, so short K loops lose by it and long ones break even; from FP8_FUSED_MIN_ROWS
-        # routed rows per expert on the two forms are within 2 % of each other on both shapes, and the
-        # fused one saves the [rows, 2I] intermediate.  Fused against two kernels, the two in turn: gemm1 of
-        # N 4096, K 7168 (65536 rows) 3.65 against 3.86 ms at 256 rows per expert, 3.07 / 3.10 at 512, 2.75
-        # / 2.77 at 1024, 2.65 / 2.65 at 2048; N 1536, K 2048 253 against 229 us at 256, 422 / 416 at 512,
-        # 393 / 387 at 1024, 377 / 376 at 2048.  fuse_activation=True / False force it.
+        # The epilogue runs on the warps that also promote the K blocks' partial sums, so short K loops lose by
+        # it and long ones break even, and it saves the [rows, 2I] intermediate, which counts at long segments:
+        # taken from FP8_FUSED_MIN_ROWS routed rows per expert on.  The layer call, fused / two kernels, us:
+        # 32 experts, hidden 7168, I 2048: 755 / 748 at 256 rows per expert, 942 / 950 at 512, 1910 / 1890 at
+        # 1024; 128 experts, hidden 2048, I 768: 380 / 355 at 256, 619 / 593 at 512, 1140 / 1090 at 1024,
+        # 2250 / 2130 at 2048.  fuse_activation=True / False force it.
         self._fp8_fused_ok = (is_block_fp8 and self._act_kind == "silu" and self.inter_size % FP8_BLOCK_SIZE == 0
                               and fuse_activation is not False)
         self._fp8_fused_min_rows = 12 if fuse_activation else FP8_FUSED_MIN_ROWS
