@@ -20,7 +20,7 @@
 // MMAs of the next).  fp8 inputs use kind::f8f6f4 per 128-wide K block; the
 // epilogue warps promote each block's partial sum into fp32 registers with
 // a_scale[row, kb] * w_scale[e, n/128, kb], as the block-scaled recipe needs.
-// (fp8 segments of 12 rows per expert or more go to the token-major kernels of
+// (fp8 segments of 7 rows per expert or more go to the token-major kernels of
 // gemm_tc_fp8t.cu, where that scale is one register per thread.)
 //
 // Every wait on an mbarrier is bounded (see sm100_ptx.cuh): on expiry the CTA

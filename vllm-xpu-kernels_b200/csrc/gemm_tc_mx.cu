@@ -65,7 +65,8 @@ constexpr int kMxMaxStages = 8;
 // fetches 256, so every fourth block comes from DRAM, and the ring is too short for that latency (stamps: 1500 to
 // 1900 cycles for that block, 750 for the others).  128 experts, N 5760, K 2880, gated, with / without: 4 rows per
 // expert 204 / 217 us, 16 rows 262 / 283, 64 rows 385 / 393; 4, 8 and 10 blocks ahead, or on into the next tile, are
-// slower.
+// slower.  Not for token tiles of 16: their calls run into the power cap when they follow one another, and the
+// asking costs energy: layer calls of 128 tokens, in short runs 342 / 349 us, in a loop of seconds 391 / 384.
 constexpr int kMxAhead = 6;
 constexpr int kMxGroup = 4;         // K blocks per scale group (one hand-over from the scale preparers)
 constexpr int kMxSlots = 4;         // scale groups in the ring, at most
@@ -87,7 +88,6 @@ struct MxParams {
   int terms;       // activation planes (1 or 2)
   int tail;        // 1: the last K block is partial, its weights are brought by the epilogue warps
   int stages;
-  int rows_ready;  // 1: prefetch_first_tiles
   int sfw_bytes;   // bytes of one staged weight-scale buffer
   uint32_t tmem_cols;
   uint32_t idesc;
@@ -201,10 +201,6 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (warp == 0) {
-    if (!kW8 && p.rows_ready)
-      prefetch_first_tiles<BT>(p.rows_per_expert, p.num_experts, 0, p.n_tiles, p.tail ? p.num_kb - 1 : p.num_kb,
-                               kPreBytes / kMxWTx, after,
-                               [&](const TileInfo& ti, int kb) { ptx::tma_prefetch_3d(&tmap_w, kb * 128, ti.n_tile * kFeat, ti.e); });
     pdl_wait();
     build_tile_walk<BT>(p.rows_per_expert, p.num_experts, p.n_tiles, after);
     if (lane == 0) {
@@ -271,7 +267,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
               else ptx::tma_load_3d_s(st + sub * kMxWBytes, &tmap_w, full, (kb0 + sub) * 128, n0, ti.e);
             }
           }
-          if (!kW8 && kb0 + kMxAhead < whole_kb) ptx::tma_prefetch_3d(&tmap_w, (kb0 + kMxAhead) * 128, n0, ti.e);
+          if (!kW8 && BT > 16 && kb0 + kMxAhead < whole_kb) ptx::tma_prefetch_3d(&tmap_w, (kb0 + kMxAhead) * 128, n0, ti.e);
           st += kStageBytes;
           if (++s == (uint32_t)stages) { s = 0; ph ^= 1; st = st0; }
         }
@@ -720,7 +716,6 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   p.w_tensor_scale = reinterpret_cast<const float*>(a->w_scale);
   p.a_scale = reinterpret_cast<const uint32_t*>(a->a_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
-  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
   p.n_tiles = (a->n + kFeat - 1) / kFeat;
   p.num_kb = (a->k + 127) / 128;

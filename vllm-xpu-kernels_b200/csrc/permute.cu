@@ -4,8 +4,8 @@
 // Both ops are a stable counting sort of the T*K routed slots by (mapped)
 // expert id.  The slots are cut into chunks of 256 handled by one warp each:
 //   1. count : every warp builds a histogram of its chunk,
-//   2. scan  : per expert an exclusive scan over the chunks, then a scan over
-//              the experts (padded to block_size for the align op),
+//   2. scan  : per expert an exclusive scan over the chunks (a warp each); every block of the next step
+//              then scans the experts itself (padded to block_size for the align op),
 //   3. rank  : every warp walks its chunk 32 slots at a time; the rank of a
 //              slot among equal ids in the same step comes from
 //              __match_any_sync, so slots of one expert keep ascending order.
