@@ -34,9 +34,10 @@ struct Plan {
   // Up to this many rows per expert the block-scaled int4 kernel (gemm_tc_i4.cu) takes the layer: it
   // streams the weights faster than the one that expands them to 16 bits (gemm_tc_dq.cu), until experts
   // need a second of its tiles of 32 tokens.  A layer of 8 experts of 4096 x 14336, 2 a token, bfloat16
-  // (float16, three planes): 106 (117) against 125 us at 1 token, 256 (285) against 305 at 8 rows an
-  // expert, 264 (287) against 307 at 12, 266 (295) against 311 at 16, 279 (306) against 315 at 20, 297
-  // (393) against 317 at 24, 373 (465) against 320 at 32.  Half a tile leaves room for uneven routing.
+  // (float16, three planes) with routing as it comes: 93 (101) against 121 us at 1 token, 215 (240) against 297 at
+  // 8 rows an expert, 230 (294) against 276 at 12, 250 (320) against 280 at 16, 318 (399) against 284 at 20, 321
+  // (404) against 285 at 24.  Half a tile leaves room for uneven routing; float16 keeps the same line, because
+  // its planes also lose less than a weight rounded after its scale.
   static constexpr int64_t kI4PlaneRows = 16;
 };
 const char* const kPlanName = "b200moe.layer_plan";
