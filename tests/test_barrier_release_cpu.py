@@ -38,3 +38,20 @@ def test_tensor_memory_waits_name_the_registers_they_wait_for(path):
     waits = [code for _, code in _statements(path) if re.search(r"tmem_wait_ld\w*\(", code)]
     assert loads and waits
     assert not [w for w in waits if "tmem_wait_ld()" in w and "break;" not in w]
+
+
+@pytest.mark.parametrize("name,kernel,seen", [("gemm_tc_fp8t.cu", "grouped_gemm_fp8t256_kernel", "sf_full0"),
+                                              ("gemm_tc_i4.cu", "grouped_gemm_i4_kernel", "sf_full0")])
+def test_promotion_warps_acquire_what_they_read_from_shared_memory(name, kernel, seen):
+    """Scales and sums are written with ordinary stores by warps that only the issuer waits for.  A
+    tcgen05.commit orders the tensor core's work, not those stores: the issuer has to arrive on the
+    accumulator's barrier itself, after its own wait for them and before (or beside) the commit."""
+    text = (PKG_DIR / "csrc" / name).read_text()
+    code = "\n".join(c for c in (line.split("//")[0].rstrip() for line in text[text.index(kernel):].splitlines()) if c.strip())
+    assert re.search(r"mbar_init\(&ctrl->acc_full\[a\], 2\);", code)
+    issuer = code[code.index("umma_commit(acc_full0"):]           # behind: the promotion warps take the accumulator alone
+    assert seen not in issuer[issuer.index("setmaxnreg_inc"):]
+    before = code[:code.index("umma_commit(acc_full0")]
+    wait = before.rindex("mbar_wait_s(" + seen)
+    free = before.rindex("mbar_wait_s(acc_empty0")                # (not before the phase before is over)
+    assert before.rfind("mbar_arrive_s(acc_full0") > max(wait, free)

@@ -419,7 +419,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       ptx::mbar_init(&ctrl->empty[s], 1);
     }
     for (int a = 0; a < kT2Acc; ++a) {
-      ptx::mbar_init(&ctrl->acc_full[a], 1);
+      ptx::mbar_init(&ctrl->acc_full[a], 2);   // the MMAs, and the issuer for the scales it has seen
       ptx::mbar_init(&ctrl->acc_empty[a], 8);
     }
     for (int g = 0; g < kT2Slots; ++g) {
@@ -486,10 +486,13 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ CUtensorMap tmap_a,
       uint64_t wdesc = wdesc0, adesc = adesc0;
       const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((256u >> 3) << 17);
       for (uint32_t i = 0; i < blocks; ++i) {
-        // (the block's scales: so that acc_full stands for them too)
+        // (the block's scales: acc_full stands for them too)
         if (i % kTGroup == 0 && !ptx::mbar_wait_s(sf_full0 + 8 * ((i >> 2) & 1), (i >> 3) & 1, abort_flag)) break;
         if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) break;
         if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) break;
+        // tcgen05.commit completes the MMAs and orders nothing else: scales and tile, written by the preparers,
+        // reach the promotion warps through this arrival (acquired above, released here)
+        ptx::mbar_arrive_s(acc_full0 + 8 * a);
         ptx::tc_fence_after();
         ptx::umma_block<true, 2, kWKn ? 4096 / 16 : 2>(tmem_base + a * 256, adesc, wdesc, idesc, 0u);
         ptx::umma_commit(acc_full0 + 8 * a);

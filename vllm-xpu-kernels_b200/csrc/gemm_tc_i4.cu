@@ -139,7 +139,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       ptx::mbar_init(&ctrl->conv_full[c], 4);
     }
     for (int a = 0; a < kI4Conv; ++a) {
-      ptx::mbar_init(&ctrl->acc_full[a], 1);
+      ptx::mbar_init(&ctrl->acc_full[a], 2);   // the MMAs, and the issuer for the sums it has seen
       ptx::mbar_init(&ctrl->acc_empty[a], 8);
     }
     for (int g = 0; g < kI4Slots; ++g) {
@@ -225,6 +225,9 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
               if ((u < kI4Issuers && !ptx::mbar_wait_s(sf_full0 + 8 * slot, slot_ph, abort_flag)) ||
                   !ptx::mbar_wait_s(conv_full0 + 8 * c, cph, abort_flag) ||
                   !ptx::mbar_wait_s(acc_empty0 + 8 * c, cph ^ 1, abort_flag)) { ok = false; break; }
+              // tcgen05.commit completes the MMAs and orders nothing else: the group's sums, written by warp 3, reach
+              // the promotion warps through this arrival (acquired above, released here)
+              ptx::mbar_arrive_s(acc_full0 + 8 * c);
               ptx::tc_fence_after();
               const uint32_t sfa = sf + 8 + c * S::kSfPer, adesc = adesc0 + s * (kStageBytes >> 4);
               const uint64_t sfd = sfdesc0 + slot * (kSlotBytes >> 4) + u * (S::kTokChunks * 32);
