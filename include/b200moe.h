@@ -338,7 +338,9 @@ typedef enum {
  * csrc/xpu/torch_bindings.cpp:46-53).
  * For each expert e with rows_e = rows_per_expert[e] > 0 and r0 = sum of the
  * earlier experts' rows:  D[r0:r0+rows_e, :] = A[r0:r0+rows_e, :] * W_e^T
- * (+ bias_e), fp32 accumulation, result cast to d_dtype. */
+ * (+ bias_e), fp32 accumulation, result cast to d_dtype.
+ * Begin with an all-zero struct and set what the call needs: members are added
+ * over time, also where there was padding (rows_ready), and zero means "as before". */
 typedef struct {
   const void* a;          /* [M,K] a_dtype, row-major, 16-byte aligned            */
   b200moe_dtype a_dtype;  /* BF16, F16, or FP8_E4M3 (with a_scale)                */
@@ -389,11 +391,11 @@ typedef struct {
                              pre-activation values (and the bias) have: they are
                              rounded to it before the activation, as the unfused
                              GEMM's output would be                                */
-  int rows_ready;         /* 1: rows_per_expert was complete before the kernel ahead
-                             of this call in the stream could let it start (a layer's
-                             second GEMM: the first has waited for it).  The kernel
-                             then brings weights of its first tiles to L2 while it
-                             waits.  Never changes the result.                     */
+  int rows_ready;         /* 1 (any other value is 0): rows_per_expert was complete
+                             before the kernel ahead of this call in the stream could
+                             let it start (a layer's second GEMM: the first has waited
+                             for it).  The kernel then brings weights of its first
+                             tiles to L2 while it waits.  Never changes the result.  */
   int64_t rows_hint;      /* 0, or the number of rows expected to be in use when `m`
                              is only a loose upper bound (buffers sized for the worst
                              case): tile sizes are picked for rows_hint / num_experts

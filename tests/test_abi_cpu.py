@@ -2,11 +2,14 @@
 declares; argument validation that needs no device; the torch op schemas."""
 import ctypes
 import re
+import shutil
+import subprocess
 
 import pytest
 import torch
 
 from conftest import PKG_DIR, ROOT
+from gemm_args import GemmArgs
 
 
 def _declared_symbols():
@@ -142,3 +145,26 @@ def test_expert_parallel_owner_map_and_workspace_size(lib):
     assert lib.b200moe_ep_dispatch(None, None, 2, None, 5, None, ctypes.c_int64(0), None, None, None,
                                    ctypes.c_size_t(0), None) == -1
     assert b"null peer table" in lib.b200moe_last_error()
+
+
+def test_gemm_args_layout(tmp_path):
+    if shutil.which("gcc") is None:
+        pytest.skip("gcc not found")
+    names = [f[0] for f in GemmArgs._fields_]
+    (tmp_path / "o.c").write_text(
+        '#include <stddef.h>\n#include <stdio.h>\n#include "b200moe.h"\nint main(void) {\n' +
+        "".join(f'printf("%zu ", offsetof(b200moe_gemm_args, {n}));\n' for n in names) +
+        'printf("%zu", sizeof(b200moe_gemm_args)); return 0; }\n')
+    subprocess.run(["gcc", "-I", str(ROOT / "include"), "-o", str(tmp_path / "o"), str(tmp_path / "o.c")], check=True)
+    got = [int(x) for x in subprocess.run([str(tmp_path / "o")], capture_output=True, text=True, check=True).stdout.split()]
+    assert got == [getattr(GemmArgs, n).offset for n in names] + [ctypes.sizeof(GemmArgs)]
+
+
+def test_a_member_in_what_was_padding_counts_only_when_it_is_1():
+    """rows_ready took the place of padding: a caller built against the header before it may hand over anything
+    there.  Only 1 may make a kernel read the counts ahead of its wait, and from any counts that walk has to end."""
+    uses = [line for f in sorted((PKG_DIR / "csrc").glob("gemm*.cu")) for line in f.read_text().splitlines() if "a->rows_ready" in line]
+    assert len(uses) == 3 and all("a->rows_ready == 1" in u for u in uses)
+    text = (PKG_DIR / "csrc" / "gemm_tc_common.cuh").read_text()
+    walk = text[text.index("void prefetch_first_tiles"):]
+    assert "if ((uint32_t)ti.n_tile >= (uint32_t)n_tiles) break;" in walk[:walk.index("host side")]

@@ -213,7 +213,8 @@ __device__ __forceinline__ void build_tile_walk(const int32_t* rows_per_expert, 
 // Weights of the CTA's first tiles to L2, in the time in which an early launched kernel only waits for the one
 // before it (6 to 10 us for the second GEMM of a decode layer: the end of the first GEMM and the activation).
 // One full warp, before pdl_wait(): `rows_per_expert` must be complete already (gemm_args.rows_ready), but
-// nothing here depends on it: the walk is built again after the wait.  `load(tile, kb)` asks for a K block.
+// nothing depends on it: from any counts the walk ends and asks for blocks of the weights only, and it is built
+// again after the wait.  `load(tile, kb)` asks for a K block.
 // Second GEMM of qwen3 fp8 at 16 tokens 33.6 -> 31.2 us, of the small 16-bit layer at 64 tokens 11.1 -> 10.4; the
 // layer calls with 128 / 256 / 512 KB a CTA: 96.9 / 96.2 / 97.1 (98.2 without) and 39.1 / 39.6 / 39.9 (39.9); one
 // Mixtral token 118.9 / 119.3 / 120.3 (119.3).
@@ -229,7 +230,8 @@ __device__ __forceinline__ void prefetch_first_tiles(const int32_t* rows_per_exp
     for (int t = blockIdx.x; t < walk.total && blocks > 0; t += gridDim.x) {
       TileInfo ti;
       locate_tile<BT>(walk, t, cursor, ti, w_experts);
-      for (int kb = 0; kb < num_kb && blocks > 0 && ti.n_tile < n_tiles; ++kb, --blocks) load(ti, kb);
+      if ((uint32_t)ti.n_tile >= (uint32_t)n_tiles) break;   // the counts were not complete: no such tile, so no more
+      for (int kb = 0; kb < num_kb && blocks > 0; ++kb, --blocks) load(ti, kb);
     }
   }
   __syncwarp();

@@ -791,7 +791,7 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   p.w_scale = reinterpret_cast<const float*>(a->w_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
-  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
+  p.rows_ready = a->rows_ready == 1 && a->m <= kEarlyLaunchRows;
   const int w_sets = (a->w_experts > 0 && a->w_experts != a->num_experts) ? a->w_experts : a->num_experts;
   p.w_experts = w_sets != a->num_experts ? w_sets : 0;
   p.n_tiles = a->n / kFeat;

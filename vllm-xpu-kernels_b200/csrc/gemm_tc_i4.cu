@@ -512,7 +512,7 @@ int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
   p.w_scale = reinterpret_cast<const uint16_t*>(a->w_scale);
   p.a_scale = reinterpret_cast<const uint32_t*>(a->a_scale);
   p.bias = a->bias; p.d = a->d; p.rows_per_expert = a->rows_per_expert; p.status = a->status;
-  p.rows_ready = a->rows_ready != 0 && a->m <= kEarlyLaunchRows;
+  p.rows_ready = a->rows_ready == 1 && a->m <= kEarlyLaunchRows;
   p.m = a->m; p.n = a->n; p.k = a->k; p.num_experts = a->num_experts;
   p.n_tiles = (a->n + kFeat - 1) / kFeat;
   p.num_kb = a->k / 128;
