@@ -36,6 +36,22 @@ def test_moe_align_exact(native, m, topk, E, bs, pad):
     assert int((s.cpu() < ids.numel()).sum()) == ids.numel()
 
 
+@pytest.mark.parametrize("bs", [1, 16, 128])
+@pytest.mark.parametrize("numel", [2048, 2050, 70000])
+@pytest.mark.parametrize("E,live", [(1, [0]), (2, [1]), (8, range(8)), (8, [0]), (8, [3, 6]), (256, [0, 1, 255]), (256, [100]),
+                                    (300, range(0, 300, 2))])
+def test_moe_align_block_table(native, E, live, numel, bs):
+    """Few large experts, empty ones at the ends and in between, in one block and in many, and room past the last block."""
+    g = torch.Generator().manual_seed(numel + E)
+    live = torch.tensor(list(live), dtype=torch.int32)
+    ids = live[torch.randint(0, len(live), (numel // 2, 2), generator=g)]
+    n, nb = align_sizes(numel, E, bs, False)
+    s, e, p = (torch.full((k,), -7, dtype=torch.int32, device=DEV) for k in (n, nb + 5, 1))
+    torch.ops._moe_C.moe_align_block_size(ids.to(DEV), E, bs, s, e, p, None)
+    os_, oe, op = co.moe_align_block_size(ids, E, bs, n, nb + 5)
+    assert torch.equal(p.cpu(), op) and torch.equal(e.cpu(), oe) and torch.equal(s.cpu(), os_)
+
+
 def test_moe_align_reference_vectors_map_determinism_dtypes(native):
     for c in load_golden("moe_align.pt"):
         emap = c["expert_map"].to(DEV) if c["expert_map"] is not None else None

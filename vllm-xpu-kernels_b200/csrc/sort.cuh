@@ -159,6 +159,26 @@ struct RemapOut {
   int32_t* row_map;
 };
 
+// The align op's block table: entry i is the bucket whose padded rows hold row i * block_size (0 past the last).  An
+// entry a thread, its bucket by bisection of `base` (exclusive sums of the padded sizes, base[nb] their total), so
+// that few large buckets are written as fast as many small ones.  moe_align_block_size of 65536 slots, a thread per
+// four buckets in one block / so: 8 experts, blocks of 16, 172 / 12.0 us; 2 experts 332 / 11.9; 256 experts 22.9 /
+// 17.3; 2048 slots, 8 experts 13.3 / 7.6.
+__device__ __forceinline__ void write_block_table(const int* base, int nb, int block_size, const AlignOut& ao, int64_t first,
+                                                  int64_t step) {
+  const int blocks = base[nb] / block_size;
+  for (int64_t blk = first; blk < ao.expert_ids_len; blk += step) {
+    int lo = 0, hi = blk < blocks ? nb - 1 : 0;
+    const int row = (int)blk * block_size;
+    while (lo < hi) {   // the last bucket that begins at or before the row (empty ones before it begin there, too)
+      const int mid = (lo + hi + 1) >> 1;
+      if (base[mid] <= row) lo = mid;
+      else hi = mid - 1;
+    }
+    ao.expert_ids[blk] = lo;
+  }
+}
+
 template <int kMode>
 __global__ void __launch_bounds__(kBlockThreads)
 sort_single_block_kernel(SortParams p, AlignOut ao, RemapOut ro) {
@@ -199,25 +219,10 @@ sort_single_block_kernel(SortParams p, AlignOut ao, RemapOut ro) {
     base[e] = (kMode == 0) ? ((run + p.block_size - 1) / p.block_size) * p.block_size : run;
   }
   __syncthreads();
-  int padded[4];  // align: remember the padded sizes for expert_ids
-#pragma unroll
-  for (int j = 0; j < 4; ++j) padded[j] = (4 * t + j < nb) ? base[4 * t + j] : 0;
   block_exclusive_scan(base, nb, warp_tot);
   if (kMode == 0) {
-    const int total = base[nb];
-    if (t == 0) ao.post_pad[0] = total;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int e = 4 * t + j;
-      if (e < nb) {
-        for (int o = 0; o < padded[j]; o += p.block_size) {
-          const int64_t blk = (base[e] + o) / p.block_size;
-          if (blk < ao.expert_ids_len) ao.expert_ids[blk] = e;
-        }
-      }
-    }
-    for (int64_t blk = total / p.block_size + t; blk < ao.expert_ids_len; blk += kBlockThreads)
-      ao.expert_ids[blk] = 0;
+    if (t == 0) ao.post_pad[0] = base[nb];
+    write_block_table(base, nb, p.block_size, ao, t, kBlockThreads);
   }
   // hist[w][e] += base[e]  -> absolute next-free position per warp and bucket
   for (int i = t; i < kWarps * nb; i += kBlockThreads)
@@ -406,7 +411,7 @@ sort_scan_kernel(SortParams p, int n_chunks, int* counts, int* sizes, RemapOut r
   }
 }
 
-// Every block scans the buckets' sizes for itself; the first one of the align op writes its block table.
+// Every block scans the buckets' sizes for itself; together they write the align op's block table.
 template <int kMode>
 __global__ void __launch_bounds__(kBlockThreads)
 sort_rank_kernel(SortParams p, int n_chunks, const int* counts, const int* sizes,
@@ -424,25 +429,10 @@ sort_rank_kernel(SortParams p, int n_chunks, const int* counts, const int* sizes
   if (chunk < n_chunks)
     for (int e = lane; e < nb; e += 32) run[e] = counts[(int64_t)e * n_chunks + chunk];
   __syncthreads();
-  int padded[4];  // align: the padded sizes, for expert_ids
-#pragma unroll
-  for (int j = 0; j < 4; ++j) padded[j] = (4 * t + j < nb) ? base[4 * t + j] : 0;
   block_exclusive_scan(base, nb, warp_tot);
-  if (kMode == 0 && blockIdx.x == 0) {
-    const int total = base[nb];
-    if (t == 0) ao.post_pad[0] = total;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int e = 4 * t + j;
-      if (e < nb) {
-        for (int o = 0; o < padded[j]; o += p.block_size) {
-          const int64_t blk = (base[e] + o) / p.block_size;
-          if (blk < ao.expert_ids_len) ao.expert_ids[blk] = e;
-        }
-      }
-    }
-    for (int64_t blk = total / p.block_size + t; blk < ao.expert_ids_len; blk += kBlockThreads)
-      ao.expert_ids[blk] = 0;
+  if (kMode == 0) {
+    if (blockIdx.x == 0 && t == 0) ao.post_pad[0] = base[nb];
+    write_block_table(base, nb, p.block_size, ao, (int64_t)blockIdx.x * kBlockThreads + t, (int64_t)gridDim.x * kBlockThreads);
   }
   if (chunk >= n_chunks) return;
   for (int e = lane; e < nb; e += 32)
