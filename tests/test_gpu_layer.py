@@ -432,8 +432,8 @@ def test_a_bounded_wait_that_runs_out_reaches_the_caller(native):
 @pytest.mark.parametrize("T", [40, 700])
 def test_fp8_layer_fused_and_unfused_activation_agree_bit_for_bit(native, T):
     """Block-scaled fp8 layer: gemm1's epilogue can apply SiLU and the 1x128 quantisation (one kernel
-    less, no [T*K, 2I] round trip; the default for many rows per expert, forced here) or the
-    two-kernel form runs (fuse_activation=False, and below 12 rows per expert).  Same values either way."""
+    less, no [T*K, 2I] round trip; on request) or the two-kernel form runs
+    (the default, and below 12 rows per expert).  Same values either way."""
     cfg = wl.scaled(wl.CONFIGS["cfg3_qwen3_fp8"], H=512, I=384, E=16)
     w = wl.make_weights(cfg, seed=8)
     x, logits, bias = wl.make_inputs(cfg, T, seed=8)

@@ -27,14 +27,16 @@ def test_which_calls_fuse_the_activation_into_gemm1(native):
     assert [rows(odd, r) for r in (1, 96, 97, 5000)] == ["epilogue", "epilogue", None, None]
     _, off = _layer(native, "cfg1_small_bf16", dict(H=256, I=256, E=4), fuse_activation=False)
     assert rows(off, 8) is None
-    # block-scaled fp8, SiLU: activation and 1x128 quantisation in the epilogue from 512 rows per expert
+    # block-scaled fp8, SiLU: two kernels are never slower, so the fused form only on request
     _, fp8 = _layer(native, "cfg4_deepseek_fp8", dict(H=256, I=256, E=8))
-    assert [rows(fp8, r) for r in (1, 511, 512, 4096)] == [None, None, "fp8", "fp8"]
+    assert [rows(fp8, r) for r in (1, 511, 512, 4096)] == [None] * 4
     _, forced = _layer(native, "cfg4_deepseek_fp8", dict(H=256, I=256, E=8), fuse_activation=True)
     assert [rows(forced, r) for r in (11, 12)] == [None, "fp8"]
     # a hint about the rows actually in use (expert parallelism: buffers sized for the worst case) decides
-    fp8.rows_hint = 512 * fp8.num_experts
-    assert fp8.fuses_activation(100 * 512 * fp8.num_experts) == "fp8" and rows(fp8, 1) == "fp8"
+    forced.rows_hint = 12 * forced.num_experts
+    assert forced.fuses_activation(100 * 12 * forced.num_experts) == "fp8" and rows(forced, 1) == "fp8"
+    forced.rows_hint = 11 * forced.num_experts
+    assert rows(forced, 100) is None
     # MXFP4 with SwigluOAI: always in the epilogue
     _, mx = _layer(native, "cfg5_gptoss_mxfp4", dict(H=256, I=256, E=4))
     assert [rows(mx, r) for r in (1, 4096)] == ["epilogue"] * 2

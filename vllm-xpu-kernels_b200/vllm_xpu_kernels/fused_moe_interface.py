@@ -34,7 +34,7 @@ except ImportError as e:  # native libraries not built
 REF_FUSED_MOE_ENV = "VLLM_XPU_FUSED_MOE_USE_REF"
 USE_MXFP4_FP8_ENV = "VLLM_XPU_FUSED_MOE_USE_MXFP4_FP8"
 FP8_BLOCK_SIZE = 128
-FP8_FUSED_MIN_ROWS = 512   # routed rows per expert from which gemm1 of an fp8 layer fuses SiLU + quantisation
+FP8_FUSED_MIN_ROWS = 12   # routed rows per expert from which fuse_activation=True takes the fused form of fp8 layers
 
 
 def _require_native():
@@ -283,15 +283,15 @@ class XpuFusedMoe:
         self._use_ref = False
         # block-scaled fp8 with SiLU: the token-major tensor-core kernel can apply the activation and the
         # 1x128 e4m3 quantisation of gemm2's input in its epilogue (same values as the two-kernel form).
-        # The epilogue runs on the warps that also promote the K blocks' partial sums, so short K loops lose by
-        # it and long ones break even, and it saves the [rows, 2I] intermediate, which counts at long segments:
-        # taken from FP8_FUSED_MIN_ROWS routed rows per expert on.  The layer call, fused / two kernels, us:
-        # 32 experts, hidden 7168, I 2048: 755 / 748 at 256 rows per expert, 942 / 950 at 512, 1910 / 1890 at
-        # 1024; 128 experts, hidden 2048, I 768: 380 / 355 at 256, 619 / 593 at 512, 1140 / 1090 at 1024,
-        # 2250 / 2130 at 2048.  fuse_activation=True / False force it.
+        # The epilogue runs on the warps that also promote the K blocks' partial sums, the kernel's bottleneck, and
+        # it is slower than a kernel of its own at every size measured, so it is taken on request only, where it
+        # saves the [rows, 2I] buffer.  The layer call, fused / two kernels, us (single bursts, which differ by
+        # 0.1 %): 128 experts, hidden 2048, I 768: 372 / 351 at 256 rows per expert, 616 / 595 at 512, 1098 / 1073 at
+        # 1024, 2068 / 2051 at 2048; 32 of 256 experts, hidden 7168, I 2048: 445 / 438 at 128, 641 / 636 at 256, 847 /
+        # 842 at 512, 2019 / 2018 at 1024; all 256 experts: 4286 / 4287 at 256.  In calls that
+        # follow one another under the power cap the two are within 1 %.
         self._fp8_fused_ok = (is_block_fp8 and self._act_kind == "silu" and self.inter_size % FP8_BLOCK_SIZE == 0
-                              and fuse_activation is not False)
-        self._fp8_fused_min_rows = 12 if fuse_activation else FP8_FUSED_MIN_ROWS
+                              and bool(fuse_activation))
         # 16-bit weights with SiLU: the tensor-core kernel pairs gate and up tiles in two
         # accumulators, which tensor memory holds for token tiles up to 128; for long expert
         # segments and K >= 4096 a CTA pair splits gate and up between its CTAs on 256-token
@@ -431,7 +431,7 @@ class XpuFusedMoe:
         None (a separate activation kernel)."""
         rows_expected = self.rows_hint if self.rows_hint > 0 else num_moe_inputs
         E = self.num_experts
-        if self._fp8_fused_ok and rows_expected >= self._fp8_fused_min_rows * E:
+        if self._fp8_fused_ok and rows_expected >= FP8_FUSED_MIN_ROWS * E:
             return "fp8"
         if self.fuse_activation or (self._w16_fused_ok and (
                 self._w16_fused_max_rows is None or rows_expected <= self._w16_fused_max_rows * E)):
