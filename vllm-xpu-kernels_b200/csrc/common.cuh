@@ -50,10 +50,12 @@ int fail(int code, const char* fmt, ...);
 // ends when every earlier kernel of the stream has completed (each of them waited for its own
 // predecessor) and its writes are visible.  A decode step is a chain of few-microsecond kernels and
 // gains 0.5 to 1 us per launch, a chain of nine at a few thousand rows as much.  Kernels of many waves lose
-// (blocks that wait take the place of blocks that work).  Layer calls without / with, us: qwen3 fp8 4096 routed
-// rows 176 / 166, 8192 rows 192 / 181, 32768 rows 353 / 351; one of 8 DeepSeek ranks at 4096 rows 303 / 295, 8192
-// rows 278 / 274; gpt-oss MXFP4 16384 rows 1520 / 1613; DeepSeek 8192 rows no difference, 32768 rows 3279 / 3410,
-// 65536 rows 5 % slower.  The line lies where none of them loses.
+// (blocks that wait take the place of blocks that work).  Layer calls with plain launches from 2048 rows on / with
+// early ones, single bursts, us: qwen3 fp8 8000 rows 191 / 179; one of 8 DeepSeek ranks at 4096 rows 270 / 261, 8192 rows
+// 278 / 271; small 16-bit layer 4096 rows 127 / 118, 8192 rows 171 / 161; Mixtral 16-bit 4096 rows 1306 / 1294, 8192 rows
+// 2209 / 2180, int4 1386 / 1377 and 2481 / 2480; DeepSeek of 256 experts 4800 rows no difference, 8000 rows 1627 / 1645 (the
+// one that loses), 32768 rows 3279 / 3410, 65536 rows 5 % slower; gpt-oss MXFP4 4096 rows 508 / 499, 8192 rows 678 / 665
+// (its GEMM apart, which has a line of its own: gemm_tc_mx.cu), 16384 rows 1419 / 1481.
 constexpr int64_t kEarlyLaunchRows = 8192;   // routed rows up to which a layer's kernels launch early
 template <typename... Params, typename... Args>
 inline cudaError_t launch_pdl(bool early, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem,

@@ -68,6 +68,11 @@ constexpr int kMxMaxStages = 8;
 // slower.  Not for token tiles of 16: their calls run into the power cap when they follow one another, and the
 // asking costs energy: layer calls of 128 tokens, in short runs 342 / 349 us, in a loop of seconds 391 / 384.
 constexpr int kMxAhead = 6;
+// Routed rows up to which this kernel launches early (launch_pdl); the layer's other kernels gain by it further on
+// (kEarlyLaunchRows), this one does not.  gpt-oss layer calls, single bursts, this kernel plain / early, us: 1 token 42.2 /
+// 39.7, 128 tokens 348 / 344, 400 tokens (1600 rows) 416.2 / 416.1, 512 tokens 428.5 / 429.1, 1024 tokens 499.5 / 505.1, 1500
+// tokens 558 / 571, 2048 tokens (8192 rows) 665 / 697.
+constexpr int64_t kMxEarlyLaunchRows = 2048;
 constexpr int kMxGroup = 4;         // K blocks per scale group (one hand-over from the scale preparers)
 constexpr int kMxSlots = 4;         // scale groups in the ring, at most
 constexpr int kMxSfwCap = 24576 + 32;    // largest weight-scale piece (128 rows x K/32 bytes) staged in shared memory
@@ -678,7 +683,7 @@ int launch_mx(const b200moe_gemm_args* a, const CUtensorMap& tw, MxParams& p, in
   const size_t smem = (size_t)fixed + (size_t)p.stages * body;
   static SmemConfig configured;
   if (int rc = configured.ensure(kern)) return rc;
-  B200_LAUNCHED("grouped_gemm_mx_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kMxThreads), smem, st, ta, tw, p));
+  B200_LAUNCHED("grouped_gemm_mx_kernel", launch_pdl(p.m <= kMxEarlyLaunchRows, kern, dim3(grid), dim3(kMxThreads), smem, st, ta, tw, p));
   return B200MOE_OK;
 }
 
