@@ -824,13 +824,16 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   // even, so leave headroom before a second token tile re-reads the weights).
   int bt;
   if (a_fp8) {
-    // fp8 pays a hand-over per 128-wide K block, so wide tiles win early.  Layer calls with tiles of 16 / 64 /
-    // 128 tokens, us: 128 experts, N 1536, K 2048: 4 rows per expert 140 / 155 / 140, 6 rows 142 / 160 / 142,
-    // 8 rows 143 / 161 / 142, 12 rows 153 / 164 / 146; 256 experts, N 4096, K 7168: 4 rows 1176 / 1248 / 1311,
-    // 5 rows 1255 / 1301 / 1338, 6 rows 1224 / 1195 / 1206, 8 rows 1361 / 1298 / 1308, 12 rows 1697 / 1437 /
-    // 1370; 32 of those experts: 6 rows 205 / 206 / 215, 8 rows 232 / 233 / 225, 12 rows 327 / 253 / 243.
-    // Nowhere is 64 the best by more than 1 %, so there is no such tile.
-    bt = avg <= 6 ? 16 : 128;
+    // fp8 pays a hand-over per 128-wide K block, so wide tiles win early, and short K loops (a tile of 768 is six
+    // blocks) want the 128-token kernel, which hands over best.  But with few rows that kernel draws the most power, so
+    // each pair of lines was measured in single bursts and in calls that follow one another under the power cap.
+    // Layer calls with tiles of 16 / 64 / 128 tokens, us, burst (cap): 256 experts, hidden 7168, I 2048: 5 rows per expert
+    // 1215 / 1240 / 1292 (1242 / 1293 / 1408), 6 rows 1227 / 1205 / 1258 (1374 / 1393 / 1504), 7 rows 1292 / 1237 / 1290
+    // (1453 / 1424 / 1519), 9 rows 1470 / 1313 / 1349 (1631 / 1516 / 1590), 11 rows 1632 / 1396 / 1393 (1772 / 1605 /
+    // 1702); 32 of those experts: 6 rows 198 / 196 / 209, 7 rows 218 / 209 / 213 (- / 213 / 227), 11 rows 281 / 241 / 240
+    // (- / 204 / 225).  128 experts, hidden 2048, I 768, 8 rows: 142 / 157 / 142 (141 / 157 / 155), gemm2 alone (K 768)
+    // 51 / 56 / 41 (51 / 56 / 48); with 64 for gemm1 and 128 for gemm2 142 (147).
+    bt = avg <= 6 ? 16 : (avg < 12 && a->k >= 2048 ? 64 : 128);
   } else {
     // Measured at 16 / 64 / 128 / 256 tokens (a CTA pair), 8 experts, N 28672, K 4096: 8 rows per expert
     // 289 / 285 / 295 / 340 us, 32 rows 336 / 291 / 301 / 342, 64 rows 539 / 320 / 307 / 344, 96 rows
@@ -910,6 +913,7 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   if (tile_bound < grid) grid = (int)tile_bound;
   if (grid < 1) grid = 1;
 
+  if (a_fp8 && bt == 64) return kn ? launch_tc<64, true, true>(ta, tw, p, grid, st) : launch_tc<64, true, false>(ta, tw, p, grid, st);
   if (a_fp8) return kn ? launch_tc<16, true, true>(ta, tw, p, grid, st) : launch_tc<16, true, false>(ta, tw, p, grid, st);
 #define B200_TC_CASE(BT_)                                                         \
   if (bt == BT_) {                                                                \
