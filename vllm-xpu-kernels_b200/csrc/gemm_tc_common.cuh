@@ -15,10 +15,11 @@ constexpr int kMaxExperts = 1024;
 constexpr size_t kMaxSmem = 227 * 1024;   // dynamic shared memory of a CTA
 
 // Depth of a ring whose blocks `sets` converter sets take in turn, each putting what it makes of a block
-// into one of `operands` stages that the MMA frees in order.  A set waits for the n-th fill of a stage by
+// into one of `operands` stages that one issuer's MMAs free in order.  A set waits for the n-th fill of a stage by
 // parity, which also looks complete while fill n - 1 is still on its way: that fill, block i - stages, has
 // landed for sure only if the MMA was done with it when the set stored its last block, i - sets, i.e. if it
-// is no later than block i - sets - operands.
+// is no later than block i - sets - operands.  (Two issuers free operands out of order: gemm_tc_i4.cu therefore also
+// keeps its depth a multiple of the sets, so that a stage's fills are all seen by the same set.)
 constexpr int converter_ring_depth(int sets, int operands) { return sets + operands; }
 
 struct TileInfo {
