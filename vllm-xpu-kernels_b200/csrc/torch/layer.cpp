@@ -33,11 +33,12 @@ struct Plan {
   double clamp = 0.0;
   // Up to this many rows per expert the block-scaled int4 kernel (gemm_tc_i4.cu) takes the layer: it
   // streams the weights faster than the one that expands them to 16 bits (gemm_tc_dq.cu), until experts
-  // need a second of its tiles of 32 tokens.  A layer of 8 experts of 4096 x 14336, 2 a token, bfloat16
-  // (float16, three planes) with routing as it comes: 93 (101) against 121 us at 1 token, 215 (240) against 297 at
-  // 8 rows an expert, 230 (294) against 276 at 12, 250 (320) against 280 at 16, 318 (399) against 284 at 20, 321
-  // (404) against 285 at 24.  Half a tile leaves room for uneven routing; float16 keeps the same line, because
-  // its planes also lose less than a weight rounded after its scale.
+  // need a second of its tiles of 32 tokens.  A layer of 8 experts of 4096 x 14336, 2 a token, with routing as it
+  // comes, this / that kernel, us: bfloat16 218 / 305 at 8 rows an expert, 235 / 289 at 12, 249 / 293 at 16, 292 / 297 at
+  // 20, 295 / 298 at 24; float16 (three planes) 241 / 304 at 8, 298 / 287 at 10, 300 / 288 at 12, 317 / 292 at 16, 365 / 295
+  // at 20.  Half a tile leaves room for uneven routing.  float16 keeps the same line although it costs 4 to 8 % from
+  // 10 rows on, because the planes are the more accurate: error of the layer's output against 64 bits (2-norm, 9 to
+  // 16 rows an expert) 5.3e-4 / 6.1e-4, where the other kernel rounds a weight after its scale; bfloat16 4.3e-3 / 4.9e-3.
   static constexpr int64_t kI4PlaneRows = 16;
 };
 const char* const kPlanName = "b200moe.layer_plan";
