@@ -292,6 +292,7 @@ class XpuFusedMoe:
         # follow one another under the power cap the two are within 1 %.
         self._fp8_fused_ok = (is_block_fp8 and self._act_kind == "silu" and self.inter_size % FP8_BLOCK_SIZE == 0
                               and bool(fuse_activation))
+        self._fp8_fused_min_rows = FP8_FUSED_MIN_ROWS
         # 16-bit weights with SiLU: the tensor-core kernel pairs gate and up tiles in two
         # accumulators, which tensor memory holds for token tiles up to 128; for long expert
         # segments and K >= 4096 a CTA pair splits gate and up between its CTAs on 256-token
@@ -431,7 +432,7 @@ class XpuFusedMoe:
         None (a separate activation kernel)."""
         rows_expected = self.rows_hint if self.rows_hint > 0 else num_moe_inputs
         E = self.num_experts
-        if self._fp8_fused_ok and rows_expected >= FP8_FUSED_MIN_ROWS * E:
+        if self._fp8_fused_ok and rows_expected >= self._fp8_fused_min_rows * E:
             return "fp8"
         if self.fuse_activation or (self._w16_fused_ok and (
                 self._w16_fused_max_rows is None or rows_expected <= self._w16_fused_max_rows * E)):
