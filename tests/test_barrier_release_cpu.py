@@ -55,3 +55,21 @@ def test_promotion_warps_acquire_what_they_read_from_shared_memory(name, kernel,
     wait = before.rindex("mbar_wait_s(" + seen)
     free = before.rindex("mbar_wait_s(acc_empty0")                # (not before the phase before is over)
     assert before.rfind("mbar_arrive_s(acc_full0") > max(wait, free)
+
+
+@pytest.mark.parametrize("path", SOURCES, ids=lambda p: p.name)
+def test_a_proxy_fence_lies_between_ordinary_stores_and_the_tensor_core(path):
+    """Scale words and partial weight blocks are stored by warps and read by tcgen05.cp / tcgen05.mma, and finished
+    rows by TMA, through the async proxy.  Either the writer fences before it arrives, or the issuer does between its
+    wait for them and its first use."""
+    text = "\n".join(code for _, code in _statements(path))
+    fences = text.count("ptx::fence_proxy_async();")
+    uses = {"gemm_tc_i4.cu": 1, "gemm_tc_mx.cu": 2, "gemm_tc_fp8t.cu": 1}.get(path.name, 0)
+    assert fences == uses
+    if path.name == "gemm_tc_i4.cu":      # the preparer, before it hands a group over
+        assert "ptx::fence_proxy_async();\n__syncwarp();\nif (lane == 0) ptx::mbar_arrive_s(sf_full0" in text
+    if path.name == "gemm_tc_mx.cu":      # the partial block's writers; the issuer, for the scale words
+        assert "ptx::fence_proxy_async();\n__syncwarp();\nif (lane == 0) ptx::mbar_arrive(&ctrl->tail_full);" in text
+        assert re.search(r"mbar_wait_s\(sf_full0 [^\n]*\n *ptx::fence_proxy_async\(\);", text)
+    if path.name == "gemm_tc_fp8t.cu":    # finished rows, before their TMA store
+        assert re.search(r"ptx::fence_proxy_async\(\);\n__syncwarp\(\);\nif \(lane == 0\) \{\nptx::tma_store_2d", text)
