@@ -179,6 +179,17 @@ __device__ __forceinline__ void write_block_table(const int* base, int nb, int b
   }
 }
 
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// The word at `p` (shared memory) of CTA `rank` of the cluster.
+__device__ __forceinline__ int cluster_load(const int* p, int rank) {
+  uint32_t at;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+
 template <int kMode>
 __global__ void __launch_bounds__(kBlockThreads)
 sort_single_block_kernel(SortParams p, AlignOut ao, RemapOut ro) {
@@ -337,6 +348,101 @@ lora_align_kernel(SortParams p, LoraAlignArgs a) {
   }
 }
 
+// ------------------------- one cluster ----------------------------------------
+// Row maps of 2049 to 65536 slots in one launch: a cluster of eight CTAs, 256 warps with up to 256 consecutive slots
+// each.  A lane keeps its slots' buckets and their ranks inside the warp in registers; the warps' histograms are
+// summed up per CTA, and the CTAs read one another's sums over the cluster's shared memory.
+constexpr int kClusterCtas = 8;
+constexpr int kClusterThreads = 1024;
+constexpr int kClusterWarps = kClusterThreads / 32;
+constexpr int kClusterSteps = 8;                 // slots a lane takes at most
+constexpr int64_t kClusterSlots = (int64_t)kClusterCtas * kClusterThreads * kClusterSteps;
+// Histograms of all warps within the 48 KB a kernel has without asking (more buckets: the three launches below).
+__host__ __device__ constexpr size_t cluster_sort_smem(int nb) { return ((size_t)(kClusterWarps + 2) * nb + kClusterWarps) * sizeof(int); }
+constexpr size_t kClusterSmem = 48 * 1024;
+
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
+sort_cluster_kernel(SortParams p, int steps, RemapOut ro) {
+  pdl_trigger();
+  extern __shared__ int smem[];
+  const int nb = p.n_buckets;
+  int* hist = smem;                              // [kClusterWarps][nb]: slots of a warp, then of the warps before it
+  int* sums = hist + kClusterWarps * nb;         // [nb] slots of this CTA, read by the others
+  int* first = sums + nb;                        // [nb] the first position of this CTA
+  int* warp_tot = first + nb;                    // [kClusterWarps]
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t rank = blockIdx.x;              // (the grid is one cluster)
+  for (int i = t; i < kClusterWarps * nb; i += kClusterThreads) hist[i] = 0;
+  pdl_wait();
+  const int64_t begin = ((int64_t)rank * kClusterWarps + warp) * steps * 32 + lane;
+  int bucket[kClusterSteps], local[kClusterSteps];
+#pragma unroll
+  for (int s = 0; s < kClusterSteps; ++s) {
+    const int64_t i = begin + s * 32;
+    bucket[s] = s < steps && i < p.numel ? bucket_of(p, i) : -1;
+  }
+  __syncthreads();
+  int* mine = hist + warp * nb;
+#pragma unroll
+  for (int s = 0; s < kClusterSteps; ++s) {
+    if (s < steps) {
+      const int b = bucket[s];
+      // Lanes without a bucket use distinct keys so they never match a real one.
+      const uint32_t peers = __match_any_sync(0xffffffffu, b >= 0 ? b : kMaxBuckets + lane);
+      const int before = __popc(peers & ((1u << lane) - 1u));
+      local[s] = b >= 0 ? mine[b] + before : 0;
+      __syncwarp();
+      if (b >= 0 && before == 0) mine[b] += __popc(peers);
+      __syncwarp();
+    }
+  }
+  __syncthreads();
+  for (int e = t; e < nb; e += kClusterThreads) {
+    int run = 0;
+#pragma unroll 8
+    for (int w = 0; w < kClusterWarps; ++w) {
+      const int c = hist[w * nb + e];
+      hist[w * nb + e] = run;
+      run += c;
+    }
+    sums[e] = run;
+  }
+  cluster_arrive();
+  cluster_wait();
+  // (a thread per bucket: nb is below the block's size)
+  int total = 0, lower = 0;
+  if (t < nb) {
+    int x[kClusterCtas];
+#pragma unroll
+    for (int c = 0; c < kClusterCtas; ++c) x[c] = cluster_load(sums + t, c);
+#pragma unroll
+    for (int c = 0; c < kClusterCtas; ++c) {
+      total += x[c];
+      if (c < (int)rank) lower += x[c];
+    }
+    if (rank == 0) ro.rows_per_expert[t] = total;
+  }
+  cluster_arrive();   // the others' sums have been read
+  int incl = total;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
+  }
+  if (lane == 31) warp_tot[warp] = incl;
+  __syncthreads();
+  int base = incl - total;
+  for (int w = 0; w < warp && w * 32 < nb; ++w) base += warp_tot[w];
+  if (t < nb) first[t] = (p.bucket_stride > 0 ? (int)(t * p.bucket_stride) : base) + lower;
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < kClusterSteps; ++s) {
+    const int64_t i = begin + s * 32;
+    if (s < steps && i < p.numel) ro.row_map[i] = bucket[s] >= 0 ? first[bucket[s]] + mine[bucket[s]] + local[s] : -1;
+  }
+  cluster_wait();     // no CTA leaves while another may still read its sums
+}
+
 // ------------------------- multi-block path ---------------------------------
 // workspace: counts[n_buckets][n_chunks] ints, then sizes[n_buckets] ints.
 __global__ void __launch_bounds__(kBlockThreads)
@@ -462,6 +568,12 @@ int run_sort(const SortParams& p, const AlignOut& ao, const RemapOut& ro,
   if (workspace == nullptr || workspace_bytes < need)
     return fail(B200MOE_E_WORKSPACE, "workspace of %zu bytes needed, got %zu", need,
                 workspace_bytes);
+  if (kMode == 1 && p.numel <= kClusterSlots && cluster_sort_smem(nb) <= kClusterSmem) {
+    const int steps = (int)((p.numel + kClusterCtas * kClusterThreads - 1) / (kClusterCtas * kClusterThreads));
+    B200_LAUNCHED("sort_cluster_kernel", launch_pdl(p.numel <= kEarlyLaunchRows, sort_cluster_kernel, dim3(kClusterCtas),
+        dim3(kClusterThreads), cluster_sort_smem(nb), st, p, steps, ro));
+    return B200MOE_OK;
+  }
   const int n_chunks = (int)((p.numel + kChunk - 1) / kChunk);
   const int n_blocks = (n_chunks + kWarps - 1) / kWarps;
   int* counts = reinterpret_cast<int*>(workspace);
