@@ -43,6 +43,30 @@ __device__ __forceinline__ int8_t f32_to_i8_rn(float x) {
   return (int8_t)fminf(fmaxf(rintf(x), -128.0f), 127.0f);
 }
 
+// silu(g) = g / (1 + 2^(-g log2 e)) with the hardware's exponential and reciprocal and nothing around them.  The range
+// steps that __expf and __fdividef add act on subnormals and beyond 2^126, where this denominator, from 1 up to
+// infinity, gives the same value without them.
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+__device__ __forceinline__ float silu_fast(float g) {
+  float e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(g, -1.4426950408889634f)));
+  return __fmul_rn(g, rcp_ftz(1.0f + e));
+}
+
+// x / 448 for x >= 0, correctly rounded where the quotient is normal: the product with the rounded reciprocal and one
+// correction by the exact remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990; all 2^23 significands compared).  An infinity stays one.
+__device__ __forceinline__ float div_448(float x) {
+  constexpr float kInv = 1.0f / 448.0f;
+  const float q = __fmul_rn(x, kInv);
+  const float fixed = fmaf(fmaf(-q, 448.0f, x), kInv, q);
+  return q == INFINITY ? q : fixed;
+}
+
 enum OutFmt { kOutE4m3 = 0, kOutI8 = 1, kOutE2m1 = 2 };
 
 struct GroupQuantArgs {
@@ -55,10 +79,6 @@ struct GroupQuantArgs {
   int64_t s_stride_row, s_stride_group;
   float eps;
   int ue8m0;
-  // optional: only the first sum(rows_per_segment[0..num_segments)) rows are in use (row
-  // buffers sized for a worst case); blocks past them return at once
-  const int32_t* rows_per_segment = nullptr;
-  int num_segments = 0;
 };
 
 // kGated: input rows are [gate(hidden) | up(hidden)] and the quantised value is
@@ -73,18 +93,6 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
   pdl_trigger();
   pdl_wait();
   constexpr int N = Vec16<T>::N;
-  if (a.rows_per_segment != nullptr) {
-    __shared__ int64_t in_use;
-    if (threadIdx.x < 32) {
-      int64_t sum = 0;
-      for (int e = threadIdx.x; e < a.num_segments; e += 32) sum += max(a.rows_per_segment[e], 0);
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, off);
-      if (threadIdx.x == 0) in_use = sum;
-    }
-    __syncthreads();
-    if (in_use < rows) rows = in_use;
-  }
   const int lanes_per_group = a.group / N;
   const int nvec = a.hidden / N;
   const int64_t in_pitch = (int64_t)a.hidden * (kGated ? 2 : 1);
@@ -115,7 +123,7 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
 #pragma unroll
           for (int i = 0; i < N; ++i) {
             const float gf = to_f32<T>(ge[i]);
-            v[i] = __fmul_rn(__fdividef(gf, 1.0f + __expf(-gf)), to_f32<T>(ue[i]));
+            v[i] = __fmul_rn(silu_fast(gf), to_f32<T>(ue[i]));
           }
         } else {
 #pragma unroll
@@ -132,7 +140,7 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
         scale = fmaxf(__fdiv_rn(amax, 127.0f), 1.1920928955078125e-07f);
       } else if (kFmt == kOutE4m3) {
         const float floor_s = 1.0f / (448.0f * 512.0f);
-        scale = fmaxf(__fdiv_rn(amax, 448.0f), floor_s);
+        scale = fmaxf(div_448(amax), floor_s);
         if (a.scale_ub != nullptr) scale = fmaxf(fminf(scale, *a.scale_ub), floor_s);
         if (a.ue8m0) scale = ceil_pow2_eps(scale, 1e-10f);
       } else {
@@ -156,7 +164,7 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
           else *reinterpret_cast<uint16_t*>(dst) = *reinterpret_cast<const uint16_t*>(o);
         } else {
           alignas(8) uint8_t o[N];
-          const float inv = __fdividef(1.0f, scale);   // the group's, once: v * inv is __fdividef(v, scale)
+          const float inv = rcp_ftz(scale);   // the group's, once: v * inv is __fdividef(v, scale)
 #pragma unroll
           for (int i = 0; i < N; i += 2) {
             const float q0 = __fmul_rn(v[i], inv), q1 = __fmul_rn(v[i + 1], inv);
@@ -173,6 +181,75 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
           else *reinterpret_cast<uint32_t*>(dst) = *reinterpret_cast<const uint32_t*>(o);
         }
       }
+    }
+  }
+}
+
+// The layer's form: SiLU, multiply and 1x128 e4m3 quantisation of the rows that the experts' segments use (the first
+// sum(rows_per_segment) of them; the buffers may be sized for a worst case), value for value the arithmetic above.
+// A warp takes pieces of 256 values, kPieces of them in flight together; as many blocks as are resident walk over
+// all pieces, so the sum over the segments is made once a block.  The last rows come first: they are what the GEMM
+// before wrote last, so they are read from L2 before the others push them out.
+// Bytes bound it: 65536 x 2048 values 190 -> 144 us (4.7 TB/s beside the write-back of what the GEMM left in L2), 65536 x
+// 768 81 -> 56, 24008 x 768 28.6 -> 20.9 (blocks of a row's width that each summed the segments, more of them than were
+// resident, first row first, __expf and __fdividef with their range steps, an IEEE division a value group).
+constexpr int kPieces = 4;
+template <typename T>
+__global__ void __launch_bounds__(256, 4)
+silu_quant_rows_kernel(uint8_t* __restrict__ out, float* __restrict__ scales, const T* __restrict__ in, int64_t max_rows,
+                       int hidden, const int32_t* __restrict__ rows_per_segment, int num_segments) {
+  pdl_trigger();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  int64_t used = 0;   // (every warp for itself)
+  for (int e = lane; e < num_segments; e += 32) used += max(__ldg(rows_per_segment + e), 0);
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) used += __shfl_xor_sync(0xffffffffu, used, off);
+  const int rows = (int)(used < max_rows ? used : max_rows);
+  const int nvec = hidden / 8, pieces = (nvec + 31) / 32, groups = hidden / 128;
+  const int warps = gridDim.x * 8, first = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const int step_row = warps / pieces, step_piece = warps - step_row * pieces;
+  int row = first / pieces, piece = first - row * pieces;   // counted from the last row
+  while (row < rows) {
+    vec16 g[kPieces], u[kPieces];
+    int64_t at[kPieces];    // row
+    int col[kPieces];       // 16-byte piece of it, or past its end
+#pragma unroll
+    for (int k = 0; k < kPieces; ++k) {
+      at[k] = rows - 1 - row;
+      col[k] = row < rows ? piece * 32 + lane : nvec;
+      if (col[k] < nvec) {
+        const T* src = in + at[k] * 2 * hidden + col[k] * 8;
+        g[k] = ld16(src);
+        u[k] = ld16(src + hidden);
+      }
+      row += step_row;
+      piece += step_piece;
+      if (piece >= pieces) { piece -= pieces; ++row; }
+    }
+#pragma unroll
+    for (int k = 0; k < kPieces; ++k) {
+      const bool active = col[k] < nvec;
+      const T *ge = reinterpret_cast<const T*>(&g[k]), *ue = reinterpret_cast<const T*>(&u[k]);
+      float v[8], amax = 0.f;
+      if (active) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          v[i] = __fmul_rn(silu_fast(to_f32<T>(ge[i])), to_f32<T>(ue[i]));
+          amax = fmaxf(amax, fabsf(v[i]));
+        }
+      }
+#pragma unroll
+      for (int off = 1; off < 16; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+      if (!active) continue;
+      const float scale = fmaxf(div_448(amax), 1.0f / (448.0f * 512.0f));
+      if ((lane & 15) == 0) scales[at[k] * groups + (col[k] >> 4)] = scale;
+      const float inv = rcp_ftz(scale);
+      uint32_t q[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)   // (the conversion saturates; the minimum makes 448 of a NaN)
+        q[i] = f32x2_to_e4m3x2(fminf(__fmul_rn(v[2 * i], inv), 448.0f), fminf(__fmul_rn(v[2 * i + 1], inv), 448.0f));
+      *reinterpret_cast<uint2*>(out + at[k] * hidden + col[k] * 8) = make_uint2(q[0] | (q[1] << 16), q[2] | (q[3] << 16));
     }
   }
 }
@@ -223,9 +300,8 @@ template <bool kGated, int kFmt>
 int launch_group_quant(b200moe_dtype dtype, const GroupQuantArgs& a, int64_t rows, cudaStream_t st,
                        const char* name) {
   const int threads = threads_for(a.hidden / (dtype == B200MOE_F32 ? 4 : 8));
-  // As many blocks as are resident together: each sums the segments once and walks over its rows.  Instructions
-  // bound the kernel (issue slots 79 % in use, DRAM 43 %): the reciprocal of a group's scale once, two values a
-  // conversion, 65536 x 2048 values with SiLU 189 -> 174 us.
+  // Instructions bound the kernel (issue slots 79 % in use, DRAM 43 %): the reciprocal of a group's scale once, two
+  // values a conversion, 65536 x 2048 values with SiLU 189 -> 174 us.
   const int64_t blocks = (rows + kRows - 1) / kRows, most = (int64_t)sm_count() * (2048 / threads);
   const dim3 grid((unsigned)(blocks < most ? blocks : most));
   auto run = [&](auto type) {
@@ -274,8 +350,18 @@ extern "C" int b200moe_silu_and_mul_per_block_quant_ragged(void* out, float* sca
   if (rows == 0 || hidden == 0) return B200MOE_OK;
   B200_CHECK_ARG(out && scales && in, "silu_and_mul_per_block_quant: null pointer");
   B200_CHECK_ARG(aligned16(in) && (((uintptr_t)out & 7) == 0), "silu_and_mul_per_block_quant: misaligned buffer");
-  GroupQuantArgs a = {in, out, scales, nullptr, hidden, 128, hidden / 128, 1, 0.f, 0, rows_per_segment, num_segments};
-  return launch_group_quant<true, kOutE4m3>(dtype, a, rows, as_stream(stream), "silu_and_mul_per_block_quant");
+  B200_CHECK_ARG(rows < ((int64_t)1 << 31), "silu_and_mul_per_block_quant_ragged: too many rows");
+  const int64_t items = rows * ((hidden + 255) / 256), blocks = (items + 8 * kPieces - 1) / (8 * kPieces);
+  const int64_t most = (int64_t)sm_count() * 4;
+  const dim3 grid((unsigned)(blocks < most ? blocks : most));
+  auto run = [&](auto type) {
+    using T = decltype(type);
+    return launch_pdl(rows <= kEarlyLaunchRows, silu_quant_rows_kernel<T>, grid, dim3(256), 0, as_stream(stream), (uint8_t*)out,
+                      scales, (const T*)in, rows, hidden, rows_per_segment, num_segments);
+  };
+  if (dtype == B200MOE_BF16) B200_LAUNCHED("silu_quant_rows_kernel", run(__nv_bfloat16()));
+  else B200_LAUNCHED("silu_quant_rows_kernel", run(__half()));
+  return B200MOE_OK;
 }
 
 extern "C" int b200moe_silu_and_mul_mxfp4_quant(void* out, float* scales, const void* in, b200moe_dtype dtype,
