@@ -358,7 +358,11 @@ typedef struct {
                              block-scaled fp8: the activated values leave the
                              kernel quantised per token and 128 features, as
                              b200moe_silu_and_mul_per_block_quant would quantise
-                             the unfused output (same values)                     */
+                             the unfused output (same values); a_dtype (FP8_E4M3 or
+                             FP8_E4M3_X2) with EPI_SWIGLUOAI on MXFP4, MXFP8 or
+                             per-tensor fp8 weights, N divisible by 64: the planes
+                             [planes][M, N/2] that b200moe_quant_mxfp8 would make of
+                             the mid_dtype output (same values)                   */
   const int32_t* rows_per_expert; /* [E] device                                   */
   int64_t m;              /* rows of A and D (upper bound of the rows in use)     */
   int n, k, num_experts;
@@ -386,7 +390,8 @@ typedef struct {
                              exchange as they arrive, grouped by source rank and by
                              local expert inside a source, need no second
                              permutation.  16-bit and block-scaled fp8 weights.     */
-  void* d_scale;          /* FP8_E4M3 output: fp32 scales [M, N/256]; else NULL     */
+  void* d_scale;          /* FP8_E4M3 output: fp32 scales [M, N/256]; planes: their
+                             scale words [planes][ceil(N/2 / 128)][M]; else NULL    */
   b200moe_dtype mid_dtype;/* FP8_E4M3 output: BF16 or F16, the type the
                              pre-activation values (and the bias) have: they are
                              rounded to it before the activation, as the unfused

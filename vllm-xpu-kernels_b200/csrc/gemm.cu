@@ -23,8 +23,14 @@ extern "C" int b200moe_grouped_gemm(const b200moe_gemm_args* a, b200moe_stream s
   B200_CHECK_ARG(a->m >= 0 && a->n >= 0 && a->k > 0 && a->num_experts >= 1,
                  "grouped_gemm: bad sizes (m=%lld n=%d k=%d experts=%d)", (long long)a->m, a->n,
                  a->k, a->num_experts);
-  const bool d_quant = a->d_dtype == B200MOE_FP8_E4M3;
-  B200_CHECK_ARG(a->d_dtype == B200MOE_BF16 || a->d_dtype == B200MOE_F16 || d_quant,
+  // the SwigluOAI form's output as the planes that the next GEMM takes
+  const bool d_planes = a->epilogue == B200MOE_EPI_SWIGLUOAI && a->d_dtype == a->a_dtype &&
+                        (a->d_dtype == B200MOE_FP8_E4M3 || a->d_dtype == B200MOE_FP8_E4M3_X2) &&
+                        (a->w_format == B200MOE_W_MXFP4_NK || a->w_format == B200MOE_W_FP8_TENSOR_KN ||
+                         a->w_format == B200MOE_W_FP8E5M2_TENSOR_KN || a->w_format == B200MOE_W_MXFP8_KN) &&
+                        a->d_scale != nullptr && (a->mid_dtype == B200MOE_BF16 || a->mid_dtype == B200MOE_F16) && a->n % 64 == 0;
+  const bool d_quant = a->d_dtype == B200MOE_FP8_E4M3 && !d_planes;
+  B200_CHECK_ARG(d_planes || a->d_dtype == B200MOE_BF16 || a->d_dtype == B200MOE_F16 || d_quant,
                  "grouped_gemm: ptr_D must be bfloat16 or float16");
   B200_CHECK_ARG(!d_quant || (a->epilogue == B200MOE_EPI_SILU_MUL && a->d_scale != nullptr &&
                               a->a_dtype == B200MOE_FP8_E4M3 &&

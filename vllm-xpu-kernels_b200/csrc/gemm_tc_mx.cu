@@ -51,6 +51,7 @@
 // rounding of the activations to MXFP8 only.
 #include "common.cuh"
 #include "gemm_tc_common.cuh"
+#include "mx_quant.cuh"
 #include "sm100_ptx.cuh"
 
 
@@ -99,6 +100,7 @@ struct MxParams {
   int out_f16;
   int swiglu;      // 1: D[m, f/2] = swigluoai(acc[m,f], acc[m,f+1]) for even f
   float alpha, limit, clamp_limit;
+  uint32_t* d_scale;   // swiglu: not null, D leaves as e4m3 planes [terms][M, n/2] with their scale words [terms][n/2 / 128][M]
 };
 
 struct MxCtrl {
@@ -111,10 +113,53 @@ struct MxCtrl {
   uint64_t sfw_full[2];
   uint64_t sfw_empty[2];
   uint64_t tail_full;    // the tile's partial block has been spread
+  uint64_t pair_full[2]; // quantised output: both halves of a 32-wide group are in shared memory
   uint32_t tmem_base;
   int abort_flag;
-  alignas(16) uint16_t xpose[4][32 * 32];
+  alignas(16) uint16_t xpose[4][32 * 32];   // a warp's transpose tile; quantised output: two buffers per pair of warps
 };
+
+// Quantised output of a gated tile: lane pair lane / 2 takes one token's group of 32 outputs, 16 values each (16-bit, as
+// they would have been stored), through the planes of quant_mxfp8_kernel, value for value.
+template <int kTerms>
+__device__ __forceinline__ void store_quantised(uint32_t src, const MxParams& p, int64_t row, bool live, int group, int lane) {
+  const int n_out = p.n >> 1, words = (n_out + 127) / 128;
+  uint32_t x[8];
+  *reinterpret_cast<uint4*>(x) = ptx::lds128(src);
+  *reinterpret_cast<uint4*>(x + 4) = ptx::lds128(src + 16);
+  float v[16], amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    if (p.out_f16) {
+      const float2 h = __half22float2(*reinterpret_cast<const __half2*>(x + i));
+      v[2 * i] = h.x; v[2 * i + 1] = h.y;
+    } else {
+      v[2 * i] = __uint_as_float(x[i] << 16); v[2 * i + 1] = __uint_as_float(x[i] & 0xffff0000u);
+    }
+  }
+#pragma unroll
+  for (int term = 0; term < kTerms; ++term) {
+    amax = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    float sc, inv;
+    const int e = mx_scale(amax, kMxLeast, sc, inv);
+    uint32_t c[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) c[i] = mx_codes4(v + 4 * i, sc, inv, term + 1 < kTerms);
+    if (live) {
+      uint8_t* to = reinterpret_cast<uint8_t*>(p.d) + (term * p.m + row) * n_out + group * 32 + (lane & 1) * 16;
+      *reinterpret_cast<uint4*>(to) = make_uint4(c[0], c[1], c[2], c[3]);
+      if ((lane & 1) == 0) {
+        uint8_t* s = reinterpret_cast<uint8_t*>(p.d_scale + ((int64_t)term * words + (group >> 2)) * p.m + row) + (group & 3);
+        *s = (uint8_t)e;
+        if ((group + 1) * 32 == n_out)    // the groups that fill the row's last word: 2^0
+          for (int g = 1; (group & 3) + g < 4; ++g) s[g] = 0x7f;
+      }
+    }
+  }
+}
 // Shared memory after the pipeline stages: one buffer for the partial K block, the ring
 // of scale groups, MxCtrl, the tile walk and two weight-scale staging buffers.
 // One group of the scale ring: per K block 512 bytes for the weight rows and 512 per 128 token rows.
@@ -231,6 +276,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
       ptx::mbar_init(&ctrl->sfw_empty[a], 4);
     }
     ptx::mbar_init(&ctrl->tail_full, 4);
+    for (int x = 0; x < 2; ++x) ptx::mbar_init(&ctrl->pair_full[x], 2);
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
   }
@@ -542,7 +588,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
     const int et = q * 32 + lane;
     const uint32_t lane_sel = (uint32_t)(q * 32) << 16;
     const int n_out = p.swiglu ? p.n / 2 : p.n;
-    uint32_t acc_it = 0;
+    uint32_t acc_it = 0, xit = 0;
     int cursor = 0, cursor_next = 0;
     bool ok = true;
     // The partial K block (K = 64 past a multiple of 128): row et's 32 packed bytes, fetched a tile
@@ -635,6 +681,24 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
               up = fminf(fmaxf(up, -p.limit), p.limit);
               out[j] = (up + 1.0f) * gate * __fdividef(1.0f, 1.0f + __expf(-gate * p.alpha));
             }
+            if (BT == 16 && p.d_scale != nullptr) {
+              // A group of 32 outputs is spread over two warps (q and q ^ 1): both put their 16 of every token into one
+              // buffer, from where the first takes them.  Two buffers in turn: who writes one again has seen the
+              // other warp arrive for the tile in between, after its reads of the tile before.
+              const uint32_t pair = q >> 1, side = q & 1;
+              const uint32_t buf = ptx::smem_u32(ctrl->xpose[pair * 2 + (xit & 1)]);
+              const uint32_t at = buf + ((lane & 1) * 32 + side * 16 + (lane >> 1)) * 2;
+#pragma unroll
+              for (int j = 0; j < kChunk / 2; ++j) ptx::sts16(at + j * 128, bits16(out[j], p.out_f16));
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive(&ctrl->pair_full[pair]);
+              if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->pair_full[pair], xit & 1, abort_flag))) { ok = false; break; }
+              ++xit;
+              const int tok = lane >> 1, group = ti.n_tile * 2 + pair;
+              if (side == 0)
+                store_quantised<kTerms>(buf + lane * 32, p, (int64_t)ti.row0 + tok, tok < ti.valid && group * 32 < n_out, group, lane);
+              continue;
+            }
             store_pairs_transposed(ctrl->xpose[warp - 6], out, p.d, p.out_f16, (int64_t)ti.row0 + c0, ti.valid - c0, p.m,
                                    n_out, (ti.n_tile * kFeat + q * 32) >> 1, lane);
           } else {
@@ -644,6 +708,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
           }
         }
       }
+      if (!ok) break;
       ptx::tc_fence_before();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&ctrl->acc_empty[a]);
@@ -749,6 +814,9 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   p.out_f16 = a->d_dtype == B200MOE_F16;
   p.swiglu = a->epilogue == B200MOE_EPI_SWIGLUOAI;
   p.alpha = a->act_alpha; p.limit = a->act_limit; p.clamp_limit = a->clamp_limit;
+  const bool quantised = a->d_dtype == B200MOE_FP8_E4M3 || a->d_dtype == B200MOE_FP8_E4M3_X2;
+  p.d_scale = quantised ? reinterpret_cast<uint32_t*>(a->d_scale) : nullptr;
+  if (quantised) p.out_f16 = a->mid_dtype == B200MOE_F16;
 
   const int64_t rows_in_use = (a->rows_hint > 0 && a->rows_hint < a->m) ? a->rows_hint : a->m;
   const int64_t avg = (rows_in_use + a->num_experts - 1) / a->num_experts;
@@ -758,6 +826,7 @@ int grouped_gemm_tc_mx(const b200moe_gemm_args* a, cudaStream_t st) {
   // and the scale columns fill the 512 columns
   if (x2 && bt > 64) bt = avg > 48 ? 96 : 64;
   if (!x2 && avg > 128) bt = 192;               // one plane: the same N = 192 instruction
+  if (quantised) bt = 16;   // (the other tiles have no such epilogue)
   // Measured, 128 experts, N 5760, K 2880.  Two planes at 16 / 64 / 96 tokens: 8 rows per expert 238 / 305
   // / 373 us, 16 rows 305 / 309 / 373, 48 rows 670 / 356 / 426, 64 rows - / 469 / 430; one plane at 16 / 64
   // / 128 / 192: 8 rows 232 / 283 / 301 / 347, 16 rows 313 / 285 / 300 / 350, 40 rows 549 / 318 / 322 / 367,

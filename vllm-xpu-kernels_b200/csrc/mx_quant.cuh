@@ -20,39 +20,46 @@ namespace {
 // lose bits and then vanish.  Planes that stand for 16-bit activations (an int4 layer's) go down to
 // 2^-100: what they leave of a bfloat16 is below 2^-109, and nothing gets near fp32's subnormals.
 constexpr int kMxLeast = 127 - 33, kMxLeastExact = 127 - 100;
+// Biased exponent of a group's scale, the scale and its inverse.
+__device__ __forceinline__ int mx_scale(float amax, int least, float& sc, float& inv) {
+  const uint32_t bits = __float_as_uint(amax);
+  int e = (int)(bits >> 23) - 8 + ((bits & 0x007fffffu) > 0x00600000u ? 1 : 0);   // biased exponent of the scale
+  e = e < least ? least : e;
+  if (bits >= 0x7f800000u) e = 255;   // an infinity in the group: the scale byte is NaN
+  sc = __uint_as_float((uint32_t)e << 23);
+  inv = e == 255 ? 0.f : __uint_as_float((uint32_t)(254 - e) << 23);
+  return e;
+}
+// Codes of four values (the first one in the low byte); `residual`: leaves what they miss in v.
+__device__ __forceinline__ uint32_t mx_codes4(float* v, float sc, float inv, bool residual) {
+  uint32_t o[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    o[j] = f32x2_to_e4m3x2(fmaxf(__fmul_rn(v[2 * j], inv), -448.f),   // saturates; the maximum makes -448 of a NaN
+                           fmaxf(__fmul_rn(v[2 * j + 1], inv), -448.f));
+  if (residual) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float2 d = e4m3x2_to_f32x2(o[j]);
+      v[2 * j] = fmaf(-d.x, sc, v[2 * j]);
+      v[2 * j + 1] = fmaf(-d.y, sc, v[2 * j + 1]);
+    }
+  }
+  return o[0] | (o[1] << 16);
+}
 __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes, int least, bool residual) {
   float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
   amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-  const uint32_t bits = __float_as_uint(amax);
-  int e = (int)(bits >> 23) - 8 + ((bits & 0x007fffffu) > 0x00600000u ? 1 : 0);   // biased exponent of the scale
-  e = e < least ? least : e;
-  if (bits >= 0x7f800000u) e = 255;   // an infinity in the group: the scale byte is NaN
-  const float sc = __uint_as_float((uint32_t)e << 23), inv = e == 255 ? 0.f : __uint_as_float((uint32_t)(254 - e) << 23);
+  float sc, inv;
+  const int e = mx_scale(amax, least, sc, inv);
   // Instructions bound the quantisers (ALU pipe 69 %, DRAM 29 %): two values a conversion, one comparison a value,
   // no residual behind the last plane, and as code * scale is exact the residual is one fused operation.
   // 8192 x 2880 values with the launch: two planes 52 -> 42 us, one 33 -> 28.
-  uint32_t c[2];
-#pragma unroll
-  for (int i = 0; i < 8; i += 4) {
-    uint32_t o[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-      o[j] = f32x2_to_e4m3x2(fmaxf(__fmul_rn(v[i + 2 * j], inv), -448.f),   // saturates; the maximum makes -448 of a NaN
-                             fmaxf(__fmul_rn(v[i + 2 * j + 1], inv), -448.f));
-    c[i >> 2] = o[0] | (o[1] << 16);
-    if (residual) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        const float2 d = e4m3x2_to_f32x2(o[j]);
-        v[i + 2 * j] = fmaf(-d.x, sc, v[i + 2 * j]);
-        v[i + 2 * j + 1] = fmaf(-d.y, sc, v[i + 2 * j + 1]);
-      }
-    }
-  }
-  codes = make_uint2(c[0], c[1]);
+  codes.x = mx_codes4(v, sc, inv, residual);
+  codes.y = mx_codes4(v + 4, sc, inv, residual);
   const uint32_t byte = (active ? (uint32_t)e : 0x7fu) << (8 * ((threadIdx.x >> 2) & 3));
   uint32_t word = byte | __shfl_xor_sync(0xffffffffu, byte, 4);
   word |= __shfl_xor_sync(0xffffffffu, word, 8);

@@ -214,7 +214,7 @@ struct Experts {
   void lay_out_second(Layout& l) {
     const int64_t I = p.inter, I2 = o.form == kUnfused ? inter2() : I;
     const bool direct_fp8 = p.block_fp8 && (o.form == kFp8 || (p.act == kSilu && I % 128 == 0));
-    if (!direct_fp8 && !gated_quant()) act = l.take(M * I2 * 2);
+    if (!direct_fp8 && !gated_quant() && !planes_out()) act = l.take(M * I2 * 2);
     if (p.block_fp8) {
       act_q = l.take(M * I2);
       act_s = l.take(M * (I2 / 128) * 4);
@@ -225,6 +225,17 @@ struct Experts {
   }
   // SiLU, multiply and the planes of gemm2's input in one pass
   bool gated_quant() const { return planes_in && o.form == kUnfused && p.act == kSilu && p.inter % 32 == 0; }
+
+  // gemm1's SwigluOAI epilogue writes the planes of gemm2's input.  That saves a launch in the chain of a small decode
+  // step; with several tiles a CTA its epilogue warps take more time from the other roles than the quantiser's launch
+  // costs.  gpt-oss layer calls, quantiser / so, us: 1 token 39.3 / 37.0, 4 tokens 69.6 / 67.2, 16 tokens 155.7 / 154.4, 32
+  // tokens 232.8 / 233.7, 64 tokens 297.4 / 300.5, 512 tokens 427 / 457, 2048 tokens (calls in a row) 768 / 813.
+  // (Only token tiles of 16 have it, which experts with 8 rows or fewer on average take.)
+  static constexpr int64_t kPlanesOutRows = 64;
+  bool planes_out() const {
+    return planes_in && !sums && o.form == kEpilogue && p.act == kSwigluOai && p.inter % 32 == 0 &&
+           M <= std::min<int64_t>(kPlanesOutRows, 8 * p.experts);
+  }
 
   void gemm(bool first, const void* a, b200moe_dtype a_dtype, const void* a_scale, void* d, b200moe_dtype d_dtype,
             void* d_scale, const int32_t* rows, b200moe_epilogue epi) const {
@@ -260,6 +271,10 @@ struct Experts {
       gemm(true, a, a_dtype, a_scale, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, rows, B200MOE_EPI_SILU_MUL);
       mark(o, gil, "gemm1");
       fp8_ready = true;
+    } else if (planes_out()) {
+      gemm(true, a, a_dtype, a_scale, ws + act_q, mx_dtype, ws + act_s, rows, B200MOE_EPI_SWIGLUOAI);
+      mark(o, gil, "gemm1");
+      planes_ready = true;
     } else if (o.form == kEpilogue) {
       gemm(true, a, a_dtype, a_scale, ws + act, out, nullptr, rows,
            p.act == kSilu ? B200MOE_EPI_SILU_MUL : B200MOE_EPI_SWIGLUOAI);
