@@ -238,58 +238,72 @@ group_quant_fp8_scalar_kernel(const T* __restrict__ x, uint8_t* __restrict__ q,
 // (one block per row with a division per group and a byte store per scale ran at 1.9 TB/s:
 // 8192 x 2880 values in 50 us).
 constexpr int kMxQuantUnroll = 2;
-template <typename T, bool kGated>
+// Instructions bound it (issue slots 74 % in use with 292 of them a piece, most of them 64-bit products for the
+// addresses and a division a step): the planes are a template argument, a step's addresses follow from two pointers, and
+// row and step advance by additions.
+template <typename T, bool kGated, int kTerms, bool kSums>
 __global__ void __launch_bounds__(256)
-quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* __restrict__ s,
-                   int64_t rows, int cols, int terms, int sums) {
+quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* __restrict__ s, uint32_t rows, int cols) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
   const int nvec = cols / 8;
   const int num_kb = (cols + 127) / 128;
   const int pieces = (num_kb + 1) / 2;                        // 256-wide pieces of a row
-  const int steps = (pieces + kMxQuantUnroll - 1) / kMxQuantUnroll;
-  const int64_t total = rows * steps;
-  for (int64_t w = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); w < total; w += (int64_t)gridDim.x * 8) {
-    const int64_t r = total <= 0xffffffffll ? (int64_t)((uint32_t)w / (uint32_t)steps) : w / steps;
-    const int j0 = (int)(w - r * steps) * kMxQuantUnroll * 32 + lane;
-    const T* xr = x + r * (int64_t)cols * (kGated ? 2 : 1);
+  const uint32_t steps = (pieces + kMxQuantUnroll - 1) / kMxQuantUnroll;
+  const uint32_t warps = gridDim.x * 8, first = blockIdx.x * 8 + (threadIdx.x >> 5);
+  const uint32_t row_step = warps / steps, step_step = warps - row_step * steps;
+  const size_t q_plane = (size_t)rows * cols, s_plane = (size_t)rows * num_kb;
+  uint32_t r = first / steps, step = first - r * steps;
+  while (r < rows) {
+    const int j0 = step * (kMxQuantUnroll * 32) + lane;
+    const T* xr = x + (size_t)r * (cols * (kGated ? 2 : 1)) + j0 * 8;
+    uint8_t* qr = q + (size_t)r * cols + j0 * 8;
+    uint32_t* sr = s + (size_t)rows * (j0 >> 4) + r;
     vec16 in[kMxQuantUnroll], up[kGated ? kMxQuantUnroll : 1];
 #pragma unroll
     for (int u = 0; u < kMxQuantUnroll; ++u) {
       if (j0 + 32 * u < nvec) {
-        in[u] = ld16(xr + (int64_t)(j0 + 32 * u) * 8);
-        if (kGated) up[kGated ? u : 0] = ld16(xr + cols + (int64_t)(j0 + 32 * u) * 8);
+        in[u] = ld16(xr + 256 * u);
+        if (kGated) up[kGated ? u : 0] = ld16(xr + cols + 256 * u);
       }
     }
 #pragma unroll
     for (int u = 0; u < kMxQuantUnroll; ++u) {
       const int j = j0 + 32 * u;
+      const bool active = j < nvec, first_of_block = (j & 15) == 0 && j < num_kb * 16;
       const T* e = reinterpret_cast<const T*>(&in[u]);
       const T* ue = reinterpret_cast<const T*>(&up[kGated ? u : 0]);
       float v[8];
       float total = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
-        v[i] = j < nvec ? to_f32<T>(e[i]) : 0.f;
-        if (kGated && j < nvec)   // the two roundings of silu_and_mul
+        v[i] = active ? to_f32<T>(e[i]) : 0.f;
+        if (kGated && active)   // the two roundings of silu_and_mul
           v[i] = to_f32<T>(from_f32<T>(to_f32<T>(from_f32<T>(silu_f32(v[i]))) * to_f32<T>(ue[i])));
-        total += v[i];
+        if (kSums) total += v[i];
       }
-      for (int term = 0; term < terms; ++term) {
+      uint8_t* qu = qr + 256 * u;
+      uint32_t* su = sr + (size_t)(2 * u) * rows;
+#pragma unroll
+      for (int term = 0; term < kTerms; ++term) {
         uint2 codes;
-        const uint32_t word = mx_quant_lane(v, j < nvec, codes, sums ? kMxLeastExact : kMxLeast, sums || term + 1 < terms);
-        if (j < nvec) *reinterpret_cast<uint2*>(q + (term * rows + r) * cols + (int64_t)j * 8) = codes;
-        if ((j & 15) == 0 && j < num_kb * 16) s[((int64_t)term * num_kb + (j >> 4)) * rows + r] = word;
+        const uint32_t word = mx_quant_lane(v, active, codes, kSums ? kMxLeastExact : kMxLeast, kSums || term + 1 < kTerms);
+        if (active) *reinterpret_cast<uint2*>(qu) = codes;
+        if (first_of_block) *su = word;
+        qu += q_plane;
+        su += s_plane;
       }
-      if (sums) {
+      if (kSums) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) total -= v[i];
         total = mx_block_sum(total);
-        if ((j & 15) == 0 && j < num_kb * 16)
-          reinterpret_cast<float*>(s)[((int64_t)terms * num_kb + (j >> 4)) * rows + r] = total;
+        if (first_of_block) *reinterpret_cast<float*>(su) = total;
       }
     }
+    r += row_step;
+    step += step_step;
+    if (step >= steps) { step -= steps; ++r; }
   }
 }
 
@@ -513,15 +527,23 @@ extern "C" int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* 
   const int64_t blocks = (rows * steps + 7) / 8;
   const int64_t most = (int64_t)sm_count() * 8;
   const dim3 grid((unsigned)(blocks < most ? blocks : most));
-  auto run = [&](auto type, auto is_gated) {
+  auto run = [&](auto type, auto is_gated, auto planes, auto with_sums) {
     using T = decltype(type);
-    return launch_pdl(rows <= kEarlyLaunchRows, quant_mxfp8_kernel<T, decltype(is_gated)::value>, grid, dim3(256), 0,
-                      as_stream(stream), (const T*)x, (uint8_t*)q, (uint32_t*)s, rows, cols, terms, block_sums);
+    return launch_pdl(rows <= kEarlyLaunchRows,
+                      quant_mxfp8_kernel<T, decltype(is_gated)::value, decltype(planes)::value, decltype(with_sums)::value>, grid,
+                      dim3(256), 0, as_stream(stream), (const T*)x, (uint8_t*)q, (uint32_t*)s, (uint32_t)rows, cols);
   };
-  if (dtype == B200MOE_BF16)
-    B200_LAUNCHED("quant_mxfp8_kernel", gated ? run(__nv_bfloat16(), std::true_type()) : run(__nv_bfloat16(), std::false_type()));
-  else
-    B200_LAUNCHED("quant_mxfp8_kernel", gated ? run(__half(), std::true_type()) : run(__half(), std::false_type()));
+  auto of_planes = [&](auto type, auto is_gated, auto with_sums) {
+    return terms == 1 ? run(type, is_gated, std::integral_constant<int, 1>(), with_sums) :
+           terms == 2 ? run(type, is_gated, std::integral_constant<int, 2>(), with_sums) :
+                        run(type, is_gated, std::integral_constant<int, 3>(), with_sums);
+  };
+  auto of_form = [&](auto type) {
+    return gated ? (block_sums ? of_planes(type, std::true_type(), std::true_type()) : of_planes(type, std::true_type(), std::false_type())) :
+                   (block_sums ? of_planes(type, std::false_type(), std::true_type()) : of_planes(type, std::false_type(), std::false_type()));
+  };
+  if (dtype == B200MOE_BF16) B200_LAUNCHED("quant_mxfp8_kernel", of_form(__nv_bfloat16()));
+  else B200_LAUNCHED("quant_mxfp8_kernel", of_form(__half()));
   return B200MOE_OK;
 }
 

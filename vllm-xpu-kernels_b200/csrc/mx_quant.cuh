@@ -23,7 +23,7 @@ constexpr int kMxLeast = 127 - 33, kMxLeastExact = 127 - 100;
 // Biased exponent of a group's scale, the scale and its inverse.
 __device__ __forceinline__ int mx_scale(float amax, int least, float& sc, float& inv) {
   const uint32_t bits = __float_as_uint(amax);
-  int e = (int)(bits >> 23) - 8 + ((bits & 0x007fffffu) > 0x00600000u ? 1 : 0);   // biased exponent of the scale
+  int e = (int)((bits + 0x001fffffu) >> 23) - 8;   // biased exponent of the scale (carries beyond a significand of 1.75)
   e = e < least ? least : e;
   if (bits >= 0x7f800000u) e = 255;   // an infinity in the group: the scale byte is NaN
   sc = __uint_as_float((uint32_t)e << 23);
@@ -47,19 +47,49 @@ __device__ __forceinline__ uint32_t mx_codes4(float* v, float sc, float inv, boo
   }
   return o[0] | (o[1] << 16);
 }
+// The largest magnitude of three, a NaN if there is one (one instruction).
+__device__ __forceinline__ float max3_abs_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
 __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, uint2& codes, int least, bool residual) {
-  float amax = 0.f;
+  // Infinities and NaN are looked for once a warp instead of ordering every value for them.
+  float amax = max3_abs_nan(max3_abs_nan(v[0], v[1], v[2]), max3_abs_nan(v[3], v[4], v[5]), max3_abs_nan(v[6], v[7], 0.f));
+  const float o1 = __shfl_xor_sync(0xffffffffu, amax, 1), o2 = __shfl_xor_sync(0xffffffffu, amax, 2),
+              o3 = __shfl_xor_sync(0xffffffffu, amax, 3);
+  amax = max3_abs_nan(amax, o1, max3_abs_nan(o2, o3, 0.f));
+  const bool special = __any_sync(0xffffffffu, !(amax < INFINITY));
+  if (special) {
+    amax = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-  amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+  }
   float sc, inv;
   const int e = mx_scale(amax, least, sc, inv);
   // Instructions bound the quantisers (ALU pipe 69 %, DRAM 29 %): two values a conversion, one comparison a value,
   // no residual behind the last plane, and as code * scale is exact the residual is one fused operation.
   // 8192 x 2880 values with the launch: two planes 52 -> 42 us, one 33 -> 28.
-  codes.x = mx_codes4(v, sc, inv, residual);
-  codes.y = mx_codes4(v + 4, sc, inv, residual);
+  float x[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) x[i] = __fmul_rn(v[i], inv);
+  if (special) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = fmaxf(x[i], -448.f);   // makes -448 of a NaN
+  }
+  uint32_t o[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    o[j] = f32x2_to_e4m3x2(x[2 * j], x[2 * j + 1]);   // saturates
+    if (residual) {
+      const float2 d = e4m3x2_to_f32x2(o[j]);
+      v[2 * j] = fmaf(-d.x, sc, v[2 * j]);
+      v[2 * j + 1] = fmaf(-d.y, sc, v[2 * j + 1]);
+    }
+  }
+  codes = make_uint2(o[0] | (o[1] << 16), o[2] | (o[3] << 16));
   const uint32_t byte = (active ? (uint32_t)e : 0x7fu) << (8 * ((threadIdx.x >> 2) & 3));
   uint32_t word = byte | __shfl_xor_sync(0xffffffffu, byte, 4);
   word |= __shfl_xor_sync(0xffffffffu, word, 8);

@@ -116,11 +116,13 @@ __device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, 
   for (int p = 0; p < a.planes; ++p) {
     uint2 codes;
     const uint32_t word = mx_quant_lane(v, in, codes, a.sums ? kMxLeastExact : kMxLeast, a.sums || p + 1 < a.planes);
+    uint8_t* q = dst_q + p * a.rows * H + (int64_t)j * 8;
+    uint32_t* s = dst_s + ((int64_t)p * num_kb + (j >> 4)) * a.rows;
     for (int k = 0; k < a.K; ++k) {
       const int r = dest[k];
       if (r >= 0) {
-        if (in) *reinterpret_cast<uint2*>(dst_q + (p * a.rows + r) * H + (int64_t)j * 8) = codes;
-        if ((j & 15) == 0 && j < num_kb * 16) dst_s[((int64_t)p * num_kb + (j >> 4)) * a.rows + r] = word;
+        if (in) *reinterpret_cast<uint2*>(q + (int64_t)r * H) = codes;
+        if ((j & 15) == 0 && j < num_kb * 16) s[r] = word;
       }
     }
   }
