@@ -26,6 +26,8 @@
 // Every wait on an mbarrier is bounded (see sm100_ptx.cuh): on expiry the CTA
 // raises an abort flag, all roles leave their loops, tensor memory is freed and
 // *status is set to 1.
+#include <algorithm>
+
 #include "common.cuh"
 #include "sm100_ptx.cuh"
 #include "gemm_tc_common.cuh"
@@ -37,6 +39,7 @@ namespace {
 
 constexpr int kWTileBytes = 16384;  // 128 rows x 128 bytes, or the same area K-by-N
 constexpr int kMaxAccStages = 8;
+constexpr int kTwoSetsAccStages = 32;   // the same with two sets of epilogue warps: all of tensor memory for 16 tokens
 constexpr int kMaxStages = 11;
 
 struct TcParams {
@@ -59,16 +62,16 @@ struct TcParams {
   float alpha, limit;
 };
 
-template <int BT, bool kFp8>
+template <int BT, bool kFp8, int kSets = 1>
 struct Ctrl {
   uint64_t full[kMaxStages];
   uint64_t empty[kMaxStages];
-  uint64_t acc_full[kMaxAccStages];
-  uint64_t acc_empty[kMaxAccStages];
+  uint64_t acc_full[kSets == 2 ? kTwoSetsAccStages : kMaxAccStages];
+  uint64_t acc_empty[kSets == 2 ? kTwoSetsAccStages : kMaxAccStages];
   uint32_t tmem_base;
   int abort_flag;
-  alignas(16) float sc[kFp8 ? 4 : 1][2][kFp8 ? BT : 4];  // per epilogue warp, double buffered
-  alignas(16) uint16_t xpose[4][32 * 32];  // per epilogue warp: output transpose tile
+  alignas(16) float sc[kFp8 ? 4 * kSets : 1][2][kFp8 ? BT : 4];  // per epilogue warp, double buffered
+  alignas(16) uint16_t xpose[4 * kSets][32 * 32];  // per epilogue warp: output transpose tile
   alignas(16) uint8_t walk[tile_walk_bytes(kMaxExperts)];
 };
 
@@ -83,44 +86,58 @@ __host__ __device__ constexpr int num_stages() {
   return (200 * 1024) / stage_bytes<BT, kGated>() > kMaxStages ? kMaxStages
                                                                 : (200 * 1024) / stage_bytes<BT, kGated>();
 }
-template <int BT, bool kFp8, bool kGated = false>
+template <int BT, bool kFp8, bool kGated = false, int kSets = 1>
 __host__ __device__ constexpr size_t smem_bytes() {
-  return 1024 + (size_t)num_stages<BT, kGated>() * stage_bytes<BT, kGated>() + sizeof(Ctrl<BT, kFp8>);
+  return 1024 + (size_t)num_stages<BT, kGated>() * stage_bytes<BT, kGated>() + sizeof(Ctrl<BT, kFp8, kSets>);
 }
 // Accumulator stages in tensor memory.  16-bit inputs hand over one whole tile
 // per stage (two are enough); fp8 hands over every 128-wide K block, so more
 // stages let the MMA issuer run ahead of the promoting epilogue warps.
-template <int BT, bool kFp8>
+template <int BT, bool kFp8, int kSets = 1>
 __host__ __device__ constexpr int acc_stages() {
-  return !kFp8 ? 2 : (512 / BT > kMaxAccStages ? kMaxAccStages : 512 / BT);
+  return kSets == 2 ? kTwoSetsAccStages : !kFp8 ? 2 : (512 / BT > kMaxAccStages ? kMaxAccStages : 512 / BT);
 }
-template <int BT, bool kFp8, bool kGated = false>
+template <int BT, bool kFp8, bool kGated = false, int kSets = 1>
 __host__ __device__ constexpr uint32_t tmem_cols() {
-  const int c = acc_stages<BT, kFp8>() * BT * (kGated ? 2 : 1);
+  const int c = acc_stages<BT, kFp8, kSets>() * BT * (kGated ? 2 : 1);
   return c <= 32 ? 32u : c <= 64 ? 64u : c <= 128 ? 128u : c <= 256 ? 256u : 512u;
 }
 // Four epilogue warps cover the 128 TMEM lanes.
 constexpr int kEpiWarps = 4;
 constexpr int kTcThreads = 64 + 32 * kEpiWarps;
+// Two sets of epilogue warps that take tiles in turn (kSets == 2): an fp8 tile's promotion, stores and change of
+// tile, one after the other in the same warps, take longer than its bytes when its K loop is short (a K block of 16 KB
+// has 670 cycles at the copy rate; 1090 were measured with six blocks a tile).  While one set stores a tile the other one
+// adds up the next.  A set waits for an accumulator's n-th completion by parity, so it must have seen the one before
+// complete: that block, one round of the stages back, has to be no later than the last block of the set's tile
+// before, which is num_kb + 1 blocks back (blocks complete in order).  So the K loop is shorter than the round of
+// stages.  Layer calls, one set / two with 8 stages (K up to 7 blocks: gemm2 alone) / two with 32, us: qwen3 at 2
+// tokens 39.8 / 39.4 / 36.8, 4 tokens 51.4 / 50.4 / 46.3, 16 tokens 95.4 / 89.0 / 86.0, 96 tokens 137.0 / 127.9 / 125.2;
+// one DeepSeek token 86.6 / 86.7 / 83.1, 64 tokens 922 / 923 / 919.  (One set is slower with 32 stages than with 8: 4
+// DeepSeek tokens 219.8 / 225.0, 16 tokens 538.7 / 545.)  With a tile a CTA at most there is nothing to
+// take in turn, and the larger block costs: one qwen3 token 26.5 / 27.5, so such calls have one set.
+constexpr int kTwoSetsMaxKb = kTwoSetsAccStages - 1;
 
-template <int BT, bool kFp8, bool kWKn, bool kGated = false>
-__global__ void __launch_bounds__(kTcThreads, 1)
+template <int BT, bool kFp8, bool kWKn, bool kGated = false, int kSets = 1>
+__global__ void __launch_bounds__(kTcThreads + 32 * kEpiWarps * (kSets - 1), 1)
 grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
                        const __grid_constant__ CUtensorMap tmap_w, const TcParams p) {
   static_assert(!kFp8 || BT <= 64, "fp8 promotion keeps BT accumulators per thread");
+  static_assert(kSets == 1 || (kSets == 2 && kFp8 && BT * kTwoSetsAccStages <= 512), "tiles in turn: fp8, stages within tensor memory");
   static_assert(!kGated || (!kFp8 && BT <= 128), "gated epilogue: 16-bit inputs, two accumulators of BT columns per stage");
   constexpr int kStages = num_stages<BT, kGated>();
   constexpr int kStageBytes = stage_bytes<BT, kGated>();
   constexpr int kAOff = (kGated ? 2 : 1) * kWTileBytes;   // activations follow the weight tile(s) in a stage
   constexpr int kAccCols = BT * (kGated ? 2 : 1);         // tensor-memory columns of one accumulator stage
   constexpr int kElemsPerKb = kFp8 ? 128 : 64;  // K elements per 128-byte row
-  constexpr int kAccStages = acc_stages<BT, kFp8>();
+  constexpr int kAccStages = acc_stages<BT, kFp8, kSets>();
   constexpr int kCols = BT;                      // token columns one epilogue warp owns
   constexpr int kChunk = kCols >= 32 ? 32 : 16;  // columns per tcgen05.ld
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  Ctrl<BT, kFp8>* ctrl = reinterpret_cast<Ctrl<BT, kFp8>*>(smem + kStages * kStageBytes);
+  using Control = Ctrl<BT, kFp8, kSets>;
+  Control* ctrl = reinterpret_cast<Control*>(smem + kStages * kStageBytes);
   volatile int* abort_flag = &ctrl->abort_flag;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -142,7 +159,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
       ptx::prefetch_tensormap(&tmap_w);
     }
   } else if (warp == 1) {
-    ptx::tmem_alloc(&ctrl->tmem_base, tmem_cols<BT, kFp8, kGated>());
+    ptx::tmem_alloc(&ctrl->tmem_base, tmem_cols<BT, kFp8, kGated, kSets>());
     ptx::tmem_relinquish();
   } else if (warp == 2 && lane == 0) {
     for (int s = 0; s < kStages; ++s) {
@@ -290,10 +307,11 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
         }
       }
     };
-    uint32_t acc_it = 0;
+    const int set = kSets == 1 ? 0 : (warp - 2) / kEpiWarps;   // this warp's tiles: every kSets-th
+    uint32_t acc_it = set * p.num_kb;
     int cursor = 0;
     bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+    for (int t = blockIdx.x + set * gridDim.x; t < total_tiles && ok; t += kSets * gridDim.x) {
       TileInfo ti;
       locate_tile<BT>(walk, t, cursor, ti, p.w_experts);
       const int feat = ti.n_tile * kFeat + et;
@@ -379,10 +397,10 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
         for (int g = 0; g < n_groups && ok; ++g) {
           if (g + 1 < n_groups) {
             fetch_group(ti, g + 1, pre);
-          } else if (t + (int)gridDim.x < total_tiles) {
+          } else if (t + kSets * (int)gridDim.x < total_tiles) {
             int cursor2 = cursor;
             TileInfo tn;
-            locate_tile<BT>(walk, t + gridDim.x, cursor2, tn, p.w_experts);
+            locate_tile<BT>(walk, t + kSets * gridDim.x, cursor2, tn, p.w_experts);
             fetch_group(tn, 0, pre);
             pre_valid = true;
           }
@@ -442,6 +460,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
             }
           }
         }
+        acc_it += (kSets - 1) * p.num_kb;   // the other set's blocks
       }
     }
   }
@@ -453,19 +472,20 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
   if (warp == 1) {
     ptx::tc_fence_after();
     if (*abort_flag != 0) __nanosleep(20000);  // let copies still in flight land
-    ptx::tmem_dealloc(tmem_base, tmem_cols<BT, kFp8, kGated>());
+    ptx::tmem_dealloc(tmem_base, tmem_cols<BT, kFp8, kGated, kSets>());
   }
   if (tid == 0 && *abort_flag != 0) report_timeout(p.status);
 }
 
-template <int BT, bool kFp8, bool kWKn, bool kGated = false>
+template <int BT, bool kFp8, bool kWKn, bool kGated = false, int kSets = 1>
 int launch_tc(const CUtensorMap& ta, const CUtensorMap& tw, const TcParams& p, int grid,
               cudaStream_t st) {
-  auto kern = grouped_gemm_tc_kernel<BT, kFp8, kWKn, kGated>;
-  static_assert(smem_bytes<BT, kFp8, kGated>() <= kMaxSmem, "shared memory");
+  auto kern = grouped_gemm_tc_kernel<BT, kFp8, kWKn, kGated, kSets>;
+  constexpr size_t kSmem = smem_bytes<BT, kFp8, kGated, kSets>();
+  static_assert(kSmem <= kMaxSmem, "shared memory");
   static SmemConfig configured;
   if (int rc = configured.ensure(kern)) return rc;
-  B200_LAUNCHED("grouped_gemm_tc_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kTcThreads), smem_bytes<BT, kFp8, kGated>(), st, ta, tw, p));
+  B200_LAUNCHED("grouped_gemm_tc_kernel", launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kTcThreads + 32 * kEpiWarps * (kSets - 1)), kSmem, st, ta, tw, p));
   return B200MOE_OK;
 }
 
@@ -914,6 +934,8 @@ int grouped_gemm_tc(const b200moe_gemm_args* a, cudaStream_t st) {
   if (grid < 1) grid = 1;
 
   if (a_fp8 && bt == 64) return kn ? launch_tc<64, true, true>(ta, tw, p, grid, st) : launch_tc<64, true, false>(ta, tw, p, grid, st);
+  if (a_fp8 && p.num_kb <= kTwoSetsMaxKb && std::min<int64_t>(a->m, a->num_experts) * p.n_tiles > grid)
+    return kn ? launch_tc<16, true, true, false, 2>(ta, tw, p, grid, st) : launch_tc<16, true, false, false, 2>(ta, tw, p, grid, st);
   if (a_fp8) return kn ? launch_tc<16, true, true>(ta, tw, p, grid, st) : launch_tc<16, true, false>(ta, tw, p, grid, st);
 #define B200_TC_CASE(BT_)                                                         \
   if (bt == BT_) {                                                                \
