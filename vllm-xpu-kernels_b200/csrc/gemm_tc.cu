@@ -199,7 +199,7 @@ grouped_gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int n0 = ti.n_tile * kFeat;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           const uint32_t full = full0 + 8 * s;
-          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::mbar_expect_tx_s(full, kStageBytes);
           const int k0 = kb * kElemsPerKb;
 #pragma unroll
@@ -596,7 +596,7 @@ grouped_gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int n0 = kGated ? (cta == 0 ? 0 : (p.n >> 1)) + ti.n_tile * kFeat : (ti.n_tile * 2 + (int)cta) * kFeat;
         const int row = ti.row0 + (int)cta * 128;
         for (int kb = 0; kb < p.num_kb; ++kb) {
-          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           if (cta == 0) ptx::mbar_expect_tx_s(full0 + 8 * s, 2 * kPairStageBytes);
           const uint32_t bar = bar0 + 8 * s;
           const int k0 = kb * 64;

@@ -238,7 +238,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const uint32_t bytes = (BT > kUnit && !second) ? kPieces * kUnit * 128 : S::kTokBytes;
         for (int hb = 0; hb < p.num_kb * kHalves; ++hb) {
           const uint32_t full = tok_full0 + 8 * s;
-          if (!ptx::mbar_wait_s(tok_empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(tok_empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::mbar_expect_tx_s(full, bytes);
 #pragma unroll
           for (int j = 0; j < kPieces; ++j)
@@ -264,7 +264,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int n0 = ti.n_tile * kFeat;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           const uint32_t full = raw_full0 + 8 * s;
-          if (!ptx::mbar_wait_s(raw_empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(raw_empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::mbar_expect_tx_s(full, kDqRawBytes);
           ptx::tma_load_3d_s(st, &tmap_w, full, kb * 64, n0, ti.e);
           st += kDqRawBytes;
@@ -379,7 +379,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
       kb += kSets;
       settle();
       if (t < total_tiles) nxt = load_scales();
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(raw_full0 + 8 * s, ph, abort_flag))) break;
+      if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(raw_full0 + 8 * s, ph, abort_flag))) break;
       const uint32_t src = src0 + s * kDqRawBytes;
       uint4 raw[4];
 #pragma unroll
@@ -402,7 +402,7 @@ grouped_gemm_dq_kernel(const __grid_constant__ CUtensorMap tmap_a,
           if (lane == 0) ptx::mbar_arrive_s(raw_empty0 + 8 * s);   // the block is in registers
         }
         if (h == 0 || kHalves == 2) {
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(slot_empty0 + 8 * c, cph, abort_flag))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(slot_empty0 + 8 * c, cph, abort_flag))) { ok = false; break; }
           ptx::tc_fence_after();
         }
         ptx::tmem_st_32x32(slot_base + c * S::kSlotCols + (kHalves == 1 ? h * 32 : 0), o);

@@ -131,7 +131,7 @@ grouped_gemm_fp8t_kernel(const __grid_constant__ CUtensorMap tmap_a,
         const int n0 = ti.n_tile * kFeat;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           const uint32_t full = full0 + 8 * s;
-          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::mbar_expect_tx_s(full, kTStageBytes);
           if (!kWKn) ptx::tma_load_3d_s(st, &tmap_w, full, kb * 128, n0, ti.e);
           else ptx::tma_load_3d_s(st, &tmap_w, full, n0, kb * 128, ti.e);
@@ -473,7 +473,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ T2TokenMaps tmap_a,
         const int quarters = (ti.valid + 31) >> 5;
         for (int kb = 0; kb < p.num_kb; ++kb) {
           const uint32_t full = full0 + 8 * s;
-          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           ptx::mbar_expect_tx_s(full, kT2StageBytes);
           // two 128-feature blocks (the second one is zero-filled past N)
           if (!kWKn) {
@@ -500,9 +500,9 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ T2TokenMaps tmap_a,
       const uint32_t idesc = (p.idesc & ~(0x3fu << 17)) | ((256u >> 3) << 17);
       for (uint32_t i = 0; i < blocks; ++i) {
         // (the block's scales: acc_full stands for them too)
-        if (i % kTGroup == 0 && !ptx::mbar_wait_s(sf_full0 + 8 * ((i >> 2) & 1), (i >> 3) & 1, abort_flag)) break;
-        if (!ptx::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) break;
-        if (!ptx::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) break;
+        if (i % kTGroup == 0 && !ptx::paced::mbar_wait_s(sf_full0 + 8 * ((i >> 2) & 1), (i >> 3) & 1, abort_flag)) break;
+        if (!ptx::paced::mbar_wait_s(full0 + 8 * s, ph, abort_flag)) break;
+        if (!ptx::paced::mbar_wait_s(acc_empty0 + 8 * a, aph, abort_flag)) break;
         // tcgen05.commit completes the MMAs and orders nothing else: scales and tile, written by the preparers,
         // reach the promotion warps through this arrival (acquired above, released here)
         ptx::mbar_arrive_s(acc_full0 + 8 * a);
@@ -559,7 +559,7 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ T2TokenMaps tmap_a,
           }
           if (in) ++kb;
         }
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, ((b / (kTGroup * kT2Slots)) & 1) ^ 1, abort_flag))) break;
+        if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(sf_empty0 + 8 * slot, ((b / (kTGroup * kT2Slots)) & 1) ^ 1, abort_flag))) break;
         T2Slot* out = &ctrl->slot[slot];
 #pragma unroll
         for (int j = 0; j < kTGroup; ++j) {

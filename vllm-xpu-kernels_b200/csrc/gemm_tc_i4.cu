@@ -189,7 +189,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           const int n0 = ti.n_tile * kFeat;
           for (int kb = 0; kb < p.num_kb; ++kb) {
             const uint32_t full = full0 + 8 * s;
-            if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+            if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
             ptx::mbar_expect_tx_s(full, kStageBytes);
             ptx::tma_load_3d_s(st, &tmap_w, full, kb * 64, n0, ti.e);
             ptx::tma_load_3d_s(st + kI4RawBytes, &tmap_a, full, kb * 128, ti.row0, 0);   // all planes
@@ -278,7 +278,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
             m[i] = (kb < p.num_kb && tok < ti.valid)
                        ? -8.0f * __ldg(sums + (int64_t)kb * p.m + ti.row0 + tok) : 0.f;
           }
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(sf_empty0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(sf_empty0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
           const uint32_t ring = ptx::smem_u32(sf_ring) + slot * kSlotBytes;
   #pragma unroll
           for (int i = 0; i < kPer; ++i) {
@@ -307,7 +307,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     uint32_t s = set, ph = 0, c = set, cph = 0;
     const uint32_t blocks = (uint32_t)my_tiles * p.num_kb;      // every tile: the same K loop
     for (uint32_t i = set; i < blocks; i += kI4Sets) {
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(full0 + 8 * s, ph, abort_flag))) break;
+      if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(full0 + 8 * s, ph, abort_flag))) break;
       const uint32_t src = src0 + s * kStageBytes;
       uint32_t o[32];
 #pragma unroll
@@ -325,7 +325,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_s(empty0 + 8 * s);
       // the operand columns are free when the MMAs of the slot's block before are complete: its accumulator is full
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait_inline_s(acc_full0 + 8 * c, cph ^ 1, abort_flag))) break;
+      if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(acc_full0 + 8 * c, cph ^ 1, abort_flag))) break;
       ptx::tc_fence_after();
       ptx::tmem_st_32x32(tmem_base + S::kConvBase + c * 32 + lane_sel, o);
       ptx::tmem_wait_st();

@@ -307,7 +307,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
         locate_tile<BT>(walk, t, cursor, ti);
         const int n0 = ti.n_tile * kFeat;
         for (int kb0 = 0; kb0 < p.num_kb; kb0 += kSub) {
-          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           const uint32_t full = full0 + 8 * s;
           ptx::mbar_expect_tx_s(full, max(0, min(kSub, whole_kb - kb0)) * kWTx);
 #pragma unroll
@@ -341,7 +341,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
         const CUtensorMap* tok_map = &tmap_a.rows[BT == 16 ? 0 : (ti.valid - 1) >> 4];
         const int tok_bytes = BT == 16 ? kABytes : ((ti.valid + 15) & ~15) * (kTerms * 128);
         for (int kb0 = 0; kb0 < p.num_kb; kb0 += kSub) {
-          if (!ptx::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
+          if (!ptx::paced::mbar_wait_s(empty0 + 8 * s, ph, abort_flag)) { ok = false; break; }
           const uint32_t full = full0 + 8 * s;
           ptx::mbar_expect_tx_s(full, min(kSub, p.num_kb - kb0) * tok_bytes);
 #pragma unroll
@@ -557,7 +557,7 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
           }
         }
         // the ring slot's previous group has been copied to tensor memory
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&ctrl->sf_empty[slot], slot_ph ^ 1, abort_flag))) {
+        if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(ptx::smem_u32(&ctrl->sf_empty[slot]), slot_ph ^ 1, abort_flag))) {
           *abort_flag = 1;
           return false;
         }
