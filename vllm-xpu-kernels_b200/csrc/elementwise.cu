@@ -289,7 +289,7 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
       for (int term = 0; term < kTerms; ++term) {
         uint2 codes;
         const uint32_t word = mx_quant_lane(v, active, codes, kSums ? kMxLeastExact : kMxLeast, kSums || term + 1 < kTerms);
-        if (active) *reinterpret_cast<uint2*>(qu) = codes;
+        if (active) *reinterpret_cast<uint2*>(qu) = kSums ? mx_evens_first(codes) : codes;
         if (first_of_block) *su = word;
         qu += q_plane;
         su += s_plane;

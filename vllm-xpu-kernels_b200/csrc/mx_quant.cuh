@@ -96,6 +96,12 @@ __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, ui
   return word;
 }
 
+// An int4 layer's codes, eight at a time: the even ones, then the odd ones (the order in which its GEMM unpacks the
+// nibbles of a word; the sum over k does not mind).
+__device__ __forceinline__ uint2 mx_evens_first(uint2 c) {
+  return make_uint2(__byte_perm(c.x, c.y, 0x6420), __byte_perm(c.x, c.y, 0x7531));
+}
+
 // Sum of a 128-wide block over its sixteen lanes: what the int4 GEMM needs to take its weights' zero
 // point out (x: the lane's values less what the planes left over).
 __device__ __forceinline__ float mx_block_sum(float x) {
