@@ -376,9 +376,9 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         }
         return r;
       };
-      float acc[kHalf];
+      float2 acc[kHalf / 2];
 #pragma unroll
-      for (int i = 0; i < kHalf; ++i) acc[i] = 0.f;
+      for (int i = 0; i < kHalf / 2; ++i) acc[i] = make_float2(0.f, 0.f);
       uint2 nxt = scales_of(0);
       for (int kb0 = 0; kb0 < p.num_kb && ok; kb0 += kI4Group) {
         const uint2 cur = nxt;
@@ -414,10 +414,8 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 #pragma unroll
             for (int i = 0; i < kHalf; i += 4) {
               const float4 m = ptx::lds128f(sums + (u * BT + i) * 4);   // -8 * the block's sum of the token
-              acc[i + 0] = fmaf(__uint_as_float(v[i + 0]) + m.x, sc[u], acc[i + 0]);
-              acc[i + 1] = fmaf(__uint_as_float(v[i + 1]) + m.y, sc[u], acc[i + 1]);
-              acc[i + 2] = fmaf(__uint_as_float(v[i + 2]) + m.z, sc[u], acc[i + 2]);
-              acc[i + 3] = fmaf(__uint_as_float(v[i + 3]) + m.w, sc[u], acc[i + 3]);
+              ptx::add_fma_f32x2(acc[i / 2], v[i], v[i + 1], m.x, m.y, sc[u]);
+              ptx::add_fma_f32x2(acc[i / 2 + 1], v[i + 2], v[i + 3], m.z, m.w, sc[u]);
             }
           }
         }
@@ -434,7 +432,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           if (col0 + c0 < ti.valid) {
             float vals[kChunk];
 #pragma unroll
-            for (int i = 0; i < kChunk; ++i) vals[i] = acc[c0 + i] + bias_v;
+            for (int i = 0; i < kChunk; ++i) vals[i] = ((i & 1) ? acc[(c0 + i) / 2].y : acc[(c0 + i) / 2].x) + bias_v;
             store_block_transposed<kChunk, 32>(ctrl->xpose[warp - 16], vals, p.d, p.out_f16, (int64_t)ti.row0 + col0 + c0,
                                                ti.valid - col0 - c0, p.m, p.n, ti.n_tile * kFeat + q * 32, lane);
           }

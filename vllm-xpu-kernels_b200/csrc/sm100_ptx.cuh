@@ -612,6 +612,13 @@ __device__ __forceinline__ void fma_f32x2(float2* acc, const uint32_t (&v)[32], 
         : "+f"(acc[i].x), "+f"(acc[i].y)
         : "r"(v[2 * i]), "r"(v[2 * i + 1]), "f"(s));
 }
+// acc += (v + m) * s for two values at once, each rounded as an addition and an fmaf round it.
+__device__ __forceinline__ void add_fma_f32x2(float2& acc, uint32_t v0, uint32_t v1, float m0, float m1, float s) {
+  asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tadd.rn.f32x2 a, a, b;\n\t"
+      "mov.b64 b, {%6, %6};\n\tmov.b64 c, {%0, %1};\n\tfma.rn.f32x2 c, a, b, c;\n\tmov.b64 {%0, %1}, c;\n\t}"
+      : "+f"(acc.x), "+f"(acc.y)
+      : "r"(v0), "r"(v1), "f"(m0), "f"(m1), "f"(s));
+}
 // umma_block's four kind::f16 instructions with the 128-row operand in tensor memory (eight columns per
 // K step, the other operand 32 bytes).
 __device__ __forceinline__ void umma_f16_block_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
