@@ -520,9 +520,13 @@ int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
   p.out_f16 = a->d_dtype == B200MOE_F16;
   const int64_t in_use = (a->rows_hint > 0 && a->rows_hint < a->m) ? a->rows_hint : a->m;
   const int64_t avg = (in_use + a->num_experts - 1) / a->num_experts;
-  // (both the MMA and the promotion cost grow with the tile: it is what the average expert fills)
-  if (planes == 2) return avg <= 8 ? launch_i4<16, 2>(a, p, st) : launch_i4<32, 2>(a, p, st);
-  return avg <= 8 ? launch_i4<16, 3>(a, p, st) : launch_i4<32, 3>(a, p, st);
+  // Both the MMA and the promotion cost grow with the tile; experts with more rows than the tile stream their weights
+  // once more, from L2.  Layer calls of 8 experts of 4096 x 14336, 2 a token, six routings (skewed), tiles of 16 / 32, us:
+  // bfloat16 8.3 rows an expert 207 / 218, 10 rows 220 / 222, 10.3 rows 222 / 221, 11 rows 230 / 223, 12 rows 247 / 226; float16
+  // (three planes, whose wide tile leaves the ring 9 stages) 8.3 rows 222 / 274, 10 rows 236 / 277, 12 rows 266 / 278, 13
+  // rows 274 / 280, 14 rows 289 / 287.
+  if (planes == 2) return avg <= 10 ? launch_i4<16, 2>(a, p, st) : launch_i4<32, 2>(a, p, st);
+  return avg <= 13 ? launch_i4<16, 3>(a, p, st) : launch_i4<32, 3>(a, p, st);
 }
 
 }  // namespace b200moe

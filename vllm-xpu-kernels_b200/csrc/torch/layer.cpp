@@ -35,9 +35,9 @@ struct Plan {
   // streams the weights faster than the one that expands them to 16 bits (gemm_tc_dq.cu), until experts
   // need a second of its tiles of 32 tokens.  A layer of 8 experts of 4096 x 14336, 2 a token, with routing as it
   // comes, this / that kernel, us: bfloat16 218 / 305 at 8 rows an expert, 235 / 289 at 12, 249 / 293 at 16, 292 / 297 at
-  // 20, 295 / 298 at 24; float16 (three planes) 241 / 304 at 8, 298 / 287 at 10, 300 / 288 at 12, 317 / 292 at 16, 365 / 295
-  // at 20.  Half a tile leaves room for uneven routing.  float16 keeps the same line although it costs 4 to 8 % from
-  // 10 rows on, because the planes are the more accurate: error of the layer's output against 64 bits (2-norm, 9 to
+  // 20, 295 / 298 at 24 (since then the first one 207 at 8, 226 at 12, 238 at 16); float16 (three planes) 222 / 304 at 8, 236 /
+  // 287 at 10, 266 / 288 at 12, 292 / 292 at 16, 365 / 295 at 20.  Half a tile leaves room for uneven routing, and the
+  // planes are the more accurate: error of the layer's output against 64 bits (2-norm, 9 to
   // 16 rows an expert) 5.3e-4 / 6.1e-4, where the other kernel rounds a weight after its scale; bfloat16 4.3e-3 / 4.9e-3.
   static constexpr int64_t kI4PlaneRows = 16;
 };
