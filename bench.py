@@ -384,15 +384,15 @@ def time_gemms(cfg, layer, ids, T, dev, iters, ep_world=1, ep_rank=0):
 
 def launches_per_step(cfg, T, layer, ep_world, transport) -> int:
     """Kernels of this repository launched by one step, counted from the code path taken:
-    routing 1; sort 3 and row copy (+quant) 1, or one kernel for both (<= 2048 slots, top-k <= 8);
-    gemm1 1; activation (+quant) 1 unless fused into gemm1; MX quantiser of gemm2's input 1; gemm2 1;
-    gather 1.  Expert parallelism
+    routing 1; sort 1 (3 beyond 65536 slots or 360 experts) and row copy (+quant) 1, or one kernel for both (<= 2048
+    slots, top-k <= 8); gemm1 1; activation (+quant) 1 unless fused into gemm1; MX quantiser of gemm2's input 1 unless
+    gemm1 writes the planes (<= 64 routed rows, 8 an expert); gemm2 1; gather 1.  Expert parallelism
     over peer memory: routing 1, dispatch sort 1|3 + dispatch 1, mask 1, the local layer without
     its gather, combine 1, final gather 1."""
     local = layer.local if ep_world > 1 else layer
     act = 0 if local.fuses_activation(T * cfg.K) else 1
-    mx = 1 if getattr(local, "mx_acts", False) else 0
-    sort = lambda slots: 1 if slots <= 2048 else 3
+    mx = 1 if getattr(local, "mx_acts", False) and T * cfg.K > min(64, 8 * cfg.E) else 0
+    sort = lambda slots: 1 if slots <= 2048 or (slots <= 65536 and cfg.E <= 360) else 3
     place = lambda slots: 1 if slots <= 2048 and cfg.K <= 8 else sort(slots) + 1
     if ep_world == 1:
         return 1 + place(T * cfg.K) + 1 + act + mx + 1 + 1

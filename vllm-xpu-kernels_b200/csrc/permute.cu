@@ -9,10 +9,9 @@
 //   3. rank  : every warp walks its chunk 32 slots at a time; the rank of a
 //              slot among equal ids in the same step comes from
 //              __match_any_sync, so slots of one expert keep ascending order.
-// Up to 2048 slots all three steps run in one block without any scratch;
-// beyond that they are three launches that exchange the histograms through a
-// caller-provided workspace.  The result is deterministic: no atomics decide
-// an order.
+// Up to 2048 slots all three steps run in one block without any scratch; beyond
+// that in one cluster of blocks (row maps) or in three launches (sort.cuh).  The
+// result is deterministic: no atomics decide an order.
 //
 // Semantics follow csrc/moe/moe_align_sum_kernels.cpp:135-273, 1034-1181 and
 // csrc/moe/remap_hidden_states.cpp:42-116, 181-330 of vllm-xpu-kernels, which

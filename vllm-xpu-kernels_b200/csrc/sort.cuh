@@ -9,9 +9,9 @@
 //   3. rank  : every warp walks its chunk 32 slots at a time; the rank of a
 //              slot among equal ids in the same step comes from
 //              __match_any_sync, so slots of one bucket keep ascending order.
-// Up to 2048 slots all three steps run in one block without any scratch;
-// beyond that they are three launches that exchange the histograms through a
-// caller-provided workspace.  The result is deterministic: no atomics decide
+// Up to 2048 slots all three steps run in one block without any scratch.  Beyond that row maps of up to 65536
+// slots and 360 buckets are made by one cluster of blocks (below), all others by three launches that exchange the
+// histograms through a caller-provided workspace.  The result is deterministic: no atomics decide
 // an order.
 #pragma once
 
@@ -565,6 +565,27 @@ sort_rank_kernel(SortParams p, int n_chunks, const int* counts, const int* sizes
   });
 }
 
+// Whether the current device runs such a cluster (a partition with few SMs per GPC may not), asked once per device.
+inline bool cluster_sort_runs() {
+  static std::atomic<int> clusters[kMaxDevices];   // 0: not asked yet
+  const int dev = current_device();
+  int n = clusters[dev].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kClusterCtas); cfg.blockDim = dim3(kClusterThreads); cfg.dynamicSmemBytes = kClusterSmem;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kClusterCtas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, sort_cluster_kernel, &cfg) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      n = -1;
+    }
+    clusters[dev].store(n, std::memory_order_relaxed);
+  }
+  return n > 0;
+}
+
 template <int kMode>
 int run_sort(const SortParams& p, const AlignOut& ao, const RemapOut& ro,
              void* workspace, size_t workspace_bytes, cudaStream_t st) {
@@ -580,7 +601,7 @@ int run_sort(const SortParams& p, const AlignOut& ao, const RemapOut& ro,
   if (workspace == nullptr || workspace_bytes < need)
     return fail(B200MOE_E_WORKSPACE, "workspace of %zu bytes needed, got %zu", need,
                 workspace_bytes);
-  if (kMode == 1 && p.numel <= kClusterSlots && cluster_sort_smem(nb) <= kClusterSmem) {
+  if (kMode == 1 && p.numel <= kClusterSlots && cluster_sort_smem(nb) <= kClusterSmem && cluster_sort_runs()) {
     const int steps = (int)((p.numel + kClusterCtas * kClusterThreads - 1) / (kClusterCtas * kClusterThreads));
     B200_LAUNCHED("sort_cluster_kernel", launch_pdl(p.numel <= kEarlyLaunchRows, sort_cluster_kernel, dim3(kClusterCtas),
         dim3(kClusterThreads), cluster_sort_smem(nb), st, p, steps, ro));
