@@ -41,3 +41,27 @@ def test_positions_are_those_of_a_stable_sort(native, T, K, E, masked, ids_dtype
     assert torch.equal(row_map.cpu().flatten(), want)
     assert torch.equal(rows.cpu().long(), torch.bincount(bucket[live], minlength=E))
     assert torch.equal(out[:order.numel()].cpu(), x.cpu()[order // K])
+
+
+def test_captured_and_replayed_with_other_ids(native):
+    T, K, E, H = 1024, 8, 64, 16
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(T, H, generator=g).to(torch.bfloat16).to(DEV)
+    ids = torch.zeros(T, K, dtype=torch.int32, device=DEV)
+    out = torch.empty(T * K, H, dtype=torch.bfloat16, device=DEV)
+    rows, row_map = torch.empty(E, dtype=torch.int32, device=DEV), torch.empty(T, K, dtype=torch.int32, device=DEV)
+    call = lambda: torch.ops._moe_C.remap_hidden_states(x, None, out, None, None, rows, row_map, ids, E, E)
+    call()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for _ in range(2):
+        new = torch.randint(0, E, (T, K), generator=g, dtype=torch.int32)
+        ids.copy_(new)
+        graph.replay()
+        order = torch.sort(new.flatten(), stable=True).indices
+        want = torch.empty(T * K, dtype=torch.int32)
+        want[order] = torch.arange(T * K, dtype=torch.int32)
+        assert torch.equal(row_map.cpu().flatten(), want)
+        assert torch.equal(rows.cpu().long(), torch.bincount(new.flatten().long(), minlength=E))

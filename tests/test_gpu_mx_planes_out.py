@@ -36,3 +36,26 @@ def test_layer_is_gemm_quantise_gemm(native, T, H, I, E, planes, how, dtype):
     want = torch.empty_like(x)
     torch.ops._moe_C.moe_gather(want, d, tw, row_map, E)
     assert torch.equal(out.view(torch.int16), want.view(torch.int16))
+
+
+@pytest.mark.parametrize("T", [1, 9, 40])
+def test_per_tensor_fp8_weights_too(native, T):
+    """The same kernel's other weights: [E, K, N] e4m3 with one scale per expert."""
+    E, K, H, I, dtype = 8, 2, 256, 160, torch.bfloat16
+    g = torch.Generator().manual_seed(T)
+    w13, w2 = ((torch.randn(E, *s, generator=g)).to(torch.float8_e4m3fn).to(DEV) for s in ((H, 2 * I), (I, H)))
+    s13, s2 = ((torch.rand(E, generator=g) * 0.1 + 0.02).to(DEV) for _ in range(2))
+    x = torch.randn(T, H, generator=g).to(dtype).to(DEV)
+    tw, ids = torch.topk(torch.softmax(torch.randn(T, E, generator=g), -1), k=K, dim=-1)
+    tw, ids = tw.to(DEV), ids.int().to(DEV)
+    layer = native.XpuFusedMoe(w13, s13, None, w2, s2, None, K, "swigluoai", E, fuse_activation=True)
+    out = torch.empty_like(x)
+    layer.apply(out, x, tw, ids)
+    rows, row_map = torch.empty(E, dtype=torch.int32, device=DEV), torch.empty(T, K, dtype=torch.int32, device=DEV)
+    xp = torch.empty(T * K, H, dtype=dtype, device=DEV)
+    torch.ops._moe_C.remap_hidden_states(x, None, xp, None, None, rows, row_map, ids, E, E)
+    mid = grouped_gemm(*quant_mxfp8(xp, 2), w13, s13, None, rows, 2 * I, H, epilogue=2, rows_out=T * K)
+    d = grouped_gemm(*quant_mxfp8(mid, 2), w2, s2, None, rows, H, I, rows_out=T * K)
+    want = torch.empty_like(x)
+    torch.ops._moe_C.moe_gather(want, d, tw, row_map, E)
+    assert torch.equal(out.view(torch.int16), want.view(torch.int16))
