@@ -30,6 +30,16 @@
 #define DM_DIV(a, b) ((a) / (b))
 #endif
 
+// x / 448 for x >= 0, correctly rounded where quotient and remainder are normal (x of 2^-93 and more): the product with
+// the rounded reciprocal and one correction by the exact remainder (Markstein, "Computation of elementary functions on
+// the IBM RISC System/6000 processor", 1990).  An infinity stays one.
+DM_HD float dm_div_448(float x) {
+  const float inv = 1.0f / 448.0f;
+  const float q = DM_MUL(x, inv);
+  const float fixed = DM_FMA(DM_FMA(-q, 448.0f, x), inv, q);
+  return q == INFINITY ? q : fixed;
+}
+
 DM_HD float dm_pow2i(int e) {  // 2^e for e in [-126, 127]
   uint32_t bits = (uint32_t)(e + 127) << 23;
   float f;

@@ -9,11 +9,13 @@
 // neighbours in a warp and combine their maxima with xor shuffles, exactly the
 // work split of the reference kernels, so the operation order per value is
 // theirs: fp32 silu(g) * u, group maximum, scale, divide (or multiply by the
-// reciprocal where the reference does), clamp, round.  Scales use IEEE
-// division; the per-value exp and divisions use the fast hardware forms (a
-// couple of ulp), which can move a value across a rounding boundary about once
-// in a million: the ops are arithmetic-bound, not HBM-bound, with the IEEE forms.
+// reciprocal where the reference does), clamp, round.  Scales are correctly
+// rounded quotients; the per-value exponential and reciprocals are the
+// hardware's approximations (a few ulp), which can move a value across a rounding
+// boundary about once in a million: the ops are arithmetic-bound, not HBM-bound,
+// with correctly rounded ones.
 #include "common.cuh"
+#include "det_math.h"
 
 namespace b200moe {
 namespace {
@@ -43,28 +45,21 @@ __device__ __forceinline__ int8_t f32_to_i8_rn(float x) {
   return (int8_t)fminf(fmaxf(rintf(x), -128.0f), 127.0f);
 }
 
-// silu(g) = g / (1 + 2^(-g log2 e)) with the hardware's exponential and reciprocal and nothing around them.  The range
-// steps that __expf and __fdividef add act on subnormals and beyond 2^126, where this denominator, from 1 up to
-// infinity, gives the same value without them.
+// The hardware's reciprocal and power of two (PTX: one unit in the last place, and 2^-22 of the value; subnormal
+// inputs and results are zero).
 __device__ __forceinline__ float rcp_ftz(float x) {
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+// silu(g) = g / (1 + e^-g) with e^-g = 2^(-g log2 e).  The denominator lies between 1 and infinity: where e^-g is
+// subnormal, and zero here, it is 1 all the same, and above 2^126 (gates below -87.33), where its reciprocal is subnormal, the
+// result is -0 instead of some -1e-36.  Elsewhere the relative error stays below 6e-7 + 7.3e-8 |g|: the exponent is
+// rounded to 2^-24 of itself, twice, and the rest is four roundings and the two instructions above.
 __device__ __forceinline__ float silu_fast(float g) {
   float e;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(g, -1.4426950408889634f)));
   return __fmul_rn(g, rcp_ftz(1.0f + e));
-}
-
-// x / 448 for x >= 0, correctly rounded where the quotient is normal: the product with the rounded reciprocal and one
-// correction by the exact remainder (Markstein, "Computation of elementary functions on the IBM RISC System/6000
-// processor", 1990; all 2^23 significands compared).  An infinity stays one.
-__device__ __forceinline__ float div_448(float x) {
-  constexpr float kInv = 1.0f / 448.0f;
-  const float q = __fmul_rn(x, kInv);
-  const float fixed = fmaf(fmaf(-q, 448.0f, x), kInv, q);
-  return q == INFINITY ? q : fixed;
 }
 
 enum OutFmt { kOutE4m3 = 0, kOutI8 = 1, kOutE2m1 = 2 };
@@ -140,7 +135,7 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
         scale = fmaxf(__fdiv_rn(amax, 127.0f), 1.1920928955078125e-07f);
       } else if (kFmt == kOutE4m3) {
         const float floor_s = 1.0f / (448.0f * 512.0f);
-        scale = fmaxf(div_448(amax), floor_s);
+        scale = fmaxf(dm_div_448(amax), floor_s);
         if (a.scale_ub != nullptr) scale = fmaxf(fminf(scale, *a.scale_ub), floor_s);
         if (a.ue8m0) scale = ceil_pow2_eps(scale, 1e-10f);
       } else {
@@ -164,7 +159,7 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
           else *reinterpret_cast<uint16_t*>(dst) = *reinterpret_cast<const uint16_t*>(o);
         } else {
           alignas(8) uint8_t o[N];
-          const float inv = rcp_ftz(scale);   // the group's, once: v * inv is __fdividef(v, scale)
+          const float inv = rcp_ftz(scale);   // the group's, once
 #pragma unroll
           for (int i = 0; i < N; i += 2) {
             const float q0 = __fmul_rn(v[i], inv), q1 = __fmul_rn(v[i + 1], inv);
@@ -192,7 +187,7 @@ group_quant_kernel(const GroupQuantArgs a, int64_t rows) {
 // before wrote last, so they are read from L2 before the others push them out.
 // Bytes bound it: 65536 x 2048 values 190 -> 144 us (4.7 TB/s beside the write-back of what the GEMM left in L2), 65536 x
 // 768 81 -> 56, 24008 x 768 28.6 -> 20.9 (blocks of a row's width that each summed the segments, more of them than were
-// resident, first row first, __expf and __fdividef with their range steps, an IEEE division a value group).
+// resident, first row first, SiLU by __expf and __fdividef, an IEEE division a group).
 constexpr int kPieces = 4;
 template <typename T>
 __global__ void __launch_bounds__(256, 4)
@@ -242,7 +237,7 @@ silu_quant_rows_kernel(uint8_t* __restrict__ out, float* __restrict__ scales, co
 #pragma unroll
       for (int off = 1; off < 16; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
       if (!active) continue;
-      const float scale = fmaxf(div_448(amax), 1.0f / (448.0f * 512.0f));
+      const float scale = fmaxf(dm_div_448(amax), 1.0f / (448.0f * 512.0f));
       if ((lane & 15) == 0) scales[at[k] * groups + (col[k] >> 4)] = scale;
       const float inv = rcp_ftz(scale);
       uint32_t q[4];
