@@ -36,7 +36,11 @@ typedef enum {
   B200MOE_FP8_E4M3_X2 = 9, /* two float8_e4m3fn planes [2][rows][cols]: value =
                               plane 0 + plane 1 (MXFP8 activations + residual) */
   B200MOE_I8 = 10, /* int8 */
-  B200MOE_FP8_E4M3_X3 = 11 /* three planes: a float16 exactly (int4 weights only) */
+  B200MOE_FP8_E4M3_X3 = 11, /* three planes: a float16 exactly (int4 weights only) */
+  /* the same planes with the codes of a row, eight at a time, in the order 0 2 4 6 1 3 5 7,
+     which an int4 GEMM multiplies without putting its weights in order (int4 weights only) */
+  B200MOE_FP8_E4M3_X2_EVENS_FIRST = 12,
+  B200MOE_FP8_E4M3_X3_EVENS_FIRST = 13
 } b200moe_dtype;
 
 /* Status codes. */
@@ -297,8 +301,8 @@ int b200moe_remap_quant_fp8(const void* hidden, b200moe_dtype dtype,
                             b200moe_stream stream);
 /* The same with MXFP8 planes (b200moe_quant_mxfp8) instead of fp8: codes
  * [planes][T*K,H], scale words [planes][ceil(H/128)][T*K]; with block_sums
- * fp32 sums [ceil(H/128)][T*K] follow the words, and the codes are in the order of
- * b200moe_quant_mxfp8_ex. */
+ * fp32 sums [ceil(H/128)][T*K] follow the words (values and order of the codes as in
+ * b200moe_quant_mxfp8_ex). */
 int b200moe_remap_quant_mxfp8(const void* hidden, b200moe_dtype dtype,
                               void* remapped_q, void* remapped_scales, int planes,
                               int block_sums,
@@ -347,9 +351,12 @@ typedef struct {
   b200moe_dtype a_dtype;  /* BF16, F16, or FP8_E4M3 (with a_scale)                */
   const void* a_scale;    /* fp8 activations: block-fp8 weights: fp32 [M,K/128];
                              MXFP4 weights (MXFP8 activations, a_dtype FP8_E4M3
-                             or FP8_E4M3_X2, _X3): e8m0 bytes as 32-bit words
+                             or FP8_E4M3_X2): e8m0 bytes as 32-bit words
                              [planes][ceil(K/128)][M], the output of
-                             b200moe_quant_mxfp8; else NULL                  */
+                             b200moe_quant_mxfp8; int4 weights (FP8_E4M3_X2, _X3
+                             and their _EVENS_FIRST forms): such words and fp32
+                             block sums [K/128][M] behind them, the output of
+                             b200moe_quant_mxfp8_ex; else NULL                  */
   const void* w;          /* weights, layout per w_format                         */
   b200moe_weight_format w_format;
   const void* w_scale;    /* per w_format, else NULL                              */
@@ -533,9 +540,12 @@ int b200moe_quant_mxfp8(const void* x, b200moe_dtype dtype, void* q, void* s,
 /* The same with up to three planes and, behind the scale words, fp32 sums
  * [ceil(cols/128)][rows] of every 128-wide block (of what the planes hold): the
  * activations of an int4 grouped GEMM, whose scales go down to 2^-100 (so that
- * small values keep their bits) and whose codes have, of every eight, the even
- * ones before the odd ones (0 2 4 6 1 3 5 7).  With `gated` x is [rows, 2 * cols] and
- * the values are silu(gate) * up as b200moe_silu_and_mul rounds them. */
+ * small values keep their bits).  block_sums: 0 = none, B200MOE_SUMS_EVENS_FIRST = with
+ * the codes of a row, eight at a time, in the order 0 2 4 6 1 3 5 7 (the GEMM's
+ * a_dtype ..._EVENS_FIRST), any other value = codes in their own order.  With
+ * `gated` x is [rows, 2 * cols] and the values are silu(gate) * up as
+ * b200moe_silu_and_mul rounds them. */
+#define B200MOE_SUMS_EVENS_FIRST 2
 int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* q, void* s,
                            int64_t rows, int cols, int terms, int block_sums,
                            int gated, b200moe_stream stream);

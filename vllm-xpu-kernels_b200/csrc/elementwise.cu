@@ -241,7 +241,9 @@ constexpr int kMxQuantUnroll = 2;
 // Instructions bound it (issue slots 74 % in use with 292 of them a piece, most of them 64-bit products for the
 // addresses and a division a step): the planes are a template argument, a step's addresses follow from two pointers, and
 // row and step advance by additions.
-template <typename T, bool kGated, int kTerms, bool kSums>
+// kSums: block sums behind the scale words, with the codes in their own order or the even ones of eight first.
+enum MxSums { kNoSums = 0, kSumsInOrder, kSumsEvensFirst };
+template <typename T, bool kGated, int kTerms, int kSums>
 __global__ void __launch_bounds__(256)
 quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* __restrict__ s, uint32_t rows, int cols) {
   pdl_trigger();
@@ -289,7 +291,7 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
       for (int term = 0; term < kTerms; ++term) {
         uint2 codes;
         const uint32_t word = mx_quant_lane(v, active, codes, kSums ? kMxLeastExact : kMxLeast, kSums || term + 1 < kTerms);
-        if (active) *reinterpret_cast<uint2*>(qu) = kSums ? mx_evens_first(codes) : codes;
+        if (active) *reinterpret_cast<uint2*>(qu) = kSums == kSumsEvensFirst ? mx_evens_first(codes) : codes;
         if (first_of_block) *su = word;
         qu += q_plane;
         su += s_plane;
@@ -538,9 +540,13 @@ extern "C" int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* 
            terms == 2 ? run(type, is_gated, std::integral_constant<int, 2>(), with_sums) :
                         run(type, is_gated, std::integral_constant<int, 3>(), with_sums);
   };
+  auto of_sums = [&](auto type, auto is_gated) {
+    return !block_sums ? of_planes(type, is_gated, std::integral_constant<int, kNoSums>()) :
+           block_sums == B200MOE_SUMS_EVENS_FIRST ? of_planes(type, is_gated, std::integral_constant<int, kSumsEvensFirst>()) :
+                                                    of_planes(type, is_gated, std::integral_constant<int, kSumsInOrder>());
+  };
   auto of_form = [&](auto type) {
-    return gated ? (block_sums ? of_planes(type, std::true_type(), std::true_type()) : of_planes(type, std::true_type(), std::false_type())) :
-                   (block_sums ? of_planes(type, std::false_type(), std::true_type()) : of_planes(type, std::false_type(), std::false_type()));
+    return gated ? of_sums(type, std::true_type()) : of_sums(type, std::false_type());
   };
   if (dtype == B200MOE_BF16) B200_LAUNCHED("quant_mxfp8_kernel", of_form(__nv_bfloat16()));
   else B200_LAUNCHED("quant_mxfp8_kernel", of_form(__half()));

@@ -38,8 +38,9 @@ extern "C" int b200moe_grouped_gemm(const b200moe_gemm_args* a, b200moe_stream s
                               (a->mid_dtype == B200MOE_BF16 || a->mid_dtype == B200MOE_F16)),
                  "grouped_gemm: e4m3 output needs the SiLU epilogue, d_scale, a 16-bit mid_dtype, fp8 "
                  "activations and block-scaled fp8 weights");
-  const bool a_x2 = a->a_dtype == B200MOE_FP8_E4M3_X2;
-  const bool a_x3 = a->a_dtype == B200MOE_FP8_E4M3_X3;
+  const bool evens_first = a->a_dtype == B200MOE_FP8_E4M3_X2_EVENS_FIRST || a->a_dtype == B200MOE_FP8_E4M3_X3_EVENS_FIRST;
+  const bool a_x2 = a->a_dtype == B200MOE_FP8_E4M3_X2 || a->a_dtype == B200MOE_FP8_E4M3_X2_EVENS_FIRST;
+  const bool a_x3 = a->a_dtype == B200MOE_FP8_E4M3_X3 || a->a_dtype == B200MOE_FP8_E4M3_X3_EVENS_FIRST;
   const bool a_fp8 = a->a_dtype == B200MOE_FP8_E4M3 || a_x2 || a_x3;
   B200_CHECK_ARG(a_fp8 || a->a_dtype == a->d_dtype,
                  "grouped_gemm: ptr_A must be fp8 (with scales) or have ptr_D's dtype");
@@ -95,6 +96,8 @@ extern "C" int b200moe_grouped_gemm(const b200moe_gemm_args* a, b200moe_stream s
   B200_CHECK_ARG(!a_x3 || a->w_format == B200MOE_W_INT4_NK, "grouped_gemm: three-plane activations need int4 weights");
   B200_CHECK_ARG(!a_x2 || a->w_format == B200MOE_W_MXFP4_NK || a->w_format == B200MOE_W_INT4_NK || w_tensor8,
                  "grouped_gemm: two-plane fp8 activations need MXFP4, MXFP8 or per-tensor fp8 weights");
+  B200_CHECK_ARG(!evens_first || a->w_format == B200MOE_W_INT4_NK,
+                 "grouped_gemm: activations with the even codes first need int4 weights");
   const bool segmented = a->w_experts > 0 && a->w_experts != a->num_experts;
   B200_CHECK_ARG(a->w_experts >= 0 && (!segmented || a->num_experts % a->w_experts == 0),
                  "grouped_gemm: w_experts must divide num_experts");

@@ -5,10 +5,10 @@
 // Weights [E,N,K/2] are two's-complement nibbles with one 16-bit scale per row and 128 or 256 K
 // elements.  A nibble u in 0..15, put into a byte, IS the e4m3 number u * 2^-9 (the subnormals and
 // the first binade of e4m3 are linear), so unpacking is the whole conversion: three instructions per
-// eight weights (their even and odd ones apart, which is the order of the tokens' codes, too; two more to
-// interleave them before: 33 tokens x top-2 of 8 experts of 4096 x 14336, a layer call 223 -> 219 us), against
-// seventeen for the 16-bit expansion of gemm_tc_dq.cu, whose integer pipe is the bound when there are few tokens.  The
-// activations are e4m3 planes with one power-of-two
+// eight weights where the tokens' codes come with the even ones first, too (a layer's do), two more to put the
+// weights in order where they don't (33 tokens x top-2 of 8 experts of 4096 x 14336, a layer call 223 -> 219 us
+// without), against seventeen for the 16-bit expansion of gemm_tc_dq.cu, whose integer pipe is the bound when there
+// are few tokens.  The activations are e4m3 planes with one power-of-two
 // scale per 32 values (mx_quant.cuh): two planes hold a bfloat16 exactly, three a float16 (values
 // 2^-14 of the group's largest and smaller excepted, whose error stays below 2^-21 of it), so
 // nothing is lost against 16-bit activations, and the weight is not rounded after its scale is applied.
@@ -104,7 +104,7 @@ struct I4Ctrl {
   alignas(16) uint16_t xpose[8][16 * 32];   // per promotion warp: output transpose tile
 };
 
-template <int BT, int kTerms>
+template <int BT, int kTerms, bool kEvensFirst>
 __global__ void __launch_bounds__(kI4Threads, 1)
 grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
                        const I4Params p) {
@@ -318,9 +318,10 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          // nibbles of even and of odd k as bytes (sign bit flipped: 0..15); the tokens' codes come in the same order
-          o[q * 8 + 2 * j] = (w[j] & 0x0f0f0f0fu) ^ 0x08080808u;
-          o[q * 8 + 2 * j + 1] = ((w[j] >> 4) & 0x0f0f0f0fu) ^ 0x08080808u;
+          // nibbles of even and of odd k as bytes (sign bit flipped: 0..15), in the order of the tokens' codes
+          const uint32_t e = (w[j] & 0x0f0f0f0fu) ^ 0x08080808u, d = ((w[j] >> 4) & 0x0f0f0f0fu) ^ 0x08080808u;
+          o[q * 8 + 2 * j] = kEvensFirst ? e : __byte_perm(e, d, 0x5140);
+          o[q * 8 + 2 * j + 1] = kEvensFirst ? d : __byte_perm(e, d, 0x7362);
         }
       }
       __syncwarp();
@@ -452,10 +453,10 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   if (tid == 0 && *abort_flag != 0) report_timeout(p.status);
 }
 
-template <int BT, int kTerms>
+template <int BT, int kTerms, bool kEvensFirst>
 int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
   using S = I4Shape<BT, kTerms>;
-  auto kern = grouped_gemm_i4_kernel<BT, kTerms>;
+  auto kern = grouped_gemm_i4_kernel<BT, kTerms, kEvensFirst>;
   p.idesc = ptx::make_idesc_mx(0u, 0u, kFeat, (uint32_t)BT);
   CUtensorMap ta, tw;
   {
@@ -498,9 +499,11 @@ int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
 
 // INT4 weights x two (bfloat16 output) or three (float16 output) e4m3 planes: a codes [planes][M,K],
 // a_scale words [planes][K/128][M] and fp32 block sums [K/128][M] behind them (what
-// b200moe_quant_mxfp8_ex writes).  Returns B200MOE_E_UNSUPPORTED (no launch) for anything else.
+// b200moe_quant_mxfp8_ex writes, in either order of the codes).  Returns B200MOE_E_UNSUPPORTED (no launch) for anything else.
 int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
-  const int planes = a->a_dtype == B200MOE_FP8_E4M3_X2 ? 2 : a->a_dtype == B200MOE_FP8_E4M3_X3 ? 3 : 0;
+  const bool evens_first = a->a_dtype == B200MOE_FP8_E4M3_X2_EVENS_FIRST || a->a_dtype == B200MOE_FP8_E4M3_X3_EVENS_FIRST;
+  const int planes = a->a_dtype == B200MOE_FP8_E4M3_X2 || a->a_dtype == B200MOE_FP8_E4M3_X2_EVENS_FIRST ? 2 :
+                     a->a_dtype == B200MOE_FP8_E4M3_X3 || a->a_dtype == B200MOE_FP8_E4M3_X3_EVENS_FIRST ? 3 : 0;
   if (a->w_format != B200MOE_W_INT4_NK || planes == 0 || a->a_scale == nullptr || a->epilogue != B200MOE_EPI_NONE)
     return fail(B200MOE_E_UNSUPPORTED, "int4 GEMM takes int4 weights and two or three e4m3 activation planes");
   if (a->num_experts > kMaxExperts || a->k % 128 != 0 || (a->group_size != 128 && a->group_size != 256) || a->n % 8 != 0)
@@ -525,8 +528,12 @@ int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
   // bfloat16 8.3 rows an expert 207 / 218, 10 rows 220 / 222, 10.3 rows 222 / 221, 11 rows 230 / 223, 12 rows 247 / 226; float16
   // (three planes, whose wide tile leaves the ring 9 stages) 8.3 rows 222 / 274, 10 rows 236 / 277, 12 rows 266 / 278, 13
   // rows 274 / 280, 14 rows 289 / 287.
-  if (planes == 2) return avg <= 10 ? launch_i4<16, 2>(a, p, st) : launch_i4<32, 2>(a, p, st);
-  return avg <= 13 ? launch_i4<16, 3>(a, p, st) : launch_i4<32, 3>(a, p, st);
+  auto run = [&](auto order) {
+    constexpr bool kEvens = decltype(order)::value;
+    if (planes == 2) return avg <= 10 ? launch_i4<16, 2, kEvens>(a, p, st) : launch_i4<32, 2, kEvens>(a, p, st);
+    return avg <= 13 ? launch_i4<16, 3, kEvens>(a, p, st) : launch_i4<32, 3, kEvens>(a, p, st);
+  };
+  return evens_first ? run(std::true_type()) : run(std::false_type());
 }
 
 }  // namespace b200moe

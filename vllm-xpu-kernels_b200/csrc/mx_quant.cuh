@@ -96,8 +96,8 @@ __device__ __forceinline__ uint32_t mx_quant_lane(float (&v)[8], bool active, ui
   return word;
 }
 
-// An int4 layer's codes, eight at a time: the even ones, then the odd ones (the order in which its GEMM unpacks the
-// nibbles of a word; the sum over k does not mind).
+// Codes eight at a time, the even ones, then the odd ones: the order in which an int4 GEMM unpacks the nibbles of a
+// word (the sum over k does not mind).
 __device__ __forceinline__ uint2 mx_evens_first(uint2 c) {
   return make_uint2(__byte_perm(c.x, c.y, 0x6420), __byte_perm(c.x, c.y, 0x7531));
 }

@@ -115,7 +115,7 @@ __device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, 
   for (int p = 0; p < a.planes; ++p) {
     uint2 codes;
     const uint32_t word = mx_quant_lane(v, in, codes, a.sums ? kMxLeastExact : kMxLeast, a.sums || p + 1 < a.planes);
-    if (a.sums) codes = mx_evens_first(codes);
+    if (a.sums == B200MOE_SUMS_EVENS_FIRST) codes = mx_evens_first(codes);
     uint8_t* q = dst_q + p * a.rows * H + (int64_t)j * 8;
     uint32_t* s = dst_s + ((int64_t)p * num_kb + (j >> 4)) * a.rows;
     for (int k = 0; k < a.K; ++k) {
