@@ -192,12 +192,14 @@ constexpr int kPieces = 4;
 template <typename T>
 __global__ void __launch_bounds__(256, 4)
 silu_quant_rows_kernel(uint8_t* __restrict__ out, float* __restrict__ scales, const T* __restrict__ in, int64_t max_rows,
-                       int hidden, const int32_t* __restrict__ rows_per_segment, int num_segments) {
+                       int hidden, const int32_t* rows_per_segment, int num_segments) {
   pdl_trigger();
   pdl_wait();
   const int lane = threadIdx.x & 31;
-  int64_t used = 0;   // (every warp for itself)
-  for (int e = lane; e < num_segments; e += 32) used += max(__ldg(rows_per_segment + e), 0);
+  // (Every warp for itself; plain loads: a kernel that started early may not read through the non-coherent path, nor ahead of
+  // its wait, what the kernel before it is still writing.)
+  int64_t used = 0;
+  for (int e = lane; e < num_segments; e += 32) used += max(rows_per_segment[e], 0);
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) used += __shfl_xor_sync(0xffffffffu, used, off);
   const int rows = (int)(used < max_rows ? used : max_rows);
