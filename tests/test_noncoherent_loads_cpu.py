@@ -12,6 +12,16 @@ def _code(path):
     return "\n".join(line.split("//")[0] for line in path.read_text().splitlines())
 
 
+def test_only_weights_are_read_through_the_non_coherent_path():
+    """Token scales and sums, rows and their positions come from the kernel ahead."""
+    weights = {"gemm_tc_mx.cu": ["src", "src + 1"], "gemm_tc_fp8t.cu": ["w0 + kb", "w0 + w1 + kb"],
+               "gemm_tc_i4.cu": ["reinterpret_cast<const uint2*>(srow + kb0)", "srow + g"],
+               "gemm_tc_dq.cu": ["s16 + ((kb * 128) >> p.group_shift)", "s16 + g", "srow + kb * 4 + u"]}
+    for path in SOURCES:
+        found = re.findall(r"__ldg\(((?:[^()]|\((?:[^()]|\([^()]*\))*\))*)\)", _code(path))
+        assert found == weights.get(path.name, []), path.name
+
+
 def test_row_counts_are_read_with_plain_loads():
     """Counts come from the sort ahead: no __ldg, and no __restrict__, by which a compiler may make one."""
     for path in SOURCES:

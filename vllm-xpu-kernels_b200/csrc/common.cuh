@@ -68,7 +68,8 @@ inline cudaError_t launch_pdl(bool early, void (*kern)(Params...), dim3 grid, di
   cfg.attrs = attr; cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, Params(std::forward<Args>(args))...);
 }
-// Every thread that touches global memory calls the wait; the trigger lets the next kernel of the
+// Every thread that touches global memory calls the wait (what an earlier kernel of the stream writes is read with plain
+// loads behind it: __ldg is for weights and their scales, which stay as they are while a kernel runs); the trigger lets the next kernel of the
 // stream be launched (it holds its own wait until this one has completed).  The grouped GEMMs
 // trigger when a CTA's last tile is done, everything else at once.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -551,9 +551,9 @@ grouped_gemm_fp8t256_kernel(const __grid_constant__ T2TokenMaps tmap_a,
           for (int i = 0; i < 2; ++i) {
             const float* src = a0 + (int64_t)(64 * i) * kbs + kb;
             if (!vec4) {
-              av[i][j] = in && live[i] ? __ldg(src) : 0.f;
+              av[i][j] = in && live[i] ? *src : 0.f;
             } else if (j == 0) {
-              const float4 v = live[i] ? __ldg(reinterpret_cast<const float4*>(src)) : make_float4(0.f, 0.f, 0.f, 0.f);
+              const float4 v = live[i] ? *reinterpret_cast<const float4*>(src) : make_float4(0.f, 0.f, 0.f, 0.f);
               av[i][0] = v.x; av[i][1] = v.y; av[i][2] = v.z; av[i][3] = v.w;
             }
           }

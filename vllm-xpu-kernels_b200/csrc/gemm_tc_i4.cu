@@ -272,13 +272,13 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
           for (int i = 0; i < kPer; ++i) {
             const int x = ft + 32 * i, n = x % kNT, kb = kb0 + x / kNT, term = n / BT, tok = n % BT;
             w[i] = (kb < p.num_kb && tok < ti.valid)
-                       ? __ldg(p.a_scale + term * plane_words + (int64_t)kb * p.m + ti.row0 + tok) : 0x7f7f7f7fu;
+                       ? p.a_scale[term * plane_words + (int64_t)kb * p.m + ti.row0 + tok] : 0x7f7f7f7fu;
           }
   #pragma unroll
           for (int i = 0; i < kPerSum; ++i) {
             const int x = ft + 32 * i, tok = x % BT, kb = kb0 + x / BT;
             m[i] = (kb < p.num_kb && tok < ti.valid)
-                       ? -8.0f * __ldg(sums + (int64_t)kb * p.m + ti.row0 + tok) : 0.f;
+                       ? -8.0f * sums[(int64_t)kb * p.m + ti.row0 + tok] : 0.f;
           }
           if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(sf_empty0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
           const uint32_t ring = ptx::smem_u32(sf_ring) + slot * kSlotBytes;

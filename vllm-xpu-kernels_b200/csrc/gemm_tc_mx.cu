@@ -470,8 +470,8 @@ grouped_gemm_mx_kernel(const __grid_constant__ MxTokenMaps<BT> tmap_a,
       const uint32_t* base = p.a_scale + (int64_t)(g * kMxGroup) * p.m + ti.row0;
 #pragma unroll
       for (int i = 0; i < kPer; ++i)
-        db[i] = (ft + 128 * i < kMxGroup * kNT && word_u(i) < p.num_kb - g * kMxGroup && word_tok(i) < ti.valid) ? __ldg(base + src[i])
-                                                                                                              : 0x7f7f7f7fu;
+        db[i] = (ft + 128 * i < kMxGroup * kNT && word_u(i) < p.num_kb - g * kMxGroup && word_tok(i) < ti.valid)
+                    ? base[src[i]] : 0x7f7f7f7fu;
     };
     int la_t = blockIdx.x, la_g = 0;
     TileInfo la_ti;

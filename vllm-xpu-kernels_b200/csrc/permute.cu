@@ -393,7 +393,7 @@ __device__ __forceinline__ void copy_bytes(unsigned char* dst, const unsigned ch
   if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src) | (uintptr_t)n) & 15) == 0) {
     const uint4* s4 = reinterpret_cast<const uint4*>(src);
     uint4* d4 = reinterpret_cast<uint4*>(dst);
-    for (int64_t i = threadIdx.x; i < n / 16; i += blockDim.x) d4[i] = __ldg(s4 + i);
+    for (int64_t i = threadIdx.x; i < n / 16; i += blockDim.x) d4[i] = s4[i];
   } else {
     for (int64_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
   }
