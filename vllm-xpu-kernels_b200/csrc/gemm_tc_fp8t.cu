@@ -816,9 +816,10 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   // A operand = tokens (K-major), B operand = weights (K-major, or MN-major for [E,K,N])
   p.idesc = ptx::make_idesc(0u, 0u, 0u, kn ? 1u : 0u, kTTok, kFeat);
 
+  const bool wide = a->n >= 256;   // 256-feature tiles; a single 128-feature block takes the narrow kernel
   T2TokenMaps ta;
   CUtensorMap tw, td;
-  for (int i = 0; i < 4; ++i) {
+  for (int i = wide ? 0 : 3; i < 4; ++i) {   // (the narrow kernel brings whole boxes)
     cuuint64_t dims[2] = {(cuuint64_t)a->k, (cuuint64_t)a->m};
     cuuint64_t strides[1] = {(cuuint64_t)a->k};
     cuuint32_t box[2] = {128, (cuuint32_t)(32 * (i + 1))};
@@ -840,7 +841,6 @@ int grouped_gemm_tc_fp8t(const b200moe_gemm_args* a, cudaStream_t st) {
   }
   int grid = sm_count();
   if (a->max_ctas > 0 && a->max_ctas < grid) grid = a->max_ctas;
-  const bool wide = a->n >= 256;   // 256-feature tiles; a single 128-feature block takes the narrow kernel
   const int64_t tile_bound = ((a->m + kTTok - 1) / kTTok + a->num_experts) * (int64_t)(wide ? (p.n_tiles + 1) / 2 : p.n_tiles);
   if (tile_bound < grid) grid = (int)tile_bound;
   if (grid < 1) grid = 1;
