@@ -37,6 +37,36 @@ def test_layer_int4(native, dtype, T, H, I, group):
     assert err < (1e-2 if dtype == torch.bfloat16 else 2e-3), err
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T,H,I", [(20, 256, 384), (21, 640, 256), (26, 384, 128), (27, 256, 640), (32, 512, 384), (30, 128, 256)])
+def test_layer_int4_on_both_sides_of_the_tile_lines(native, dtype, T, H, I):
+    """Rows per expert (half of T) around the lines of 10 (bfloat16) and 13 (float16), and up to the 16 at which another
+    kernel takes over: 16- and 32-token tiles of two and three planes, several tiles an expert (routing as it comes)."""
+    test_layer_int4(native, dtype, T, H, I, 128)
+
+
+@pytest.mark.parametrize("ctas", [1, 3])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("T", [24, 30])
+def test_int4_tiles_that_follow_one_another(native, dtype, T, ctas):
+    """Few CTAs that walk many tiles give what one tile a CTA gives, bit for bit; some experts have none, some several."""
+    E, K, H, I, group = 4, 2, 384, 640, 128
+    g = torch.Generator().manual_seed(T)
+    w13, w2 = (torch.randint(0, 256, s, generator=g, dtype=torch.int32).to(torch.uint8).to(DEV)
+               for s in ((E, 2 * I, H // 2), (E, H, I // 2)))
+    s13, s2 = ((torch.rand(E, n, k // group, generator=g) * 0.2 + 0.1).mul(k ** -0.5).to(dtype).to(DEV) for n, k in ((2 * I, H), (H, I)))
+    x = torch.randn(T, H, generator=g).to(dtype).to(DEV)
+    ids = torch.tensor([[0, 2]] * (T - 3) + [[2, 3]] * 3, dtype=torch.int32, device=DEV)
+    tw = torch.rand(T, K, generator=g).to(DEV)
+    layer = native.XpuFusedMoe(w13, s13, None, w2, s2, None, K, "silu", E)
+    outs = []
+    for n in (0, ctas):
+        layer.gemm_max_ctas = n
+        outs.append(torch.full_like(x, float("nan")))
+        layer.apply(outs[-1], x, tw, ids)
+    assert not outs[0].isnan().any() and torch.equal(*outs)
+
+
 @pytest.mark.parametrize("T", [9, 70])
 @pytest.mark.parametrize("size", [1e-6, 1e-11, 1e-14])
 def test_layer_int4_keeps_small_activations(native, T, size):
