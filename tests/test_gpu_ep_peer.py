@@ -46,7 +46,7 @@ def _oracle_full(cfg, w, x, tw, ids):
     ("cfg1_small_bf16", dict(H=256, I=128, E=8), 4, (33, 0, 64, 7), 2e-2, True),        # experts placed by load
     ("cfg4_deepseek_fp8", dict(H=512, I=256, E=64), 4, (50, 64, 1, 23), 5e-2, False),
     ("cfg4_deepseek_fp8", dict(H=512, I=256, E=64), 4, (50, 64, 1, 23), 5e-2, True),
-    ("cfg4_deepseek_fp8", dict(H=512, I=256, E=64), 8, (300, 290, 310, 5, 300, 0, 299, 320), 5e-2, False),  # multi-block sort
+    ("cfg4_deepseek_fp8", dict(H=512, I=256, E=64), 8, (300, 290, 310, 5, 300, 0, 299, 320), 5e-2, False),  # cluster sort
 ])
 def test_peer_ep_layer_matches_the_single_process_oracle(native, cfg_name, dims, ep, tokens, tol, placed):
     from vllm_xpu_kernels.ep_moe import balanced_expert_slots
@@ -128,6 +128,28 @@ def test_peer_ep_quantised_rows_are_the_group_quantiser(native):
         scales = layers[d].recv_scales.cpu().view(ep, cap, cfg.H // 128)[0]
         assert torch.equal(rows[idx], q.view(torch.uint8)[sent])
         assert torch.equal(scales[idx], s[sent])
+
+
+@pytest.mark.parametrize("T", [8192, 8193])
+def test_peer_ep_dispatch_of_many_tokens(native, T):
+    """(token, rank) slots into fixed regions on both sides of what one cluster sorts, 65536: beyond it in three launches."""
+    cfg = wl.scaled(wl.CONFIGS["cfg1_small_bf16"], H=64, I=64, E=8)
+    ep, cap = 8, T + 7
+    _, layers = _build(native, cfg, ep, cap, seed=2)
+    g = torch.Generator().manual_seed(T)
+    x = torch.randn(T, cfg.H, generator=g).to(torch.bfloat16)
+    ids = torch.topk(torch.rand(T, cfg.E, generator=g), cfg.K, dim=-1).indices.to(torch.int32)
+    ids[torch.rand(T, cfg.K, generator=g) < 0.02] = -1
+    tw = torch.rand(T, cfg.K, generator=g)
+    layers[3].dispatch(x.to(DEV), tw.to(DEV), ids.to(DEV))
+    torch.cuda.synchronize()
+    counts, pos, loc = to.ep_dispatch_plan(ids, ep, cfg.E // ep, cap)
+    assert torch.equal(layers[3].send_counts.cpu(), counts) and torch.equal(layers[3].send_pos[:T].cpu(), pos)
+    for d in range(ep):
+        sent = pos[:, d] >= 0
+        idx = (pos[sent, d] - d * cap).long()
+        assert torch.equal(layers[d].recv_rows.cpu().view(ep, cap, cfg.H)[3][idx], x[sent])
+        assert torch.equal(layers[d].recv_ids.cpu().view(ep, cap, cfg.K)[3][idx], loc[sent, d])
 
 
 def test_peer_ep_rejects_more_tokens_than_its_regions_hold(native):
