@@ -259,7 +259,7 @@ quant_mxfp8_kernel(const T* __restrict__ x, uint8_t* __restrict__ q, uint32_t* _
   uint32_t r = first / steps, step = first - r * steps;
   while (r < rows) {
     const int j0 = step * (kMxQuantUnroll * 32) + lane;
-    const T* xr = x + (size_t)r * (cols * (kGated ? 2 : 1)) + j0 * 8;
+    const T* xr = x + (size_t)r * cols * (kGated ? 2 : 1) + j0 * 8;
     uint8_t* qr = q + (size_t)r * cols + j0 * 8;
     uint32_t* sr = s + (size_t)rows * (j0 >> 4) + r;
     vec16 in[kMxQuantUnroll], up[kGated ? kMxQuantUnroll : 1];
