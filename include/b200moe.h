@@ -301,8 +301,8 @@ int b200moe_remap_quant_fp8(const void* hidden, b200moe_dtype dtype,
                             b200moe_stream stream);
 /* The same with MXFP8 planes (b200moe_quant_mxfp8) instead of fp8: codes
  * [planes][T*K,H], scale words [planes][ceil(H/128)][T*K]; with block_sums
- * fp32 sums [ceil(H/128)][T*K] follow the words (values and order of the codes as in
- * b200moe_quant_mxfp8_ex). */
+ * fp32 sums [ceil(H/128)][T*K] follow the words (values, `planes` and order of the
+ * codes as with the `terms` of b200moe_quant_mxfp8_ex). */
 int b200moe_remap_quant_mxfp8(const void* hidden, b200moe_dtype dtype,
                               void* remapped_q, void* remapped_scales, int planes,
                               int block_sums,
@@ -540,12 +540,11 @@ int b200moe_quant_mxfp8(const void* x, b200moe_dtype dtype, void* q, void* s,
 /* The same with up to three planes and, behind the scale words, fp32 sums
  * [ceil(cols/128)][rows] of every 128-wide block (of what the planes hold): the
  * activations of an int4 grouped GEMM, whose scales go down to 2^-100 (so that
- * small values keep their bits).  block_sums: 0 = none, B200MOE_SUMS_EVENS_FIRST = with
- * the codes of a row, eight at a time, in the order 0 2 4 6 1 3 5 7 (the GEMM's
- * a_dtype ..._EVENS_FIRST), any other value = codes in their own order.  With
- * `gated` x is [rows, 2 * cols] and the values are silu(gate) * up as
- * b200moe_silu_and_mul rounds them. */
-#define B200MOE_SUMS_EVENS_FIRST 2
+ * small values keep their bits).  terms + B200MOE_PLANES_EVENS_FIRST (with block_sums
+ * only): the codes of a row, eight at a time, in the order 0 2 4 6 1 3 5 7 (the GEMM's
+ * a_dtype ..._EVENS_FIRST).  With `gated` x is [rows, 2 * cols] and the values are
+ * silu(gate) * up as b200moe_silu_and_mul rounds them. */
+#define B200MOE_PLANES_EVENS_FIRST 16
 int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* q, void* s,
                            int64_t rows, int cols, int terms, int block_sums,
                            int gated, b200moe_stream stream);

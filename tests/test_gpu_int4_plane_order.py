@@ -13,7 +13,7 @@ from gpu_utils import DEV
 pytestmark = pytest.mark.gpu
 
 F16, BF16, E4M3_X2, E4M3_X3, X2_EVENS_FIRST, X3_EVENS_FIRST, I32, INT4_NK = 1, 2, 9, 11, 12, 13, 5, 7
-IN_ORDER, EVENS_FIRST = 1, 2
+IN_ORDER, EVENS_FIRST = 0, 16
 ORDER = [0, 2, 4, 6, 1, 3, 5, 7]
 
 
@@ -32,12 +32,12 @@ def _stream():
     return ct.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
-def _quantise(lib, x, planes, block_sums, gated=0):
+def _quantise(lib, x, planes, order, gated=0, block_sums=1):
     rows, cols = x.shape[0], x.shape[1] // (2 if gated else 1)
     q = torch.empty(planes, rows, cols, dtype=torch.uint8, device=DEV)
     s = torch.empty(planes + 1, (cols + 127) // 128, rows, dtype=torch.int32, device=DEV)
     rc = lib.b200moe_quant_mxfp8_ex(_ptr(x), F16 if x.dtype == torch.float16 else BF16, _ptr(q), _ptr(s), ct.c_int64(rows), cols,
-                                    planes, block_sums, gated, _stream())
+                                    planes + order, block_sums, gated, _stream())
     assert rc == 0, lib.b200moe_last_error()
     return q, s
 
@@ -90,6 +90,9 @@ def test_quantiser_writes_both_orders(lib, rows, cols, dtype, planes, gated):
     g = torch.Generator().manual_seed(cols)
     x = torch.randn(rows, cols * (1 + gated), generator=g).to(dtype).to(DEV)
     q, s = _quantise(lib, x, planes, IN_ORDER, gated)
+    for other in (2, 16, -1):                            # any value but zero asks for the sums, and for nothing else
+        again = _quantise(lib, x, planes, IN_ORDER, gated, other)
+        assert torch.equal(q, again[0]) and torch.equal(s, again[1])
     q2, s2 = _quantise(lib, x, planes, EVENS_FIRST, gated)
     assert torch.equal(s, s2)
     assert torch.equal(q.view(planes, rows, cols // 8, 8)[..., ORDER].reshape_as(q), q2)
@@ -110,12 +113,12 @@ def test_remap_and_quantise_as_the_quantiser_does(lib, dtype, planes):
     x = torch.randn(T, H, generator=g).to(dtype).to(DEV)
     ids = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(T)]).int().to(DEV)
     order = torch.sort(ids.flatten(), stable=True).indices
-    for block_sums in (IN_ORDER, EVENS_FIRST):
-        want_q, want_s = _quantise(lib, x[order // K].contiguous(), planes, block_sums)
+    for codes, block_sums in ((IN_ORDER, 1), (IN_ORDER, 2), (EVENS_FIRST, 1)):
+        want_q, want_s = _quantise(lib, x[order // K].contiguous(), planes, codes)
         q, s = torch.empty_like(want_q), torch.empty_like(want_s)
         rows, row_map = torch.empty(E, dtype=torch.int32, device=DEV), torch.empty(T, K, dtype=torch.int32, device=DEV)
-        rc = lib.b200moe_remap_quant_mxfp8(_ptr(x), F16 if dtype == torch.float16 else BF16, _ptr(q), _ptr(s), planes, block_sums,
-                                           None, _ptr(rows), _ptr(row_map), _ptr(ids), I32, ct.c_int64(T), H, K, E, E, None,
+        rc = lib.b200moe_remap_quant_mxfp8(_ptr(x), F16 if dtype == torch.float16 else BF16, _ptr(q), _ptr(s), planes + codes,
+                                           block_sums, None, _ptr(rows), _ptr(row_map), _ptr(ids), I32, ct.c_int64(T), H, K, E, E, None,
                                            ct.c_size_t(0), _stream())
         assert rc == 0, lib.b200moe_last_error()
         assert torch.equal(q, want_q) and torch.equal(s, want_s)
@@ -127,3 +130,10 @@ def test_other_weights_refuse_the_order(lib):
         args = GemmArgs(a=a.data_ptr(), a_dtype=a_dtype, a_scale=a.data_ptr(), w=a.data_ptr(), w_format=5, w_scale=a.data_ptr(),
                         d=a.data_ptr(), d_dtype=BF16, rows_per_expert=a.data_ptr(), m=1, n=64, k=128, num_experts=1)
         assert lib.b200moe_grouped_gemm(ct.byref(args), _stream()) == -1
+
+
+@pytest.mark.parametrize("terms,block_sums", [(EVENS_FIRST + 2, 0), (EVENS_FIRST, 1), (EVENS_FIRST + 4, 1), (4, 1), (0, 1), (-14, 1)])
+def test_quantiser_refuses_other_plane_counts(lib, terms, block_sums):
+    x = torch.zeros(4, 256, dtype=torch.bfloat16, device=DEV)
+    q, s = torch.empty(5, 4, 256, dtype=torch.uint8, device=DEV), torch.empty(5, 2, 4, dtype=torch.int32, device=DEV)
+    assert lib.b200moe_quant_mxfp8_ex(_ptr(x), BF16, _ptr(q), _ptr(s), ct.c_int64(4), 256, terms, block_sums, 0, _stream()) == -1

@@ -520,6 +520,8 @@ extern "C" int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* 
                                       int terms, int block_sums, int gated, b200moe_stream stream) {
   B200_CHECK_ARG(dtype == B200MOE_BF16 || dtype == B200MOE_F16, "quant_mxfp8: input must be bfloat16 or float16");
   B200_CHECK_ARG(rows >= 0 && cols >= 0 && cols % 32 == 0, "quant_mxfp8: the row length must be a multiple of 32");
+  const bool evens_first = terms > B200MOE_PLANES_EVENS_FIRST && block_sums;
+  if (evens_first) terms -= B200MOE_PLANES_EVENS_FIRST;
   B200_CHECK_ARG(terms >= 1 && terms <= 3, "quant_mxfp8: terms must be 1, 2 or 3");
   if (rows == 0 || cols == 0) return B200MOE_OK;
   B200_CHECK_ARG(x && q && s, "quant_mxfp8: null pointer");
@@ -542,8 +544,8 @@ extern "C" int b200moe_quant_mxfp8_ex(const void* x, b200moe_dtype dtype, void* 
   };
   auto of_sums = [&](auto type, auto is_gated) {
     return !block_sums ? of_planes(type, is_gated, std::integral_constant<int, kNoSums>()) :
-           block_sums == B200MOE_SUMS_EVENS_FIRST ? of_planes(type, is_gated, std::integral_constant<int, kSumsEvensFirst>()) :
-                                                    of_planes(type, is_gated, std::integral_constant<int, kSumsInOrder>());
+           evens_first ? of_planes(type, is_gated, std::integral_constant<int, kSumsEvensFirst>()) :
+                         of_planes(type, is_gated, std::integral_constant<int, kSumsInOrder>());
   };
   auto of_form = [&](auto type) {
     return gated ? of_sums(type, std::true_type()) : of_sums(type, std::false_type());

@@ -40,6 +40,7 @@ struct RowJob {
   int64_t rows;          // mx: rows of a plane (T * K)
   int planes;            // mx: 1 to 3
   int sums;              // mx: fp32 block sums [ceil(H/128)][rows] follow the scale words
+  int evens_first;       // mx with sums: the even codes of eight before the odd ones
 };
 
 __device__ __forceinline__ void copy_scales(const RowJob& a, int64_t tok, const int* dest) {
@@ -115,7 +116,7 @@ __device__ __forceinline__ void quant_piece_mx(const RowJob& a, int j, bool in, 
   for (int p = 0; p < a.planes; ++p) {
     uint2 codes;
     const uint32_t word = mx_quant_lane(v, in, codes, a.sums ? kMxLeastExact : kMxLeast, a.sums || p + 1 < a.planes);
-    if (a.sums == B200MOE_SUMS_EVENS_FIRST) codes = mx_evens_first(codes);
+    if (a.evens_first) codes = mx_evens_first(codes);
     uint8_t* q = dst_q + p * a.rows * H + (int64_t)j * 8;
     uint32_t* s = dst_s + ((int64_t)p * num_kb + (j >> 4)) * a.rows;
     for (int k = 0; k < a.K; ++k) {
@@ -704,6 +705,8 @@ extern "C" int b200moe_remap_quant_mxfp8(
   B200_CHECK_ARG(dtype == B200MOE_BF16 || dtype == B200MOE_F16,
                  "remap_quant_mxfp8: activations must be bfloat16 or float16");
   B200_CHECK_ARG(hidden_size % 32 == 0, "remap_quant_mxfp8: hidden_size must be a multiple of 32");
+  const bool evens_first = planes > B200MOE_PLANES_EVENS_FIRST && block_sums;
+  if (evens_first) planes -= B200MOE_PLANES_EVENS_FIRST;
   B200_CHECK_ARG(planes >= 1 && planes <= 3, "remap_quant_mxfp8: one to three planes");
   SortParams p;
   if (int rc = remap_params(p, expert_map, rows_per_expert, row_map, topk_ids, ids_dtype, num_rows, topk,
@@ -713,7 +716,7 @@ extern "C" int b200moe_remap_quant_mxfp8(
                  "remap_quant_mxfp8: buffers must be 16-byte aligned");
   RowJob job = {};
   job.src = hidden; job.dst = remapped_q; job.dst_s = remapped_scales; job.H = hidden_size; job.K = topk;
-  job.rows = num_rows * topk; job.planes = planes; job.sums = block_sums;
+  job.rows = num_rows * topk; job.planes = planes; job.sums = block_sums; job.evens_first = evens_first;
   auto run = dtype == B200MOE_BF16 ? remap_rows<__nv_bfloat16, kRowMx> : remap_rows<__half, kRowMx>;
   return run(p, job, rows_per_expert, row_map, num_rows, workspace, workspace_bytes, as_stream(stream));
 }

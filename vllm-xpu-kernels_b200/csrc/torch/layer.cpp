@@ -267,7 +267,7 @@ struct Experts {
     const b200moe_dtype mx_dtype =
         sums ? (planes == 3 ? B200MOE_FP8_E4M3_X3_EVENS_FIRST : B200MOE_FP8_E4M3_X2_EVENS_FIRST) :
         planes == 2 ? B200MOE_FP8_E4M3_X2 : B200MOE_FP8_E4M3;
-    const int block_sums = sums ? B200MOE_SUMS_EVENS_FIRST : 0;
+    const int terms = planes + (sums ? B200MOE_PLANES_EVENS_FIRST : 0);
     const b200moe_dtype a_dtype = a_fp8 ? B200MOE_FP8_E4M3 : planes_in ? mx_dtype : out;
     bool fp8_ready = false, planes_ready = false;
     if (o.form == kFp8) {
@@ -298,7 +298,7 @@ struct Experts {
                                                                  (int)I, rows, segments, stream));
         fp8_ready = true;
       } else if (gated_quant()) {
-        check_status(b200moe_quant_mxfp8_ex(ws + g1, out, ws + act_q, ws + act_s, M, (int)I, planes, block_sums, 1, stream));
+        check_status(b200moe_quant_mxfp8_ex(ws + g1, out, ws + act_q, ws + act_s, M, (int)I, terms, sums, 1, stream));
         planes_ready = true;
       } else {
         void *to = ws + act, *from = ws + g1;
@@ -321,7 +321,7 @@ struct Experts {
       gemm(false, ws + act_q, B200MOE_FP8_E4M3, ws + act_s, d, out, nullptr, rows, B200MOE_EPI_NONE);
     } else if (planes_in) {
       if (!planes_ready)
-        check_status(b200moe_quant_mxfp8_ex(ws + act, out, ws + act_q, ws + act_s, M, (int)I2, planes, block_sums, 0, stream));
+        check_status(b200moe_quant_mxfp8_ex(ws + act, out, ws + act_q, ws + act_s, M, (int)I2, terms, sums, 0, stream));
       gemm(false, ws + act_q, mx_dtype, ws + act_s, d, out, nullptr, rows, B200MOE_EPI_NONE);
     } else {
       gemm(false, ws + act, out, nullptr, d, out, nullptr, rows, B200MOE_EPI_NONE);
@@ -489,8 +489,9 @@ PyObject* layer_run(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                          st));
   else if (planes_in)
     check_status(b200moe_remap_quant_mxfp8(x.data_ptr(), float_dtype(x, "hidden_states"), ws + a_at, ws + as_at,
-                                           planes, i4 ? B200MOE_SUMS_EVENS_FIRST : 0, emap, rows, row_map, ids.data_ptr(), index_dtype(ids), T, (int)H,
-                                           (int)K, (int)p.total_experts, (int)p.experts, ws + sort_at, sort_bytes, st));
+                                           planes + (i4 ? B200MOE_PLANES_EVENS_FIRST : 0), i4, emap, rows, row_map,
+                                           ids.data_ptr(), index_dtype(ids), T, (int)H, (int)K, (int)p.total_experts,
+                                           (int)p.experts, ws + sort_at, sort_bytes, st));
   else
     check_status(b200moe_remap_hidden_states(
         x.data_ptr(), a1q.has_value() ? a1q->data_ptr() : nullptr, ws + a_at, a1q.has_value() ? ws + as_at : nullptr,
