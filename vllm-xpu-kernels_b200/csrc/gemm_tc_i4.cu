@@ -38,6 +38,8 @@
 // 33 tokens x top-2 of 8 experts, 28672 x 4096 and 4096 x 14336: 144 -> 135 and 97 -> 94.5 us; the next in the
 // row are the promotion warps (540 cycles a block).
 // Waits are bounded as in the other kernels (sm100_ptx.cuh).
+#include <algorithm>
+
 #include "common.cuh"
 #include "gemm_tc_common.cuh"
 #include "sm100_ptx.cuh"
@@ -71,11 +73,14 @@ struct I4Params {
   int n, k, num_experts;
   int n_tiles, num_kb;
   int groups, kb_shift;      // scales per weight row; scale index = K block >> kb_shift
-  int stages;
+  int stages, stages_wide;   // of the ring (with the 32-token tile, where the kernel chooses)
+  int ctrl_at;
   int rows_ready;            // 1: prefetch_first_tiles
   uint32_t idesc;
   int out_f16;
 };
+
+constexpr uint32_t kI4Tmem = 512;    // columns
 
 template <int BT, int kTerms>
 struct I4Shape {
@@ -86,9 +91,8 @@ struct I4Shape {
   static constexpr uint32_t kConvBase = kI4Conv * BT;
   static constexpr uint32_t kSfBase = kConvBase + kI4Conv * 32;   // weights' scale columns (constant), then the tokens'
   static constexpr uint32_t kCols = kSfBase + 8 + kI4Conv * kSfPer;
-  static constexpr uint32_t kTmem = kCols <= 256 ? 256u : 512u;
   static constexpr int kSlotBytes = kI4Group * (512 * kTokChunks + BT * 4);
-  static_assert(BT <= 32 && kCols <= 512, "tensor memory");
+  static_assert(BT <= 32 && kCols <= kI4Tmem, "tensor memory");
 };
 
 struct I4Ctrl {
@@ -104,21 +108,18 @@ struct I4Ctrl {
   alignas(16) uint16_t xpose[8][16 * 32];   // per promotion warp: output transpose tile
 };
 
-template <int BT, int kTerms, bool kEvensFirst>
-__global__ void __launch_bounds__(kI4Threads, 1)
-grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
-                       const I4Params p) {
-  using S = I4Shape<BT, kTerms>;
-  constexpr int kStageBytes = S::kStageBytes, kSlotBytes = S::kSlotBytes;
+// Shared memory: ring and token scales, then from p.ctrl_at on the control block and the tile walk (or two).
+constexpr int kI4CtrlBytes = (int)((sizeof(I4Ctrl) + 15) & ~(size_t)15);
+__device__ __forceinline__ uint8_t* i4_smem() {
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int stages = p.stages;
-  uint8_t* sf_ring = smem + stages * kStageBytes;
-  I4Ctrl* ctrl = reinterpret_cast<I4Ctrl*>(sf_ring + kI4Slots * kSlotBytes);
-  uint8_t* walk_mem = reinterpret_cast<uint8_t*>(ctrl) + ((sizeof(I4Ctrl) + 15) & ~(size_t)15);
-  volatile int* abort_flag = &ctrl->abort_flag;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  return reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+}
 
+// Everything that comes before the first tile; with kEither the walk over 32-token tiles, too, behind the other one.
+template <int BT, bool kEither>
+__device__ __forceinline__ void grouped_gemm_i4_kernel_prologue(const CUtensorMap& tmap_a, const CUtensorMap& tmap_w,
+                                                                const I4Params& p, I4Ctrl* ctrl, uint8_t* walk_mem) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0) {
     if (p.rows_ready)
       prefetch_first_tiles<BT>(p.rows_per_expert, p.num_experts, 0, p.n_tiles, p.num_kb, kPreBytes / kI4RawBytes, walk_mem,
@@ -130,7 +131,7 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
       ptx::prefetch_tensormap(&tmap_w);
     }
   } else if (warp == 1) {
-    ptx::tmem_alloc(&ctrl->tmem_base, S::kTmem);
+    ptx::tmem_alloc(&ctrl->tmem_base, kI4Tmem);
     ptx::tmem_relinquish();
   } else if (warp == 2 && lane == 0) {
     for (int s = 0; s < kI4MaxStages; ++s) {
@@ -150,11 +151,25 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     }
     ctrl->abort_flag = 0;
     ptx::fence_barrier_init();
+  } else if (kEither && warp == 3) {
+    pdl_wait();
+    build_tile_walk<32>(p.rows_per_expert, p.num_experts, p.n_tiles, walk_mem + tile_walk_bytes(p.num_experts));
   }
   pdl_wait();
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
+}
+
+template <int BT, int kTerms, bool kEvensFirst>
+__device__ __forceinline__ void grouped_gemm_i4_kernel_body(const CUtensorMap& tmap_a, const CUtensorMap& tmap_w,
+                                                            const I4Params& p, int stages, uint8_t* smem, I4Ctrl* ctrl,
+                                                            const uint8_t* walk_mem) {
+  using S = I4Shape<BT, kTerms>;
+  constexpr int kStageBytes = S::kStageBytes, kSlotBytes = S::kSlotBytes;
+  uint8_t* sf_ring = smem + stages * kStageBytes;
+  volatile int* abort_flag = &ctrl->abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t tmem_base = ctrl->tmem_base;
   if (warp >= 4 && warp < 8) {
     // the weights' scale factors: 2^9 everywhere, which makes the codes the integers 0..15
@@ -255,9 +270,9 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
     } else {
       // ------------------------ tokens' scales and sums ---------------------------
       const int ft = lane;
-      constexpr int kNT = kTerms * BT, kPer = kI4Group * kNT / 32, kPerSum = kI4Group * BT / 32;
+      constexpr int kPer = kI4Group * kTerms * BT / 32, kPerSum = kI4Group * BT / 32;
+      const int tok = ft % BT;
       const int64_t plane_words = (int64_t)p.num_kb * p.m;
-      const float* sums = reinterpret_cast<const float*>(p.a_scale + kTerms * plane_words);
       uint32_t slot = 0, slot_ph = 1;
       int cursor = 0;
       bool ok = true;
@@ -266,26 +281,27 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
         TileInfo ti;
         locate_tile<BT>(walk, t, cursor, ti);
         for (int kb0 = 0; kb0 < p.num_kb; kb0 += kI4Group) {
+          const uint32_t* words = p.a_scale + ((int64_t)kb0 * p.m + ti.row0 + tok);
           uint32_t w[kPer];
           float m[kPerSum];
+          // token, plane and K block of a word: lane % BT, then planes, then blocks (with all three from one number, lane +
+          // 32 * i, the addresses did not fit the registers: three planes in the choosing kernel 4 to 5 % slower)
   #pragma unroll
           for (int i = 0; i < kPer; ++i) {
-            const int x = ft + 32 * i, n = x % kNT, kb = kb0 + x / kNT, term = n / BT, tok = n % BT;
-            w[i] = (kb < p.num_kb && tok < ti.valid)
-                       ? p.a_scale[term * plane_words + (int64_t)kb * p.m + ti.row0 + tok] : 0x7f7f7f7fu;
+            const int j = i * (32 / BT) + ft / BT, u = j / kTerms, kb = kb0 + u;
+            w[i] = (kb < p.num_kb && tok < ti.valid) ? words[(j % kTerms) * plane_words + (int64_t)u * p.m] : 0x7f7f7f7fu;
           }
   #pragma unroll
           for (int i = 0; i < kPerSum; ++i) {
-            const int x = ft + 32 * i, tok = x % BT, kb = kb0 + x / BT;
-            m[i] = (kb < p.num_kb && tok < ti.valid)
-                       ? -8.0f * sums[(int64_t)kb * p.m + ti.row0 + tok] : 0.f;
+            const int u = i * (32 / BT) + ft / BT, kb = kb0 + u;
+            m[i] = (kb < p.num_kb && tok < ti.valid) ? -8.0f * __uint_as_float(words[kTerms * plane_words + (int64_t)u * p.m]) : 0.f;
           }
           if (!__all_sync(0xffffffffu, ptx::paced::mbar_wait_s(sf_empty0 + 8 * slot, slot_ph, abort_flag))) { ok = false; break; }
           const uint32_t ring = ptx::smem_u32(sf_ring) + slot * kSlotBytes;
   #pragma unroll
           for (int i = 0; i < kPer; ++i) {
             // plane `term` takes the columns 2 * term and 2 * term + 1 (an MMA's scales start on an even one)
-            const int x = ft + 32 * i, n = x % kNT, u = x / kNT, term = n / BT, tok = n % BT;
+            const int j = i * (32 / BT) + ft / BT, u = j / kTerms, term = j % kTerms;
             ptx::sts32(ring + u * (S::kTokChunks * 512) + (term >> 1) * 512 + (tok & 31) * 16 + ((2 * term + (tok >> 5)) & 3) * 4,
                        w[i]);
           }
@@ -448,23 +464,73 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
   if (warp == 1) {
     ptx::tc_fence_after();
     if (*abort_flag != 0) __nanosleep(20000);
-    ptx::tmem_dealloc(tmem_base, S::kTmem);
+    ptx::tmem_dealloc(tmem_base, kI4Tmem);
   }
   if (tid == 0 && *abort_flag != 0) report_timeout(p.status);
 }
 
 template <int BT, int kTerms, bool kEvensFirst>
-int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
+__global__ void __launch_bounds__(kI4Threads, 1)
+grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_w,
+                       const I4Params p) {
+  uint8_t *smem = i4_smem(), *walk = smem + p.ctrl_at + kI4CtrlBytes;
+  I4Ctrl* ctrl = reinterpret_cast<I4Ctrl*>(smem + p.ctrl_at);
+  grouped_gemm_i4_kernel_prologue<BT, false>(tmap_a, tmap_w, p, ctrl, walk);
+  grouped_gemm_i4_kernel_body<BT, kTerms, kEvensFirst>(tmap_a, tmap_w, p, p.stages, smem, ctrl, walk);
+}
+
+// The tile by the rows that the experts really have, which the host does not know: 32 tokens where the tiles of 16
+// would be more by an eighth (two planes) or a third (three); see grouped_gemm_tc_i4.  Both walks are made at once and
+// all else ahead of them as in the other kernel: it costs nothing there (Mixtral, 33 tokens 221.3 / 221.2 us; with the
+// count and a barrier in front of the other kernel's start 217.2 / 219.4).
+template <int kTerms, bool kEvensFirst>
+__global__ void __launch_bounds__(kI4Threads, 1)
+grouped_gemm_i4_either_kernel(const __grid_constant__ CUtensorMap tmap_a16, const __grid_constant__ CUtensorMap tmap_a32,
+                              const __grid_constant__ CUtensorMap tmap_w, const I4Params p) {
+  uint8_t *smem = i4_smem(), *walk16 = smem + p.ctrl_at + kI4CtrlBytes, *walk32 = walk16 + tile_walk_bytes(p.num_experts);
+  I4Ctrl* ctrl = reinterpret_cast<I4Ctrl*>(smem + p.ctrl_at);
+  grouped_gemm_i4_kernel_prologue<16, true>(tmap_a16, tmap_w, p, ctrl, walk16);
+  const int64_t tiles16 = tile_walk_at(walk16, p.num_experts).total, tiles32 = tile_walk_at(walk32, p.num_experts).total;
+  if (kTerms == 2 ? 8 * tiles16 > 9 * tiles32 : 3 * tiles16 > 4 * tiles32)
+    grouped_gemm_i4_kernel_body<32, kTerms, kEvensFirst>(tmap_a32, tmap_w, p, p.stages_wide, smem, ctrl, walk32);
+  else
+    grouped_gemm_i4_kernel_body<16, kTerms, kEvensFirst>(tmap_a16, tmap_w, p, p.stages, smem, ctrl, walk16);
+}
+
+template <int BT, int kTerms>
+int i4_token_map(CUtensorMap* map, const b200moe_gemm_args* a) {
+  cuuint64_t dims[3] = {(cuuint64_t)a->k, (cuuint64_t)a->m, (cuuint64_t)kTerms};
+  cuuint64_t strides[2] = {(cuuint64_t)a->k, (cuuint64_t)a->k * (cuuint64_t)a->m};
+  cuuint32_t box[3] = {128, (cuuint32_t)BT, (cuuint32_t)kTerms};
+  return encode_map(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->a, dims, strides, box);
+}
+
+// Stages of the ring, and in ctrl_at (at least) the end of ring and token scales.
+template <int BT, int kTerms>
+int i4_ring(int walk_bytes, int& ctrl_at) {
   using S = I4Shape<BT, kTerms>;
-  auto kern = grouped_gemm_i4_kernel<BT, kTerms, kEvensFirst>;
-  p.idesc = ptx::make_idesc_mx(0u, 0u, kFeat, (uint32_t)BT);
-  CUtensorMap ta, tw;
-  {
-    cuuint64_t dims[3] = {(cuuint64_t)a->k, (cuuint64_t)a->m, (cuuint64_t)kTerms};
-    cuuint64_t strides[2] = {(cuuint64_t)a->k, (cuuint64_t)a->k * (cuuint64_t)a->m};
-    cuuint32_t box[3] = {128, (cuuint32_t)BT, (cuuint32_t)kTerms};
-    if (int rc = encode_map(&ta, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->a, dims, strides, box)) return rc;
-  }
+  constexpr int kScales = kI4Slots * S::kSlotBytes, kOther = 1024 + kScales + kI4CtrlBytes;
+  // A multiple of the converter sets: then a stage is always read by the same set, which has seen the fill before
+  // the one that it waits for by parity (the issuers finish blocks out of order).  And deeper than the slots: a
+  // stage is released when the block kI4Conv further on is stored.
+  constexpr int kLeast = ((int)kMaxSmem - kOther - 2 * tile_walk_bytes(kMaxExperts)) / S::kStageBytes;
+  constexpr int kDepth = converter_ring_depth(kI4Sets, kI4Conv);
+  static_assert(kLeast / kI4Sets * kI4Sets >= kDepth && kI4MaxStages >= kDepth && kI4MaxStages % kI4Sets == 0,
+                "ring depth that the converters' waits need");
+  int stages = ((int)kMaxSmem - kOther - walk_bytes) / S::kStageBytes / kI4Sets * kI4Sets;
+  if (stages > kI4MaxStages) stages = kI4MaxStages;
+  ctrl_at = std::max(ctrl_at, stages * S::kStageBytes + kScales);
+  return stages;
+}
+
+// kEither: the kernel chooses between BT and 32 tokens.
+template <int BT, int kTerms, bool kEvensFirst, bool kEither = false>
+int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
+  p.idesc = ptx::make_idesc_mx(0u, 0u, kFeat, (uint32_t)BT);   // (a tile puts its number of columns in)
+  CUtensorMap ta, ta32, tw;
+  if (int rc = i4_token_map<BT, kTerms>(&ta, a)) return rc;
+  if (kEither)
+    if (int rc = i4_token_map<32, kTerms>(&ta32, a)) return rc;
   {
     cuuint64_t dims[3] = {(cuuint64_t)(a->k / 2), (cuuint64_t)a->n, (cuuint64_t)a->num_experts};
     cuuint64_t strides[2] = {(cuuint64_t)(a->k / 2), (cuuint64_t)(a->k / 2) * a->n};
@@ -472,26 +538,27 @@ int launch_i4(const b200moe_gemm_args* a, I4Params& p, cudaStream_t st) {
     if (int rc = encode_map(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, a->w, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_64B))
       return rc;
   }
-  constexpr int kFixed = 1024 + kI4Slots * S::kSlotBytes + (int)((sizeof(I4Ctrl) + 15) & ~(size_t)15);
-  // A multiple of the converter sets: then a stage is always read by the same set, which has seen the fill before
-  // the one that it waits for by parity (the issuers finish blocks out of order).  And deeper than the slots: a
-  // stage is released when the block kI4Conv further on is stored.
-  constexpr int kLeast = ((int)kMaxSmem - kFixed - tile_walk_bytes(kMaxExperts)) / S::kStageBytes;
-  constexpr int kDepth = converter_ring_depth(kI4Sets, kI4Conv);
-  static_assert(kLeast / kI4Sets * kI4Sets >= kDepth && kI4MaxStages >= kDepth && kI4MaxStages % kI4Sets == 0,
-                "ring depth that the converters' waits need");
-  const int fixed = kFixed + tile_walk_bytes(p.num_experts);
-  p.stages = ((int)kMaxSmem - fixed) / S::kStageBytes / kI4Sets * kI4Sets;
-  if (p.stages > kI4MaxStages) p.stages = kI4MaxStages;
-  const size_t smem = (size_t)fixed + (size_t)p.stages * S::kStageBytes;
-  static SmemConfig configured;
-  if (int rc = configured.ensure(kern)) return rc;
+  const int walk_bytes = (kEither ? 2 : 1) * tile_walk_bytes(p.num_experts);
+  p.ctrl_at = 0;
+  p.stages = i4_ring<BT, kTerms>(walk_bytes, p.ctrl_at);
+  p.stages_wide = kEither ? i4_ring<32, kTerms>(walk_bytes, p.ctrl_at) : 0;
+  const size_t smem = 1024 + (size_t)p.ctrl_at + kI4CtrlBytes + walk_bytes;
   const int64_t tile_bound = ((a->m + BT - 1) / BT + a->num_experts) * (int64_t)p.n_tiles;
   int grid = sm_count();
   if (a->max_ctas > 0 && a->max_ctas < grid) grid = a->max_ctas;
   if (tile_bound < grid) grid = (int)tile_bound;
-  B200_LAUNCHED("grouped_gemm_i4_kernel",
-                launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kI4Threads), smem, st, ta, tw, p));
+  static SmemConfig configured;
+  if constexpr (kEither) {
+    auto kern = grouped_gemm_i4_either_kernel<kTerms, kEvensFirst>;
+    if (int rc = configured.ensure(kern)) return rc;
+    B200_LAUNCHED("grouped_gemm_i4_either_kernel",
+                  launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kI4Threads), smem, st, ta, ta32, tw, p));
+  } else {
+    auto kern = grouped_gemm_i4_kernel<BT, kTerms, kEvensFirst>;
+    if (int rc = configured.ensure(kern)) return rc;
+    B200_LAUNCHED("grouped_gemm_i4_kernel",
+                  launch_pdl(p.m <= kEarlyLaunchRows, kern, dim3(grid), dim3(kI4Threads), smem, st, ta, tw, p));
+  }
   return B200MOE_OK;
 }
 
@@ -523,15 +590,23 @@ int grouped_gemm_tc_i4(const b200moe_gemm_args* a, cudaStream_t st) {
   p.out_f16 = a->d_dtype == B200MOE_F16;
   const int64_t in_use = (a->rows_hint > 0 && a->rows_hint < a->m) ? a->rows_hint : a->m;
   const int64_t avg = (in_use + a->num_experts - 1) / a->num_experts;
-  // Both the MMA and the promotion cost grow with the tile; experts with more rows than the tile stream their weights
-  // once more, from L2.  Layer calls of 8 experts of 4096 x 14336, 2 a token, six routings (skewed), tiles of 16 / 32, us:
-  // bfloat16 8.3 rows an expert 207 / 218, 10 rows 220 / 222, 10.3 rows 222 / 221, 11 rows 230 / 223, 12 rows 247 / 226; float16
-  // (three planes, whose wide tile leaves the ring 9 stages) 8.3 rows 222 / 274, 10 rows 236 / 277, 12 rows 266 / 278, 13
-  // rows 274 / 280, 14 rows 289 / 287.
+  // Both the MMA and the promotion cost grow with the tile; experts with more rows than the tile take another, whose
+  // weights come from L2.  How many do is not known here, so from 9 to 10 rows per expert (13 for float16, whose three
+  // planes make the wide tile dearer) the kernel chooses.  Layer calls, time with 16-token tiles / with the kernel's
+  // choice, each against 32-token tiles in the same run (calls that follow one another, outputs the same bit for bit), where
+  // the router's logits have an offset per expert of deviation 0, 0.5, 1, 2 and 4:
+  //   8 experts of 4096 x 14336, top 2, bfloat16, 9 rows    .94 / .96   .97 / .97    .99 / 1.00  1.02 / 1.00  1.09 / 1.00  (of 171 to 240 us)
+  //   64 experts of 2048 x 1408, top 6, bfloat16, 9 rows    .96 / .96   1.01 / 1.01  1.05 / 1.01  1.13 / 1.01  1.17 / 1.01  (of 72 to 114)
+  //   the same, float16, 9 rows                             .84 / .85   .90 / .93    .95 / .99   1.03 / .98   1.09 / .96  (of 83 to 138)
+  //   the 8 experts, float16, 13 rows                       .88 / .94   1.01 / .99   1.04 / 1.01  1.11 / 1.00  1.04 / .99  (of 251 to 310)
+  // By those, 16 tokens win while their tiles are no more than by a tenth to a sixth (two planes) or 0.28 to 0.35 (three) as
+  // many again: a wide tile multiplies only columns that have rows.
   auto run = [&](auto order) {
     constexpr bool kEvens = decltype(order)::value;
-    if (planes == 2) return avg <= 10 ? launch_i4<16, 2, kEvens>(a, p, st) : launch_i4<32, 2, kEvens>(a, p, st);
-    return avg <= 13 ? launch_i4<16, 3, kEvens>(a, p, st) : launch_i4<32, 3, kEvens>(a, p, st);
+    if (planes == 2) return avg <= 8 ? launch_i4<16, 2, kEvens>(a, p, st) : avg <= 10 ? launch_i4<16, 2, kEvens, true>(a, p, st) :
+                                                                                       launch_i4<32, 2, kEvens>(a, p, st);
+    return avg <= 8 ? launch_i4<16, 3, kEvens>(a, p, st) : avg <= 13 ? launch_i4<16, 3, kEvens, true>(a, p, st) :
+                                                                      launch_i4<32, 3, kEvens>(a, p, st);
   };
   return evens_first ? run(std::true_type()) : run(std::false_type());
 }
