@@ -481,8 +481,8 @@ grouped_gemm_i4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_
 
 // The tile by the rows that the experts really have, which the host does not know: 32 tokens where the tiles of 16
 // would be more by an eighth (two planes) or a third (three); see grouped_gemm_tc_i4.  Both walks are made at once and
-// all else ahead of them as in the other kernel: it costs nothing there (Mixtral, 33 tokens 221.3 / 221.2 us; with the
-// count and a barrier in front of the other kernel's start 217.2 / 219.4).
+// all else ahead of them as in the other kernel.  The choice costs 0 to 1 % (Mixtral, 33 tokens, 16-token tiles alone / so, on
+// four inputs: 211.8 / 214.5, 221.0 / 223.5, 222.8 / 224.3, 226.4 / 227.4 us).
 template <int kTerms, bool kEvensFirst>
 __global__ void __launch_bounds__(kI4Threads, 1)
 grouped_gemm_i4_either_kernel(const __grid_constant__ CUtensorMap tmap_a16, const __grid_constant__ CUtensorMap tmap_a32,

@@ -107,9 +107,10 @@ __device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, volat
 // converters for theirs): without a call, whose way back stood between the phase's end and the next load, and with both
 // bounds looked at after every poll, which makes polls rarer: they take turns in one unit with the arrivals and
 // waits of the roles that are behind (eight polls in a row without anything between them cost the int4 kernel 4 %, the
-// MXFP4 one 2 %; a sleep between them 1 to 2 %).  Layer calls, call and counter / so, us: DeepSeek at 8192 tokens 4625 / 4470, one
-// of its 8 ranks at 1024 tokens 253 / 248, qwen3 at 3001 tokens 271 / 266, gpt-oss at 128 tokens 342 / 337, 2048 tokens
-// 672 / 661, int4 Mixtral at 33 tokens 227 / 224.
+// MXFP4 one 2 %; a sleep between them 1 to 2 %).  Layer calls that follow one another, call and counter / so, us: DeepSeek at
+// 8192 tokens 4929 / 4737, one of its 8 ranks at 1024 tokens 280.5 / 275.9, qwen3 at 3001 tokens 307.6 / 301.1, gpt-oss at 2048
+// tokens 764 / 751, at 128 tokens 391.8 / 389.9 (no difference: runs of one side differ by 0.7 %; in bursts of 20 ms after
+// a rest 342 / 337), int4 Mixtral at 33 tokens 231.5 / 230.0.
 namespace paced {
 __device__ __forceinline__ bool mbar_wait_s(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (mbar_try_wait_s(bar, parity)) return true;

@@ -227,9 +227,11 @@ struct Experts {
   bool gated_quant() const { return planes_in && o.form == kUnfused && p.act == kSilu && p.inter % 32 == 0; }
 
   // gemm1's SwigluOAI epilogue writes the planes of gemm2's input.  That saves a launch in the chain of a small decode
-  // step; with several tiles a CTA its epilogue warps take more time from the other roles than the quantiser's launch
-  // costs.  gpt-oss layer calls, quantiser / so, us: 1 token 39.3 / 37.0, 4 tokens 69.6 / 67.2, 16 tokens 155.7 / 154.4, 32
-  // tokens 232.8 / 233.7, 64 tokens 297.4 / 300.5, 512 tokens 427 / 457, 2048 tokens (calls in a row) 768 / 813.
+  // step; with many tiles a CTA its epilogue warps take more time from the other roles than the quantiser's launch
+  // costs.  Layer calls in a row, quantiser / so, us: 128 experts of 2880 x 2880, top 4, 1 token 39.7 / 37.1, 4 tokens 69.5 /
+  // 67.5, 8 tokens 106.6 / 105.7, 16 tokens 174.9 / 174.9, 2048 tokens 768 / 813 (bursts: 32 tokens 232.8 / 233.7, 64 tokens
+  // 297.4 / 300.5, 512 tokens 427 / 457); 32 such experts 16 tokens 105.3 / 103.8, with very uneven routing 56.6 / 54.4; 8 of
+  // 4096 x 6144, top 2, 8 and 32 tokens 83.5 / 81.9 and 89.9 / 88.6; 16 of 1024 x 512, 32 tokens 23.6 / 22.7.
   // (Only token tiles of 16 have it, which experts with 8 rows or fewer on average take.)
   static constexpr int64_t kPlanesOutRows = 64;
   bool planes_out() const {
